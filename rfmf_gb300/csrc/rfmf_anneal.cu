@@ -15,8 +15,9 @@
 //     side on that one copy.  Chains never synchronise with each other: a
 //     chain's barriers are __syncwarp (W == 1) or a named barrier of its own.
 //   * All mutable chain state stays in shared memory for the whole window:
-//     D[v] = spin[v]*S[v] (the per-vertex gain; int8 with a +128 bias when
-//     the max weighted degree B <= 127, else int32), the spins as bits, and
+//     D[v] = spin[v]*S[v] (the per-vertex gain; as an int8 field S with a
+//     bias that one xor with the spin mask turns into D when the max weighted
+//     degree B <= 127, else int32 D), the spins as mask bytes and bits, and
 //     the best-so-far spins as bits.  Graphs too big for shared memory walk
 //     their CSR in HBM instead, in the most compact entry form they allow
 //     (2, 4 or 8 bytes); the chain state stays resident.
@@ -24,9 +25,11 @@
 //     hoisted (rounds 1-3 lose 3 multiplies and 3 xors per block) and three
 //     vertex blocks are in flight per thread.
 //   * The group argmax keeps eight register accumulators per thread (one per
-//     Philox lane j) whenever every thread's lane j lands in one group, folds
-//     them with warp shuffles, and stores one packed (biased score, ~v) key
-//     per group; other P fall back to shared-memory atomics.
+//     Philox lane j) whenever every thread's lane j lands in one group.  For
+//     256 % P == 0, P <= 128 each warp transposes its 256 accumulators through
+//     shared memory and reduces them in registers; the winners stay there
+//     (one-warp chains) or pass through one partial per warp and group.  Other
+//     P go through shared-memory slots with atomics.
 //   * FLIP has no winner-winner correction walk.  With D kept per vertex,
 //     negating the winners' D and scattering 2*w*s_b*s_x into D[x] over the
 //     winners' rows leaves every winner holding D_final, and the cut gain of
@@ -40,6 +43,13 @@
 #include <type_traits>
 
 #include "rfmf_device.h"
+
+// Gain bytes this translation unit compiles the kernels for (each leaves the
+// other width's helpers unreferenced).
+#ifndef RFMF_GAIN_BYTES
+#define RFMF_GAIN_BYTES 1
+#endif
+#pragma nv_diag_suppress 177
 
 namespace rfmf {
 
@@ -68,9 +78,20 @@ struct ChainKeys {
     uint32_t k1[10];
 };
 
+// A value that is the same in every lane of the (converged) warp, as one the
+// compiler knows to be uniform: redux.sync delivers to a uniform register,
+// where a chain's constants cost no per-thread registers.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_or_sync(0xFFFFFFFFu, x); }
+__device__ __forceinline__ int32_t uniform(int32_t x) { return static_cast<int32_t>(uniform(static_cast<uint32_t>(x))); }
+__device__ __forceinline__ uint64_t uniform(uint64_t x) {
+    return (static_cast<uint64_t>(uniform(static_cast<uint32_t>(x >> 32))) << 32) | uniform(static_cast<uint32_t>(x));
+}
+__device__ __forceinline__ int64_t uniform(int64_t x) { return static_cast<int64_t>(uniform(static_cast<uint64_t>(x))); }
+template <class T>
+__device__ __forceinline__ T* uniform(T* x) { return reinterpret_cast<T*>(uniform(reinterpret_cast<uint64_t>(x))); }
 __device__ __forceinline__ ChainKeys make_keys(uint64_t seed) {
     ChainKeys k;
-    uint32_t a = static_cast<uint32_t>(seed), b = static_cast<uint32_t>(seed >> 32);
+    uint32_t a = uniform(static_cast<uint32_t>(seed)), b = uniform(static_cast<uint32_t>(seed >> 32));
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
         k.k0[r] = a;
@@ -174,35 +195,41 @@ __device__ __forceinline__ void group_sync(int grp, int T) {
     }
 }
 
-// ------------------------------------------------------------ D storage
-// int32 gains: plain words.
+// ------------------------------------------------------- gain storage
+// A chain keeps one value per vertex and its spin as a mask byte (sb: 0x00
+// for +1, 0xFF for -1).  D[v] = spin[v] * S[v] is the gain SELECT scores,
+// S[v] = sum_u w(v,u) spin[u].
+//
+// int32 gains: D itself, plain words (a row walk reads the neighbour's spin
+// to know the sign of its change).
 struct D32 {
+    static constexpr bool kField = false;
     static constexpr int32_t kBias = 0;
     // Stored values (D + kBias) of block b; D32 stores D itself.
-    __device__ static __forceinline__ void load8raw(const unsigned char* D, int b, int32_t d[8]) {
-        load8(D, b, d);
-    }
-    __device__ static __forceinline__ void load8(const unsigned char* D, int b, int32_t d[8]) {
+    __device__ static __forceinline__ void load8raw(const unsigned char* D, const unsigned char*, int b, int32_t d[8]) {
         const int4 a = *reinterpret_cast<const int4*>(D + 32 * b);
         const int4 c = *reinterpret_cast<const int4*>(D + 32 * b + 16);
         d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;
         d[4] = c.x; d[5] = c.y; d[6] = c.z; d[7] = c.w;
     }
-    __device__ static __forceinline__ int32_t get(const unsigned char* D, int v) {
+    __device__ static __forceinline__ void load8(const unsigned char* D, const unsigned char* sb, int b, int32_t d[8]) {
+        load8raw(D, sb, b, d);
+    }
+    __device__ static __forceinline__ int32_t get(const unsigned char* D, const unsigned char*, int v) {
         return reinterpret_cast<const int32_t*>(D)[v];
     }
-    __device__ static __forceinline__ void set(unsigned char* D, int v, int32_t d) {
+    __device__ static __forceinline__ void set(unsigned char* D, const unsigned char*, int v, int32_t d) {
         reinterpret_cast<int32_t*>(D)[v] = d;
+    }
+    // Vertex v (gain d, mask byte m before) flips.
+    __device__ static __forceinline__ void flip(unsigned char* D, int v, int32_t d, uint32_t) {
+        reinterpret_cast<int32_t*>(D)[v] = -d;
     }
     __device__ static __forceinline__ void add(unsigned char* D, int v, int32_t delta) {
         atomicAdd(reinterpret_cast<int*>(D) + v, delta);
     }
 };
 
-// int8 gains stored as D + 128 in [1, 255] (|D| <= B <= 127).  Every partial
-// sum during a scatter is the gain of some spin configuration, so it stays in
-// range and a shifted 32-bit atomicAdd on the containing word never carries
-// into the neighbouring byte.  (x ^ 0x80) read as int8 is D.
 // Byte k of x sign-extended to 32 bits: prmt with selector nibbles whose msb
 // requests sign replication (the __byte_perm intrinsic drops that bit).
 template <int k>
@@ -231,12 +258,29 @@ __device__ __forceinline__ int32_t ubyte(uint32_t x) {
     return r;
 }
 
+// int8 gains (|S| <= B <= 127): the byte q holds S + 128 while the vertex's
+// spin is +1 and S + 127 while it is -1, so that q ^ mask is D + 128 either
+// way (255 - (S + 127) = -S + 128).  SELECT pays one 8-byte mask load and two
+// xors per block of 8 vertices; a flipped vertex changes its neighbours' q by
+// 2 * w * (its new spin) whatever their spins are, so FLIP's row walk needs
+// no load of the neighbour's spin (one of its three dependent shared-memory
+// accesses per entry, each with ~3 bank-conflict wavefronts).
+// Every partial sum during a scatter is the S of some spin configuration, so
+// a byte stays in [0, 255] and a shifted 32-bit atomicAdd on the containing
+// word never carries into the neighbouring byte.
 struct D8 {
+    static constexpr bool kField = true;
     static constexpr int32_t kBias = 128;
-    // Stored values D + 128 of block b (no sign handling: callers fold the
-    // bias into a constant).
-    __device__ static __forceinline__ void load8raw(const unsigned char* D, int b, int32_t d[8]) {
+    __device__ static __forceinline__ uint2 words(const unsigned char* D, const unsigned char* sb, int b) {
         const uint2 w = *reinterpret_cast<const uint2*>(D + 8 * b);
+        const uint2 m = *reinterpret_cast<const uint2*>(sb + 8 * b);
+        return make_uint2(w.x ^ m.x, w.y ^ m.y);
+    }
+    // D + 128 of block b's vertices (no sign handling: callers fold the bias
+    // into a constant).
+    __device__ static __forceinline__ void load8raw(const unsigned char* D, const unsigned char* sb, int b,
+                                                    int32_t d[8]) {
+        const uint2 w = words(D, sb, b);
         d[0] = ubyte<0>(w.x);
         d[1] = ubyte<1>(w.x);
         d[2] = ubyte<2>(w.x);
@@ -246,8 +290,8 @@ struct D8 {
         d[6] = ubyte<2>(w.y);
         d[7] = ubyte<3>(w.y);
     }
-    __device__ static __forceinline__ void load8(const unsigned char* D, int b, int32_t d[8]) {
-        const uint2 w = *reinterpret_cast<const uint2*>(D + 8 * b);
+    __device__ static __forceinline__ void load8(const unsigned char* D, const unsigned char* sb, int b, int32_t d[8]) {
+        const uint2 w = words(D, sb, b);
         const uint32_t a = w.x ^ 0x80808080u, c = w.y ^ 0x80808080u;
         d[0] = sbyte<0>(a);
         d[1] = sbyte<1>(a);
@@ -258,11 +302,15 @@ struct D8 {
         d[6] = sbyte<2>(c);
         d[7] = sbyte<3>(c);
     }
-    __device__ static __forceinline__ int32_t get(const unsigned char* D, int v) {
-        return static_cast<int32_t>(static_cast<int8_t>(D[v] ^ 0x80u));
+    __device__ static __forceinline__ int32_t get(const unsigned char* D, const unsigned char* sb, int v) {
+        return static_cast<int32_t>(D[v] ^ sb[v]) - 128;
     }
-    __device__ static __forceinline__ void set(unsigned char* D, int v, int32_t d) {
-        D[v] = static_cast<unsigned char>(d + 128);
+    __device__ static __forceinline__ void set(unsigned char* D, const unsigned char* sb, int v, int32_t d) {
+        D[v] = static_cast<unsigned char>((d + 128) ^ sb[v]);
+    }
+    // Vertex v (gain d, mask byte m before) flips: S stays, D changes sign.
+    __device__ static __forceinline__ void flip(unsigned char* D, int v, int32_t d, uint32_t m) {
+        D[v] = static_cast<unsigned char>((128 - d) ^ (m ^ 0xFFu));
     }
     __device__ static __forceinline__ void add(unsigned char* D, int v, int32_t delta) {
         atomicAdd(reinterpret_cast<unsigned int*>(D + (v & ~3)),
@@ -357,7 +405,7 @@ struct ChainSmem {
     unsigned char* D;
     uint32_t* bits;
     uint32_t* best;
-    unsigned char* sb;           // spins as bytes (1 = +1), kept equal to bits
+    unsigned char* sb;           // spins as mask bytes (0x00 = +1, 0xFF = -1), kept equal to bits
     unsigned long long* slots;   // int32 mode: packed keys
     long long* scores;           // int64 mode: max score per group (aliases slots)
     int32_t* ids;                // int64 mode: winner id per group
@@ -394,16 +442,15 @@ __device__ __forceinline__ int64_t group_sum(int64_t v, const ChainSmem& s, int 
     return tot;
 }
 
-// int32 sum over a chain's warp group with redux.sync (int8 gains: the sums
-// of a sweep's winner gains are bounded by 2 * 127 * P, far inside int32).
-__device__ __forceinline__ int32_t group_sum32(int32_t v, const ChainSmem& s, int t, int T, int grp) {
-    v = __reduce_add_sync(0xFFFFFFFFu, v);
-    if (T == 32) return v;
-    if ((t & 31) == 0) s.red[t >> 5] = v;
-    group_sync(grp, T);
-    int64_t tot = 0;
-    for (int w = 0; w < (T >> 5); ++w) tot += s.red[w];
-    return static_cast<int32_t>(tot);
+// Exact warp sums with redux.sync.  int8 gains: the winners' gains of a sweep
+// sum to at most 2 * 127 * P, far inside int32.  int32 gains: a lane's |v| is
+// below 2^34, split into a low 24-bit part and the rest so that neither sum
+// of 32 lanes leaves int32.
+__device__ __forceinline__ int32_t warp_sum(int32_t v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ int64_t warp_sum(int64_t v) {
+    const int32_t lo = __reduce_add_sync(0xFFFFFFFFu, static_cast<int32_t>(v & 0xFFFFFF));
+    const int32_t hi = __reduce_add_sync(0xFFFFFFFFu, static_cast<int32_t>(v >> 24));
+    return (static_cast<int64_t>(hi) << 24) + lo;
 }
 
 // ---------------------------------------------------------------- SELECT
@@ -413,29 +460,32 @@ __device__ __forceinline__ int32_t group_sum32(int32_t v, const ChainSmem& s, in
 
 // Per-phase constants, recomputed only when P changes (no integer division
 // or modulo by P inside a sweep).
+//
+// kPathWarp: 256 % P == 0 and P <= 128.  Every (lane, j) accumulator belongs
+// to one group, each warp reduces its 256 accumulators to P winners
+// (warp_argmax) and the winners stay in registers (one-warp chains) or pass
+// through one 8-byte partial per warp and group (wider ones).  Other P go
+// through the group slots: kPathPrivate when 8T % P == 0 (one atomic per
+// accumulator), else kPathVertex (one atomic per vertex).
+enum PhasePath : int { kPathWarp = 0, kPathPrivate = 1, kPathVertex = 2 };
+
 struct PhaseCfg {
     int P;
-    int mode;       // 0: P | 256, groups repeat every P/8 lanes (register fold +
-                    //    warp reduction); 1: 8T % P == 0, thread-private groups;
-                    // 2: general P, one shared atomic per vertex
-    int period;     // mode 0: P/8 (or 1 for P < 8); lanes l and l + period share groups
-    int g0;         // mode 1: (8 t) mod P
-    int laneShift;  // FLIP scatter: log2 of the lanes that share one row
-    uint32_t gmask; // mode 0, P >= 16: the lanes sharing this lane's groups
+    int path;       // PhasePath
+    int g0;         // kPathPrivate: (8 t) mod P
+    int laneShift;  // FLIP: log2 of the lanes that share one winner's row
+    int rows;       // FLIP: rows a thread takes part in on kPathWarp (1, 2 or 4)
 };
 
-__device__ __forceinline__ PhaseCfg phase_cfg(int P, int t, int T) {
+__device__ __forceinline__ PhaseCfg phase_cfg(int P, int t, int T, bool slots) {
     PhaseCfg c;
     c.P = P;
-    c.mode = ((256 % P) == 0) ? 0 : (((8 * T) % P) == 0 ? 1 : 2);
-    c.period = (P >= 8) ? (P >> 3) : 1;
+    c.path = (!slots && P <= 128 && (256 % P) == 0) ? kPathWarp : ((8 * T) % P) == 0 ? kPathPrivate : kPathVertex;
     c.g0 = (8 * t) % P;
     int sh = 0;
     while ((2 << sh) * P <= T && sh < 5) ++sh;
     c.laneShift = sh;
-    const uint32_t rep = (c.period >= 32) ? 1u : (c.period == 16) ? 0x00010001u
-                       : (c.period == 8) ? 0x01010101u : (c.period == 4) ? 0x11111111u : 0x55555555u;
-    c.gmask = rep << ((t & 31) & (c.period - 1));
+    c.rows = (P + T - 1) / T;
     return c;
 }
 
@@ -530,12 +580,12 @@ __device__ __forceinline__ void score_blocks(int32_t acc[8], const ChainSmem& s,
         // loaded just before it is scored so that they fit the registers.
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
-            DP::load8raw(s.D, b + q * T, d[0]);
+            DP::load8raw(s.D, s.sb, b + q * T, d[0]);
             score8_key<kMasked, kF0>(acc, x[q], d[0], betaK, tkb - q, kc, lim);
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < NB; ++q) DP::load8raw(s.D, b + q * T, d[q]);
+        for (int q = 0; q < NB; ++q) DP::load8raw(s.D, s.sb, b + q * T, d[q]);
 #pragma unroll
         for (int q = 0; q < NB; ++q) score8_key<kMasked, kF0>(acc, x[q], d[q], betaK, tkb - q, kc, lim);
     }
@@ -564,72 +614,121 @@ __device__ __forceinline__ void select_blocks(int32_t acc[8], const ChainSmem& s
     }
 }
 
-// FLIP step 1 for one winner v (or none, v < 0) of group g: publish it, add
-// its pre-sweep gain to loc, negate the gain, flip the spin bit and byte.
-template <class DP, class Loc>
-__device__ __forceinline__ void flip_winner(const ChainSmem& s, int g, int v, Loc& loc) {
-    s.win[g] = v;
-    if (v >= 0) {
-        const int32_t d = DP::get(s.D, v);
-        loc += d;
-        DP::set(s.D, v, -d);
-        atomicXor(&s.bits[v >> 5], 1u << (v & 31));
-        s.sb[v] ^= 1u;
-    }
+// The winner of one group among a warp's 256 accumulators: its compact key
+// and the accumulator it came from (8 * lane + j).  Equal keys mean equal
+// score and block iteration, so the smaller accumulator is the smaller vertex.
+__device__ __forceinline__ bool beats(int32_t ka, int32_t aa, int32_t kb, int32_t ab) {
+    return ka > kb || (ka == kb && aa < ab);
 }
 
-// FLIP step 2 of a one-warp chain at P >= 64 with +-1 weights in the 16-bit
-// CSR (entry = col << 1 | w < 0) and int8 gains: one lane per winner row,
-// four entries in flight.  With spins as bits (1 = +1), D[col] changes by +2
-// when s_b, s_col and the weight bit XOR to 0, else by -2, added into byte
-// lane col & 3 of word col >> 2 (the biased bytes never carry, see D8).
-// (At smaller P the generic walk, which spreads a row over several lanes,
-// is faster.)
-template <int kFmt>
-__device__ __forceinline__ void flip2_unit16_d8_warp(const ChainSmem& s, const CsrView& csr, int P, int lane) {
-    unsigned int* Dw = reinterpret_cast<unsigned int*>(s.D);
-    const unsigned char* sb = s.sb;
-    for (int gi = lane; gi < P; gi += 32) {
-        const int v = s.win[gi];
-        if (v < 0) continue;
-        const uint32_t sv = sb[v];
-        uint32_t i, hi;
-        Csr<kFmt>::row(csr, v, i, hi);
-        for (; i + 4 <= hi; i += 4) {
-            uint32_t e[4], sx[4];
+// Per-warp scratch of warp_argmax: the 256 accumulators as words, j >= 4 in a
+// second half that starts 16 banks later, so that both the vector stores
+// (4 words per lane) and the transposed reads (lanes at consecutive
+// accumulators) are free of bank conflicts.  Wider chains reuse it for the
+// warp's partials (8 bytes per group, P <= 128).
+constexpr int kHalf = 144;
+
+// Groups of a warp's accumulators for P = 32 Q, or P <= 32 with Q = 1:
+// accumulator a belongs to group a mod P; lane l gets the winners of groups
+// l + 32 q (of group l mod P when P < 32, in every lane of that residue).
+// The accumulators are transposed through shared memory, where eight reads
+// and a register tree replace log2(256 / P) shuffles of each of the eight
+// accumulators and a ballot per Philox lane to find the winning lane.  Wider
+// chains used to merge their warps' winners with 64-bit shared atomic maxima
+// (a compare-and-swap loop each), 1,900 to 2,900 cycles of a sweep on GB300.
+// us per sweep before / with this and the settled gain (see run_chain):
+// 1024 one-warp chains of ER n = 2000 P = 16 3.55 / 2.97, P = 128 7.55 / 6.75;
+// 32 four-warp chains of ER n = 800 P = 16 2.93 / 1.94; 80 eight-warp chains
+// of the 100x200 torus P = 16 4.36 / 3.75.
+template <int Q>
+__device__ __forceinline__ void warp_argmax(const int32_t acc[8], int32_t* scr, int lane, int P, int32_t key[4],
+                                            int32_t at[4]) {
+    *reinterpret_cast<int4*>(scr + 4 * lane) = make_int4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<int4*>(scr + kHalf + 4 * lane) = make_int4(acc[4], acc[5], acc[6], acc[7]);
+    __syncwarp();
+    const int32_t* mine = scr + 4 * (lane >> 3) + (lane & 3) + kHalf * ((lane >> 2) & 1);
+    int32_t k[8], a[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) e[j] = Csr<kFmt>::raw(csr, i + j);
+    for (int i = 0; i < 8; ++i) {
+        k[i] = mine[16 * i];   // accumulator lane + 32 i
+        a[i] = lane + 32 * i;
+    }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sx[j] = sb[e[j] >> 1];
+    for (int d = Q; d < 8; d *= 2) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t neg = (sv ^ sx[j] ^ e[j]) & 1u;
-                atomicAdd(Dw + (e[j] >> 3), (neg ? 0xFFFFFFFEu : 2u) << ((e[j] & 6u) << 2));
+        for (int i = 0; i + d < 8; ++i) {
+            if ((i / Q) % (2 * d / Q) == 0 && k[i + d] > k[i]) {
+                k[i] = k[i + d];
+                a[i] = a[i + d];
             }
         }
-        for (; i < hi; ++i) {
-            const uint32_t e0 = Csr<kFmt>::raw(csr, i);
-            const uint32_t neg = (sv ^ sb[e0 >> 1] ^ e0) & 1u;
-            atomicAdd(Dw + (e0 >> 3), (neg ? 0xFFFFFFFEu : 2u) << ((e0 & 6u) << 2));
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        key[q] = k[q];
+        at[q] = a[q];
+    }
+    if (Q == 1) {
+        for (int m = 16; m >= P; m >>= 1) {
+            const int32_t ok = __shfl_xor_sync(0xFFFFFFFFu, key[0], m);
+            const int32_t oa = __shfl_xor_sync(0xFFFFFFFFu, at[0], m);
+            if (beats(ok, oa, key[0], at[0])) {
+                key[0] = ok;
+                at[0] = oa;
+            }
         }
     }
 }
 
-// How select32 hands its winners to FLIP step 1.
-enum WinnerHandoff : int {
-    kWinSlots = 0,      // packed keys in the group slots (any warp count, any P)
-    kWinFlipped = 1,    // FLIP step 1 done here (one-warp chains, P <= 8)
-    kWinPublished = 2   // winner ids in s.win (one-warp chains, P >= 16)
-};
+// P = 1: fold the eight accumulators in registers, one warp max, and the
+// lowest lane holding it; every lane gets the winner.
+__device__ __forceinline__ void warp_argmax_one(const int32_t acc[8], int32_t& key, int32_t& at) {
+    int32_t k[8];
+    int jb[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { k[j] = acc[j]; jb[j] = j; }
+#pragma unroll
+    for (int d = 1; d < 8; d *= 2) {
+#pragma unroll
+        for (int j = 0; j < 8; j += 2 * d)
+            if (k[j + d] > k[j]) { k[j] = k[j + d]; jb[j] = jb[j + d]; }
+    }
+    key = __reduce_max_sync(0xFFFFFFFFu, k[0]);
+    const int src = __ffs(__ballot_sync(0xFFFFFFFFu, k[0] == key)) - 1;
+    at = 8 * src + __shfl_sync(0xFFFFFFFFu, jb[0], src);
+}
 
-template <class DP, class Loc>
-__device__ int select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
+// A wider chain's partial: one warp's winner of one group, ordered as an
+// unsigned 64-bit number by key, then smaller vertex; 0 is none.  int8 gains
+// carry the winner's spin sign and gain byte along (FLIP needs the gain from
+// before any neighbour's flip, and so saves the barrier between reading it
+// and scattering); v < 2^23 there (a chain keeps two bytes per vertex in
+// shared memory).
+template <class DP>
+__device__ __forceinline__ unsigned long long make_partial(const ChainSmem& s, int32_t key, int v) {
+    uint32_t lo;
+    if constexpr (DP::kField) {
+        const uint32_t m = s.sb[v];
+        lo = ((~static_cast<uint32_t>(v) & 0x7FFFFFu) << 9) | ((m & 1u) << 8) |
+             static_cast<uint32_t>(static_cast<unsigned char>(s.D[v] ^ m));
+    } else {
+        lo = ~static_cast<uint32_t>(v);
+    }
+    return (static_cast<unsigned long long>(static_cast<uint32_t>(key) ^ 0x80000000u) << 32) | lo;
+}
+
+// SELECT of the int32 path on kPathWarp: on return lane l of a one-warp chain
+// holds the winners v[q] of groups l + 32 q (-1: none); a wider chain has its
+// partials in place (a barrier is due).  On the other paths the winners are
+// packed keys in the group slots (a barrier is due).
+template <bool kOne, class DP>
+__device__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
                          const PhaseCfg& pc, int32_t beta, uint64_t step, const ChainKeys& keys,
-                         int t, int T, Loc& loc) {
+                         int t, int T, int32_t v[4]) {
     const SweepConst sc = make_sweep(step, keys);
     const int P = pc.P;
     const int M = (1 << kc.kb) - 1;
-    if (pc.mode != 2) {
+    if (pc.path != kPathVertex) {
         const int32_t betaK = beta * (1 << kc.kb);
         int32_t acc[8];
 #pragma unroll
@@ -639,110 +738,29 @@ __device__ int select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc
                                                     static_cast<uint32_t>(DP::kBias) * static_cast<uint32_t>(betaK));
         if (kc.kb == 4) select_blocks<true, DP>(acc, s, sc, keys, n, t, T, betaK, tkBase, kc);
         else select_blocks<false, DP>(acc, s, sc, keys, n, t, T, betaK, tkBase, kc);
-        const int wb = t & ~31;
-        // Group argmax on the compact keys.  Equal keys mean equal score and
-        // block iteration k, so they differ only in the thread t (vertex
-        // 8(t + kT) + j): the lowest lane holding the maximum wins.  Only the
-        // winners are widened to packed (score, v) keys for the slots.
-        const int lane = t & 31;
-        if (P == 1) {
-            // One group: fold the eight accumulators in registers (on equal
-            // keys the smaller j, i.e. the smaller vertex, stays), then one
-            // warp max; the lowest lane holding it has the smallest vertex
-            // (equal keys share the block iteration k) and, in a one-warp
-            // chain, flips it itself, so no lane needs its j; in a wider
-            // chain it offers its packed key to the group slot (one atomic
-            // per warp).  Measured on GB300 at 2048 one-warp chains: -2.4%
-            // per P = 1 sweep on ER n = 2000, -13% on n = 256; folding at
-            // P = 4 and 8 was slower (the winners' broadcast).
-            int32_t m = acc[0];
-            int jb = 0;
+        if (pc.path == kPathWarp) {
+            const int lane = t & 31;
+            int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
+                                                      (kOne ? 0 : (t >> 5) * kWarpScratch));
+            int32_t key[4], at[4];
+            if (P == 1) warp_argmax_one(acc, key[0], at[0]);
+            else if (P <= 32) warp_argmax<1>(acc, scr, lane, P, key, at);
+            else if (P == 64) warp_argmax<2>(acc, scr, lane, P, key, at);
+            else warp_argmax<4>(acc, scr, lane, P, key, at);
+            const int Q = (P + 31) >> 5;
+            if (!kOne) __syncwarp();   // the scratch is rewritten below
 #pragma unroll
-            for (int j = 1; j < 8; ++j)
-                if (acc[j] > m) { m = acc[j]; jb = j; }
-            const int32_t mx = __reduce_max_sync(0xFFFFFFFFu, m);
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, m == mx);
-            if (lane == __ffs(bal) - 1) {
-                const int kk = M - (mx & M);
-                const int v = (mx != INT32_MIN) ? 8 * (wb + lane + kk * T) + jb : -1;
-                if (T == 32) flip_winner<DP>(s, 0, v, loc);
-                else if (v >= 0) atomicMax(&s.slots[0], pack_key(mx >> kc.kb, v));
-            }
-            return (T == 32) ? kWinFlipped : kWinSlots;
-        }
-        if (pc.mode == 0 && P <= 8) {
-            int32_t mj[8];
-            int32_t vj[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                mj[j] = __reduce_max_sync(0xFFFFFFFFu, acc[j]);
-                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, acc[j] == mj[j]);
-                const int kk = M - (mj[j] & M);
-                vj[j] = 8 * (wb + (__ffs(bal) - 1) + kk * T) + j;
-            }
-            // Groups g < P collect j = g, g + P, ...: larger key, then smaller v.
-            if (P <= 4) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (mj[j + 4] > mj[j] || (mj[j + 4] == mj[j] && vj[j + 4] < vj[j])) {
-                        mj[j] = mj[j + 4];
-                        vj[j] = vj[j + 4];
-                    }
-            }
-            if (P <= 2) {
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    if (mj[j + 2] > mj[j] || (mj[j + 2] == mj[j] && vj[j + 2] < vj[j])) {
-                        mj[j] = mj[j + 2];
-                        vj[j] = vj[j + 2];
-                    }
-            }
-            if (P == 1 && (mj[1] > mj[0] || (mj[1] == mj[0] && vj[1] < vj[0]))) {
-                mj[0] = mj[1];
-                vj[0] = vj[1];
-            }
-            if (T == 32) {
-                // Every lane holds every group's winner: lane g flips group g.
-                int mine = -1;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (lane == j) mine = (mj[j] != INT32_MIN) ? vj[j] : -1;
-                if (lane < P) flip_winner<DP>(s, lane, mine, loc);
-                return kWinFlipped;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (lane == j && j < P && mj[j] != INT32_MIN)
-                    atomicMax(&s.slots[j], pack_key(mj[j] >> kc.kb, vj[j]));
-            }
-        } else if (pc.mode == 0) {
-            // P = 8p, p = P/8 in {2..32}: lanes r, r + p, ... share group 8r + j.
-            // Shuffle steps outermost so the eight chains overlap, then one
-            // divergent block for the p writing lanes.
-            int32_t mx[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) mx[j] = acc[j];
-#pragma unroll
-            for (int m = 16; m >= 2; m >>= 1) {
-                if (m >= pc.period) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) mx[j] = max(mx[j], __shfl_xor_sync(0xFFFFFFFFu, mx[j], m));
+            for (int q = 0; q < 4; ++q) {
+                if (q >= Q) break;
+                const int kk = M - (key[q] & M);
+                v[q] = (key[q] != INT32_MIN) ? 8 * (t & ~31) + at[q] + 8 * kk * T : -1;
+                if (!kOne) {
+                    const int g = lane + 32 * q;
+                    if (g < P)
+                        reinterpret_cast<unsigned long long*>(scr)[g] =
+                            (v[q] >= 0) ? make_partial<DP>(s, key[q], v[q]) : 0ull;
                 }
             }
-            uint32_t bal[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) bal[j] = __ballot_sync(0xFFFFFFFFu, acc[j] == mx[j]) & pc.gmask;
-            if (lane < pc.period) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int kk = M - (mx[j] & M);
-                    const int v = 8 * (wb + (__ffs(bal[j]) - 1) + kk * T) + j;
-                    const int g = 8 * lane + j;
-                    if (T == 32) s.win[g] = (mx[j] != INT32_MIN) ? v : -1;
-                    else if (mx[j] != INT32_MIN) atomicMax(&s.slots[g], pack_key(mx[j] >> kc.kb, v));
-                }
-            }
-            if (T == 32) return kWinPublished;
         } else {
             int g = pc.g0;
 #pragma unroll
@@ -760,21 +778,20 @@ __device__ int select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc
             uint32_t x[4];
             int32_t d[8];
             philox_block(static_cast<uint32_t>(bb), sc, keys, x);
-            DP::load8(s.D, bb, d);
+            DP::load8(s.D, s.sb, bb, d);
             int g = (8 * bb) % P;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int v = 8 * bb + j;
-                if (v < n) {
+                const int vv = 8 * bb + j;
+                if (vv < n) {
                     const uint32_t r = field(x, j);
                     const int32_t sv = lut[r & 15u] + static_cast<int32_t>(r >> 4) + beta * d[j];
-                    atomicMax(&s.slots[g], pack_key(sv, v));
+                    atomicMax(&s.slots[g], pack_key(sv, vv));
                 }
                 if (++g == P) g = 0;
             }
         }
     }
-    return kWinSlots;
 }
 
 // int64 scores (the reference's two-pass path, src/anneal_kernels.cu:348-378,
@@ -804,7 +821,7 @@ __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const Ph
                          int grp) {
     const SweepConst sc = make_sweep(step, keys);
     const int P = pc.P;
-    const bool priv = pc.mode != 2;
+    const bool priv = pc.path != kPathVertex;
     if (priv) {
         Acc64 a;
 #pragma unroll
@@ -813,7 +830,7 @@ __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const Ph
             uint32_t x[4];
             int32_t d[8];
             philox_block(static_cast<uint32_t>(b), sc, keys, x);
-            DP::load8(s.D, b, d);
+            DP::load8(s.D, s.sb, b, d);
             const int lim = (n - 8 * b < 8) ? (n - 8 * b) : 8;
             score8_64(a, x, d, beta, lut, static_cast<uint32_t>(b), lim);
         }
@@ -833,7 +850,7 @@ __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const Ph
                 uint32_t x[4];
                 int32_t d[8];
                 philox_block(static_cast<uint32_t>(b), sc, keys, x);
-                DP::load8(s.D, b, d);
+                DP::load8(s.D, s.sb, b, d);
                 int g = (8 * b) % P;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -852,6 +869,184 @@ __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const Ph
             if (pass == 0) group_sync(grp, T);
         }
     }
+}
+
+// ------------------------------------------------------------------- FLIP
+// S[x] (or D[x]) changes over winner v's row after its flip: 2 w s_v for
+// neighbour x, times the neighbour's spin for int32 gains.  `neg`: v's new
+// spin is -1.  `lanes` threads share the row (this one is `sub`), four
+// entries in flight.
+template <class DP, int kFmt>
+__device__ __forceinline__ void scatter_row(const ChainSmem& s, const CsrView& csr, int v, uint32_t neg, int sub,
+                                            int lanes) {
+    uint32_t i, hi;
+    Csr<kFmt>::row(csr, v, i, hi);
+    i += sub;
+    if constexpr (DP::kField && (kFmt == kCsrUnit16 || kFmt == kCsrGlobal16)) {
+        // entry = col << 1 | w < 0: +2 or -2 added into byte lane col & 3 of
+        // word col >> 2.
+        unsigned int* Dw = reinterpret_cast<unsigned int*>(s.D);
+        for (; i + 3 * lanes < hi; i += 4 * lanes) {
+            uint32_t e[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) e[j] = Csr<kFmt>::raw(csr, i + j * lanes);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                atomicAdd(Dw + (e[j] >> 3), (((neg ^ e[j]) & 1u) ? 0xFFFFFFFEu : 2u) << ((e[j] & 6u) << 2));
+        }
+        for (; i < hi; i += lanes) {
+            const uint32_t e = Csr<kFmt>::raw(csr, i);
+            atomicAdd(Dw + (e >> 3), (((neg ^ e) & 1u) ? 0xFFFFFFFEu : 2u) << ((e & 6u) << 2));
+        }
+    } else {
+        for (; i + 3 * lanes < hi; i += 4 * lanes) {
+            int c[4], w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) Csr<kFmt>::entry(csr, i + j * lanes, c[j], w[j]);
+            uint32_t x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = DP::kField ? 0u : s.sb[c[j]] & 1u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) DP::add(s.D, c[j], (neg ^ x[j]) ? -2 * w[j] : 2 * w[j]);
+        }
+        for (; i < hi; i += lanes) {
+            int c, w;
+            Csr<kFmt>::entry(csr, i, c, w);
+            const uint32_t x = DP::kField ? 0u : s.sb[c] & 1u;
+            DP::add(s.D, c, (neg ^ x) ? -2 * w : 2 * w);
+        }
+    }
+}
+
+// Winner v (gain d, mask byte m before) flips: its stored value, its spin.
+template <class DP>
+__device__ __forceinline__ void flip_vertex(const ChainSmem& s, int v, int32_t d, uint32_t m) {
+    DP::flip(s.D, v, d, m);
+    atomicXor(&s.bits[v >> 5], 1u << (v & 31));
+    s.sb[v] = static_cast<unsigned char>(m ^ 0xFFu);
+}
+
+// FLIP on kPathWarp.  Row r = (t >> laneShift) + q T of the P winners is
+// flipped by its first lane and walked by all 2^laneShift of them; v[q] comes
+// from SELECT's registers (one-warp chains) or the warps' partials.  Returns
+// this thread's part of sum(D before) - sum(D after), which is twice the cut
+// gain once summed over the chain.
+//
+// With int8 gains nothing a row's walk reads is changed by another row (a
+// flip adds +-1 to its own byte, a walk +-2w to its neighbours': they
+// commute), so after the gains are read there is one barrier, at the end.
+// With int32 gains a walk reads its neighbours' new spins, so the flips are
+// fenced off from the walks.
+template <bool kOne, class DP, int kFmt, class Loc>
+__device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
+                                         int grp, int32_t v[4]) {
+    const int sub = t & ((1 << pc.laneShift) - 1);
+    uint32_t m[4];
+    int32_t d[4];
+    Loc loc = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= pc.rows) break;
+        const int r = (t >> pc.laneShift) + q * T;
+        if constexpr (kOne) {
+            if (q == 0 && pc.laneShift) v[0] = __shfl_sync(0xFFFFFFFFu, v[0], r);
+        } else {
+            unsigned long long p = 0;
+            v[q] = -1;
+            if (r < pc.P) {
+                const unsigned char* part = reinterpret_cast<const unsigned char*>(s.slots) + 8 * r;
+                for (int w = 0; w < (T >> 5); w += 2) {
+                    const unsigned long long a = *reinterpret_cast<const unsigned long long*>(part + w * kWarpScratch);
+                    const unsigned long long b =
+                        *reinterpret_cast<const unsigned long long*>(part + (w + 1) * kWarpScratch);
+                    const unsigned long long ab = a > b ? a : b;
+                    p = ab > p ? ab : p;
+                }
+                const uint32_t lo = static_cast<uint32_t>(p);
+                if constexpr (DP::kField) {
+                    v[q] = p ? static_cast<int32_t>(~(lo >> 9) & 0x7FFFFFu) : -1;
+                    m[q] = (lo & 0x100u) ? 0xFFu : 0u;
+                    d[q] = static_cast<int32_t>(lo & 0xFFu) - 128;
+                } else {
+                    v[q] = p ? static_cast<int32_t>(~lo) : -1;
+                }
+            }
+        }
+        if ((kOne || !DP::kField) && v[q] >= 0) {
+            m[q] = s.sb[v[q]];
+            d[q] = DP::get(s.D, s.sb, v[q]);
+        }
+        if (v[q] >= 0 && sub == 0) loc += d[q];
+    }
+    if (kOne || !DP::kField) __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= pc.rows) break;
+        if (v[q] >= 0 && sub == 0) {
+            if constexpr (DP::kField) {
+                // q' = q - 1 (+1 -> -1) or q + 1: an add, as a neighbour's
+                // walk may be adding to this byte.
+                DP::add(s.D, v[q], m[q] ? 1 : -1);
+                atomicXor(&s.bits[v[q] >> 5], 1u << (v[q] & 31));
+                s.sb[v[q]] = static_cast<unsigned char>(m[q] ^ 0xFFu);
+            } else {
+                flip_vertex<DP>(s, v[q], d[q], m[q]);
+            }
+        }
+    }
+    if (!DP::kField) group_sync(grp, T);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= pc.rows) break;
+        if (v[q] >= 0) scatter_row<DP, kFmt>(s, csr, v[q], (m[q] & 1u) ^ 1u, sub, 1 << pc.laneShift);
+    }
+    group_sync(grp, T);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= pc.rows) break;
+        if (v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
+    }
+    return loc;
+}
+
+// FLIP of winners in the group slots (other paths, int64 scores; a barrier
+// since SELECT's atomics has passed): publish and flip them, walk the rows,
+// read the gains again.
+template <class DP, int kFmt, bool kS64, class Loc>
+__device__ __forceinline__ Loc flip_slots(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
+                                          int grp) {
+    Loc loc = 0;
+    for (int gi = t; gi < pc.P; gi += T) {
+        int v;
+        if constexpr (kS64) {
+            const int32_t id = s.ids[gi];
+            v = (id == INT32_MAX) ? -1 : id;
+            s.scores[gi] = LLONG_MIN;
+            s.ids[gi] = INT32_MAX;
+        } else {
+            const unsigned long long k = s.slots[gi];
+            s.slots[gi] = 0ull;
+            v = k ? key_vertex(k) : -1;
+        }
+        s.win[gi] = v;
+        if (v >= 0) {
+            const int32_t d = DP::get(s.D, s.sb, v);
+            loc += d;
+            flip_vertex<DP>(s, v, d, s.sb[v]);
+        }
+    }
+    group_sync(grp, T);
+    const int lanes = 1 << pc.laneShift;
+    for (int gi = t >> pc.laneShift; gi < pc.P; gi += T >> pc.laneShift) {
+        const int v = s.win[gi];
+        if (v >= 0) scatter_row<DP, kFmt>(s, csr, v, s.sb[v] & 1u, t & (lanes - 1), lanes);
+    }
+    group_sync(grp, T);
+    for (int gi = t; gi < pc.P; gi += T) {
+        const int v = s.win[gi];
+        if (v >= 0) loc -= DP::get(s.D, s.sb, v);
+    }
+    return loc;
 }
 
 // ------------------------------------------------------------------ chain
@@ -880,22 +1075,26 @@ __device__ __forceinline__ int slowest_chain(const volatile int* prog) {
     return m;
 }
 
-template <class DP, int kFmt, bool kS64>
+template <bool kOne, class DP, int kFmt, bool kS64>
 __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView& csr,
-                          const int32_t* lut, int ci, int t, int T, int grp) {
+                          const int32_t* lut, int ci, int t, int threads, int grp) {
+    const int T = kOne ? 32 : threads;
     volatile int* prog = pace_state();
     DevChain& ch = L.chains[ci];
-    if (ch.sweepsDone >= ch.sweepsTotal && ch.cur != kUnsetCut) {
+    if (uniform(static_cast<int>(ch.sweepsDone >= ch.sweepsTotal && ch.cur != kUnsetCut))) {
         if (t == 0) prog[grp] = INT_MAX;
         return;
     }
-    const DevGraph& g = L.graphs[ch.graph];
-    const DevSchedule sch = L.scheds[ch.sched];
-    const int n = g.n;
-    const int words = g.words;
+    const DevGraph& g = L.graphs[uniform(ch.graph)];
+    DevSchedule sch = L.scheds[uniform(ch.sched)];
+    sch.phaseP = uniform(sch.phaseP);
+    sch.phaseIters = uniform(sch.phaseIters);
+    sch.nphases = uniform(sch.nphases);
+    const int n = uniform(g.n);
+    const int words = (n + 31) >> 5;
 
     // ---- state in: spin bits and best bits; empty group slots
-    const bool fresh = (ch.cur == kUnsetCut);
+    const bool fresh = uniform(static_cast<int>(ch.cur == kUnsetCut));
     for (int w = t; w < words; w += T) {
         const uint32_t sb = ch.spinBits[w];
         s.bits[w] = sb;
@@ -909,7 +1108,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     group_sync(grp, T);
     const int nPad = (n + 7) & ~7;
     for (int v = t; v < nPad; v += T)
-        s.sb[v] = (v < n) ? static_cast<unsigned char>(spin_of(s.bits, v)) : 0;
+        s.sb[v] = (v < n && !spin_of(s.bits, v)) ? 0xFFu : 0u;
     group_sync(grp, T);
 
     // ---- D[v] = spin[v] * sum_u w(v,u) spin[u]; padding past n is 0
@@ -923,25 +1122,27 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             for (uint32_t i = lo; i < hi; ++i) {
                 int col, w;
                 Csr<kFmt>::entry(csr, i, col, w);
-                acc += s.sb[col] ? w : -w;
+                acc += s.sb[col] ? -w : w;
             }
-            d = s.sb[v] ? acc : -acc;
+            d = s.sb[v] ? -acc : acc;
             dsum += d;
         }
-        DP::set(s.D, v, d);
+        DP::set(s.D, s.sb, v, d);
     }
     // cut = (sum over directed entries of w - sum_v D[v]) / 4, exactly.
     const int64_t cutD = (g.wsum2 - group_sum(dsum, s, t, T, grp)) / 4;
-    int64_t cur = ch.cur, best = ch.best;
+    int64_t cur = uniform(ch.cur);
+    int64_t best = uniform(ch.best);
     if (fresh) {
-        cur = best = cutD;
+        cur = best = uniform(cutD);
     } else if (cur != cutD) {
         if (t == 0) raise_error(L, kDevCutMismatch, ci);
     }
 
     // ---- window, beta cursor (first run with end > s0), phase cursor
-    const uint64_t s0 = ch.sweepsDone;
-    const uint64_t s1 = (ch.sweepsTotal - s0 > L.window) ? s0 + L.window : ch.sweepsTotal;
+    const uint64_t s0 = uniform(ch.sweepsDone);
+    const uint64_t sEnd = uniform(ch.sweepsTotal);
+    const uint64_t s1 = (sEnd - s0 > L.window) ? s0 + L.window : sEnd;
     int64_t run = 0;
     {
         int64_t lo = 0, hi = ch.betaRuns;
@@ -949,7 +1150,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             const int64_t mid = (lo + hi) >> 1;
             if (static_cast<uint64_t>(ch.betaEnd[mid]) > s0) hi = mid; else lo = mid + 1;
         }
-        run = lo;
+        run = uniform(lo);
     }
     if (s1 > s0 && (run >= ch.betaRuns ||
                     static_cast<uint64_t>(ch.betaEnd[ch.betaRuns - 1]) < s1)) {
@@ -965,32 +1166,52 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     {
         uint64_t acc = 0;
         for (p = 0; p < sch.nphases; ++p) {
-            if (sch.phaseP[p] == 0) continue;
-            if (acc + sch.phaseIters[p] > s0) break;
-            acc += sch.phaseIters[p];
+            if (uniform(sch.phaseP[p]) == 0) continue;
+            const uint64_t iters = uniform(sch.phaseIters[p]);
+            if (acc + iters > s0) break;
+            acc += iters;
         }
         if (p < sch.nphases) {
-            phaseEnd = acc + sch.phaseIters[p];
-            P = static_cast<int>(umin(sch.phaseP[p], static_cast<uint32_t>(n)));
+            phaseEnd = acc + uniform(sch.phaseIters[p]);
+            P = static_cast<int>(umin(uniform(sch.phaseP[p]), static_cast<uint32_t>(n)));
         }
     }
-    PhaseCfg pc = phase_cfg(P, t, T);
+    PhaseCfg pc = phase_cfg(P, t, T, kS64);
 
     const ChainKeys keys = make_keys(ch.solverSeed);
     // Beta cursor in registers, with the following run prefetched one run
     // ahead (read-only path): a run change costs no dependent global load.
-    const int64_t* __restrict__ bEnd = ch.betaEnd;
-    const int32_t* __restrict__ bVal = ch.betaVal;
-    const int64_t nRuns = ch.betaRuns;
-    uint64_t betaNext = (s1 > s0) ? static_cast<uint64_t>(__ldg(bEnd + run)) : 0;
-    int32_t beta = (s1 > s0) ? __ldg(bVal + run) : 0;
-    uint64_t pfEnd = ~0ull;
+    const int64_t* __restrict__ bEnd = uniform(ch.betaEnd);
+    const int32_t* __restrict__ bVal = uniform(ch.betaVal);
+    const int64_t nRuns = uniform(ch.betaRuns);
+    uint64_t betaNext = (s1 > s0) ? uniform(static_cast<uint64_t>(__ldg(bEnd + run))) : 0;
+    int32_t beta = (s1 > s0) ? uniform(__ldg(bVal + run)) : 0;
+    uint64_t pfEnd = ~uint64_t(0);
     int32_t pfVal = 0;
     if (s1 > s0 && run + 1 < nRuns) {
         pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 1));
         pfVal = __ldg(bVal + run + 1);
     }
     uint64_t improved = 0;
+    using Loc = typename std::conditional<DP::kField, int32_t, int64_t>::type;
+    // The last sweep's gain is settled when the next one is about to flip (or
+    // at the window's end): the loads and the warp sum behind it overlap
+    // SELECT, and wider chains pass the warps' sums through s.red under
+    // SELECT's own barrier instead of one more.
+    Loc loc = 0;
+    auto settle = [&](uint64_t sw) {
+        if (sw == s0) return;
+        Loc gain;
+        if constexpr (kOne) gain = warp_sum(loc);
+        else gain = warp_sum(static_cast<Loc>((t & 31) < (T >> 5) ? s.red[t & 31] : 0));
+        cur += gain / 2;
+        if (cur > best) {
+            best = cur;
+            ++improved;
+            for (int w = t; w < words; w += T) s.best[w] = s.bits[w];
+            group_sync(grp, T);
+        }
+    };
     group_sync(grp, T);
 
     for (uint64_t sw = s0; sw < s1; ++sw) {
@@ -998,17 +1219,24 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             while (sw >= phaseEnd) {
                 ++p;
                 if (p >= sch.nphases) break;
-                if (sch.phaseP[p] == 0) continue;
-                phaseEnd += sch.phaseIters[p];
-                P = static_cast<int>(umin(sch.phaseP[p], static_cast<uint32_t>(n)));
+                if (uniform(sch.phaseP[p]) == 0) continue;
+                phaseEnd += uniform(sch.phaseIters[p]);
+                P = static_cast<int>(umin(uniform(sch.phaseP[p]), static_cast<uint32_t>(n)));
             }
-            pc = phase_cfg(P, t, T);
+            const bool warp = pc.path == kPathWarp;
+            pc = phase_cfg(P, t, T, kS64);
+            if (warp && pc.path != kPathWarp) {
+                // The slots held scratch and partials: empty them (all their
+                // readers are past the last sweep's barrier).
+                for (int i = t; i < L.pmax; i += T) s.slots[i] = 0ull;
+                group_sync(grp, T);
+            }
         }
         if (sw >= betaNext) {
             // Runs are never empty, so one step of the cursor per sweep.
             ++run;
-            betaNext = pfEnd;
-            beta = pfVal;
+            betaNext = uniform(pfEnd);
+            beta = uniform(pfVal);
             if (run + 1 < nRuns) {
                 pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 1));
                 pfVal = __ldg(bVal + run + 1);
@@ -1025,90 +1253,21 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         }
         const uint64_t step = sw + 1;   // 1-based sweep id
 
-        using Loc = typename std::conditional<std::is_same<DP, D8>::value, int32_t, int64_t>::type;
-        Loc loc = 0;
-        int handoff = kWinSlots;
+        int32_t v[4];
         if constexpr (kS64) select64<DP>(s, lut, n, pc, beta, step, keys, t, T, grp);
-        else handoff = select32<DP>(s, lut, kc, n, pc, beta, step, keys, t, T, loc);
-
-        // ---- FLIP 1: winners; negate their gains, flip their spins
-        if (handoff != kWinFlipped) {
-            group_sync(grp, T);
-            for (int gi = t; gi < P; gi += T) {
-                int v;
-                if constexpr (kS64) {
-                    const int32_t id = s.ids[gi];
-                    v = (id == INT32_MAX) ? -1 : id;
-                    s.scores[gi] = LLONG_MIN;
-                    s.ids[gi] = INT32_MAX;
-                } else if (handoff == kWinPublished) {
-                    v = s.win[gi];
-                } else {
-                    const unsigned long long k = s.slots[gi];
-                    s.slots[gi] = 0ull;
-                    v = k ? key_vertex(k) : -1;
-                }
-                flip_winner<DP>(s, gi, v, loc);
-            }
-        }
-        group_sync(grp, T);
-
-        // ---- FLIP 2: D[x] += 2 w s_b s_x over the winners' rows (new spins);
-        // `lanes` consecutive threads share a row, four entries in flight.
-        bool walked = false;
-        if constexpr ((kFmt == kCsrUnit16 || kFmt == kCsrGlobal16) && std::is_same<DP, D8>::value) {
-            if (T == 32 && P >= 64) {
-                flip2_unit16_d8_warp<kFmt>(s, csr, P, t);
-                walked = true;
-            }
-        }
-        if (!walked) {
-            const int lanes = 1 << pc.laneShift;
-            const int sub = t & (lanes - 1);
-            for (int gi = t >> pc.laneShift; gi < P; gi += T >> pc.laneShift) {
-                const int v = s.win[gi];
-                if (v < 0) continue;
-                const int sv = s.sb[v];
-                uint32_t lo, hi;
-                Csr<kFmt>::row(csr, v, lo, hi);
-                uint32_t i = lo + sub;
-                for (; i + 3 * lanes < hi; i += 4 * lanes) {
-                    int c0, w0, c1, w1, c2, w2, c3, w3;
-                    Csr<kFmt>::entry(csr, i, c0, w0);
-                    Csr<kFmt>::entry(csr, i + lanes, c1, w1);
-                    Csr<kFmt>::entry(csr, i + 2 * lanes, c2, w2);
-                    Csr<kFmt>::entry(csr, i + 3 * lanes, c3, w3);
-                    const int s0b = s.sb[c0], s1b = s.sb[c1];
-                    const int s2b = s.sb[c2], s3b = s.sb[c3];
-                    DP::add(s.D, c0, (sv == s0b) ? 2 * w0 : -2 * w0);
-                    DP::add(s.D, c1, (sv == s1b) ? 2 * w1 : -2 * w1);
-                    DP::add(s.D, c2, (sv == s2b) ? 2 * w2 : -2 * w2);
-                    DP::add(s.D, c3, (sv == s3b) ? 2 * w3 : -2 * w3);
-                }
-                for (; i < hi; i += lanes) {
-                    int c0, w0;
-                    Csr<kFmt>::entry(csr, i, c0, w0);
-                    DP::add(s.D, c0, (sv == s.sb[c0]) ? 2 * w0 : -2 * w0);
-                }
-            }
-        }
-        group_sync(grp, T);
-
-        // ---- FLIP 3: gain = (sum delta_pre - sum D_final) / 2
-        for (int gi = t; gi < P; gi += T) {
-            const int v = s.win[gi];
-            if (v >= 0) loc -= DP::get(s.D, v);
-        }
-        int64_t gain;
-        if constexpr (std::is_same<DP, D8>::value) gain = group_sum32(loc, s, t, T, grp) / 2;
-        else gain = group_sum(loc, s, t, T, grp) / 2;
-        cur += gain;
-        if (cur > best) {
-            best = cur;
-            ++improved;
-            for (int w = t; w < words; w += T) s.best[w] = s.bits[w];
+        else select32<kOne, DP>(s, lut, kc, n, pc, beta, step, keys, t, T, v);
+        const bool slots = kS64 || pc.path != kPathWarp;
+        if (!kOne || slots) group_sync(grp, T);
+        settle(sw);
+        if (slots) loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
+        else loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+        if (!kOne) {
+            loc = warp_sum(loc);
+            if ((t & 31) == 0) s.red[t >> 5] = loc;
         }
     }
+    if (!kOne) group_sync(grp, T);
+    settle(s1);
     if (t == 0) prog[grp] = INT_MAX;
     group_sync(grp, T);
 
@@ -1187,8 +1346,11 @@ __device__ bool stage_csr(const DevGraph& g, unsigned char* dst, uint64_t* mbar,
     return ok;
 }
 
-// kDBytes: 1 -> D8, 4 -> D32.
-template <int kDBytes, int kFmt, bool kS64>
+// kDBytes: 1 -> D8, 4 -> D32.  kOne: chains of one warp, whose barriers are
+// __syncwarp and whose winners stay in registers; a kernel of its own, as both
+// forms in one do not fit 128 registers (they spill ~200 bytes).  The int64
+// score path is one kernel for every width.
+template <int kDBytes, int kFmt, bool kS64, bool kOne>
 __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) {
     using DP = typename std::conditional<kDBytes == 1, D8, D32>::type;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1199,8 +1361,8 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
     unsigned char* csrBase = smem + kSmemHeader;
     unsigned char* chainBase = csrBase + L.csrBytes;
 
-    const int T = 32 * L.warpsPerChain;
-    const int grp = threadIdx.x / T;
+    const int T = kOne ? 32 : 32 * L.warpsPerChain;
+    const int grp = uniform(static_cast<int>(threadIdx.x) / T);
     const int t = threadIdx.x - grp * T;
     const ChainSmem cs = carve_chain(chainBase + static_cast<size_t>(grp) * L.chainBytes, L, kDBytes);
 
@@ -1213,9 +1375,12 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
     for (;;) {
         if (threadIdx.x == 0) *sItem = atomicAdd(L.queue, 1);
         __syncthreads();
-        const int it = *sItem;
+        const int it = uniform(*sItem);
         if (it >= L.nitems) break;
-        const DevItem item = L.items[it];
+        DevItem item = L.items[it];
+        item.graph = uniform(item.graph);
+        item.first = uniform(item.first);
+        item.count = uniform(item.count);
         if (item.graph < 0 || item.graph >= L.ngraphs) {
             if (threadIdx.x == 0) raise_error(L, kDevBadItem, it);
             __syncthreads();
@@ -1255,8 +1420,10 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
         if (threadIdx.x < 16) sProg[threadIdx.x] = (static_cast<int>(threadIdx.x) < active) ? 0 : INT_MAX;
         if (threadIdx.x == 0) sProg[16] = active;
         __syncthreads();
-        if (grp < active)
-            run_chain<DP, kFmt, kS64>(L, cs, csr, lut, L.order[item.first + grp], t, T, grp);
+        if (grp < active) {
+            const int ci = uniform(L.order[item.first + grp]);
+            run_chain<kOne, DP, kFmt, kS64>(L, cs, csr, lut, ci, t, T, grp);
+        }
         __syncthreads();
         if (threadIdx.x == 0 && L.itemNs) {
             uint64_t t1;
@@ -1270,28 +1437,43 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
 
 // ------------------------------------------------------------ host hooks
 // Kernel variants: D width {1, 4} x CSR format {unit16, packed32, HBM 8-byte,
-// HBM 16-bit, HBM 32-bit} x score {int32, int64}.
-template <int DB, bool S>
+// HBM 16-bit, HBM 32-bit} x {int32 scores one-warp, int32 scores wider, int64
+// scores}.  The two D widths compile as two translation units (this file, and
+// rfmf_anneal_i32.cu, which includes it), side by side.
+namespace {
+template <int DB, bool S, bool One>
 const void* kernel_for_format(int fmt) {
     switch (fmt) {
-        case kCsrUnit16: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrUnit16, S>);
-        case kCsrPacked32: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrPacked32, S>);
-        case kCsrGlobal16: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal16, S>);
-        case kCsrGlobal32: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal32, S>);
-        default: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal, S>);
+        case kCsrUnit16: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrUnit16, S, One>);
+        case kCsrPacked32: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrPacked32, S, One>);
+        case kCsrGlobal16: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal16, S, One>);
+        case kCsrGlobal32: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal32, S, One>);
+        default: return reinterpret_cast<const void*>(&rfmf_anneal_kernel<DB, kCsrGlobal, S, One>);
     }
 }
 
-const void* kernel_ptr(int dbytes, int fmt, bool s64) {
-    if (dbytes == 1) return s64 ? kernel_for_format<1, true>(fmt) : kernel_for_format<1, false>(fmt);
-    return s64 ? kernel_for_format<4, true>(fmt) : kernel_for_format<4, false>(fmt);
+template <int DB>
+const void* kernel_for(int fmt, bool s64, int warps) {
+    if (s64) return kernel_for_format<DB, true, false>(fmt);
+    return warps == 1 ? kernel_for_format<DB, false, true>(fmt) : kernel_for_format<DB, false, false>(fmt);
+}
+}  // namespace
+
+#if RFMF_GAIN_BYTES == 4
+const void* kernel_ptr_i32(int fmt, bool s64, int warps) { return kernel_for<4>(fmt, s64, warps); }
+#else
+const void* kernel_ptr_i32(int fmt, bool s64, int warps);
+
+const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps) {
+    return dbytes == 1 ? kernel_for<1>(fmt, s64, warps) : kernel_ptr_i32(fmt, s64, warps);
 }
 
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream) {
     void* args[] = {const_cast<DevLaunch*>(&L)};
-    return cudaLaunchKernel(kernel_ptr(dbytes, fmt, s64), dim3(grid), dim3(threads), args, smem,
+    return cudaLaunchKernel(kernel_ptr(dbytes, fmt, s64, L.warpsPerChain), dim3(grid), dim3(threads), args, smem,
                             stream);
 }
+#endif
 
 }  // namespace rfmf

@@ -128,7 +128,7 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
         perGraph.push_back(static_cast<int64_t>(k.chainsOf[q].size()));
     }
     k.pmax = std::max(1, std::min(k.pmax, maxN));
-    const void* kern = kernel_ptr(k.dbytes, k.fmt, k.score64);
+    const void* kern = kernel_ptr(k.dbytes, k.fmt, k.score64, k.warps);
     cudaFuncAttributes fa{};
     const int64_t dynMax = dyn_smem_max(b.ctx, kern, fa);
     if (dynMax < 0) return fail(RFMF_ERR_CUDA, "kernel attributes unavailable");
@@ -687,7 +687,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                                       static_cast<int64_t>(std::max(1, 8 / Wc)), perSm}));
             auto fits = [&](int f) {
                 cudaFuncAttributes fa{};
-                const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, f, pk.s64), fa);
+                const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, f, pk.s64, Wc), fa);
                 return dynMax > 0 &&
                        static_cast<int64_t>(kSmemHeader) + csr_bytes(g, f) + kWant * chainB <= dynMax;
             };
@@ -705,7 +705,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             // the 8-byte pairs are asked for.
             if (pk.fmt == kCsrGlobal && c.csr_format != 4) pk.fmt = hbm_format(g);
             cudaFuncAttributes fa{};
-            const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, pk.fmt, pk.s64), fa);
+            const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, pk.fmt, pk.s64, Wc), fa);
             const int64_t room = dynMax - static_cast<int64_t>(kSmemHeader) -
                                  (csr_in_hbm(pk.fmt) ? 0 : static_cast<int64_t>(csr_bytes(g, pk.fmt)));
             const int64_t warpCap = std::min(16 / Wc, Wc > 1 ? 15 : 16);
@@ -762,7 +762,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             if (csr_in_hbm(b->cls[ci].fmt)) continue;
             cudaFuncAttributes fa{};
             const int64_t dynMax =
-                dyn_smem_max(ctx, kernel_ptr(b->cls[ci].dbytes, b->cls[ci].fmt, b->cls[ci].score64), fa);
+                dyn_smem_max(ctx, kernel_ptr(b->cls[ci].dbytes, b->cls[ci].fmt, b->cls[ci].score64, b->cls[ci].warps), fa);
             while (!b->cls[ci].graphs.empty()) {
                 BatchClass& k = b->cls[ci];
                 auto chainOf = [&](int64_t n) {

@@ -140,13 +140,17 @@ constexpr uint32_t kSmemHeader = 256;
 RFMF_HD uint32_t align16(uint32_t x) { return (x + 15u) & ~15u; }
 
 // Per-chain shared-memory region, in order: gains D (nPad * dbytes), spin
-// bits, best-spin bits, spins as bytes (0/1, for one-load neighbour lookups
-// in FLIP), group key slots (8 B), ids (4 B), winners (4 B),
-// reduction partials (8 B per warp).
+// bits, best-spin bits, spins as mask bytes (0x00 / 0xFF), group key slots
+// (8 B per group, or the warps' argmax scratch and partials), ids (4 B),
+// winners (4 B), reduction partials (8 B per warp).
 // Host and kernel both carve with this.
 struct ChainLayout {
     uint32_t d, bits, best, sb, slots, ids, win, red, total;
 };
+
+// Argmax scratch of one warp: 256 keys in two halves 16 banks apart, reused
+// for up to 128 partials of 8 bytes.
+constexpr uint32_t kWarpScratch = (144 + 128) * 4;
 
 RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, int dbytes) {
     ChainLayout c;
@@ -156,7 +160,8 @@ RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, in
     c.bits = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.best = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.sb = o;    o = align16(o + nPad);
-    c.slots = o; o = align16(o + static_cast<uint32_t>(pmax) * 8u);
+    const uint32_t slots = static_cast<uint32_t>(pmax) * 8u, scratch = static_cast<uint32_t>(warps) * kWarpScratch;
+    c.slots = o; o = align16(o + (slots > scratch ? slots : scratch));
     c.ids = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);
     c.win = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);
     c.red = o;   o = align16(o + static_cast<uint32_t>(warps) * 8u);

@@ -41,7 +41,7 @@ inline void host_alloc_point() {
 }
 
 // Kernel entry points (rfmf_anneal.cu).
-const void* kernel_ptr(int dbytes, int fmt, bool s64);
+const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream);
 

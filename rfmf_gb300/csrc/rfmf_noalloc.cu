@@ -49,7 +49,7 @@
 namespace rfmf {
 int set_last_error(int code, const char* msg);
 int fail(int code, const char* fmt, ...);
-const void* kernel_ptr(int dbytes, int fmt, bool s64);
+const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream);
 }  // namespace rfmf
@@ -223,7 +223,7 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
         return nerr(RFMF_ERR_CUDA, "device attribute query failed");
-    const void* kern = kernel_ptr(dbytes, kCsrGlobal, s64);
+    const void* kern = kernel_ptr(dbytes, kCsrGlobal, s64, W);
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return nerr(RFMF_ERR_CUDA, "kernel attributes");
     const int dynMax = optin - static_cast<int>(fa.sharedSizeBytes);

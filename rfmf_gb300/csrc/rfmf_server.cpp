@@ -410,7 +410,7 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
             pmax = std::max(pmax, r->pmax);
             csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
         }
-        const void* kern = kernel_ptr(k.dbytes, k.fmt, k.s64);
+        const void* kern = kernel_ptr(k.dbytes, k.fmt, k.s64, k.W);
         if (int rc = ensure_attr(s, kern)) return rc;
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kern));
@@ -829,7 +829,7 @@ static int rfmf_submit_impl(rfmf_server* s, const rfmf_graph* g, int64_t nchains
     // the request's chains, if fewer), else the CSR is walked in HBM.
     {
         cudaFuncAttributes fa{};
-        CU(cudaFuncGetAttributes(&fa, kernel_ptr(r->dbytes, fmt, r->s64)));
+        CU(cudaFuncGetAttributes(&fa, kernel_ptr(r->dbytes, fmt, r->s64, r->W)));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
         const uint32_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax,
                                              r->W, r->dbytes).total;
