@@ -245,16 +245,20 @@ __device__ __forceinline__ int32_t sbyte(uint32_t x) {
     return r;
 }
 
-// Byte k of x zero-extended to 32 bits.
+// Byte k of x zero-extended to 32 bits, as a dot product with a unit byte: it
+// issues on the FMA pipe, while a byte permute or a shift would take the ALU
+// pipe that bounds SELECT (see score8_key).
 template <int k>
 __device__ __forceinline__ int32_t ubyte(uint32_t x) {
     int32_t r;
-    if constexpr (k == 3) {
-        r = static_cast<int32_t>(x >> 24);
-    } else {
-        constexpr uint32_t sel = static_cast<uint32_t>(k) | 0x4440u;
-        asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(x), "n"(sel));
-    }
+    asm("dp4a.u32.u32 %0, %1, %2, 0;" : "=r"(r) : "r"(x), "r"(1u << (8 * k)));
+    return r;
+}
+
+// c + b * (half k of x, 16 bits), b < 256, on the FMA pipe: b arrives as byte k.
+__device__ __forceinline__ uint32_t add_half(uint32_t x, uint32_t bytes, uint32_t c) {
+    uint32_t r;
+    asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(x), "r"(bytes), "r"(c));
     return r;
 }
 
@@ -506,14 +510,23 @@ __device__ __forceinline__ PhaseCfg phase_cfg(int P, int t, int T, bool slots) {
 // TK[L & 15]) and is read with one shuffle whose source lane is the Philox
 // word itself (a shuffle takes its source lane modulo 32, and lanes L and
 // L + 16 hold the same entry, so the low word needs no masking and the high
-// one a single shift); the field's multiple f * 2^(kb-4) is one multiply-add
-// on the FMA pipe (a mul.hi for the high half-word, whose field sits at bit
-// 16); the final add and max fuse into one add-max.
+// one a single shift); beta * gain is one multiply-add; the field is a mask
+// folded into the add + max when kb == 4, else its multiple is added by a
+// 16-bit dot product.
+//
+// Measured on GB300, cycles per warp instruction and scheduler: logic, shifts,
+// permutes, max and add-max 2 on the ALU pipe; 32-bit multiply-add and the dot
+// products 2 on the FMA pipe; a wide or high multiply 4 on the FMA pipe and 2
+// on the ALU pipe.  A block of 8 vertices' Philox takes 74 ALU / 72 FMA
+// cycles; its scoring adds 44 / 32, having moved the byte extraction of int8
+// gains off the ALU pipe (60 / 16 before; the loop alone at four warps per
+// scheduler 143 -> 134 cycles a block).  Adding some of the fields with dot
+// products too (114 / 112 on paper) was slower, 138.
 struct KeyCfg {
     int kb;          // bits of the block-iteration field
-    uint32_t mulF;   // 2^(kb-4): f * mulF for a low-half field
-    uint32_t mulHi;  // 2^(kb+12): umulhi(x & 0x07FF0000, mulHi) = f * 2^(kb-4)
+    uint32_t mulF;   // 2^(kb-4), the field's multiple; below 256 (a chain of 2^19 vertices would not fit)
     int32_t tkLane;  // TK[lane & 15]
+    int iters;       // block iterations of this thread's warp
 };
 
 __device__ __forceinline__ int key_bits(int n, int T) {
@@ -527,7 +540,8 @@ __device__ __forceinline__ KeyCfg key_cfg(int n, int T, int t, const int32_t* lu
     KeyCfg kc;
     kc.kb = key_bits(n, T);
     kc.mulF = 1u << (kc.kb - 4);
-    kc.mulHi = 1u << (kc.kb + 12);
+    const int ahead = ((n + 7) >> 3) - (t & ~31);   // blocks from the warp's first on
+    kc.iters = uniform(ahead > 0 ? (ahead + T - 1) / T : 0);
     const int i = t & 15;
     kc.tkLane = lut[i] * (1 << kc.kb) - i * static_cast<int32_t>(kc.mulF);
     return kc;
@@ -548,70 +562,69 @@ __device__ __forceinline__ void score8_key(int32_t acc[8], const uint32_t x[4], 
         const uint32_t xs = x[w] >> 16;
         const int32_t tk0 = __shfl_sync(0xFFFFFFFFu, tkb, static_cast<int>(x[w]));
         const int32_t tk1 = __shfl_sync(0xFFFFFFFFu, tkb, static_cast<int>(xs));
-        int32_t f0, f1;
-        if constexpr (kF0) {
-            f0 = static_cast<int32_t>(x[w] & 0x7FFu);
-            f1 = static_cast<int32_t>(xs & 0x7FFu);
-        } else {
-            f0 = static_cast<int32_t>((x[w] & 0x7FFu) * kc.mulF);
-            f1 = static_cast<int32_t>(__umulhi(x[w] & 0x07FF0000u, kc.mulHi));
-        }
         const int32_t k0 = static_cast<int32_t>(static_cast<uint32_t>(betaK) * static_cast<uint32_t>(d[2 * w]) +
                                                 static_cast<uint32_t>(tk0));
         const int32_t k1 = static_cast<int32_t>(static_cast<uint32_t>(betaK) * static_cast<uint32_t>(d[2 * w + 1]) +
                                                 static_cast<uint32_t>(tk1));
-        if (!kMasked || 2 * w < lim) acc[2 * w] = __viaddmax_s32(k0, f0, acc[2 * w]);
-        if (!kMasked || 2 * w + 1 < lim) acc[2 * w + 1] = __viaddmax_s32(k1, f1, acc[2 * w + 1]);
+        if constexpr (kF0) {
+            if (!kMasked || 2 * w < lim)
+                acc[2 * w] = __viaddmax_s32(k0, static_cast<int32_t>(x[w] & 0x7FFu), acc[2 * w]);
+            if (!kMasked || 2 * w + 1 < lim)
+                acc[2 * w + 1] = __viaddmax_s32(k1, static_cast<int32_t>(xs & 0x7FFu), acc[2 * w + 1]);
+        } else {
+            const uint32_t f = x[w] & 0x07FF07FFu;
+            const int32_t s0 = static_cast<int32_t>(add_half(f, kc.mulF, static_cast<uint32_t>(k0)));
+            const int32_t s1 = static_cast<int32_t>(add_half(f, kc.mulF << 8, static_cast<uint32_t>(k1)));
+            if (!kMasked || 2 * w < lim) acc[2 * w] = max(acc[2 * w], s0);
+            if (!kMasked || 2 * w + 1 < lim) acc[2 * w + 1] = max(acc[2 * w + 1], s1);
+        }
     }
 }
 
 // NB vertex blocks b, b + T, ... (block iterations k, k + 1, ...) scored with
-// their Philox draws in flight together.
-template <int NB, bool kMasked, bool kF0, class DP>
+// their Philox draws in flight together.  kTail: the last of them may be
+// ragged: a lane past the last block scores that block's place again with
+// lim = 0, one on a partial block has lim = n & 7.
+template <int NB, bool kTail, bool kF0, class DP>
 __device__ __forceinline__ void score_blocks(int32_t acc[8], const ChainSmem& s, const SweepConst& sc,
-                                             const ChainKeys& keys, int b, int T, int32_t betaK,
-                                             int32_t tkb, const KeyCfg& kc, int lim) {
+                                             const ChainKeys& keys, int b, int T, int n, int32_t betaK,
+                                             int32_t tkb, const KeyCfg& kc) {
     uint32_t x[NB][4];
-    int32_t d[NB][8];
+    int last = b + (NB - 1) * T, lim = 8;
+    if (kTail) {
+        const int nfull = n >> 3, nblk = (n + 7) >> 3;
+        lim = (last < nfull) ? 8 : ((last == nfull) ? (n & 7) : 0);
+        last = (last < nblk) ? last : nblk - 1;
+    }
 #pragma unroll
-    for (int q = 0; q < NB; ++q) philox_block(static_cast<uint32_t>(b + q * T), sc, keys, x[q]);
-    if constexpr (NB >= 3) {
-        // Three blocks' Philox words in flight; each block's gains are
-        // loaded just before it is scored so that they fit the registers.
+    for (int q = 0; q < NB; ++q)
+        philox_block(static_cast<uint32_t>(q == NB - 1 ? last : b + q * T), sc, keys, x[q]);
+    // Each block's gains are loaded just before it is scored so that three
+    // blocks' Philox words fit the registers.
 #pragma unroll
-        for (int q = 0; q < NB; ++q) {
-            DP::load8raw(s.D, s.sb, b + q * T, d[0]);
-            score8_key<kMasked, kF0>(acc, x[q], d[0], betaK, tkb - q, kc, lim);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < NB; ++q) DP::load8raw(s.D, s.sb, b + q * T, d[q]);
-#pragma unroll
-        for (int q = 0; q < NB; ++q) score8_key<kMasked, kF0>(acc, x[q], d[q], betaK, tkb - q, kc, lim);
+    for (int q = 0; q < NB; ++q) {
+        int32_t d[8];
+        DP::load8raw(s.D, s.sb, q == NB - 1 ? last : b + q * T, d);
+        if (kTail && q == NB - 1) score8_key<true, kF0>(acc, x[q], d, betaK, tkb - q, kc, lim);
+        else score8_key<false, kF0>(acc, x[q], d, betaK, tkb - q, kc, 8);
     }
 }
 
-// The block loop of select32 (trip counts uniform per warp: its blocks at
-// step k are wb + kT .. wb + kT + 31, so the table shuffles run converged):
-// three blocks in flight while the whole warp has three full blocks left,
-// then two, then a clamped, masked single-block tail.
+// The block loop of select32: the warp's iterations (uniform, so the table
+// shuffles run converged), three in flight, the last one to three together:
+// all of them full but the very last.  One iteration alone takes 250 cycles
+// on GB300 against 180 each for two or three in flight, so the remainder is
+// never walked one by one.
 template <bool kF0, class DP>
 __device__ __forceinline__ void select_blocks(int32_t acc[8], const ChainSmem& s, const SweepConst& sc,
-                                              const ChainKeys& keys, int n, int t, int T,
-                                              int32_t betaK, int32_t tkBase, const KeyCfg& kc) {
-    const int nfull = n >> 3;
-    const int nblk = (n + 7) >> 3;
-    const int wb = t & ~31;
-    int b = t, k = 0;
-    for (; wb + 2 * T + 31 < nfull - k * T; b += 3 * T, k += 3)
-        score_blocks<3, false, kF0, DP>(acc, s, sc, keys, b, T, betaK, tkBase - k, kc, 8);
-    for (; wb + T + 31 < nfull - k * T; b += 2 * T, k += 2)
-        score_blocks<2, false, kF0, DP>(acc, s, sc, keys, b, T, betaK, tkBase - k, kc, 8);
-    for (; wb + k * T < nblk; b += T, ++k) {
-        const int bb = (b < nblk) ? b : nblk - 1;
-        const int lim = (b < nfull) ? 8 : ((b == nfull) ? (n & 7) : 0);
-        score_blocks<1, true, kF0, DP>(acc, s, sc, keys, bb, T, betaK, tkBase - k, kc, lim);
-    }
+                                              const ChainKeys& keys, int n, int t, int T, int left,
+                                              int32_t betaK, int32_t tkb, const KeyCfg& kc) {
+    int b = t;
+    for (; left > 3; left -= 3, b += 3 * T, tkb -= 3)
+        score_blocks<3, false, kF0, DP>(acc, s, sc, keys, b, T, n, betaK, tkb, kc);
+    if (left == 3) score_blocks<3, true, kF0, DP>(acc, s, sc, keys, b, T, n, betaK, tkb, kc);
+    else if (left == 2) score_blocks<2, true, kF0, DP>(acc, s, sc, keys, b, T, n, betaK, tkb, kc);
+    else if (left == 1) score_blocks<1, true, kF0, DP>(acc, s, sc, keys, b, T, n, betaK, tkb, kc);
 }
 
 // The winner of one group among a warp's 256 accumulators: its compact key
@@ -723,9 +736,8 @@ __device__ __forceinline__ unsigned long long make_partial(const ChainSmem& s, i
 // packed keys in the group slots (a barrier is due).
 template <bool kOne, class DP>
 __device__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
-                         const PhaseCfg& pc, int32_t beta, uint64_t step, const ChainKeys& keys,
+                         const PhaseCfg& pc, int32_t beta, const SweepConst& sc, const ChainKeys& keys,
                          int t, int T, int32_t v[4]) {
-    const SweepConst sc = make_sweep(step, keys);
     const int P = pc.P;
     const int M = (1 << kc.kb) - 1;
     if (pc.path != kPathVertex) {
@@ -736,8 +748,8 @@ __device__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& k
         // Per-sweep part of the table register: (2^kb - 1) - bias * beta * 2^kb.
         const int32_t tkBase = static_cast<int32_t>(static_cast<uint32_t>(kc.tkLane) + static_cast<uint32_t>(M) -
                                                     static_cast<uint32_t>(DP::kBias) * static_cast<uint32_t>(betaK));
-        if (kc.kb == 4) select_blocks<true, DP>(acc, s, sc, keys, n, t, T, betaK, tkBase, kc);
-        else select_blocks<false, DP>(acc, s, sc, keys, n, t, T, betaK, tkBase, kc);
+        if (kc.kb == 4) select_blocks<true, DP>(acc, s, sc, keys, n, t, T, kc.iters, betaK, tkBase, kc);
+        else select_blocks<false, DP>(acc, s, sc, keys, n, t, T, kc.iters, betaK, tkBase, kc);
         if (pc.path == kPathWarp) {
             const int lane = t & 31;
             int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
@@ -817,9 +829,8 @@ __device__ __forceinline__ void score8_64(Acc64& a, const uint32_t x[4], const i
 
 template <class DP>
 __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const PhaseCfg& pc,
-                         int32_t beta, uint64_t step, const ChainKeys& keys, int t, int T,
+                         int32_t beta, const SweepConst& sc, const ChainKeys& keys, int t, int T,
                          int grp) {
-    const SweepConst sc = make_sweep(step, keys);
     const int P = pc.P;
     const bool priv = pc.path != kPathVertex;
     if (priv) {
@@ -941,11 +952,12 @@ template <bool kOne, class DP, int kFmt, class Loc>
 __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
                                          int grp, int32_t v[4]) {
     const int sub = t & ((1 << pc.laneShift) - 1);
-    uint32_t m[4];
-    int32_t d[4];
+    constexpr int kRows = kOne ? 4 : 2;   // P <= 128 over at least 32 or 64 threads
+    uint32_t m[kRows];
+    int32_t d[kRows];
     Loc loc = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRows; ++q) {
         if (q >= pc.rows) break;
         const int r = (t >> pc.laneShift) + q * T;
         if constexpr (kOne) {
@@ -980,7 +992,7 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
     }
     if (kOne || !DP::kField) __syncwarp();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRows; ++q) {
         if (q >= pc.rows) break;
         if (v[q] >= 0 && sub == 0) {
             if constexpr (DP::kField) {
@@ -996,13 +1008,13 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
     }
     if (!DP::kField) group_sync(grp, T);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRows; ++q) {
         if (q >= pc.rows) break;
         if (v[q] >= 0) scatter_row<DP, kFmt>(s, csr, v[q], (m[q] & 1u) ^ 1u, sub, 1 << pc.laneShift);
     }
     group_sync(grp, T);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRows; ++q) {
         if (q >= pc.rows) break;
         if (v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
     }
@@ -1179,18 +1191,25 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     PhaseCfg pc = phase_cfg(P, t, T, kS64);
 
     const ChainKeys keys = make_keys(ch.solverSeed);
-    // Beta cursor in registers, with the following run prefetched one run
-    // ahead (read-only path): a run change costs no dependent global load.
+    // Beta cursor: the current run and the next one as uniform values, the one
+    // after as loads in flight (read-only path), so that a change of run costs
+    // neither a dependent global load nor a reduction before SELECT.
     const int64_t* __restrict__ bEnd = uniform(ch.betaEnd);
     const int32_t* __restrict__ bVal = uniform(ch.betaVal);
     const int64_t nRuns = uniform(ch.betaRuns);
-    uint64_t betaNext = (s1 > s0) ? uniform(static_cast<uint64_t>(__ldg(bEnd + run))) : 0;
-    int32_t beta = (s1 > s0) ? uniform(__ldg(bVal + run)) : 0;
-    uint64_t pfEnd = ~uint64_t(0);
-    int32_t pfVal = 0;
-    if (s1 > s0 && run + 1 < nRuns) {
-        pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 1));
-        pfVal = __ldg(bVal + run + 1);
+    uint64_t betaNext = ~uint64_t(0), nextEnd = ~uint64_t(0), pfEnd = ~uint64_t(0);
+    int32_t beta = 0, nextVal = 0, pfVal = 0;
+    if (s1 > s0) {
+        betaNext = uniform(static_cast<uint64_t>(__ldg(bEnd + run)));
+        beta = uniform(__ldg(bVal + run));
+        if (run + 1 < nRuns) {
+            nextEnd = uniform(static_cast<uint64_t>(__ldg(bEnd + run + 1)));
+            nextVal = uniform(__ldg(bVal + run + 1));
+        }
+        if (run + 2 < nRuns) {
+            pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 2));
+            pfVal = __ldg(bVal + run + 2);
+        }
     }
     uint64_t improved = 0;
     using Loc = typename std::conditional<DP::kField, int32_t, int64_t>::type;
@@ -1214,7 +1233,9 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     };
     group_sync(grp, T);
 
-    for (uint64_t sw = s0; sw < s1; ++sw) {
+    uint64_t sw = s0;
+    SweepConst sc = make_sweep(s0 + 1, keys);   // the sweep id is 1-based
+    while (sw < s1) {
         if (sw >= phaseEnd) {
             while (sw >= phaseEnd) {
                 ++p;
@@ -1232,17 +1253,8 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
                 group_sync(grp, T);
             }
         }
-        if (sw >= betaNext) {
-            // Runs are never empty, so one step of the cursor per sweep.
-            ++run;
-            betaNext = uniform(pfEnd);
-            beta = uniform(pfVal);
-            if (run + 1 < nRuns) {
-                pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 1));
-                pfVal = __ldg(bVal + run + 1);
-            }
-        }
-        if (((sw - s0) & (kPaceEvery - 1)) == 0) {
+        const uint32_t paced = static_cast<uint32_t>(sw - s0) & (kPaceEvery - 1);
+        if (paced == 0) {
             const int mine = static_cast<int>(sw - s0);
             if (t == 0) prog[grp] = mine;
             int lead = mine - slowest_chain(prog);
@@ -1251,20 +1263,43 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
                 lead = mine - slowest_chain(prog);
             }
         }
-        const uint64_t step = sw + 1;   // 1-based sweep id
-
-        int32_t v[4];
-        if constexpr (kS64) select64<DP>(s, lut, n, pc, beta, step, keys, t, T, grp);
-        else select32<kOne, DP>(s, lut, kc, n, pc, beta, step, keys, t, T, v);
-        const bool slots = kS64 || pc.path != kPathWarp;
-        if (!kOne || slots) group_sync(grp, T);
-        settle(sw);
-        if (slots) loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
-        else loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
-        if (!kOne) {
-            loc = warp_sum(loc);
-            if ((t & 31) == 0) s.red[t >> 5] = loc;
-        }
+        // Sweeps up to the next pacing point, end of phase or of the window.
+        uint32_t left = kPaceEvery - paced;
+        if (phaseEnd > sw && phaseEnd - sw < left) left = static_cast<uint32_t>(phaseEnd - sw);
+        if (s1 - sw < left) left = static_cast<uint32_t>(s1 - sw);
+        do {
+            bool turn = false;
+            if (sw >= betaNext) {
+                // Runs are never empty, so one step of the cursor per sweep.
+                ++run;
+                betaNext = nextEnd;
+                beta = nextVal;
+                turn = true;
+            }
+            int32_t v[4];
+            if constexpr (kS64) select64<DP>(s, lut, n, pc, beta, sc, keys, t, T, grp);
+            else select32<kOne, DP>(s, lut, kc, n, pc, beta, sc, keys, t, T, v);
+            ++sw;
+            sc = make_sweep(sw + 1, keys);
+            if (turn) {
+                nextEnd = uniform(pfEnd);
+                nextVal = uniform(pfVal);
+                pfEnd = ~uint64_t(0);
+                if (run + 2 < nRuns) {
+                    pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 2));
+                    pfVal = __ldg(bVal + run + 2);
+                }
+            }
+            const bool slots = kS64 || pc.path != kPathWarp;
+            if (!kOne || slots) group_sync(grp, T);
+            settle(sw - 1);
+            if (slots) loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
+            else loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+            if (!kOne) {
+                loc = warp_sum(loc);
+                if ((t & 31) == 0) s.red[t >> 5] = loc;
+            }
+        } while (--left);
     }
     if (!kOne) group_sync(grp, T);
     settle(s1);
