@@ -269,9 +269,10 @@ __device__ __forceinline__ uint32_t add_half(uint32_t x, uint32_t bytes, uint32_
 // 2 * w * (its new spin) whatever their spins are, so FLIP's row walk needs
 // no load of the neighbour's spin (one of its three dependent shared-memory
 // accesses per entry, each with ~3 bank-conflict wavefronts).
-// Every partial sum during a scatter is the S of some spin configuration, so
-// a byte stays in [0, 255] and a shifted 32-bit atomicAdd on the containing
-// word never carries into the neighbouring byte.
+// Changes are shifted 32-bit atomic adds on the containing word.  They commute
+// and the word is the exact sum of its bytes' values times powers of 256, so
+// whatever carries happen on the way, once a sweep's adds are all in (the only
+// time a byte is read) every byte is back in [0, 255].
 struct D8 {
     static constexpr bool kField = true;
     static constexpr int32_t kBias = 128;
@@ -324,83 +325,56 @@ struct D8 {
 
 // ------------------------------------------------------------ CSR access
 struct CsrView {
-    const uint32_t* off;
+    const uint32_t* off;   // row words (compact formats) or plain offsets
     const void* ent;
 };
 
+// A word of the CSR: from the CTA's shared-memory copy, or from HBM through
+// the read-only path.
+template <bool kHbm, class T>
+__device__ __forceinline__ T csr_load(const T* p) {
+    if constexpr (kHbm) return __ldg(p);
+    else return *p;
+}
+
 template <int kFmt>
-struct Csr;
-
-template <>
-struct Csr<kCsrUnit16> {
+struct Csr {
+    static constexpr bool kHbm = csr_in_hbm(kFmt);
+    static constexpr bool kPlain = kFmt == kCsrGlobal;                          // {col, w} pairs, rows not padded
+    static constexpr bool kUnit = kFmt == kCsrUnit16 || kFmt == kCsrGlobal16;   // 16-bit entries
+    // Row v as two words: plain offsets, or row words (first entry | padding,
+    // next row's).
     __device__ static __forceinline__ void row(const CsrView& c, int v, uint32_t& lo, uint32_t& hi) {
-        lo = c.off[v];
-        hi = c.off[v + 1];
+        lo = csr_load<kHbm>(c.off + v);
+        hi = csr_load<kHbm>(c.off + v + 1);
     }
-    __device__ static __forceinline__ uint32_t raw(const CsrView& c, uint32_t i) {
-        return static_cast<const uint16_t*>(c.ent)[i];
+    // The row's entries [i, end).
+    __device__ static __forceinline__ void entries(const CsrView& c, int v, uint32_t& i, uint32_t& end) {
+        row(c, v, i, end);
+        if constexpr (!kPlain) {
+            end = (end & ~3u) - (i & 3u);
+            i &= ~3u;
+        }
     }
     __device__ static __forceinline__ void entry(const CsrView& c, uint32_t i, int& col, int& w) {
-        const uint32_t e = static_cast<const uint16_t*>(c.ent)[i];
-        col = static_cast<int>(e >> 1);
-        w = 1 - 2 * static_cast<int>(e & 1u);
+        if constexpr (kPlain) {
+            const int2 e = csr_load<kHbm>(static_cast<const int2*>(c.ent) + i);
+            col = e.x;
+            w = e.y;
+        } else if constexpr (kUnit) {
+            const uint32_t e = csr_load<kHbm>(static_cast<const unsigned short*>(c.ent) + i);
+            col = static_cast<int>(e & 0x7FFFu);
+            w = 1 - 2 * static_cast<int>(e >> 15);
+        } else {
+            const uint32_t e = csr_load<kHbm>(static_cast<const unsigned int*>(c.ent) + i);
+            col = static_cast<int>(e & 0xFFFFu);
+            w = static_cast<int32_t>(e) >> 16;
+        }
     }
-};
-
-template <>
-struct Csr<kCsrPacked32> {
-    __device__ static __forceinline__ void row(const CsrView& c, int v, uint32_t& lo, uint32_t& hi) {
-        lo = c.off[v];
-        hi = c.off[v + 1];
-    }
-    __device__ static __forceinline__ void entry(const CsrView& c, uint32_t i, int& col, int& w) {
-        const uint32_t e = static_cast<const uint32_t*>(c.ent)[i];
-        col = static_cast<int>(e & 0xFFFFu);
-        w = static_cast<int32_t>(e) >> 16;
-    }
-};
-
-template <>
-struct Csr<kCsrGlobal> {
-    __device__ static __forceinline__ void row(const CsrView& c, int v, uint32_t& lo, uint32_t& hi) {
-        lo = __ldg(c.off + v);
-        hi = __ldg(c.off + v + 1);
-    }
-    __device__ static __forceinline__ void entry(const CsrView& c, uint32_t i, int& col, int& w) {
-        const int2 e = __ldg(static_cast<const int2*>(c.ent) + i);
-        col = e.x;
-        w = e.y;
-    }
-};
-
-// The compact entries read from HBM on the read-only path: a quarter (16-bit)
-// or half (32-bit) of the bytes of the {col, w} pairs per entry.
-template <>
-struct Csr<kCsrGlobal16> {
-    __device__ static __forceinline__ void row(const CsrView& c, int v, uint32_t& lo, uint32_t& hi) {
-        lo = __ldg(c.off + v);
-        hi = __ldg(c.off + v + 1);
-    }
-    __device__ static __forceinline__ uint32_t raw(const CsrView& c, uint32_t i) {
-        return __ldg(static_cast<const unsigned short*>(c.ent) + i);
-    }
-    __device__ static __forceinline__ void entry(const CsrView& c, uint32_t i, int& col, int& w) {
-        const uint32_t e = raw(c, i);
-        col = static_cast<int>(e >> 1);
-        w = 1 - 2 * static_cast<int>(e & 1u);
-    }
-};
-
-template <>
-struct Csr<kCsrGlobal32> {
-    __device__ static __forceinline__ void row(const CsrView& c, int v, uint32_t& lo, uint32_t& hi) {
-        lo = __ldg(c.off + v);
-        hi = __ldg(c.off + v + 1);
-    }
-    __device__ static __forceinline__ void entry(const CsrView& c, uint32_t i, int& col, int& w) {
-        const uint32_t e = __ldg(static_cast<const unsigned int*>(c.ent) + i);
-        col = static_cast<int>(e & 0xFFFFu);
-        w = static_cast<int32_t>(e) >> 16;
+    // Vector q: entries 4q .. 4q + 3 (two to a word for 16-bit entries).
+    using Vec = typename std::conditional<kUnit, uint2, uint4>::type;
+    __device__ static __forceinline__ Vec vec(const CsrView& c, uint32_t q) {
+        return csr_load<kHbm>(static_cast<const Vec*>(c.ent) + q);
     }
 };
 
@@ -883,37 +857,62 @@ __device__ void select64(const ChainSmem& s, const int32_t* lut, int n, const Ph
 }
 
 // ------------------------------------------------------------------- FLIP
+// One 16-bit entry (the low half of e): the neighbour's byte changes by +2 or
+// -2, added into byte lane col & 3 of its word (the shift wraps at 32, so it
+// needs no mask).  `nm`: 0x8000 when the winner's new spin is -1.
+__device__ __forceinline__ void add_unit(unsigned char* D, uint32_t e, uint32_t nm) {
+    const uint32_t val = ((e ^ nm) & 0x8000u) ? 0xFFFFFFFEu : 2u;
+    atomicAdd(reinterpret_cast<unsigned int*>(D + (e & 0x7FFCu)), __funnelshift_l(0u, val, e << 3));
+}
+
+// One 32-bit entry w << 16 | col.  `neg`: the winner's new spin is -1.
+template <class DP>
+__device__ __forceinline__ void add_packed(const ChainSmem& s, uint32_t e, uint32_t neg) {
+    const int c = static_cast<int>(e & 0xFFFFu), w2 = 2 * (static_cast<int32_t>(e) >> 16);
+    const uint32_t x = DP::kField ? 0u : s.sb[c] & 1u;
+    DP::add(s.D, c, (neg ^ x) ? -w2 : w2);
+}
+
+// A vector of four entries of a compact row.
+template <class DP, int kFmt>
+__device__ __forceinline__ void add_vec(const ChainSmem& s, const typename Csr<kFmt>::Vec& e, uint32_t neg) {
+    if constexpr (!Csr<kFmt>::kUnit) {
+        add_packed<DP>(s, e.x, neg);
+        add_packed<DP>(s, e.y, neg);
+        add_packed<DP>(s, e.z, neg);
+        add_packed<DP>(s, e.w, neg);
+    } else {
+        static_assert(DP::kField, "16-bit entries of int32 gains are walked one by one");
+        const uint32_t nm = neg << 15;
+        add_unit(s.D, e.x, nm);
+        add_unit(s.D, e.x >> 16, nm);
+        add_unit(s.D, e.y, nm);
+        add_unit(s.D, e.y >> 16, nm);
+    }
+}
+
 // S[x] (or D[x]) changes over winner v's row after its flip: 2 w s_v for
 // neighbour x, times the neighbour's spin for int32 gains.  `neg`: v's new
-// spin is -1.  `lanes` threads share the row (this one is `sub`), four
-// entries in flight.
+// spin is -1; lo, hi: its row words.  `lanes` threads share the row (this one
+// is `sub`).
+//
+// Compact rows are walked as aligned vectors of four entries, the next one
+// loaded ahead, without a remainder: the padding entries change v itself by a
+// known amount, which its flip takes out again (own_padding).
 template <class DP, int kFmt>
-__device__ __forceinline__ void scatter_row(const ChainSmem& s, const CsrView& csr, int v, uint32_t neg, int sub,
-                                            int lanes) {
-    uint32_t i, hi;
-    Csr<kFmt>::row(csr, v, i, hi);
-    i += sub;
-    if constexpr (DP::kField && (kFmt == kCsrUnit16 || kFmt == kCsrGlobal16)) {
-        // entry = col << 1 | w < 0: +2 or -2 added into byte lane col & 3 of
-        // word col >> 2.
-        unsigned int* Dw = reinterpret_cast<unsigned int*>(s.D);
-        for (; i + 3 * lanes < hi; i += 4 * lanes) {
-            uint32_t e[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) e[j] = Csr<kFmt>::raw(csr, i + j * lanes);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                atomicAdd(Dw + (e[j] >> 3), (((neg ^ e[j]) & 1u) ? 0xFFFFFFFEu : 2u) << ((e[j] & 6u) << 2));
+__device__ __forceinline__ void scatter_row(const ChainSmem& s, const CsrView& csr, uint32_t lo, uint32_t hi,
+                                            uint32_t neg, int sub, int lanes) {
+    using C = Csr<kFmt>;
+    if constexpr (C::kPlain || (C::kUnit && !DP::kField)) {
+        if constexpr (!C::kPlain) {
+            hi = (hi & ~3u) - (lo & 3u);
+            lo &= ~3u;
         }
-        for (; i < hi; i += lanes) {
-            const uint32_t e = Csr<kFmt>::raw(csr, i);
-            atomicAdd(Dw + (e >> 3), (((neg ^ e) & 1u) ? 0xFFFFFFFEu : 2u) << ((e & 6u) << 2));
-        }
-    } else {
+        uint32_t i = lo + sub;
         for (; i + 3 * lanes < hi; i += 4 * lanes) {
             int c[4], w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) Csr<kFmt>::entry(csr, i + j * lanes, c[j], w[j]);
+            for (int j = 0; j < 4; ++j) C::entry(csr, i + j * lanes, c[j], w[j]);
             uint32_t x[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) x[j] = DP::kField ? 0u : s.sb[c[j]] & 1u;
@@ -922,11 +921,56 @@ __device__ __forceinline__ void scatter_row(const ChainSmem& s, const CsrView& c
         }
         for (; i < hi; i += lanes) {
             int c, w;
-            Csr<kFmt>::entry(csr, i, c, w);
+            C::entry(csr, i, c, w);
             const uint32_t x = DP::kField ? 0u : s.sb[c] & 1u;
             DP::add(s.D, c, (neg ^ x) ? -2 * w : 2 * w);
         }
+    } else {
+        uint32_t q = (lo >> 2) + sub;
+        const uint32_t end = hi >> 2;
+        if (q >= end) return;
+        typename C::Vec e = C::vec(csr, q);
+        for (q += lanes; q < end; q += lanes) {
+            const typename C::Vec f = C::vec(csr, q);
+            add_vec<DP, kFmt>(s, e, neg);
+            e = f;
+        }
+        add_vec<DP, kFmt>(s, e, neg);
     }
+}
+
+// Two whole rows walked by one lane as one list: the lanes of a warp then wait
+// for the longest pair, not for the longest row twice (mean degree 19: 13
+// vectors for two rows of 5 instead of 16).  An absent row has equal words.
+template <class DP, int kFmt>
+__device__ __forceinline__ void scatter_two(const ChainSmem& s, const CsrView& csr, const uint32_t lo[2],
+                                            const uint32_t hi[2], const uint32_t neg[2]) {
+    using C = Csr<kFmt>;
+    if constexpr (C::kPlain || (C::kUnit && !DP::kField)) {
+        scatter_row<DP, kFmt>(s, csr, lo[0], hi[0], neg[0], 0, 1);
+        scatter_row<DP, kFmt>(s, csr, lo[1], hi[1], neg[1], 0, 1);
+    } else {
+        const uint32_t n0 = (hi[0] >> 2) - (lo[0] >> 2), n = n0 + (hi[1] >> 2) - (lo[1] >> 2);
+        const uint32_t at0 = lo[0] >> 2, at1 = (lo[1] >> 2) - n0;
+        if (n == 0) return;
+        typename C::Vec e = C::vec(csr, n0 ? at0 : at1);
+        uint32_t ng = n0 ? neg[0] : neg[1];
+        for (uint32_t i = 1; i < n; ++i) {
+            const typename C::Vec f = C::vec(csr, i + (i < n0 ? at0 : at1));
+            add_vec<DP, kFmt>(s, e, ng);
+            e = f;
+            ng = i < n0 ? neg[0] : neg[1];
+        }
+        add_vec<DP, kFmt>(s, e, ng);
+    }
+}
+
+// What a walk of row `lo` adds to the row's own vertex through the padding:
+// nothing but for 16-bit entries, whose padding weighs +1.
+template <class DP, int kFmt>
+__device__ __forceinline__ int32_t own_padding(uint32_t lo, uint32_t neg) {
+    if constexpr (Csr<kFmt>::kUnit && DP::kField) return static_cast<int32_t>(lo & 3u) * (neg ? -2 : 2);
+    else return 0;
 }
 
 // Winner v (gain d, mask byte m before) flips: its stored value, its spin.
@@ -944,21 +988,22 @@ __device__ __forceinline__ void flip_vertex(const ChainSmem& s, int v, int32_t d
 // gain once summed over the chain.
 //
 // With int8 gains nothing a row's walk reads is changed by another row (a
-// flip adds +-1 to its own byte, a walk +-2w to its neighbours': they
-// commute), so after the gains are read there is one barrier, at the end.
-// With int32 gains a walk reads its neighbours' new spins, so the flips are
-// fenced off from the walks.
+// flip adds +-1 to its own byte, a walk +-2w to its neighbours': they commute
+// as 32-bit adds, whatever the bytes pass through on the way), so after the
+// gains are read there is one barrier, at the end.  With int32 gains a walk
+// reads its neighbours' new spins, so the flips are fenced off from the walks.
 template <bool kOne, class DP, int kFmt, class Loc>
 __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
                                          int grp, int32_t v[4]) {
-    const int sub = t & ((1 << pc.laneShift) - 1);
     constexpr int kRows = kOne ? 4 : 2;   // P <= 128 over at least 32 or 64 threads
-    uint32_t m[kRows];
+    const int sub = t & ((1 << pc.laneShift) - 1);
+    uint32_t lo[kRows], hi[kRows], neg[kRows];
     int32_t d[kRows];
     Loc loc = 0;
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
-        if (q >= pc.rows) break;
+        lo[q] = hi[q] = neg[q] = 0;
+        if (q >= pc.rows) continue;
         const int r = (t >> pc.laneShift) + q * T;
         if constexpr (kOne) {
             if (q == 0 && pc.laneShift) v[0] = __shfl_sync(0xFFFFFFFFu, v[0], r);
@@ -974,50 +1019,52 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
                     const unsigned long long ab = a > b ? a : b;
                     p = ab > p ? ab : p;
                 }
-                const uint32_t lo = static_cast<uint32_t>(p);
+                const uint32_t low = static_cast<uint32_t>(p);
                 if constexpr (DP::kField) {
-                    v[q] = p ? static_cast<int32_t>(~(lo >> 9) & 0x7FFFFFu) : -1;
-                    m[q] = (lo & 0x100u) ? 0xFFu : 0u;
-                    d[q] = static_cast<int32_t>(lo & 0xFFu) - 128;
+                    v[q] = p ? static_cast<int32_t>(~(low >> 9) & 0x7FFFFFu) : -1;
+                    neg[q] = ((low >> 8) & 1u) ^ 1u;
+                    d[q] = static_cast<int32_t>(low & 0xFFu) - 128;
                 } else {
-                    v[q] = p ? static_cast<int32_t>(~lo) : -1;
+                    v[q] = p ? static_cast<int32_t>(~low) : -1;
                 }
             }
         }
-        if ((kOne || !DP::kField) && v[q] >= 0) {
-            m[q] = s.sb[v[q]];
-            d[q] = DP::get(s.D, s.sb, v[q]);
+        if (v[q] >= 0) {
+            if (kOne || !DP::kField) {
+                neg[q] = (s.sb[v[q]] & 1u) ^ 1u;
+                d[q] = DP::get(s.D, s.sb, v[q]);
+            }
+            Csr<kFmt>::row(csr, v[q], lo[q], hi[q]);
+            if (sub == 0) loc += d[q];
         }
-        if (v[q] >= 0 && sub == 0) loc += d[q];
     }
     if (kOne || !DP::kField) __syncwarp();
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
-        if (q >= pc.rows) break;
-        if (v[q] >= 0 && sub == 0) {
+        if (q < pc.rows && v[q] >= 0 && sub == 0) {
             if constexpr (DP::kField) {
                 // q' = q - 1 (+1 -> -1) or q + 1: an add, as a neighbour's
                 // walk may be adding to this byte.
-                DP::add(s.D, v[q], m[q] ? 1 : -1);
+                DP::add(s.D, v[q], (neg[q] ? -1 : 1) - own_padding<DP, kFmt>(lo[q], neg[q]));
                 atomicXor(&s.bits[v[q] >> 5], 1u << (v[q] & 31));
-                s.sb[v[q]] = static_cast<unsigned char>(m[q] ^ 0xFFu);
+                s.sb[v[q]] = neg[q] ? 0xFFu : 0u;
             } else {
-                flip_vertex<DP>(s, v[q], d[q], m[q]);
+                flip_vertex<DP>(s, v[q], d[q], neg[q] ? 0u : 0xFFu);
             }
         }
     }
     if (!DP::kField) group_sync(grp, T);
+    if (pc.rows == 1) {
+        scatter_row<DP, kFmt>(s, csr, lo[0], hi[0], neg[0], sub, 1 << pc.laneShift);
+    } else {
 #pragma unroll
-    for (int q = 0; q < kRows; ++q) {
-        if (q >= pc.rows) break;
-        if (v[q] >= 0) scatter_row<DP, kFmt>(s, csr, v[q], (m[q] & 1u) ^ 1u, sub, 1 << pc.laneShift);
+        for (int q = 0; q < kRows; q += 2)
+            if (q < pc.rows) scatter_two<DP, kFmt>(s, csr, lo + q, hi + q, neg + q);
     }
     group_sync(grp, T);
 #pragma unroll
-    for (int q = 0; q < kRows; ++q) {
-        if (q >= pc.rows) break;
-        if (v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
-    }
+    for (int q = 0; q < kRows; ++q)
+        if (q < pc.rows && v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
     return loc;
 }
 
@@ -1051,7 +1098,16 @@ __device__ __forceinline__ Loc flip_slots(const ChainSmem& s, const CsrView& csr
     const int lanes = 1 << pc.laneShift;
     for (int gi = t >> pc.laneShift; gi < pc.P; gi += T >> pc.laneShift) {
         const int v = s.win[gi];
-        if (v >= 0) scatter_row<DP, kFmt>(s, csr, v, s.sb[v] & 1u, t & (lanes - 1), lanes);
+        if (v >= 0) {
+            uint32_t lo, hi;
+            Csr<kFmt>::row(csr, v, lo, hi);
+            const uint32_t neg = s.sb[v] & 1u;
+            const int sub = t & (lanes - 1);
+            // Past the barrier only: the plain byte stores above do not mix
+            // with an add that may carry through a neighbouring byte.
+            if (sub == 0 && (Csr<kFmt>::kUnit && DP::kField)) DP::add(s.D, v, -own_padding<DP, kFmt>(lo, neg));
+            scatter_row<DP, kFmt>(s, csr, lo, hi, neg, sub, lanes);
+        }
     }
     group_sync(grp, T);
     for (int gi = t; gi < pc.P; gi += T) {
@@ -1129,7 +1185,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         int32_t d = 0;
         if (v < n) {
             uint32_t lo, hi;
-            Csr<kFmt>::row(csr, v, lo, hi);
+            Csr<kFmt>::entries(csr, v, lo, hi);
             int32_t acc = 0;
             for (uint32_t i = lo; i < hi; ++i) {
                 int col, w;
@@ -1360,13 +1416,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
 // outcome (false: its polls ran out); the caller makes it CTA-uniform and
 // advances the phase.
 __device__ bool stage_csr(const DevGraph& g, unsigned char* dst, uint64_t* mbar, uint32_t phase) {
-    const uint32_t total = g.offBytes + g.entBytes;
+    const uint32_t total = g.rowBytes + g.entBytes;
     if (threadIdx.x == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(mbar, total);
-        const unsigned char* srcs[2] = {reinterpret_cast<const unsigned char*>(g.offsets),
+        const unsigned char* srcs[2] = {reinterpret_cast<const unsigned char*>(g.rows),
                                         static_cast<const unsigned char*>(g.compact)};
-        const uint32_t sizes[2] = {g.offBytes, g.entBytes};
+        const uint32_t sizes[2] = {g.rowBytes, g.entBytes};
         uint32_t o = 0;
         for (int k = 0; k < 2; ++k) {
             for (uint32_t c = 0; c < sizes[k]; c += 65536u) {
@@ -1426,7 +1482,7 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
         const DevGraph& g = L.graphs[item.graph];
         CsrView csr;
         if constexpr (csr_in_hbm(kFmt)) {
-            csr.off = g.offsets;
+            csr.off = (kFmt == kCsrGlobal) ? g.offsets : g.rows;
             csr.ent = (kFmt == kCsrGlobal) ? static_cast<const void*>(g.edges) : g.compact;
         } else {
             if (item.graph != loaded) {
@@ -1449,7 +1505,7 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
                 loaded = item.graph;
             }
             csr.off = reinterpret_cast<const uint32_t*>(csrBase);
-            csr.ent = csrBase + g.offBytes;
+            csr.ent = csrBase + g.rowBytes;
         }
         const int active = (item.count < L.chainsPerCta) ? item.count : L.chainsPerCta;
         if (threadIdx.x < 16) sProg[threadIdx.x] = (static_cast<int>(threadIdx.x) < active) ? 0 : INT_MAX;

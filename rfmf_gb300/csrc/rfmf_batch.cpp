@@ -101,12 +101,6 @@ struct rfmf_batch {
 
 namespace {
 
-uint32_t csr_bytes(const rfmf_graph* g, int fmt) {
-    if (fmt == kCsrUnit16) return g->offBytes + g->u16Bytes;
-    if (fmt == kCsrPacked32) return g->offBytes + g->p32Bytes;
-    return 0;
-}
-
 int64_t dyn_smem_max(const rfmf_context* ctx, const void* kern, cudaFuncAttributes& fa) {
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return -1;
     return static_cast<int64_t>(ctx->smemOptin) - static_cast<int64_t>(fa.sharedSizeBytes);
@@ -859,12 +853,13 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         const int fmt = b->cls[graphClass[gi]].fmt;
         hg[gi].offsets = g->offsets.as<uint32_t>();
         hg[gi].edges = g->edges.as<Edge>();
+        hg[gi].rows = g->rows.as<uint32_t>();
         hg[gi].compact = compact_entries(g, fmt);
         hg[gi].n = static_cast<int32_t>(g->n);
         hg[gi].words = static_cast<int32_t>((g->n + 31) / 32);
         hg[gi].wsum2 = g->wsum2;
-        hg[gi].offBytes = g->offBytes;
-        hg[gi].entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->offBytes : 0;
+        hg[gi].rowBytes = g->rowBytes;
+        hg[gi].entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;
     }
 
     // Per-chain spin words and initial state.

@@ -19,7 +19,7 @@ struct alignas(8) Edge {
 // the graph's own arrays through L1/L2 (graphs too large for shared memory
 // beside their chains), with the most compact entries the graph allows.
 enum CsrFormat : int32_t {
-    kCsrUnit16 = 0,    // uint16 entry = (col << 1) | (w < 0); |w| == 1, n <= 32768
+    kCsrUnit16 = 0,    // uint16 entry = col | (w < 0) << 15; |w| == 1, n <= 32768
     kCsrPacked32 = 1,  // uint32 entry = (w << 16) | col;  |w| < 2^15, n <= 65536
     kCsrGlobal = 2,    // Edge {col, w} in HBM
     kCsrGlobal16 = 3,  // the unit16 entries, in HBM
@@ -34,17 +34,25 @@ enum CsrFormat : int32_t {
 // Formats walked in HBM (no shared-memory copy of the CSR).
 RFMF_CHD bool csr_in_hbm(int fmt) { return fmt == kCsrGlobal || fmt == kCsrGlobal16 || fmt == kCsrGlobal32; }
 
+// The compact formats keep every row at a multiple of four entries, so that a
+// row is read as aligned vectors of four: row word r of vertex v holds its
+// first entry (a multiple of four) and, in the low two bits, how many of its
+// last vector's entries are padding (0..3); its vectors end where row v + 1's
+// begin.  Padding entries name vertex v itself, with weight +1 (16-bit) or 0
+// (32-bit).
+//
 // One CSR graph in HBM, read-only, shared by every chain that anneals it.
 // Rows are sorted ascending by neighbour (the reference's AnnealCsr order,
 // src/immutable_graph.hpp:83-101); each undirected edge is stored twice.
 struct DevGraph {
     const uint32_t* offsets;   // n + 1 (padded to 16 B)
     const Edge*     edges;     // 2m  {col, weight}
-    const void*     compact;   // 2m compact entries of the launch's format (padded to 16 B)
+    const uint32_t* rows;      // n + 1 row words of the compact entries (padded to 16 B)
+    const void*     compact;   // compact entries of the launch's format, rows padded to four (16 B in all)
     int32_t         n;
     int32_t         words;     // ceil(n / 32): spin bit-words per chain
     int64_t         wsum2;     // sum of weight over directed entries (2 * sum over edges)
-    uint32_t        offBytes;  // bytes of offsets, multiple of 16
+    uint32_t        rowBytes;  // bytes of rows, multiple of 16
     uint32_t        entBytes;  // bytes of compact entries, multiple of 16
 };
 

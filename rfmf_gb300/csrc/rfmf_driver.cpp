@@ -528,10 +528,12 @@ static int rfmf_graph_create_impl(rfmf_context* ctx, int64_t n, const uint32_t* 
     g->m = static_cast<int64_t>(m2 / 2);
     g->B = B;
     g->wsum2 = wsum2;
-    g->unit16 = unit && n <= 32768 && m2 < (uint64_t(1) << 31);
-    g->packed32 = small && n <= 65536 && m2 < (uint64_t(1) << 30);
+    // Rows of the compact formats: padded to four entries.
+    uint64_t mPad = 0;
+    for (int64_t v = 0; v < n; ++v) mPad += (static_cast<uint64_t>(offsets[v + 1] - offsets[v]) + 3u) & ~uint64_t(3);
+    g->unit16 = unit && n <= 32768 && mPad < (uint64_t(1) << 31);
+    g->packed32 = small && n <= 65536 && mPad < (uint64_t(1) << 30);
     const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
-    g->offBytes = ob > 0xFFFFFFF0ull ? 0xFFFFFFF0u : static_cast<uint32_t>(ob);
     std::vector<uint32_t> ho(ob / 4, offsets[n]);
     std::memcpy(ho.data(), offsets, (n + 1) * sizeof(uint32_t));
     std::vector<Edge> he(m2);
@@ -543,21 +545,43 @@ static int rfmf_graph_create_impl(rfmf_context* ctx, int64_t n, const uint32_t* 
     cudaStream_t st = ctx->stream;
     CU(cudaMemcpyAsync(g->offsets.p, ho.data(), ob, cudaMemcpyHostToDevice, st));
     if (m2) CU(cudaMemcpyAsync(g->edges.p, he.data(), m2 * sizeof(Edge), cudaMemcpyHostToDevice, st));
+    std::vector<uint32_t> hr, h32;
     std::vector<uint16_t> h16;
-    std::vector<uint32_t> h32;
+    if (g->unit16 || g->packed32) {
+        g->rowBytes = static_cast<uint32_t>(ob);
+        hr.assign(ob / 4, static_cast<uint32_t>(mPad));
+        if (g->unit16) {
+            g->u16Bytes = align16(static_cast<uint32_t>(mPad * 2));
+            h16.assign(g->u16Bytes / 2, 0);
+        }
+        if (g->packed32) {
+            g->p32Bytes = align16(static_cast<uint32_t>(mPad * 4));
+            h32.assign(g->p32Bytes / 4, 0);
+        }
+        uint32_t o = 0;
+        for (int64_t v = 0; v < n; ++v) {
+            const uint32_t deg = offsets[v + 1] - offsets[v], len = (deg + 3u) & ~3u;
+            hr[v] = o | (len - deg);
+            for (uint32_t k = 0; k < deg; ++k) {
+                const uint32_t i = offsets[v] + k;
+                if (g->unit16) h16[o + k] = static_cast<uint16_t>(col[i] | (weight[i] < 0 ? 0x8000 : 0));
+                if (g->packed32)
+                    h32[o + k] = (static_cast<uint32_t>(weight[i]) << 16) | static_cast<uint32_t>(col[i]);
+            }
+            for (uint32_t k = deg; k < len; ++k) {   // padding: the vertex itself
+                if (g->unit16) h16[o + k] = static_cast<uint16_t>(v);
+                if (g->packed32) h32[o + k] = static_cast<uint32_t>(v);
+            }
+            o += len;
+        }
+        if ((rc = g->rows.alloc(ob))) return rc;
+        CU(cudaMemcpyAsync(g->rows.p, hr.data(), ob, cudaMemcpyHostToDevice, st));
+    }
     if (g->unit16) {
-        g->u16Bytes = align16(static_cast<uint32_t>(m2 * 2));
-        h16.assign(g->u16Bytes / 2, 0);
-        for (uint64_t i = 0; i < m2; ++i)
-            h16[i] = static_cast<uint16_t>((static_cast<uint32_t>(col[i]) << 1) | (weight[i] < 0 ? 1u : 0u));
         if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
         CU(cudaMemcpyAsync(g->u16.p, h16.data(), g->u16Bytes, cudaMemcpyHostToDevice, st));
     }
     if (g->packed32) {
-        g->p32Bytes = align16(static_cast<uint32_t>(m2 * 4));
-        h32.assign(g->p32Bytes / 4, 0);
-        for (uint64_t i = 0; i < m2; ++i)
-            h32[i] = (static_cast<uint32_t>(weight[i]) << 16) | static_cast<uint32_t>(col[i]);
         if ((rc = g->p32.alloc(g->p32Bytes))) return rc;
         CU(cudaMemcpyAsync(g->p32.p, h32.data(), g->p32Bytes, cudaMemcpyHostToDevice, st));
     }

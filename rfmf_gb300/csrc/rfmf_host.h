@@ -306,8 +306,8 @@ struct CtxHold {
 }  // namespace rfmf
 
 // A graph in device memory: offsets and 8-byte entries for HBM walks, plus
-// the compact entry arrays the shared-memory formats stage from (present
-// when the graph qualifies).  All arrays are padded to 16 bytes.
+// the compact rows the other formats stage or walk (present when the graph
+// qualifies).  All arrays are padded to 16 bytes.
 struct rfmf_graph {
     rfmf::CtxHold ctxHold;   // first member: released last
     rfmf_context* ctx = nullptr;
@@ -316,8 +316,8 @@ struct rfmf_graph {
     mutable std::atomic<int> holders{1};
     int64_t n = 0, m = 0, B = 0, wsum2 = 0;
     bool unit16 = false, packed32 = false;
-    uint32_t offBytes = 0, u16Bytes = 0, p32Bytes = 0;
-    rfmf::DevBuf offsets, edges, u16, p32;
+    uint32_t rowBytes = 0, u16Bytes = 0, p32Bytes = 0;
+    rfmf::DevBuf offsets, edges, rows, u16, p32;
     // Learned costs: device time per sweep of one work item, by plan (warps
     // per chain, CSR format), phase group count P and scheduler level (the
     // warps an item puts on each of the SM's four schedulers,
@@ -408,6 +408,14 @@ struct GraphHolds {
 // The HBM-walk format of a graph: the most compact entries it has.
 inline int hbm_format(const rfmf_graph* g) {
     return g->unit16 ? kCsrGlobal16 : (g->packed32 ? kCsrGlobal32 : kCsrGlobal);
+}
+
+// Bytes of the graph's compact copy (row words and entries) in a format staged
+// in shared memory; 0 for the HBM formats.
+inline uint32_t csr_bytes(const rfmf_graph* g, int fmt) {
+    if (fmt == kCsrUnit16) return g->rowBytes + g->u16Bytes;
+    if (fmt == kCsrPacked32) return g->rowBytes + g->p32Bytes;
+    return 0;
 }
 
 // The entry array a launch of format `fmt` reads for graph g (the 8-byte

@@ -360,8 +360,9 @@ __global__ void scatter_entries(const int64_t* u, const int64_t* v, const int64_
 }
 
 // One thread per row: insertion sort by (col, idx); then the first entry of
-// each col run survives.  Writes the surviving count of the row.
-__global__ void sort_rows(RawEntry* ent, const int32_t* rowStart, int32_t n, int32_t* keep) {
+// each col run survives.  Writes the surviving count of the row and, in the
+// high half, that count padded to four (both are scanned together).
+__global__ void sort_rows(RawEntry* ent, const int32_t* rowStart, int32_t n, uint64_t* keep) {
     for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const int32_t lo = rowStart[r], hi = rowStart[r + 1];
         for (int32_t i = lo + 1; i < hi; ++i) {
@@ -376,15 +377,15 @@ __global__ void sort_rows(RawEntry* ent, const int32_t* rowStart, int32_t n, int
         int32_t k = 0;
         for (int32_t i = lo; i < hi; ++i)
             if (i == lo || ent[i].col != ent[i - 1].col) ++k;
-        keep[r] = k;
+        keep[r] = (static_cast<uint64_t>((k + 3) & ~3) << 32) | static_cast<uint32_t>(k);
     }
 }
 
-__global__ void compact_rows(const RawEntry* ent, const int32_t* rowStart, const int32_t* outStart,
+__global__ void compact_rows(const RawEntry* ent, const int32_t* rowStart, const uint64_t* outStart,
                              int32_t n, uint32_t* offsets, Edge* edges, BuildFlags* f) {
     for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const int32_t lo = rowStart[r], hi = rowStart[r + 1];
-        int32_t o = outStart[r];
+        int32_t o = static_cast<int32_t>(outStart[r]);
         offsets[r] = static_cast<uint32_t>(o);
         long long b = 0, s = 0;
         bool unit = true, small = true;
@@ -410,15 +411,19 @@ __global__ void orig_ids(const int32_t* present, const int32_t* dense, int64_t m
         if (present[i]) out[dense[i]] = i;
 }
 
-__global__ void make_compact(const Edge* edges, int64_t m2, int fmt, void* out) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < m2;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const Edge e = edges[i];
-        if (fmt == kCsrUnit16)
-            static_cast<uint16_t*>(out)[i] =
-                static_cast<uint16_t>((static_cast<uint32_t>(e.col) << 1) | (e.w < 0 ? 1u : 0u));
-        else
-            static_cast<uint32_t*>(out)[i] = (static_cast<uint32_t>(e.w) << 16) | static_cast<uint32_t>(e.col);
+// The compact entries (u16 and/or p32, whichever are given) and the row words,
+// eight lanes a row: the high half of start[r] is row r's first compact entry.
+__global__ void make_compact(const Edge* edges, const uint32_t* offsets, const uint64_t* start, int32_t n,
+                             uint32_t* rows, uint16_t* u16, uint32_t* p32) {
+    const int sub = threadIdx.x & 7;
+    for (int32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; r < n; r += (gridDim.x * blockDim.x) >> 3) {
+        const uint32_t lo = offsets[r], deg = offsets[r + 1] - lo, o = static_cast<uint32_t>(start[r] >> 32);
+        for (uint32_t k = sub; k < ((deg + 3u) & ~3u); k += 8) {
+            const Edge e = k < deg ? edges[lo + k] : Edge{r, 0};   // padding: the vertex itself
+            if (u16) u16[o + k] = static_cast<uint16_t>(e.col | (e.w < 0 ? 0x8000 : 0));
+            if (p32) p32[o + k] = (static_cast<uint32_t>(e.w) << 16) | static_cast<uint32_t>(e.col);
+        }
+        if (sub == 0) rows[r] = o | ((0u - deg) & 3u);
     }
 }
 
@@ -494,11 +499,11 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     DevBuf dDeg, dRow, dFill, dEnt, dKeep, dOut;
     if ((rc = dDeg.alloc((static_cast<int64_t>(n) + 1) * 4)) || (rc = dRow.alloc((static_cast<int64_t>(n) + 1) * 4)) ||
         (rc = dFill.alloc((static_cast<int64_t>(n) + 1) * 4)) || (rc = dEnt.alloc(std::max<int64_t>(2 * E, 1) * sizeof(RawEntry))) ||
-        (rc = dKeep.alloc((static_cast<int64_t>(n) + 1) * 4)) || (rc = dOut.alloc((static_cast<int64_t>(n) + 1) * 4)))
+        (rc = dKeep.alloc((static_cast<int64_t>(n) + 1) * 8)) || (rc = dOut.alloc((static_cast<int64_t>(n) + 1) * 8)))
         return rc;
     CU(cudaMemsetAsync(dDeg.p, 0, (static_cast<int64_t>(n) + 1) * 4, st));
     CU(cudaMemsetAsync(dFill.p, 0, (static_cast<int64_t>(n) + 1) * 4, st));
-    CU(cudaMemsetAsync(dKeep.p, 0, (static_cast<int64_t>(n) + 1) * 4, st));
+    CU(cudaMemsetAsync(dKeep.p, 0, (static_cast<int64_t>(n) + 1) * 8, st));
     if (E) count_degrees<<<grid_for(E), 256, 0, st>>>(dU.as<int64_t>(), dV.as<int64_t>(), E,
                                                       dDense.as<int32_t>(), dDeg.as<int32_t>());
     CU(cudaGetLastError());
@@ -508,13 +513,15 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
                                                         dDense.as<int32_t>(), dRow.as<int32_t>(),
                                                         dFill.as<int32_t>(), dEnt.as<RawEntry>());
     CU(cudaGetLastError());
-    if (n) sort_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), n, dKeep.as<int32_t>());
+    if (n) sort_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), n, dKeep.as<uint64_t>());
     CU(cudaGetLastError());
-    if ((rc = exclusive_scan<int32_t>(dKeep.as<int32_t>(), dOut.as<int32_t>(), static_cast<int64_t>(n) + 1, st)))
+    if ((rc = exclusive_scan<uint64_t>(dKeep.as<uint64_t>(), dOut.as<uint64_t>(), static_cast<int64_t>(n) + 1, st)))
         return rc;
-    int32_t m2 = 0;
-    CU(cudaMemcpyAsync(&m2, dOut.as<int32_t>() + n, 4, cudaMemcpyDeviceToHost, st));
+    uint64_t kept = 0;
+    CU(cudaMemcpyAsync(&kept, dOut.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
+    const int32_t m2 = static_cast<int32_t>(kept);
+    const uint32_t mPad = static_cast<uint32_t>(kept >> 32);   // entries of the padded compact rows
 
     auto g = std::unique_ptr<rfmf_graph>(new (std::nothrow) rfmf_graph());
     if (!g) return fail(RFMF_ERR_NOMEM, "host allocation failed");
@@ -523,9 +530,8 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     g->n = n;
     g->m = m2 / 2;
     const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
-    g->offBytes = static_cast<uint32_t>(ob);
     if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(std::max<int64_t>(m2, 1) * sizeof(Edge)))) return rc;
-    if (n) compact_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), dOut.as<int32_t>(), n,
+    if (n) compact_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), dOut.as<uint64_t>(), n,
                                                      g->offsets.as<uint32_t>(), g->edges.as<Edge>(),
                                                      dFlags.as<BuildFlags>());
     CU(cudaGetLastError());
@@ -539,18 +545,25 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     if (g->B > std::numeric_limits<int32_t>::max())
         return fail(RFMF_ERR_CAPACITY, "max weighted degree %lld exceeds int32", (long long)g->B);
     g->unit16 = !hf.notUnit && n <= 32768;
-    g->packed32 = !hf.notSmall && n <= 65536 && m2 < (1 << 30);
-    if (g->unit16) {
-        g->u16Bytes = align16(static_cast<uint32_t>(m2) * 2u);
-        if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
-        CU(cudaMemsetAsync(g->u16.p, 0, g->u16Bytes, st));
-        if (m2) make_compact<<<grid_for(m2), 256, 0, st>>>(g->edges.as<Edge>(), m2, kCsrUnit16, g->u16.p);
-    }
-    if (g->packed32) {
-        g->p32Bytes = align16(static_cast<uint32_t>(m2) * 4u);
-        if ((rc = g->p32.alloc(g->p32Bytes))) return rc;
-        CU(cudaMemsetAsync(g->p32.p, 0, g->p32Bytes, st));
-        if (m2) make_compact<<<grid_for(m2), 256, 0, st>>>(g->edges.as<Edge>(), m2, kCsrPacked32, g->p32.p);
+    g->packed32 = !hf.notSmall && n <= 65536 && mPad < (1u << 30);
+    if (g->unit16 || g->packed32) {
+        g->rowBytes = static_cast<uint32_t>(ob);
+        if ((rc = g->rows.alloc(ob))) return rc;
+        if (g->unit16) {
+            g->u16Bytes = align16(mPad * 2u);
+            if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
+            CU(cudaMemsetAsync(g->u16.p, 0, g->u16Bytes, st));
+        }
+        if (g->packed32) {
+            g->p32Bytes = align16(mPad * 4u);
+            if ((rc = g->p32.alloc(g->p32Bytes))) return rc;
+            CU(cudaMemsetAsync(g->p32.p, 0, g->p32Bytes, st));
+        }
+        if (n)
+            make_compact<<<grid_for(8 * static_cast<int64_t>(n)), 256, 0, st>>>(
+                g->edges.as<Edge>(), g->offsets.as<uint32_t>(), dOut.as<uint64_t>(), n, g->rows.as<uint32_t>(),
+                g->unit16 ? g->u16.as<uint16_t>() : nullptr, g->packed32 ? g->p32.as<uint32_t>() : nullptr);
+        fill_tail_u32<<<1, 32, 0, st>>>(g->rows.as<uint32_t>(), n, static_cast<int64_t>(ob / 4), mPad);
     }
     CU(cudaGetLastError());
     // dense id -> original id, kept on the host with the graph

@@ -199,19 +199,14 @@ DevGraph dev_graph(const rfmf_graph* g, int fmt) {
     DevGraph d{};
     d.offsets = g->offsets.as<uint32_t>();
     d.edges = g->edges.as<Edge>();
+    d.rows = g->rows.as<uint32_t>();
     d.compact = compact_entries(g, fmt);
     d.n = static_cast<int32_t>(g->n);
     d.words = static_cast<int32_t>((g->n + 31) / 32);
     d.wsum2 = g->wsum2;
-    d.offBytes = g->offBytes;
-    d.entBytes = (fmt == kCsrUnit16) ? g->u16Bytes : (fmt == kCsrPacked32 ? g->p32Bytes : 0);
+    d.rowBytes = g->rowBytes;
+    d.entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;
     return d;
-}
-
-uint32_t csr_bytes(const rfmf_graph* g, int fmt) {
-    if (fmt == kCsrUnit16) return g->offBytes + g->u16Bytes;
-    if (fmt == kCsrPacked32) return g->offBytes + g->p32Bytes;
-    return 0;
 }
 
 // Device state of a newly admitted request (worker thread).
