@@ -66,6 +66,9 @@ constexpr uint32_t kW1 = 0xBB67AE85u;
 // work and the launch reports kDevCopyTimeout.
 constexpr int kMaxCopyPolls = 1 << 22;
 
+// max |Gumbel key| (Q20 table plus the field's upper bits).
+constexpr int64_t kGumMaxMag = 3617486 + 127;
+
 __device__ __forceinline__ void mulwide(uint32_t a, uint32_t b, uint32_t& hi, uint32_t& lo) {
     const uint64_t p = static_cast<uint64_t>(a) * b;
     hi = static_cast<uint32_t>(p >> 32);
@@ -439,31 +442,55 @@ __device__ __forceinline__ int64_t warp_sum(int64_t v) {
 // Per-phase constants, recomputed only when P changes (no integer division
 // or modulo by P inside a sweep).
 //
-// kPathWarp: 256 % P == 0 and P <= 128.  Every (lane, j) accumulator belongs
-// to one group, each warp reduces its 256 accumulators to P winners
-// (warp_argmax) and the winners stay in registers (one-warp chains) or pass
-// through one 8-byte partial per warp and group (wider ones).  Other P go
-// through the group slots: kPathPrivate when 8T % P == 0 (one atomic per
-// accumulator), else kPathVertex (one atomic per vertex).
+// kPathWarp: P <= 128 and private groups.  The block loop strides by S blocks,
+// 8 S a multiple of P, so that every (lane, j) accumulator belongs to one
+// group; each warp reduces its 256 accumulators to P winners (warp_argmax) and
+// the winners stay in registers (one-warp chains) or pass through one 8-byte
+// partial per warp and group (wider ones).  S is T when 8 T % P == 0 (any
+// power of two), else the largest multiple of P / gcd(P, 8) up to T, the
+// remaining threads idle in SELECT; when that is above 32, a one-warp chain
+// plays its ceil(S / 32) warps one after another.
+// Other P go through the group slots: kPathPrivate when 8 T % P == 0 (one
+// atomic per accumulator), else kPathVertex (one atomic per vertex).
 enum PhasePath : int { kPathWarp = 0, kPathPrivate = 1, kPathVertex = 2 };
 
 struct PhaseCfg {
     int P;
     int path;       // PhasePath
-    int g0;         // kPathPrivate: (8 t) mod P
     int laneShift;  // FLIP: log2 of the lanes that share one winner's row
-    int rows;       // FLIP: rows a thread takes part in on kPathWarp (1, 2 or 4)
+    int rows;       // FLIP: rows a thread takes part in on kPathWarp (1 to 4)
+    int S;          // block stride (T but on kPathWarp; above 32 a one-warp chain
+                    //    plays several warps)
+    int step;       // kPathWarp: 256 mod P, a warp's shift of the groups
+    int warpG;      // kPathWarp: (256 warp) mod P
 };
 
-__device__ __forceinline__ PhaseCfg phase_cfg(int P, int t, int T, bool slots) {
+__device__ __forceinline__ int key_bits(int n, int T) {
+    const int iters = ((n + 7) / 8 + T - 1) / T;
+    int kb = 4;
+    while ((1 << kb) < iters) ++kb;
+    return kb;
+}
+
+// kbMax: bits the chain's keys can spare for the block iteration; `slots`:
+// the group slots are wanted (int64 scores).
+__device__ __forceinline__ PhaseCfg phase_cfg(int P, int n, int t, int T, bool one, int kbMax, bool slots) {
     PhaseCfg c;
     c.P = P;
-    c.path = (!slots && P <= 128 && (256 % P) == 0) ? kPathWarp : ((8 * T) % P) == 0 ? kPathPrivate : kPathVertex;
-    c.g0 = (8 * t) % P;
+    c.S = T;
+    const int twos = P & -P;
+    const int s0 = P / (twos < 8 ? twos : 8);
+    int S = T;
+    if ((8 * T) % P != 0) S = s0 <= T ? T / s0 * s0 : (one ? s0 : 0);
+    const bool warp = !slots && P <= 128 && S > 0 && key_bits(n, S > 0 ? S : 1) <= kbMax;
+    c.S = uniform(warp ? S : T);
+    c.path = uniform(static_cast<int>(warp ? kPathWarp : ((8 * T) % P) == 0 ? kPathPrivate : kPathVertex));
+    c.step = uniform(256 % P);
+    c.warpG = uniform((8 * (t & ~31)) % P);
     int sh = 0;
     while ((2 << sh) * P <= T && sh < 5) ++sh;
-    c.laneShift = sh;
-    c.rows = (P + T - 1) / T;
+    c.laneShift = uniform(sh);
+    c.rows = uniform((P + T - 1) / T);
     return c;
 }
 
@@ -500,25 +527,28 @@ struct KeyCfg {
     int kb;          // bits of the block-iteration field
     uint32_t mulF;   // 2^(kb-4), the field's multiple; below 256 (a chain of 2^19 vertices would not fit)
     int32_t tkLane;  // TK[lane & 15]
-    int iters;       // block iterations of this thread's warp
+    int full;        // block iterations of a stride S over all blocks: `full`,
+    int extra;       //   and one more for the threads below `extra`
 };
 
-__device__ __forceinline__ int key_bits(int n, int T) {
-    const int iters = ((n + 7) / 8 + T - 1) / T;
-    int kb = 4;
-    while ((1 << kb) < iters) ++kb;
-    return kb;
-}
-
-__device__ __forceinline__ KeyCfg key_cfg(int n, int T, int t, const int32_t* lut) {
+__device__ __forceinline__ KeyCfg key_cfg(int n, int S, int t, const int32_t* lut) {
     KeyCfg kc;
-    kc.kb = key_bits(n, T);
+    kc.kb = uniform(key_bits(n, S));
     kc.mulF = 1u << (kc.kb - 4);
-    const int ahead = ((n + 7) >> 3) - (t & ~31);   // blocks from the warp's first on
-    kc.iters = uniform(ahead > 0 ? (ahead + T - 1) / T : 0);
+    kc.full = uniform(((n + 7) >> 3) / S);
+    kc.extra = uniform(((n + 7) >> 3) % S);
     const int i = t & 15;
     kc.tkLane = lut[i] * (1 << kc.kb) - i * static_cast<int32_t>(kc.mulF);
     return kc;
+}
+
+// The most block-iteration bits the compact keys of a chain can carry: its
+// largest score is betaMax * B + max|gum|.
+__device__ __forceinline__ int key_room(int32_t betaMax, int64_t B) {
+    const int64_t top = static_cast<int64_t>(betaMax) * B + kGumMaxMag + 1;
+    int kb = 0;
+    while (kb < 12 && (top << (kb + 1)) < 2147483647) ++kb;
+    return kb;
 }
 
 // Keys of one block's 8 vertices folded into acc; lanes j >= lim are skipped
@@ -667,6 +697,52 @@ __device__ __forceinline__ void warp_argmax(const int32_t acc[8], int32_t* scr, 
     }
 }
 
+// The same for any P <= 128: class c = a mod P (the group but for the warp's
+// shift).  With P <= 32, 32 / P lanes share a class and fold pairwise into its
+// first lane; four reads go out together.
+__device__ __forceinline__ void warp_argmax_any(const int32_t acc[8], int32_t* scr, int lane, int P, int32_t key[4],
+                                                int32_t at[4]) {
+    *reinterpret_cast<int4*>(scr + 4 * lane) = make_int4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<int4*>(scr + kHalf + 4 * lane) = make_int4(acc[4], acc[5], acc[6], acc[7]);
+    __syncwarp();
+    int share = P <= 32 ? 32 / P : 1;
+    const int width = share * P;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        key[q] = INT32_MIN;
+        at[q] = 0;
+        const int c = lane + 32 * q;
+        if (c < width) {
+            for (int a = c; a < 256; a += 4 * width) {
+                int32_t k[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int x = a + i * width < 256 ? a + i * width : a;   // past the end: the first again
+                    k[i] = scr[4 * (x >> 3) + (x & 3) + kHalf * ((x >> 2) & 1)];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (k[i] > key[q]) {
+                        key[q] = k[i];
+                        at[q] = a + i * width;
+                    }
+                }
+            }
+        }
+    }
+    while (share > 1) {
+        const int half = (share + 1) >> 1;
+        const int32_t ok = __shfl_down_sync(0xFFFFFFFFu, key[0], half * P);
+        const int32_t oa = __shfl_down_sync(0xFFFFFFFFu, at[0], half * P);
+        if (lane < (share - half) * P && beats(ok, oa, key[0], at[0])) {
+            key[0] = ok;
+            at[0] = oa;
+        }
+        share = half;
+    }
+    if (lane >= P) key[0] = INT32_MIN;
+}
+
 // P = 1: fold the eight accumulators in registers, one warp max, and the
 // lowest lane holding it; every lane gets the winner.
 __device__ __forceinline__ void warp_argmax_one(const int32_t acc[8], int32_t& key, int32_t& at) {
@@ -704,62 +780,58 @@ __device__ __forceinline__ unsigned long long make_partial(const ChainSmem& s, i
     return (static_cast<unsigned long long>(static_cast<uint32_t>(key) ^ 0x80000000u) << 32) | lo;
 }
 
-// SELECT of the int32 path on kPathWarp: on return lane l of a one-warp chain
-// holds the winners v[q] of groups l + 32 q (-1: none); a wider chain has its
-// partials in place (a barrier is due).  On the other paths the winners are
-// packed keys in the group slots (a barrier is due).
+// The accumulators of one warp over its `iters` block iterations at stride S
+// (thread t of it).
+template <bool kF0, class DP>
+__device__ __forceinline__ void select_warp(int32_t acc[8], const ChainSmem& s, const SweepConst& sc,
+                                            const ChainKeys& keys, int n, const KeyCfg& kc, int t, int S, int iters,
+                                            int32_t beta) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = INT32_MIN;
+    const int32_t betaK = beta * (1 << kc.kb);
+    // Per-sweep part of the table register: (2^kb - 1) - bias * beta * 2^kb.
+    const int32_t tkBase = static_cast<int32_t>(static_cast<uint32_t>(kc.tkLane) + (1u << kc.kb) - 1u -
+                                                static_cast<uint32_t>(DP::kBias) * static_cast<uint32_t>(betaK));
+    select_blocks<kF0, DP>(acc, s, sc, keys, n, t, S, iters, betaK, tkBase, kc);
+}
+
+// The winners of a warp's P classes as its partials (wider chains) or in
+// registers (v).
 template <bool kOne, class DP>
-__device__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
-                         const PhaseCfg& pc, int32_t beta, const SweepConst& sc, const ChainKeys& keys,
-                         int t, int T, int32_t v[4]) {
-    const int P = pc.P;
+__device__ __forceinline__ void warp_winners(const ChainSmem& s, const PhaseCfg& pc, const KeyCfg& kc, int32_t* scr,
+                                             int first, int lane, int S, const int32_t key[4], const int32_t at[4],
+                                             int32_t v[4]) {
     const int M = (1 << kc.kb) - 1;
-    if (pc.path != kPathVertex) {
-        const int32_t betaK = beta * (1 << kc.kb);
-        int32_t acc[8];
+    const int Q = (pc.P + 31) >> 5;
+    if (!kOne) __syncwarp();   // the scratch is rewritten below
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = INT32_MIN;
-        // Per-sweep part of the table register: (2^kb - 1) - bias * beta * 2^kb.
-        const int32_t tkBase = static_cast<int32_t>(static_cast<uint32_t>(kc.tkLane) + static_cast<uint32_t>(M) -
-                                                    static_cast<uint32_t>(DP::kBias) * static_cast<uint32_t>(betaK));
-        if (kc.kb == 4) select_blocks<true, DP>(acc, s, sc, keys, n, t, T, kc.iters, betaK, tkBase, kc);
-        else select_blocks<false, DP>(acc, s, sc, keys, n, t, T, kc.iters, betaK, tkBase, kc);
-        if (pc.path == kPathWarp) {
-            const int lane = t & 31;
-            int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
-                                                      (kOne ? 0 : (t >> 5) * kWarpScratch));
-            int32_t key[4], at[4];
-            if (P == 1) warp_argmax_one(acc, key[0], at[0]);
-            else if (P <= 32) warp_argmax<1>(acc, scr, lane, P, key, at);
-            else if (P == 64) warp_argmax<2>(acc, scr, lane, P, key, at);
-            else warp_argmax<4>(acc, scr, lane, P, key, at);
-            const int Q = (P + 31) >> 5;
-            if (!kOne) __syncwarp();   // the scratch is rewritten below
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q >= Q) break;
-                const int kk = M - (key[q] & M);
-                v[q] = (key[q] != INT32_MIN) ? 8 * (t & ~31) + at[q] + 8 * kk * T : -1;
-                if (!kOne) {
-                    const int g = lane + 32 * q;
-                    if (g < P)
-                        reinterpret_cast<unsigned long long*>(scr)[g] =
-                            (v[q] >= 0) ? make_partial<DP>(s, key[q], v[q]) : 0ull;
-                }
-            }
-        } else {
-            int g = pc.g0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (acc[j] != INT32_MIN) {
-                    const int kk = M - (acc[j] & M);
-                    atomicMax(&s.slots[g], pack_key(acc[j] >> kc.kb, 8 * (t + kk * T) + j));
-                }
-                if (++g == P) g = 0;
+    for (int q = 0; q < 4; ++q) {
+        if (q >= Q) break;
+        const int kk = M - (key[q] & M);
+        v[q] = (key[q] != INT32_MIN) ? 8 * first + at[q] + 8 * kk * S : -1;
+        if (!kOne) {
+            const int c = lane + 32 * q;
+            if (c < pc.P) {
+                const int g = c + pc.warpG < pc.P ? c + pc.warpG : c + pc.warpG - pc.P;
+                reinterpret_cast<unsigned long long*>(scr)[g] =
+                    (v[q] >= 0) ? make_partial<DP>(s, key[q], v[q]) : 0ull;
             }
         }
-    } else {
-        // General P: one shared atomic per vertex, plain score.
+    }
+}
+
+// SELECT off the main path: private groups at a stride S below T (or, for
+// one-warp chains, above 32: the warps played one after another, each one's
+// winners merged into a table with one lane per group), and the slots.  Code
+// of its own: a variable stride in the main path's block loop cost every
+// phase 8 to 13% on GB300.
+template <bool kOne, class DP>
+__device__ __forceinline__ void select32_general(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
+                                                 const PhaseCfg& pc, int32_t beta, const SweepConst& sc,
+                                                 const ChainKeys& keys, int t, int T, int32_t v[4]) {
+    const int P = pc.P;
+    if (pc.path == kPathVertex) {
+        // One shared atomic per vertex, plain score.
         for (int bb = t; 8 * bb < n; bb += T) {
             uint32_t x[4];
             int32_t d[8];
@@ -777,7 +849,90 @@ __device__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& k
                 if (++g == P) g = 0;
             }
         }
+        return;
     }
+    const int lane = t & 31, S = pc.S, M = (1 << kc.kb) - 1;
+    int shift = 0;   // (256 round) mod P
+    for (int first = t & ~31;; first += 32) {
+        // Threads from S on idle: they score the last one's blocks and drop
+        // them.
+        int32_t acc[8], key[4], at[4];
+        const int iters = first < S ? kc.full + (first < kc.extra ? 1 : 0) : 0;
+        select_warp<false, DP>(acc, s, sc, keys, n, kc, first + lane < S ? first + lane : S - 1, S, iters, beta);
+        if (pc.path == kPathPrivate) {
+            int g = (8 * t) % P;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (acc[j] != INT32_MIN) {
+                    const int kk = M - (acc[j] & M);
+                    atomicMax(&s.slots[g], pack_key(acc[j] >> kc.kb, 8 * (t + kk * T) + j));
+                }
+                if (++g == P) g = 0;
+            }
+            return;
+        }
+        if (first + lane >= S) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = INT32_MIN;
+        }
+        int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
+                                                  (kOne ? 0 : (t >> 5) * kWarpScratch));
+        warp_argmax_any(acc, scr, lane, P, key, at);
+        if (!kOne || S <= 32) {
+            warp_winners<kOne, DP>(s, pc, kc, scr, first, lane, S, key, at, v);
+            return;
+        }
+        unsigned long long* table = reinterpret_cast<unsigned long long*>(s.ids);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int c = lane + 32 * q;
+            if (c < P) {
+                const int g = c + shift < P ? c + shift : c + shift - P;
+                const unsigned long long mine =
+                    key[q] != INT32_MIN ? pack_key(key[q], 8 * first + at[q] + 8 * (M - (key[q] & M)) * S) : 0ull;
+                if (first == 0 || mine > table[g]) table[g] = mine;
+            }
+        }
+        shift = shift + pc.step < P ? shift + pc.step : shift + pc.step - P;
+        __syncwarp();
+        if (first + 32 >= S) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int g = lane + 32 * q;
+                const unsigned long long p = g < P ? table[g] : 0ull;
+                v[q] = p ? key_vertex(p) : -1;
+            }
+            __syncwarp();
+            return;
+        }
+    }
+}
+
+// SELECT of the int32 path.  On kPathWarp, on return lane l of a one-warp chain
+// holds the winners v[q] of groups l + 32 q (-1: none) and a wider chain has
+// its partials in place (a barrier is due); else the winners are packed keys
+// in the group slots (a barrier is due).
+template <bool kOne, class DP>
+__device__ __forceinline__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
+                                         const PhaseCfg& pc, int32_t beta, const SweepConst& sc,
+                                         const ChainKeys& keys, int t, int T, int32_t v[4]) {
+    if (pc.path != kPathWarp || pc.step != 0) {
+        select32_general<kOne, DP>(s, lut, kc, n, pc, beta, sc, keys, t, T, v);
+        return;
+    }
+    const int P = pc.P;
+    const int lane = t & 31, first = kOne ? 0 : t & ~31;
+    int32_t acc[8], key[4], at[4];
+    const int iters = kc.full + (first < kc.extra ? 1 : 0);
+    if (kc.kb == 4) select_warp<true, DP>(acc, s, sc, keys, n, kc, t, T, iters, beta);
+    else select_warp<false, DP>(acc, s, sc, keys, n, kc, t, T, iters, beta);
+    int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
+                                              (kOne ? 0 : (t >> 5) * kWarpScratch));
+    if (P == 1) warp_argmax_one(acc, key[0], at[0]);
+    else if (P <= 32) warp_argmax<1>(acc, scr, lane, P, key, at);
+    else if (P == 64) warp_argmax<2>(acc, scr, lane, P, key, at);
+    else warp_argmax<4>(acc, scr, lane, P, key, at);
+    warp_winners<kOne, DP>(s, pc, kc, scr, first, lane, T, key, at, v);
 }
 
 // int64 scores (the reference's two-pass path, src/anneal_kernels.cu:348-378,
@@ -1006,7 +1161,10 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
         if (q >= pc.rows) continue;
         const int r = (t >> pc.laneShift) + q * T;
         if constexpr (kOne) {
-            if (q == 0 && pc.laneShift) v[0] = __shfl_sync(0xFFFFFFFFu, v[0], r);
+            if (q == 0 && pc.laneShift) {
+                v[0] = __shfl_sync(0xFFFFFFFFu, v[0], r);
+                if (r >= pc.P) v[0] = -1;
+            }
         } else {
             unsigned long long p = 0;
             v[q] = -1;
@@ -1172,7 +1330,6 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         s.slots[i] = kS64 ? static_cast<unsigned long long>(LLONG_MIN) : 0ull;
         s.ids[i] = INT32_MAX;
     }
-    const KeyCfg kc = key_cfg(n, T, t, lut);
     group_sync(grp, T);
     const int nPad = (n + 7) & ~7;
     for (int v = t; v < nPad; v += T)
@@ -1244,7 +1401,10 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             P = static_cast<int>(umin(uniform(sch.phaseP[p]), static_cast<uint32_t>(n)));
         }
     }
-    PhaseCfg pc = phase_cfg(P, t, T, kS64);
+    // The last beta run holds the schedule's largest beta.
+    const int kbMax = kS64 ? 0 : uniform(key_room(__ldg(ch.betaVal + ch.betaRuns - 1), g.B));
+    PhaseCfg pc = phase_cfg(P, n, t, T, kOne, kbMax, kS64);
+    KeyCfg kc = key_cfg(n, pc.S, t, lut);
 
     const ChainKeys keys = make_keys(ch.solverSeed);
     // Beta cursor: the current run and the next one as uniform values, the one
@@ -1301,7 +1461,8 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
                 P = static_cast<int>(umin(uniform(sch.phaseP[p]), static_cast<uint32_t>(n)));
             }
             const bool warp = pc.path == kPathWarp;
-            pc = phase_cfg(P, t, T, kS64);
+            pc = phase_cfg(P, n, t, T, kOne, kbMax, kS64);
+            kc = key_cfg(n, pc.S, t, lut);
             if (warp && pc.path != kPathWarp) {
                 // The slots held scratch and partials: empty them (all their
                 // readers are past the last sweep's barrier).

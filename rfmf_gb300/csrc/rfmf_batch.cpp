@@ -857,6 +857,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         hg[gi].compact = compact_entries(g, fmt);
         hg[gi].n = static_cast<int32_t>(g->n);
         hg[gi].words = static_cast<int32_t>((g->n + 31) / 32);
+        hg[gi].B = g->B;
         hg[gi].wsum2 = g->wsum2;
         hg[gi].rowBytes = g->rowBytes;
         hg[gi].entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;

@@ -51,6 +51,7 @@ struct DevGraph {
     const void*     compact;   // compact entries of the launch's format, rows padded to four (16 B in all)
     int32_t         n;
     int32_t         words;     // ceil(n / 32): spin bit-words per chain
+    int64_t         B;         // max weighted degree: no gain exceeds it
     int64_t         wsum2;     // sum of weight over directed entries (2 * sum over edges)
     uint32_t        rowBytes;  // bytes of rows, multiple of 16
     uint32_t        entBytes;  // bytes of compact entries, multiple of 16

@@ -260,6 +260,7 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     g.compact = nullptr;
     g.n = static_cast<int32_t>(n);
     g.words = words;
+    g.B = max_weighted_deg;
     g.wsum2 = 0;
     g.rowBytes = 0;
     g.entBytes = 0;

@@ -203,6 +203,7 @@ DevGraph dev_graph(const rfmf_graph* g, int fmt) {
     d.compact = compact_entries(g, fmt);
     d.n = static_cast<int32_t>(g->n);
     d.words = static_cast<int32_t>((g->n + 31) / 32);
+    d.B = g->B;
     d.wsum2 = g->wsum2;
     d.rowBytes = g->rowBytes;
     d.entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;

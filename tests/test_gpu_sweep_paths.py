@@ -2,7 +2,7 @@
 (integer work: tolerance zero): group counts that reduce per warp, per thread
 and per vertex, chain widths, gain widths, and vertex counts at the edges of a
 warp's block loop (32 W blocks of 8 vertices an iteration, three iterations in
-flight)."""
+flight), and past the 16 iterations a one-warp chain's keys number in 4 bits."""
 import numpy as np
 import pytest
 
@@ -32,7 +32,10 @@ def _graph(rfmf, n, wmax):
 @pytest.mark.parametrize("phases", sorted(PHASES))
 @pytest.mark.parametrize("threads", [32, 64, 128, 256])
 def test_sweep_routes(rfmf, ctx, oracle, threads, phases, wmax):
-    for n in (5, 255, 257, 8 * threads - 1, 24 * threads + 9, 32 * threads + 8):
+    sizes = [5, 255, 257, 8 * threads - 1, 24 * threads + 9, 32 * threads + 8]
+    if threads == 32:
+        sizes.append(4231)
+    for n in sizes:
         g = _graph(rfmf, n, wmax)
         seeds, t0s = [3, 4, 5], [35.0 * wmax, 120.0 * wmax, 400.0 * wmax]
         init, solver = chains_for(g, seeds)
