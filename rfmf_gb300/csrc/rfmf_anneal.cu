@@ -1037,12 +1037,16 @@ __device__ __forceinline__ void add_vec(const ChainSmem& s, const typename Csr<k
         add_packed<DP>(s, e.z, neg);
         add_packed<DP>(s, e.w, neg);
     } else {
-        static_assert(DP::kField, "16-bit entries of int32 gains are walked one by one");
-        const uint32_t nm = neg << 15;
-        add_unit(s.D, e.x, nm);
-        add_unit(s.D, e.x >> 16, nm);
-        add_unit(s.D, e.y, nm);
-        add_unit(s.D, e.y >> 16, nm);
+        const uint32_t h[4] = {e.x, e.x >> 16, e.y, e.y >> 16};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if constexpr (DP::kField) {
+                add_unit(s.D, h[j], neg << 15);
+            } else {
+                const int c = static_cast<int>(h[j] & 0x7FFFu);
+                DP::add(s.D, c, (((h[j] >> 15) ^ neg ^ s.sb[c]) & 1u) ? -2 : 2);
+            }
+        }
     }
 }
 
@@ -1058,11 +1062,7 @@ template <class DP, int kFmt>
 __device__ __forceinline__ void scatter_row(const ChainSmem& s, const CsrView& csr, uint32_t lo, uint32_t hi,
                                             uint32_t neg, int sub, int lanes) {
     using C = Csr<kFmt>;
-    if constexpr (C::kPlain || (C::kUnit && !DP::kField)) {
-        if constexpr (!C::kPlain) {
-            hi = (hi & ~3u) - (lo & 3u);
-            lo &= ~3u;
-        }
+    if constexpr (C::kPlain) {
         uint32_t i = lo + sub;
         for (; i + 3 * lanes < hi; i += 4 * lanes) {
             int c[4], w[4];
@@ -1101,7 +1101,7 @@ template <class DP, int kFmt>
 __device__ __forceinline__ void scatter_two(const ChainSmem& s, const CsrView& csr, const uint32_t lo[2],
                                             const uint32_t hi[2], const uint32_t neg[2]) {
     using C = Csr<kFmt>;
-    if constexpr (C::kPlain || (C::kUnit && !DP::kField)) {
+    if constexpr (C::kPlain) {
         scatter_row<DP, kFmt>(s, csr, lo[0], hi[0], neg[0], 0, 1);
         scatter_row<DP, kFmt>(s, csr, lo[1], hi[1], neg[1], 0, 1);
     } else {
@@ -1121,10 +1121,11 @@ __device__ __forceinline__ void scatter_two(const ChainSmem& s, const CsrView& c
 }
 
 // What a walk of row `lo` adds to the row's own vertex through the padding:
-// nothing but for 16-bit entries, whose padding weighs +1.
+// nothing but for 16-bit entries, whose padding weighs +1 (2 s_v to the field;
+// to the gain, 2 s_v s_v).
 template <class DP, int kFmt>
 __device__ __forceinline__ int32_t own_padding(uint32_t lo, uint32_t neg) {
-    if constexpr (Csr<kFmt>::kUnit && DP::kField) return static_cast<int32_t>(lo & 3u) * (neg ? -2 : 2);
+    if constexpr (Csr<kFmt>::kUnit) return static_cast<int32_t>(lo & 3u) * (DP::kField && neg ? -2 : 2);
     else return 0;
 }
 
@@ -1207,7 +1208,7 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
                 atomicXor(&s.bits[v[q] >> 5], 1u << (v[q] & 31));
                 s.sb[v[q]] = neg[q] ? 0xFFu : 0u;
             } else {
-                flip_vertex<DP>(s, v[q], d[q], neg[q] ? 0u : 0xFFu);
+                flip_vertex<DP>(s, v[q], d[q] + own_padding<DP, kFmt>(lo[q], neg[q]), neg[q] ? 0u : 0xFFu);
             }
         }
     }
@@ -1263,7 +1264,7 @@ __device__ __forceinline__ Loc flip_slots(const ChainSmem& s, const CsrView& csr
             const int sub = t & (lanes - 1);
             // Past the barrier only: the plain byte stores above do not mix
             // with an add that may carry through a neighbouring byte.
-            if (sub == 0 && (Csr<kFmt>::kUnit && DP::kField)) DP::add(s.D, v, -own_padding<DP, kFmt>(lo, neg));
+            if (sub == 0 && Csr<kFmt>::kUnit) DP::add(s.D, v, -own_padding<DP, kFmt>(lo, neg));
             scatter_row<DP, kFmt>(s, csr, lo, hi, neg, sub, lanes);
         }
     }
