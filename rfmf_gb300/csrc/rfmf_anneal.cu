@@ -396,7 +396,7 @@ struct ChainSmem {
 
 __device__ __forceinline__ ChainSmem carve_chain(unsigned char* base, const DevLaunch& L,
                                                  int dbytes) {
-    const ChainLayout c = chain_layout(L.maxN, L.maxWords, L.pmax, L.warpsPerChain, dbytes);
+    const ChainLayout c = chain_layout(L.maxN, L.maxWords, L.pmax, L.warpsPerChain, dbytes, !L.slotsOnly);
     ChainSmem s;
     s.D = base + c.d;
     s.bits = reinterpret_cast<uint32_t*>(base + c.bits);
@@ -473,7 +473,7 @@ __device__ __forceinline__ int key_bits(int n, int T) {
 }
 
 // kbMax: bits the chain's keys can spare for the block iteration; `slots`:
-// the group slots are wanted (int64 scores).
+// the group slots are wanted (int64 scores, chains without argmax scratch).
 __device__ __forceinline__ PhaseCfg phase_cfg(int P, int n, int t, int T, bool one, int kbMax, bool slots) {
     PhaseCfg c;
     c.P = P;
@@ -484,7 +484,8 @@ __device__ __forceinline__ PhaseCfg phase_cfg(int P, int n, int t, int T, bool o
     if ((8 * T) % P != 0) S = s0 <= T ? T / s0 * s0 : (one ? s0 : 0);
     const bool warp = !slots && P <= 128 && S > 0 && key_bits(n, S > 0 ? S : 1) <= kbMax;
     c.S = uniform(warp ? S : T);
-    c.path = uniform(static_cast<int>(warp ? kPathWarp : ((8 * T) % P) == 0 ? kPathPrivate : kPathVertex));
+    const bool priv = (8 * T) % P == 0 && key_bits(n, T) <= kbMax;
+    c.path = uniform(static_cast<int>(warp ? kPathWarp : priv ? kPathPrivate : kPathVertex));
     c.step = uniform(256 % P);
     c.warpG = uniform((8 * (t & ~31)) % P);
     int sh = 0;
@@ -1403,8 +1404,9 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         }
     }
     // The last beta run holds the schedule's largest beta.
-    const int kbMax = kS64 ? 0 : uniform(key_room(__ldg(ch.betaVal + ch.betaRuns - 1), g.B));
-    PhaseCfg pc = phase_cfg(P, n, t, T, kOne, kbMax, kS64);
+    const int kbMax = kS64 ? 31 : uniform(key_room(__ldg(ch.betaVal + ch.betaRuns - 1), g.B));
+    const bool slotsOnly = kS64 || L.slotsOnly;
+    PhaseCfg pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
     KeyCfg kc = key_cfg(n, pc.S, t, lut);
 
     const ChainKeys keys = make_keys(ch.solverSeed);
@@ -1462,7 +1464,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
                 P = static_cast<int>(umin(uniform(sch.phaseP[p]), static_cast<uint32_t>(n)));
             }
             const bool warp = pc.path == kPathWarp;
-            pc = phase_cfg(P, n, t, T, kOne, kbMax, kS64);
+            pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
             kc = key_cfg(n, pc.S, t, lut);
             if (warp && pc.path != kPathWarp) {
                 // The slots held scratch and partials: empty them (all their

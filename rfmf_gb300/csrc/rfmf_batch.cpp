@@ -126,13 +126,18 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
     cudaFuncAttributes fa{};
     const int64_t dynMax = dyn_smem_max(b.ctx, kern, fa);
     if (dynMax < 0) return fail(RFMF_ERR_CUDA, "kernel attributes unavailable");
-    const uint32_t chainB = chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes).total;
+    bool argmax = !k.score64;
+    uint32_t chainB = chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes, argmax).total;
     // Warp groups per CTA: named barriers 1..15, and the variant's register
     // budget bounds the CTA's threads.
     const int W = k.warps;
     const int kCap = std::min(std::min(16 / W, W > 1 ? 15 : 16), fa.maxThreadsPerBlock / (32 * W));
     if (kCap < 1) return fail(RFMF_ERR_CAPACITY, "a %d-thread chain exceeds the kernel's CTA limit", 32 * W);
     const int64_t room = dynMax - kSmemHeader - csrB;
+    if (argmax && room < chainB) {   // the largest graphs fit without the argmax scratch only
+        argmax = false;
+        chainB = chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes, argmax).total;
+    }
     int Kmax = room > 0 ? static_cast<int>(std::min<int64_t>(kCap, room / chainB)) : 0;
     if (c.chains_per_cta) {
         if (c.chains_per_cta < 1 || c.chains_per_cta > kCap)
@@ -190,7 +195,23 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
     k.L.pmax = k.pmax;
     k.L.csrBytes = csrB;
     k.L.chainBytes = chainB;
+    k.L.slotsOnly = argmax ? 0 : 1;
     return RFMF_OK;
+}
+
+// Whether one chain of class k fits a CTA beside its largest CSR with the rows
+// packed and without argmax scratch (see packed_csr_bytes).
+bool fits_packed(const rfmf_batch& b, const BatchClass& k) {
+    int64_t maxN = 0, csr = 0;
+    for (int gi : k.graphs) {
+        maxN = std::max(maxN, b.glist[gi]->n);
+        csr = std::max(csr, packed_csr_bytes(b.glist[gi], k.fmt));
+    }
+    cudaFuncAttributes fa{};
+    const int64_t dynMax = dyn_smem_max(b.ctx, kernel_ptr(k.dbytes, k.fmt, k.score64, k.warps), fa);
+    const int n = static_cast<int>(maxN);
+    return dynMax - kSmemHeader - csr >=
+           static_cast<int64_t>(chain_layout(n, (n + 31) / 32, k.pmax, k.warps, k.dbytes, false).total);
 }
 
 // Per-graph chains per item: graph q may use item sizes cand[q] (chain
@@ -446,24 +467,33 @@ int rebalance(rfmf_batch* b, uint32_t P, bool* changed = nullptr) {
     return RFMF_OK;
 }
 
-// Warps per chain for phases of group count P in a batch whose width
-// follows the phase (one class, one graph, the rule's width W, every chain
-// resident at 2W): 2W while the winners' rows hold at least half as many
-// entries as the graph has vertices (P >= 64), W otherwise.  GB300, us per
-// sweep at W / 2W: 1024 chains of ER n = 2000 d = 19 (W = 1) P = 128
-// 10.0 / 8.08, P = 64 6.11 / 5.43, P = 32 4.14 / 4.60, P = 1 2.41 / 2.88;
-// 32 chains of ER n = 800 d = 48 (W = 4) P = 128 5.56 / 4.39, P = 64
-// 3.92 / 3.49, P = 1 1.72 / 1.78; the 50x60 torus (512 row entries at
-// P = 128) is faster at one warp in every phase.
-bool wide_phase(const rfmf_graph* g, uint32_t P) {
+// Whether a batch whose width follows the phase (one class, one graph, the
+// rule's width) doubles it for phases of group count P: the row-heavy ones, P >=
+// 64 with at least half as many entries in the winners' rows as the graph has
+// vertices, while that leaves an SM few enough warps: 10 from one or two warps
+// per chain, 8 from four, or 16 from four when the rows hold four times the
+// vertices.  GB300, us per sweep at P = 128, narrow / doubled: from one warp ER
+// n = 1500 d = 12 600 chains (8 warps per SM) 5.06 / 3.98, ER n = 2000 d = 19 700
+// chains (9) 4.50 / 4.47 and 1024 chains (14) 4.58 / 5.15; from four ER n = 800
+// d = 48 (rows 7.7 times the vertices) 32 chains 2.98 / 2.51, 300 chains (16)
+// 3.37 / 3.14, ER n = 2000 64 chains 2.34 / 2.11, 200 chains (11; 1.2 times)
+// 2.58 / 2.67.
+bool wide_phase(const rfmf_graph* g, uint32_t P, int warps, int64_t warpsPerSm) {
     const double n = static_cast<double>(g->n);
     const double rows = std::min(static_cast<double>(P), n);
-    return P >= 64 && 2.0 * rows * (2.0 * static_cast<double>(g->m) / n) >= n;
+    const double entries = rows * (2.0 * static_cast<double>(g->m) / n);
+    if (P < 64 || 2.0 * entries < n) return false;
+    return warpsPerSm <= (warps < 4 ? 10 : entries >= 4.0 * n ? 16 : 8);
+}
+
+// Warps an SM would hold at twice the class's planned width.
+int64_t doubled_load(const rfmf_batch& b, const BatchClass& k) {
+    return (b.C * 2 * k.baseWarps + b.ctx->sms - 1) / b.ctx->sms;
 }
 
 int phase_warps(const rfmf_batch& b, const BatchClass& k, uint32_t P) {
     if (!b.phaseWarps) return k.warps;
-    return wide_phase(b.glist[k.graphs[0]], P) ? 2 * k.baseWarps : k.baseWarps;
+    return wide_phase(b.glist[k.graphs[0]], P, k.baseWarps, doubled_load(b, k)) ? 2 * k.baseWarps : k.baseWarps;
 }
 
 // Re-plans class k at `warps` per chain (CTA shape, items) for phase P.  A
@@ -671,7 +701,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                     return fail(RFMF_ERR_INVALID, "int32 scores would overflow for this (t0, B, sweeps)");
             }
             const int64_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>((g->n + 31) / 32), pmaxG,
-                                                Wc, dbytes).total;
+                                                Wc, dbytes, !pk.s64).total;
             // A shared-memory CSR pays only while it leaves room for the chains
             // a CTA should hold: about 8 warps, fewer when the graph has fewer
             // chains or the batch fewer than that per SM.  Otherwise its rows
@@ -762,7 +792,8 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 auto chainOf = [&](int64_t n) {
                     const int ni = static_cast<int>(n);
                     return static_cast<int64_t>(
-                        chain_layout(ni, (ni + 31) / 32, std::max(1, std::min(k.pmax, ni)), k.warps, k.dbytes).total);
+                        chain_layout(ni, (ni + 31) / 32, std::max(1, std::min(k.pmax, ni)), k.warps, k.dbytes,
+                                     !k.score64).total);
                 };
                 int64_t maxN = 0, maxCsr = 0, maxCh = 0;
                 for (size_t q = 0; q < k.graphs.size(); ++q) {
@@ -819,10 +850,16 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     const bool exact = b->cls.size() > 1;
     for (BatchClass& k : b->cls) {
         int rc = plan_class(*b, k, c, exact);
-        if (rc == RFMF_ERR_CAPACITY && !csr_in_hbm(k.fmt) && c.csr_format == 0) {
+        if (rc == RFMF_ERR_CAPACITY && !csr_in_hbm(k.fmt) && (c.csr_format == 0 || fits_packed(*b, k))) {
             // The class's largest CSR and largest n together do not fit: its
             // graphs (all of them 16-bit or all 32-bit capable) walk HBM.
             k.fmt = (k.fmt == kCsrUnit16) ? kCsrGlobal16 : kCsrGlobal32;
+            rc = plan_class(*b, k, c, exact);
+        }
+        while (rc == RFMF_ERR_CAPACITY && c.threads_per_chain == 0 && k.warps > 1) {
+            // A wider chain keeps a few bytes more; the largest graphs fit at
+            // a narrower one only.
+            k.warps /= 2;
             rc = plan_class(*b, k, c, exact);
         }
         if (rc) return rc;
@@ -830,9 +867,9 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     b->cfg = c;
     for (BatchClass& k : b->cls) k.baseWarps = k.warps;
     if (b->cls.size() == 1 && b->cls[0].graphs.size() == 1 && c.threads_per_chain == 0 &&
-        2 * b->cls[0].warps <= kMaxLatencyWarps && b->C * 2 * b->cls[0].warps <= int64_t(16) * ctx->sms) {
+        2 * b->cls[0].warps <= kMaxLatencyWarps) {
         for (uint32_t P : b->phaseP)
-            b->phaseWarps = b->phaseWarps || (P && wide_phase(b->glist[b->cls[0].graphs[0]], P));
+            b->phaseWarps = b->phaseWarps || (P && wide_phase(b->glist[b->cls[0].graphs[0]], P, b->cls[0].baseWarps, doubled_load(*b, b->cls[0])));
     }
     {
         uint64_t end = 0;

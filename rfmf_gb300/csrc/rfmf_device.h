@@ -124,6 +124,7 @@ struct DevLaunch {
     int32_t            pmax;            // group slots per chain: min(max P, max n)
     uint32_t           csrBytes;        // shared-memory CSR region (0 for kCsrGlobal)
     uint32_t           chainBytes;      // shared-memory bytes per chain
+    int32_t            slotsOnly;       // chains have no argmax scratch: every phase goes through the group slots
     int32_t*           queue;       // work-queue head (zeroed before the launch)
     int32_t*           error;       // first device error (DevError)
     int32_t*           errorItem;   // chain/item that raised it
@@ -161,7 +162,9 @@ struct ChainLayout {
 // for up to 128 partials of 8 bytes.
 constexpr uint32_t kWarpScratch = (144 + 128) * 4;
 
-RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, int dbytes) {
+// argmax: false for the int64 score path, which needs none, and for chains
+// that fit a CTA only without it.
+RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, int dbytes, bool argmax) {
     ChainLayout c;
     const uint32_t nPad = (static_cast<uint32_t>(maxN) + 7u) & ~7u;
     uint32_t o = 0;
@@ -169,7 +172,7 @@ RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, in
     c.bits = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.best = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.sb = o;    o = align16(o + nPad);
-    const uint32_t slots = static_cast<uint32_t>(pmax) * 8u, scratch = static_cast<uint32_t>(warps) * kWarpScratch;
+    const uint32_t slots = static_cast<uint32_t>(pmax) * 8u, scratch = argmax ? static_cast<uint32_t>(warps) * kWarpScratch : 0u;
     c.slots = o; o = align16(o + (slots > scratch ? slots : scratch));
     c.ids = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);
     c.win = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);

@@ -613,41 +613,38 @@ extern "C" int rfmf_graph_info(const rfmf_graph* g, int64_t* n, int64_t* m, int6
 }
 // ------------------------------------------------------------------ batch
 namespace rfmf {
-// Warps per chain: one unless a chain has enough vertex blocks to keep more
-// warps busy (about 384 blocks of 8 vertices per extra warp).
+// Warps per chain: one per ~768 vertex blocks (up to four), more while the
+// chains leave the SMs short of warps and the threads keep vertex blocks.
+// Chains alone fill an SM best; below that wider chains shorten the sweep, to
+// two warps while that makes at most 10 warps per SM (from 1024 vertices on),
+// to four up to 16, to
+// eight up to 8 (one chain per SM) on graphs of at least 6144 vertices and up
+// to 16 from 16384 on.  GB300, us per sweep summed over P = 128, 32, 8 and 1 at
+// 1 / 2 / 4 / 8 warps:
+//   ER n = 2000 d = 19   200 chains 10.1 / 8.9 / 7.8 / 8.6, 400 10.1 / 10.2 /
+//                        9.0 / 17, 700 12.3 / 11.9 / 17.7, 1024 12.4 / 13.6
+//   50x60 torus          400 chains 9.8 / 9.7 / 9.0, 700 12.5 / 11.7 / 17.7,
+//                        1024 12.5 / 13.6
+//   ER n = 800 d = 48    32 chains 10.9 / 9.8 / 7.4 / 7.1, 300 10.9 / 9.8 / 8.4
+//   ER n = 5000 d = 5    80 chains 14.3 / 10.5 / 8.3 / 7.6, 256 14.2 / 10.6 /
+//                        9.4 / 10.1, 600 14.2 / 12.9 / 12.8
+//   70x100 torus         80 chains 16.8 / 12.4 / 8.5 / 8.3, 300 16.8 / 12.4 /
+//                        10.3 / 11.1, 600 16.9 / 15.3 / 14.7
+//   100x200 torus        80 chains 46.8 / 27.5 / 16.4 / 13.7, 256 - / 27.6 /
+//                        20.8 / 19.2, 400 - / 35.4 / 25.7 / 38.1
+// (sixteen warps lost to eight everywhere.)
 int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms) {
     if (c.threads_per_chain) return c.threads_per_chain / 32;
     int W = 1;
     const int nblk = (maxN + 7) / 8;
-    // About 768 vertex blocks per warp.
     while (W < 4 && nblk >= 384 * 2 * W) W *= 2;
-    // Too few chains to fill the SMs: widen each chain while all chains stay
-    // within 8 warps per SM and the current width still has a vertex block
-    // per thread.  One warp per chain is the most efficient form once chains
-    // alone fill the SMs; below that, per-chain latency is what the extra
-    // warps buy (GB300, 256 chains of ER n = 2000: 67.5 -> 88.6 M
-    // chain-steps/s from one warp to four; 32 chains of ER n = 800: 6.7 -> 11.0).
-    const int sized = W;
-    while (W < kMaxAutoWarps && chains > 0 && chains * 2 * W <= int64_t(8) * sms && nblk >= 32 * W)
-        W *= 2;
-    // Two warps for latency alone lose to one on graphs of under 4096
-    // vertices (16 vertex blocks per lane) outside the phases heavy in
-    // winner rows, which a one-graph batch widens by itself (GB300, 512
-    // chains, us per sweep at one / two warps: ER n = 2000 d = 19 P = 128
-    // 9.10 / 6.84 but P = 8 2.37 / 3.15 and P = 1 1.98 / 2.23; the 50x60
-    // torus 4.11 / 4.10 at P = 128, 2.44 / 3.20 at P = 8); on larger ones
-    // two win at every phase (ER n = 5000 d = 5 P = 1 3.57 / 3.15, P = 16
-    // 4.43 / 4.24; 70x70 torus and random tree n = 5000 alike); four, where
-    // the chains are few enough, win at every phase (256 chains: ER n = 2000
-    // 4.65 / 9.10 at P = 128 and 1.89 / 1.98 at P = 1 for four / one).
-    if (sized == 1 && W == 2 && nblk < 512) W = 1;
-    // Past four warps only for large graphs, where each thread keeps at
-    // least four vertex blocks (GB300, 32-64 chains: torus n = 20000 +15% at
-    // P = 128 and +29% at P = 1 from four warps to eight, tree n = 10000 +2%
-    // / +10%; ER n = 5000 -1% / +5%, so it stays at four).
-    while (W >= kMaxAutoWarps && W < kMaxLatencyWarps && chains > 0 && chains * 2 * W <= int64_t(8) * sms &&
-           nblk >= 256 * W)
-        W *= 2;
+    if (chains <= 0) return W;
+    auto fits = [&](int wider, int warpsPerSm) {
+        return chains * wider <= static_cast<int64_t>(warpsPerSm) * sms && nblk >= 16 * wider;
+    };
+    if (W == 1 && (fits(4, 16) || (nblk >= 128 && fits(2, 10)))) W = 2;
+    if (W == 2 && fits(4, 16)) W = 4;
+    if (W == 4 && ((nblk >= 768 && fits(8, 8)) || (nblk >= 2048 && fits(8, 16)))) W = 8;
     return W;
 }
 

@@ -323,10 +323,10 @@ struct rfmf_graph {
     // warps an item puts on each of the SM's four schedulers,
     // sched_level), from the item timings of earlier launches (weight =
     // sweeps observed).  An item's chains run at the pace of its busiest
-    // scheduler: on GB300, 13 to 16 one-warp chains of the 50x60 torus take
-    // 4.53 us per sweep at P = 1 and 12 take 3.74; and two graphs' relative
-    // cost depends on P (at P = 128 a dense graph's row walks double its
-    // sweep; at P = 1 its vertex count decides).  They size the work items
+    // scheduler: on GB300, 13 to 16 one-warp chains of a graph take the same
+    // time per sweep and 12 less; and two graphs' relative cost depends on P
+    // (at P = 128 a dense graph's row walks double its sweep; at P = 1 its
+    // vertex count decides).  They size the work items
     // of later launches of the same plan; they never affect results.
     struct LearnedCost {
         double ns = 0.0, weight = 0.0;
@@ -334,8 +334,9 @@ struct rfmf_graph {
     mutable std::map<std::tuple<int, int, uint32_t, int>, LearnedCost> costs;
     // The item time per sweep at (plan, P, level): from the nearest P (in
     // log2 P) learned under the plan, at the nearest level learned there,
-    // scaled to `level` by (level + 3) / (learned level + 3) (measured
-    // level-4 / level-3 ratios 1.11 to 1.21); 0 when the plan has none.
+    // scaled to `level` by (level + 2) / (learned level + 2) (measured
+    // level-2 / level-4 ratios 0.65 to 0.68, level-1 / level-4 0.51 to 0.54);
+    // 0 when the plan has none.
     double cost(int warps, int fmt, uint32_t P, int level) const {
         const double lp = std::log2(static_cast<double>(P > 0 ? P : 1));
         double pd = 1e300;
@@ -354,20 +355,20 @@ struct rfmf_graph {
             const int L = std::get<3>(it->first);
             if (!bestL || std::abs(L - level) < std::abs(bestL - level)) { bestL = L; ns = it->second.ns; }
         }
-        return ns * (level + 3.0) / (bestL + 3.0);
+        return ns * (level + 2.0) / (bestL + 2.0);
     }
     // Before any timing: an estimate of the same quantity from the graph's
     // shape, fitted on GB300 to one-warp chains at 16 per SM (50x60 torus
-    // and ER n = 2000 d = 19, phases 128..1): 1.65 us + 1.03 ns per vertex +
-    // 3.5 ns per winner-row entry (min(P, n) rows of mean degree 2m/n), the
+    // and ER n = 2000 d = 19, phases 128..1): 1.49 us + 1.0 ns per vertex +
+    // 1.4 ns per winner-row entry (min(P, n) rows of mean degree 2m/n), the
     // vertex and entry terms spread over the chain's warps, scaled by level
-    // as above.  Within 7% of the measured sweep on both graphs at every P.
+    // as above.  Within 5% of the measured sweep on both graphs at every P.
     double model_cost(int warps, uint32_t P, int level) const {
         const double nn = static_cast<double>(n > 0 ? n : 1);
         const double rows = std::min(static_cast<double>(P > 0 ? P : 1), nn);
-        const double us = 1.65 + (1.03e-3 * nn + 3.5e-3 * rows * (2.0 * static_cast<double>(m) / nn)) /
+        const double us = 1.49 + (1.0e-3 * nn + 1.4e-3 * rows * (2.0 * static_cast<double>(m) / nn)) /
                                      static_cast<double>(warps > 0 ? warps : 1);
-        return 1e3 * us * (level + 3.0) / 7.0;
+        return 1e3 * us * (level + 2.0) / 6.0;
     }
     // Whether a cost was learned under the plan at phase P itself (any level).
     bool learned_at(int warps, int fmt, uint32_t P) const {
@@ -416,6 +417,14 @@ inline uint32_t csr_bytes(const rfmf_graph* g, int fmt) {
     if (fmt == kCsrUnit16) return g->rowBytes + g->u16Bytes;
     if (fmt == kCsrPacked32) return g->rowBytes + g->p32Bytes;
     return 0;
+}
+
+// The same with rows packed one after another.  A shared-memory format that a
+// caller asks for and that fits a CTA only without the padding is walked in
+// HBM instead of refused.
+inline int64_t packed_csr_bytes(const rfmf_graph* g, int fmt) {
+    if (csr_in_hbm(fmt)) return 0;
+    return ((4 * (g->n + 1) + 15) & ~int64_t(15)) + ((2 * g->m * (fmt == kCsrUnit16 ? 2 : 4) + 15) & ~int64_t(15));
 }
 
 // The entry array a launch of format `fmt` reads for graph g (the 8-byte

@@ -49,6 +49,8 @@
 namespace rfmf {
 int set_last_error(int code, const char* msg);
 int fail(int code, const char* fmt, ...);
+int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms);
+int key_bits(int64_t n, int T);
 const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream);
@@ -201,13 +203,18 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
         if (phases[p]) { total += iters[p]; maxP = std::max<uint64_t>(maxP, phases[p]); }
     }
 
-    // Launch plan: CSR walked in HBM (the caller's buffers), one warp per
-    // chain, int8 gains when B <= 127, compact int32 keys when the range
-    // allows (else the int64 score path), K chains per CTA from occupancy.
-    const int W = 1, T = 32;
+    // Launch plan: CSR walked in HBM (the caller's buffers), warps per chain
+    // by the planner's rule, int8 gains when B <= 127, compact int32 keys when
+    // the range allows (else the int64 score path), K chains per CTA from
+    // occupancy.  GB300, 150 chains of n = 3000, ms a call at one warp per
+    // chain / at the rule's four: 34.6 / 18.2.
+    int sms = 0, optin = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+        return nerr(RFMF_ERR_CUDA, "device attribute query failed");
+    int W = choose_warps(static_cast<int>(n), rfmf_launch_config{}, C, sms);
     const int dbytes = (max_weighted_deg <= 127) ? 1 : 4;
-    int kb = 4;
-    while ((int64_t(1) << kb) < ((n + 7) / 8 + T - 1) / T) ++kb;
+    const int kb = key_bits(n, 32 * W);
     bool s64 = false;
     for (int64_t c = 0; c < C && !s64; ++c) {
         const double bmax = std::round(std::log(1.0 + static_cast<double>(std::max<uint64_t>(total, 1))) /
@@ -218,18 +225,24 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     }
     const int words = static_cast<int>((n + 31) / 32);
     const int pmax = static_cast<int>(std::min<uint64_t>(maxP, static_cast<uint64_t>(n)));
-    const uint32_t chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes).total;
-    int sms = 0, optin = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
-        return nerr(RFMF_ERR_CUDA, "device attribute query failed");
+    // A wider chain keeps a few bytes more; the largest graphs fit at one warp
+    // only.
+    if (static_cast<int64_t>(optin) - kSmemHeader <
+        static_cast<int64_t>(chain_layout(static_cast<int>(n), words, pmax, W, dbytes, false).total))
+        W = 1;
     const void* kern = kernel_ptr(dbytes, kCsrGlobal, s64, W);
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return nerr(RFMF_ERR_CUDA, "kernel attributes");
     const int dynMax = optin - static_cast<int>(fa.sharedSizeBytes);
     const int64_t room = static_cast<int64_t>(dynMax) - kSmemHeader;
+    bool argmax = !s64;
+    uint32_t chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, argmax).total;
+    if (argmax && room < chainBytes) {   // the largest graphs fit without the argmax scratch only
+        argmax = false;
+        chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, argmax).total;
+    }
     const int Kmax = static_cast<int>(
-        std::min<int64_t>(std::min(16, fa.maxThreadsPerBlock / (32 * W)), room / chainBytes));
+        std::min<int64_t>(std::min(16 / W, fa.maxThreadsPerBlock / (32 * W)), room / chainBytes));
     if (Kmax < 1) return nerr(RFMF_ERR_CAPACITY, "chain state does not fit shared memory");
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dynMax) != cudaSuccess)
         return nerr(RFMF_ERR_CUDA, "kernel attribute");
@@ -334,6 +347,7 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     L.pmax = pmax;
     L.csrBytes = 0;
     L.chainBytes = chainBytes;
+    L.slotsOnly = argmax ? 0 : 1;
     L.queue = ctl;
     L.error = ctl + 1;
     L.errorItem = ctl + 2;

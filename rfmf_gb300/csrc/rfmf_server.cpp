@@ -411,9 +411,14 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kern));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
-        const uint32_t chainB = chain_layout(maxN, maxWords, pmax, k.W, k.dbytes).total;
+        bool argmax = !k.s64;
+        uint32_t chainB = chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, argmax).total;
         const int kCap = std::min(std::min(16 / k.W, k.W > 1 ? 15 : 16), fa.maxThreadsPerBlock / (32 * k.W));
         const int64_t room = dynMax - kSmemHeader - csrB;
+        if (argmax && room < chainB) {   // the largest graphs fit without the argmax scratch only
+            argmax = false;
+            chainB = chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, argmax).total;
+        }
         const int Kmax = room > 0 ? static_cast<int>(std::min<int64_t>(kCap, room / chainB)) : 0;
         if (Kmax < 1)
             return fail(RFMF_ERR_CAPACITY, "launch class needs %u B CSR + %u B per chain", csrB, chainB);
@@ -469,6 +474,7 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         L.pmax = pmax;
         L.csrBytes = csrB;
         L.chainBytes = chainB;
+        L.slotsOnly = argmax ? 0 : 1;
         L.queue = s->dCtl.as<int32_t>() + 4 * ci;
         L.error = L.queue + 1;
         L.errorItem = L.queue + 2;
@@ -827,15 +833,25 @@ static int rfmf_submit_impl(rfmf_server* s, const rfmf_graph* g, int64_t nchains
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kernel_ptr(r->dbytes, fmt, r->s64, r->W)));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
-        const uint32_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax,
-                                             r->W, r->dbytes).total;
+        auto chain_bytes = [&](bool argmax) {
+            return chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax, r->W, r->dbytes, argmax)
+                .total;
+        };
+        // (A wider chain keeps a few bytes more; the largest graphs fit at a
+        // narrower one only.)
+        while (c.threads_per_chain == 0 && r->W > 1 &&
+               static_cast<int64_t>(kSmemHeader) + chain_bytes(false) > dynMax)
+            r->W /= 2;
+        const uint32_t chainB = chain_bytes(!r->s64), leastB = chain_bytes(false);
         const int64_t kWant = std::min<int64_t>(nchains, std::max(1, 8 / r->W));
         if (!csr_in_hbm(fmt) && static_cast<int64_t>(kSmemHeader) + csr_bytes(g, fmt) + kWant * chainB > dynMax) {
-            if (c.csr_format != 0) return fail(RFMF_ERR_CAPACITY, "the shared-memory CSR does not fit");
+            if (c.csr_format != 0 &&
+                static_cast<int64_t>(kSmemHeader) + packed_csr_bytes(g, fmt) + kWant * leastB > dynMax)
+                return fail(RFMF_ERR_CAPACITY, "the shared-memory CSR does not fit");
             fmt = hbm_format(g);
         }
-        if (static_cast<int64_t>(kSmemHeader) + chainB > dynMax)
-            return fail(RFMF_ERR_CAPACITY, "one chain needs %u B of shared memory", chainB);
+        if (static_cast<int64_t>(kSmemHeader) + leastB > dynMax)
+            return fail(RFMF_ERR_CAPACITY, "one chain needs %u B of shared memory", leastB);
     }
     r->fmt = fmt;
     if (nchains * r->words > (int64_t(1) << 34)) return fail(RFMF_ERR_CAPACITY, "request too large");
