@@ -1149,10 +1149,9 @@ __device__ __forceinline__ void flip_vertex(const ChainSmem& s, int v, int32_t d
 // as 32-bit adds, whatever the bytes pass through on the way), so after the
 // gains are read there is one barrier, at the end.  With int32 gains a walk
 // reads its neighbours' new spins, so the flips are fenced off from the walks.
-template <bool kOne, class DP, int kFmt, class Loc>
-__device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
+template <bool kOne, int kRows, class DP, int kFmt, class Loc>
+__device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
                                          int grp, int32_t v[4]) {
-    constexpr int kRows = kOne ? 4 : 2;   // P <= 128 over at least 32 or 64 threads
     const int sub = t & ((1 << pc.laneShift) - 1);
     uint32_t lo[kRows], hi[kRows], neg[kRows];
     int32_t d[kRows];
@@ -1160,12 +1159,13 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
         lo[q] = hi[q] = neg[q] = 0;
-        if (q >= pc.rows) continue;
         const int r = (t >> pc.laneShift) + q * T;
         if constexpr (kOne) {
-            if (q == 0 && pc.laneShift) {
+            if (kRows == 1) {
                 v[0] = __shfl_sync(0xFFFFFFFFu, v[0], r);
                 if (r >= pc.P) v[0] = -1;
+            } else if (q >= pc.rows) {
+                v[q] = -1;
             }
         } else {
             unsigned long long p = 0;
@@ -1201,7 +1201,7 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
     if (kOne || !DP::kField) __syncwarp();
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
-        if (q < pc.rows && v[q] >= 0 && sub == 0) {
+        if (v[q] >= 0 && sub == 0) {
             if constexpr (DP::kField) {
                 // q' = q - 1 (+1 -> -1) or q + 1: an add, as a neighbour's
                 // walk may be adding to this byte.
@@ -1214,19 +1214,30 @@ __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr,
         }
     }
     if (!DP::kField) group_sync(grp, T);
-    if (pc.rows == 1) {
+    if constexpr (kRows == 1) {
         scatter_row<DP, kFmt>(s, csr, lo[0], hi[0], neg[0], sub, 1 << pc.laneShift);
     } else {
 #pragma unroll
-        for (int q = 0; q < kRows; q += 2)
-            if (q < pc.rows) scatter_two<DP, kFmt>(s, csr, lo + q, hi + q, neg + q);
+        for (int q = 0; q < kRows; q += 2) scatter_two<DP, kFmt>(s, csr, lo + q, hi + q, neg + q);
     }
     group_sync(grp, T);
+    if (kRows == 1 && pc.P == 1) return 2 * loc;   // a lone winner's gain just changes sign
 #pragma unroll
     for (int q = 0; q < kRows; ++q)
-        if (q < pc.rows && v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
+        if (v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
     return loc;
 }
+
+// P <= 128 over at least 32 (one-warp chains) or 64 threads: one to four rows,
+// or one or two, a thread.
+template <bool kOne, class DP, int kFmt, class Loc>
+__device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
+                                         int grp, int32_t v[4]) {
+    if (pc.rows == 1) return flip_rows<kOne, 1, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+    if (!kOne || pc.rows == 2) return flip_rows<kOne, 2, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+    return flip_rows<kOne, 4, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+}
+
 
 // FLIP of winners in the group slots (other paths, int64 scores; a barrier
 // since SELECT's atomics has passed): publish and flip them, walk the rows,
@@ -1437,8 +1448,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     // SELECT, and wider chains pass the warps' sums through s.red under
     // SELECT's own barrier instead of one more.
     Loc loc = 0;
-    auto settle = [&](uint64_t sw) {
-        if (sw == s0) return;
+    auto settle = [&]() {
         Loc gain;
         if constexpr (kOne) gain = warp_sum(loc);
         else gain = warp_sum(static_cast<Loc>((t & 31) < (T >> 5) ? s.red[t & 31] : 0));
@@ -1450,6 +1460,8 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             group_sync(grp, T);
         }
     };
+    group_sync(grp, T);   // s.red is read
+    if (t < (T >> 5)) s.red[t] = 0;
     group_sync(grp, T);
 
     uint64_t sw = s0;
@@ -1487,15 +1499,19 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         uint32_t left = kPaceEvery - paced;
         if (phaseEnd > sw && phaseEnd - sw < left) left = static_cast<uint32_t>(phaseEnd - sw);
         if (s1 - sw < left) left = static_cast<uint32_t>(s1 - sw);
+        // The sweep of them at which the beta run changes, if any does (runs
+        // are never empty: one step of the cursor per sweep).
+        auto turn_in = [&]() { return betaNext - sw < kPaceEvery ? static_cast<uint32_t>(betaNext - sw) : ~0u; };
+        uint32_t toTurn = sw >= betaNext ? 0u : turn_in();
         do {
-            bool turn = false;
-            if (sw >= betaNext) {
-                // Runs are never empty, so one step of the cursor per sweep.
+            const bool turn = toTurn == 0;
+            if (turn) {
                 ++run;
                 betaNext = nextEnd;
                 beta = nextVal;
-                turn = true;
+                toTurn = turn_in();
             }
+            --toTurn;
             int32_t v[4];
             if constexpr (kS64) select64<DP>(s, lut, n, pc, beta, sc, keys, t, T, grp);
             else select32<kOne, DP>(s, lut, kc, n, pc, beta, sc, keys, t, T, v);
@@ -1512,7 +1528,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             }
             const bool slots = kS64 || pc.path != kPathWarp;
             if (!kOne || slots) group_sync(grp, T);
-            settle(sw - 1);
+            settle();
             if (slots) loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
             else loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
             if (!kOne) {
@@ -1522,7 +1538,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         } while (--left);
     }
     if (!kOne) group_sync(grp, T);
-    settle(s1);
+    settle();
     if (t == 0) prog[grp] = INT_MAX;
     group_sync(grp, T);
 

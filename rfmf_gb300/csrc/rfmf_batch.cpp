@@ -674,113 +674,121 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     using Key = std::tuple<int, int, int, int>;   // dbytes, fmt, W, s64
     std::map<Key, int> classOf;
     std::vector<int> graphClass(G);
-    for (size_t gi = 0; gi < G; ++gi) {
-        const rfmf_graph* g = b->glist[gi];
-        const int dbytes = c.gain_width ? c.gain_width : (g->B <= 127 ? 1 : 4);
-        if (dbytes == 1 && g->B > 127)
-            return fail(RFMF_ERR_INVALID, "int8 gains need max weighted degree <= 127 (B=%lld)", (long long)g->B);
-        const int pmaxG = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(maxP, static_cast<uint64_t>(g->n))));
-        const int64_t perSm = (b->C + ctx->sms - 1) / std::max(ctx->sms, 1);
-        // Kernel variant, CSR format and chains resident per SM of this graph
-        // at Wc warps per chain.
-        struct Pick {
-            bool s64 = false;
-            int fmt = kCsrGlobal;
-            int64_t resident = 0;
-        };
-        auto pick = [&](int Wc, Pick& pk) -> int {
-            pk = Pick{};
-            pk.s64 = (c.score_path == 2);
-            if (!pk.s64) {
-                for (int32_t ch : chainsOfGraph[gi])
-                    if (!compact_key_safe(static_cast<int64_t>(total), t0s[ch], g->B, key_bits(g->n, 32 * Wc))) {
-                        pk.s64 = true;
-                        break;
-                    }
-                if (pk.s64 && c.score_path == 1)
-                    return fail(RFMF_ERR_INVALID, "int32 scores would overflow for this (t0, B, sweeps)");
-            }
-            const int64_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>((g->n + 31) / 32), pmaxG,
-                                                Wc, dbytes, !pk.s64).total;
-            // A shared-memory CSR pays only while it leaves room for the chains
-            // a CTA should hold: about 8 warps, fewer when the graph has fewer
-            // chains or the batch fewer than that per SM.  Otherwise its rows
-            // are walked in HBM (L2-resident) and the CTA holds more chains.
-            const int64_t kWant = std::max<int64_t>(
-                1, std::min<int64_t>({static_cast<int64_t>(chainsOfGraph[gi].size()),
-                                      static_cast<int64_t>(std::max(1, 8 / Wc)), perSm}));
-            auto fits = [&](int f) {
-                cudaFuncAttributes fa{};
-                const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, f, pk.s64, Wc), fa);
-                return dynMax > 0 &&
-                       static_cast<int64_t>(kSmemHeader) + csr_bytes(g, f) + kWant * chainB <= dynMax;
+    // hbm: every graph's rows are walked in HBM; width: warps per chain of all
+    // graphs (0: the rule for each).
+    auto classify = [&](bool hbm, int width) -> int {
+        classOf.clear();
+        b->cls.clear();
+        for (size_t gi = 0; gi < G; ++gi) {
+            const rfmf_graph* g = b->glist[gi];
+            const int dbytes = c.gain_width ? c.gain_width : (g->B <= 127 ? 1 : 4);
+            if (dbytes == 1 && g->B > 127)
+                return fail(RFMF_ERR_INVALID, "int8 gains need max weighted degree <= 127 (B=%lld)", (long long)g->B);
+            const int pmaxG = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(maxP, static_cast<uint64_t>(g->n))));
+            const int64_t perSm = (b->C + ctx->sms - 1) / std::max(ctx->sms, 1);
+            // Kernel variant, CSR format and chains resident per SM of this graph
+            // at Wc warps per chain.
+            struct Pick {
+                bool s64 = false;
+                int fmt = kCsrGlobal;
+                int64_t resident = 0;
             };
-            if (c.csr_format == 1) {
-                if (!g->unit16) return fail(RFMF_ERR_INVALID, "unit16 CSR needs |w| == 1 and n <= 32768");
-                pk.fmt = kCsrUnit16;
-            } else if (c.csr_format == 2) {
-                if (!g->packed32) return fail(RFMF_ERR_INVALID, "packed32 CSR needs |w| < 2^15 and n <= 65536");
-                pk.fmt = kCsrPacked32;
-            } else if (c.csr_format == 0) {
-                if (g->unit16 && fits(kCsrUnit16)) pk.fmt = kCsrUnit16;
-                else if (g->packed32 && fits(kCsrPacked32)) pk.fmt = kCsrPacked32;
+            auto pick = [&](int Wc, Pick& pk) -> int {
+                pk = Pick{};
+                pk.s64 = (c.score_path == 2);
+                if (!pk.s64) {
+                    for (int32_t ch : chainsOfGraph[gi])
+                        if (!compact_key_safe(static_cast<int64_t>(total), t0s[ch], g->B, key_bits(g->n, 32 * Wc))) {
+                            pk.s64 = true;
+                            break;
+                        }
+                    if (pk.s64 && c.score_path == 1)
+                        return fail(RFMF_ERR_INVALID, "int32 scores would overflow for this (t0, B, sweeps)");
+                }
+                const int64_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>((g->n + 31) / 32), pmaxG,
+                                                    Wc, dbytes, !pk.s64).total;
+                // A shared-memory CSR pays only while it leaves room for the chains
+                // a CTA should hold: about 8 warps, fewer when the graph has fewer
+                // chains or the batch fewer than that per SM.  Otherwise its rows
+                // are walked in HBM (L2-resident) and the CTA holds more chains.
+                const int64_t kWant = std::max<int64_t>(
+                    1, std::min<int64_t>({static_cast<int64_t>(chainsOfGraph[gi].size()),
+                                          static_cast<int64_t>(std::max(1, 8 / Wc)), perSm}));
+                auto fits = [&](int f) {
+                    cudaFuncAttributes fa{};
+                    const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, f, pk.s64, Wc), fa);
+                    return dynMax > 0 &&
+                           static_cast<int64_t>(kSmemHeader) + csr_bytes(g, f) + kWant * chainB <= dynMax;
+                };
+                if (c.csr_format == 1) {
+                    if (!g->unit16) return fail(RFMF_ERR_INVALID, "unit16 CSR needs |w| == 1 and n <= 32768");
+                    pk.fmt = kCsrUnit16;
+                } else if (c.csr_format == 2) {
+                    if (!g->packed32) return fail(RFMF_ERR_INVALID, "packed32 CSR needs |w| < 2^15 and n <= 65536");
+                    pk.fmt = kCsrPacked32;
+                } else if (c.csr_format == 0 && !hbm) {
+                    if (g->unit16 && fits(kCsrUnit16)) pk.fmt = kCsrUnit16;
+                    else if (g->packed32 && fits(kCsrPacked32)) pk.fmt = kCsrPacked32;
+                }
+                // Walked in HBM: the most compact entries the graph has, unless
+                // the 8-byte pairs are asked for.
+                if (pk.fmt == kCsrGlobal && c.csr_format != 4) pk.fmt = hbm_format(g);
+                cudaFuncAttributes fa{};
+                const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, pk.fmt, pk.s64, Wc), fa);
+                const int64_t room = dynMax - static_cast<int64_t>(kSmemHeader) -
+                                     (csr_in_hbm(pk.fmt) ? 0 : static_cast<int64_t>(csr_bytes(g, pk.fmt)));
+                const int64_t warpCap = std::min(16 / Wc, Wc > 1 ? 15 : 16);
+                pk.resident = std::max<int64_t>(0, std::min<int64_t>({perSm, warpCap, room / chainB}));
+                return RFMF_OK;
+            };
+            int W = width ? width : choose_warps(static_cast<int>(g->n), c, b->C, ctx->sms);
+            Pick pk;
+            if (int rc = pick(W, pk)) return rc;
+            // When shared memory (not the chain count) keeps an SM's chains from
+            // all being resident, wider chains fill the idle warp slots: widen
+            // while that raises the warps resident per SM (GB300, 2432 chains:
+            // ER n = 5000 d = 5 169 -> 216 M chain-steps/s at two warps, random
+            // tree n = 10000 106 -> 112 at four).  Only within about two waves of
+            // one-warp chains per SM: deeper queues keep every warp slot busy
+            // anyway and one warp per chain does more per slot (512 graphs x 64
+            // chains: 1.52e8 -> 1.44e8 when widened).
+            if (c.threads_per_chain == 0 && width == 0 && perSm <= 32) {
+                while (W < kMaxAutoWarps && pk.resident < perSm) {
+                    Pick wider;
+                    if (int rc = pick(2 * W, wider)) return rc;
+                    if (2 * W * wider.resident <= W * pk.resident) break;
+                    W *= 2;
+                    pk = wider;
+                }
             }
-            // Walked in HBM: the most compact entries the graph has, unless
-            // the 8-byte pairs are asked for.
-            if (pk.fmt == kCsrGlobal && c.csr_format != 4) pk.fmt = hbm_format(g);
-            cudaFuncAttributes fa{};
-            const int64_t dynMax = dyn_smem_max(ctx, kernel_ptr(dbytes, pk.fmt, pk.s64, Wc), fa);
-            const int64_t room = dynMax - static_cast<int64_t>(kSmemHeader) -
-                                 (csr_in_hbm(pk.fmt) ? 0 : static_cast<int64_t>(csr_bytes(g, pk.fmt)));
-            const int64_t warpCap = std::min(16 / Wc, Wc > 1 ? 15 : 16);
-            pk.resident = std::max<int64_t>(0, std::min<int64_t>({perSm, warpCap, room / chainB}));
-            return RFMF_OK;
-        };
-        int W = choose_warps(static_cast<int>(g->n), c, b->C, ctx->sms);
-        Pick pk;
-        if (int rc = pick(W, pk)) return rc;
-        // When shared memory (not the chain count) keeps an SM's chains from
-        // all being resident, wider chains fill the idle warp slots: widen
-        // while that raises the warps resident per SM (GB300, 2432 chains:
-        // ER n = 5000 d = 5 169 -> 216 M chain-steps/s at two warps, random
-        // tree n = 10000 106 -> 112 at four).  Only within about two waves of
-        // one-warp chains per SM: deeper queues keep every warp slot busy
-        // anyway and one warp per chain does more per slot (512 graphs x 64
-        // chains: 1.52e8 -> 1.44e8 when widened).
-        if (c.threads_per_chain == 0 && perSm <= 32) {
-            while (W < kMaxAutoWarps && pk.resident < perSm) {
-                Pick wider;
-                if (int rc = pick(2 * W, wider)) return rc;
-                if (2 * W * wider.resident <= W * pk.resident) break;
-                W *= 2;
-                pk = wider;
+            const bool s64 = pk.s64;
+            const int fmt = pk.fmt;
+            const Key key{dbytes, fmt, W, s64 ? 1 : 0};
+            auto it = classOf.find(key);
+            if (it == classOf.end()) {
+                it = classOf.emplace(key, static_cast<int>(b->cls.size())).first;
+                b->cls.emplace_back();
+                BatchClass& k = b->cls.back();
+                k.dbytes = dbytes;
+                k.fmt = fmt;
+                k.warps = W;
+                k.score64 = s64;
+                k.pmax = static_cast<int>(std::max<uint64_t>(1, maxP));
             }
+            graphClass[gi] = it->second;
+            BatchClass& k = b->cls[it->second];
+            k.graphs.push_back(static_cast<int>(gi));
+            k.chainsOf.push_back(chainsOfGraph[gi]);
         }
-        const bool s64 = pk.s64;
-        const int fmt = pk.fmt;
-        const Key key{dbytes, fmt, W, s64 ? 1 : 0};
-        auto it = classOf.find(key);
-        if (it == classOf.end()) {
-            it = classOf.emplace(key, static_cast<int>(b->cls.size())).first;
-            b->cls.emplace_back();
-            BatchClass& k = b->cls.back();
-            k.dbytes = dbytes;
-            k.fmt = fmt;
-            k.warps = W;
-            k.score64 = s64;
-            k.pmax = static_cast<int>(std::max<uint64_t>(1, maxP));
-        }
-        graphClass[gi] = it->second;
-        BatchClass& k = b->cls[it->second];
-        k.graphs.push_back(static_cast<int>(gi));
-        k.chainsOf.push_back(chainsOfGraph[gi]);
-    }
+        return RFMF_OK;
+    };
+    if (int rc = classify(false, 0)) return rc;
     // A shared-memory class's CTA holds the class's largest CSR beside K
     // chains sized for its largest graph.  While that leaves room for fewer
     // chains than a CTA should hold (as above, over the class), the graph
     // demanding the most moves to the HBM class of the same key, so that a
     // few large graphs do not shrink every CTA of the class.
-    if (c.csr_format == 0) {
+    auto spread = [&]() {
         const int64_t perSm = (b->C + ctx->sms - 1) / std::max(ctx->sms, 1);
         for (size_t ci = 0; ci < b->cls.size(); ++ci) {
             if (csr_in_hbm(b->cls[ci].fmt)) continue;
@@ -846,6 +854,32 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         }
         b->cls = std::move(kept);
         for (size_t gi = 0; gi < G; ++gi) graphClass[gi] = remap[graphClass[gi]];
+    };
+    if (c.csr_format == 0) spread();
+    // Several classes share the SMs, each sized as if alone: their CSR copies
+    // crowd the chains out of shared memory.  Up to two chains per SM, and from
+    // sixteen on, such a batch walks every graph's rows in HBM instead; between
+    // two and five per SM, at four warps per chain for all, so that (but for
+    // gain widths) it is one class whose items the work queue levels.  Only
+    // with graphs whose copies are large (4096 vertices).  GB300, ms for 1,200
+    // sweeps, before / this: 16 graphs n 807..14,000 x 4 chains 3.4 / 3.5, x 16
+    // 5.1 / 4.1, x 48 10.3 / 7.2, x 160 19.8 / 15.5, x 300 26.8 / 23.7; three
+    // sparse graphs x 64 4.9 / 4.2, x 256 13.7 / 9.7; four graphs n 11,000 to
+    // 17,000 x 200 14.1 / 12.6; 64 graphs x 64 18.5 / 15.1 (between five and
+    // sixteen per SM neither form is always ahead: 64 graphs x 16 7.9 / 8.8, 16
+    // graphs x 96 12.9 / 11.9).
+    if (b->cls.size() > 1 && c.csr_format == 0 && c.threads_per_chain == 0) {
+        int64_t maxN = 0;
+        for (const rfmf_graph* g : b->glist) maxN = std::max(maxN, g->n);
+        const int64_t sms = std::max(ctx->sms, 1);
+        const bool few = b->C <= 2 * sms, some = 4 * b->C <= 21 * sms, many = b->C >= 16 * sms;
+        if (maxN >= 4096 && (few || some || many)) {
+            if (classify(true, !few && some ? kMaxAutoWarps : 0) != RFMF_OK) {
+                // int32 scores asked for that this width has no room for
+                if (int rc = classify(false, 0)) return rc;
+                spread();
+            }
+        }
     }
     const bool exact = b->cls.size() > 1;
     for (BatchClass& k : b->cls) {
