@@ -396,7 +396,7 @@ struct ChainSmem {
 
 __device__ __forceinline__ ChainSmem carve_chain(unsigned char* base, const DevLaunch& L,
                                                  int dbytes) {
-    const ChainLayout c = chain_layout(L.maxN, L.maxWords, L.pmax, L.warpsPerChain, dbytes, !L.slotsOnly);
+    const ChainLayout c = chain_layout(L.maxN, L.maxWords, L.pmax, L.warpsPerChain, dbytes, L.layout);
     ChainSmem s;
     s.D = base + c.d;
     s.bits = reinterpret_cast<uint32_t*>(base + c.bits);
@@ -1339,9 +1339,11 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         s.bits[w] = sb;
         s.best[w] = fresh ? sb : ch.bestBits[w];
     }
-    for (int i = t; i < L.pmax; i += T) {
-        s.slots[i] = kS64 ? static_cast<unsigned long long>(LLONG_MIN) : 0ull;
-        s.ids[i] = INT32_MAX;
+    if (L.layout != kLayoutMain) {
+        for (int i = t; i < L.pmax; i += T) {
+            s.slots[i] = kS64 ? static_cast<unsigned long long>(LLONG_MIN) : 0ull;
+            s.ids[i] = INT32_MAX;
+        }
     }
     group_sync(grp, T);
     const int nPad = (n + 7) & ~7;
@@ -1416,9 +1418,18 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     }
     // The last beta run holds the schedule's largest beta.
     const int kbMax = kS64 ? 31 : uniform(key_room(__ldg(ch.betaVal + ch.betaRuns - 1), g.B));
-    const bool slotsOnly = kS64 || L.slotsOnly;
+    const bool slotsOnly = kS64 || L.layout == kLayoutSlots;
+    const bool table = L.layout != kLayoutMain;
     PhaseCfg pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
     KeyCfg kc = key_cfg(n, pc.S, t, lut);
+    if (!table && (pc.path != kPathWarp || pc.step != 0)) {
+        // The host plans a table for every schedule that needs one.
+        if (t == 0) {
+            raise_error(L, kDevBadItem, ci);
+            prog[grp] = INT_MAX;
+        }
+        return;
+    }
 
     const ChainKeys keys = make_keys(ch.solverSeed);
     // Beta cursor: the current run and the next one as uniform values, the one
@@ -1478,6 +1489,10 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             const bool warp = pc.path == kPathWarp;
             pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
             kc = key_cfg(n, pc.S, t, lut);
+            if (!table && (pc.path != kPathWarp || pc.step != 0)) {
+                if (t == 0) raise_error(L, kDevBadItem, ci);
+                break;
+            }
             if (warp && pc.path != kPathWarp) {
                 // The slots held scratch and partials: empty them (all their
                 // readers are past the last sweep's barrier).

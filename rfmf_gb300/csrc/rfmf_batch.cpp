@@ -55,6 +55,7 @@ struct BatchClass {
     std::vector<int> Kg;                          // per class graph: chains per item
     std::vector<DevItem> items;
     std::vector<int32_t> order;
+    bool table = false;          // phases may leave the main path (kLayoutAny)
     bool balanced = false;       // items sized from graph costs (learned or modelled)
     uint64_t pendingSweeps = 0;  // sweeps of the last launch, whose item times are unread
     uint32_t pendingP = 0;       // its phase P (0: it spanned several phases)
@@ -126,17 +127,21 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
     cudaFuncAttributes fa{};
     const int64_t dynMax = dyn_smem_max(b.ctx, kern, fa);
     if (dynMax < 0) return fail(RFMF_ERR_CUDA, "kernel attributes unavailable");
-    bool argmax = !k.score64;
-    uint32_t chainB = chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes, argmax).total;
+    int layout = k.score64 ? kLayoutSlots : kLayoutMain;
+    for (int gi : k.graphs)
+        for (uint32_t P : b.phaseP)
+            if (layout == kLayoutMain && (k.table || !main_phase(P, static_cast<int>(b.glist[gi]->n)))) layout = kLayoutAny;
+    auto chain_bytes = [&](int kind) { return chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes, kind).total; };
+    uint32_t chainB = chain_bytes(layout);
     // Warp groups per CTA: named barriers 1..15, and the variant's register
     // budget bounds the CTA's threads.
     const int W = k.warps;
     const int kCap = std::min(std::min(16 / W, W > 1 ? 15 : 16), fa.maxThreadsPerBlock / (32 * W));
     if (kCap < 1) return fail(RFMF_ERR_CAPACITY, "a %d-thread chain exceeds the kernel's CTA limit", 32 * W);
     const int64_t room = dynMax - kSmemHeader - csrB;
-    if (argmax && room < chainB) {   // the largest graphs fit without the argmax scratch only
-        argmax = false;
-        chainB = chain_layout(maxN, maxWords, k.pmax, k.warps, k.dbytes, argmax).total;
+    if (room < chainB && chain_bytes(kLayoutSlots) < chainB) {   // the largest graphs fit without scratch only
+        layout = kLayoutSlots;
+        chainB = chain_bytes(layout);
     }
     int Kmax = room > 0 ? static_cast<int>(std::min<int64_t>(kCap, room / chainB)) : 0;
     if (c.chains_per_cta) {
@@ -195,7 +200,7 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
     k.L.pmax = k.pmax;
     k.L.csrBytes = csrB;
     k.L.chainBytes = chainB;
-    k.L.slotsOnly = argmax ? 0 : 1;
+    k.L.layout = layout;
     return RFMF_OK;
 }
 
@@ -211,7 +216,7 @@ bool fits_packed(const rfmf_batch& b, const BatchClass& k) {
     const int64_t dynMax = dyn_smem_max(b.ctx, kernel_ptr(k.dbytes, k.fmt, k.score64, k.warps), fa);
     const int n = static_cast<int>(maxN);
     return dynMax - kSmemHeader - csr >=
-           static_cast<int64_t>(chain_layout(n, (n + 31) / 32, k.pmax, k.warps, k.dbytes, false).total);
+           static_cast<int64_t>(chain_layout(n, (n + 31) / 32, k.pmax, k.warps, k.dbytes, kLayoutSlots).total);
 }
 
 // Per-graph chains per item: graph q may use item sizes cand[q] (chain
@@ -686,6 +691,9 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 return fail(RFMF_ERR_INVALID, "int8 gains need max weighted degree <= 127 (B=%lld)", (long long)g->B);
             const int pmaxG = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(maxP, static_cast<uint64_t>(g->n))));
             const int64_t perSm = (b->C + ctx->sms - 1) / std::max(ctx->sms, 1);
+            int kind = kLayoutMain;
+            for (uint32_t P : b->phaseP)
+                if (!main_phase(P, static_cast<int>(g->n))) kind = kLayoutAny;
             // Kernel variant, CSR format and chains resident per SM of this graph
             // at Wc warps per chain.
             struct Pick {
@@ -706,7 +714,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                         return fail(RFMF_ERR_INVALID, "int32 scores would overflow for this (t0, B, sweeps)");
                 }
                 const int64_t chainB = chain_layout(static_cast<int>(g->n), static_cast<int>((g->n + 31) / 32), pmaxG,
-                                                    Wc, dbytes, !pk.s64).total;
+                                                    Wc, dbytes, pk.s64 ? kLayoutSlots : kind).total;
                 // A shared-memory CSR pays only while it leaves room for the chains
                 // a CTA should hold: about 8 warps, fewer when the graph has fewer
                 // chains or the batch fewer than that per SM.  Otherwise its rows
@@ -797,11 +805,15 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 dyn_smem_max(ctx, kernel_ptr(b->cls[ci].dbytes, b->cls[ci].fmt, b->cls[ci].score64, b->cls[ci].warps), fa);
             while (!b->cls[ci].graphs.empty()) {
                 BatchClass& k = b->cls[ci];
+                int kind = k.score64 ? kLayoutSlots : kLayoutMain;
+                for (int gi : k.graphs)
+                    for (uint32_t P : b->phaseP)
+                        if (kind == kLayoutMain && !main_phase(P, static_cast<int>(b->glist[gi]->n))) kind = kLayoutAny;
                 auto chainOf = [&](int64_t n) {
                     const int ni = static_cast<int>(n);
                     return static_cast<int64_t>(
-                        chain_layout(ni, (ni + 31) / 32, std::max(1, std::min(k.pmax, ni)), k.warps, k.dbytes,
-                                     !k.score64).total);
+                        chain_layout(ni, (ni + 31) / 32, std::max(1, std::min(k.pmax, ni)), k.warps, k.dbytes, kind)
+                            .total);
                 };
                 int64_t maxN = 0, maxCsr = 0, maxCh = 0;
                 for (size_t q = 0; q < k.graphs.size(); ++q) {
@@ -894,6 +906,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             // A wider chain keeps a few bytes more; the largest graphs fit at
             // a narrower one only.
             k.warps /= 2;
+            k.table = true;   // the narrower chain's keys may lack room
             rc = plan_class(*b, k, c, exact);
         }
         if (rc) return rc;

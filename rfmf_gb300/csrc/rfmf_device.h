@@ -124,7 +124,7 @@ struct DevLaunch {
     int32_t            pmax;            // group slots per chain: min(max P, max n)
     uint32_t           csrBytes;        // shared-memory CSR region (0 for kCsrGlobal)
     uint32_t           chainBytes;      // shared-memory bytes per chain
-    int32_t            slotsOnly;       // chains have no argmax scratch: every phase goes through the group slots
+    int32_t            layout;          // which per-chain arrays there are (LayoutKind)
     int32_t*           queue;       // work-queue head (zeroed before the launch)
     int32_t*           error;       // first device error (DevError)
     int32_t*           errorItem;   // chain/item that raised it
@@ -162,9 +162,23 @@ struct ChainLayout {
 // for up to 128 partials of 8 bytes.
 constexpr uint32_t kWarpScratch = (144 + 128) * 4;
 
-// argmax: false for the int64 score path, which needs none, and for chains
-// that fit a CTA only without it.
-RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, int dbytes, bool argmax) {
+// What a chain's region holds besides its state.  The group table (slots
+// aside: ids and winners) serves the phases off the kernel's main path; the
+// argmax scratch the int32 score path.
+enum LayoutKind : int32_t {
+    kLayoutMain = 0,    // scratch only: every phase has 256 % P == 0, P <= 128
+    kLayoutAny = 1,     // scratch and table
+    kLayoutSlots = 2,   // table only: int64 scores, and chains that fit a CTA only so;
+                        // every phase goes through the group slots
+};
+
+// Whether a phase of P groups (clamped to n) runs on the main path.
+RFMF_HD bool main_phase(uint32_t P, int n) {
+    const uint32_t p = P < static_cast<uint32_t>(n) ? P : static_cast<uint32_t>(n);
+    return p == 0 || (p <= 128 && 256 % p == 0);
+}
+
+RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, int dbytes, int kind) {
     ChainLayout c;
     const uint32_t nPad = (static_cast<uint32_t>(maxN) + 7u) & ~7u;
     uint32_t o = 0;
@@ -172,10 +186,11 @@ RFMF_HD ChainLayout chain_layout(int maxN, int maxWords, int pmax, int warps, in
     c.bits = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.best = o;  o = align16(o + static_cast<uint32_t>(maxWords) * 4u);
     c.sb = o;    o = align16(o + nPad);
-    const uint32_t slots = static_cast<uint32_t>(pmax) * 8u, scratch = argmax ? static_cast<uint32_t>(warps) * kWarpScratch : 0u;
+    const uint32_t scratch = kind == kLayoutSlots ? 0u : static_cast<uint32_t>(warps) * kWarpScratch;
+    const uint32_t groups = kind == kLayoutMain ? 0u : static_cast<uint32_t>(pmax), slots = groups * 8u;
     c.slots = o; o = align16(o + (slots > scratch ? slots : scratch));
-    c.ids = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);
-    c.win = o;   o = align16(o + static_cast<uint32_t>(pmax) * 4u);
+    c.ids = o;   o = align16(o + groups * 4u);
+    c.win = o;   o = align16(o + groups * 4u);
     c.red = o;   o = align16(o + static_cast<uint32_t>(warps) * 8u);
     c.total = o;
     return c;

@@ -228,18 +228,20 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     // A wider chain keeps a few bytes more; the largest graphs fit at one warp
     // only.
     if (static_cast<int64_t>(optin) - kSmemHeader <
-        static_cast<int64_t>(chain_layout(static_cast<int>(n), words, pmax, W, dbytes, false).total))
+        static_cast<int64_t>(chain_layout(static_cast<int>(n), words, pmax, W, dbytes, kLayoutSlots).total))
         W = 1;
     const void* kern = kernel_ptr(dbytes, kCsrGlobal, s64, W);
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return nerr(RFMF_ERR_CUDA, "kernel attributes");
     const int dynMax = optin - static_cast<int>(fa.sharedSizeBytes);
     const int64_t room = static_cast<int64_t>(dynMax) - kSmemHeader;
-    bool argmax = !s64;
-    uint32_t chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, argmax).total;
-    if (argmax && room < chainBytes) {   // the largest graphs fit without the argmax scratch only
-        argmax = false;
-        chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, argmax).total;
+    // (With the group table for any schedule: the keys' room follows the
+    // caller's own beta table.)
+    int layout = s64 ? kLayoutSlots : kLayoutAny;
+    uint32_t chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, layout).total;
+    if (room < chainBytes) {   // the largest graphs fit without the argmax scratch only
+        layout = kLayoutSlots;
+        chainBytes = chain_layout(static_cast<int>(n), words, pmax, W, dbytes, layout).total;
     }
     const int Kmax = static_cast<int>(
         std::min<int64_t>(std::min(16 / W, fa.maxThreadsPerBlock / (32 * W)), room / chainBytes));
@@ -347,7 +349,7 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     L.pmax = pmax;
     L.csrBytes = 0;
     L.chainBytes = chainBytes;
-    L.slotsOnly = argmax ? 0 : 1;
+    L.layout = layout;
     L.queue = ctl;
     L.error = ctl + 1;
     L.errorItem = ctl + 2;

@@ -47,6 +47,7 @@ struct Request {
     std::vector<uint64_t> phaseIters;
     uint64_t total = 0;
     int pmax = 1;
+    bool table = false;   // a phase may leave the kernel's main path (kLayoutAny)
     std::vector<uint32_t> initBits;   // C * words
     ChainBeta beta;                   // the context's shared device beta tables
     // launch class
@@ -399,11 +400,13 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         const ClassKey& k = kv.first;
         std::vector<Request*>& reqs = kv.second;
         int maxN = 0, maxWords = 0, pmax = 1;
+        int layout = k.s64 ? kLayoutSlots : kLayoutMain;
         uint32_t csrB = 0;
         for (Request* r : reqs) {
             maxN = std::max<int>(maxN, static_cast<int>(r->n));
             maxWords = std::max<int>(maxWords, static_cast<int>(r->words));
             pmax = std::max(pmax, r->pmax);
+            if (r->table && layout == kLayoutMain) layout = kLayoutAny;
             csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
         }
         const void* kern = kernel_ptr(k.dbytes, k.fmt, k.s64, k.W);
@@ -411,13 +414,13 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kern));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
-        bool argmax = !k.s64;
-        uint32_t chainB = chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, argmax).total;
+        auto chain_bytes = [&](int kind) { return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total; };
+        uint32_t chainB = chain_bytes(layout);
         const int kCap = std::min(std::min(16 / k.W, k.W > 1 ? 15 : 16), fa.maxThreadsPerBlock / (32 * k.W));
         const int64_t room = dynMax - kSmemHeader - csrB;
-        if (argmax && room < chainB) {   // the largest graphs fit without the argmax scratch only
-            argmax = false;
-            chainB = chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, argmax).total;
+        if (room < chainB && chain_bytes(kLayoutSlots) < chainB) {   // the largest graphs fit without scratch only
+            layout = kLayoutSlots;
+            chainB = chain_bytes(layout);
         }
         const int Kmax = room > 0 ? static_cast<int>(std::min<int64_t>(kCap, room / chainB)) : 0;
         if (Kmax < 1)
@@ -474,7 +477,7 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         L.pmax = pmax;
         L.csrBytes = csrB;
         L.chainBytes = chainB;
-        L.slotsOnly = argmax ? 0 : 1;
+        L.layout = layout;
         L.queue = s->dCtl.as<int32_t>() + 4 * ci;
         L.error = L.queue + 1;
         L.errorItem = L.queue + 2;
@@ -785,6 +788,8 @@ static int rfmf_submit_impl(rfmf_server* s, const rfmf_graph* g, int64_t nchains
         if (!(t0s[c] > 0.0)) return fail(RFMF_ERR_INVALID, "t0s[%lld] must be > 0", static_cast<long long>(c));
     r->total = total;
     r->pmax = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(maxP, static_cast<uint64_t>(g->n))));
+    for (int64_t p = 0; p < nphases; ++p)
+        if (!main_phase(static_cast<uint32_t>(phases[p]), static_cast<int>(g->n))) r->table = true;
     // Run tables on the submitting thread, never on the worker, where
     // building or uploading them would stall the launch windows: the
     // context's device copies when another batch or request holds the same
@@ -833,16 +838,21 @@ static int rfmf_submit_impl(rfmf_server* s, const rfmf_graph* g, int64_t nchains
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kernel_ptr(r->dbytes, fmt, r->s64, r->W)));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
-        auto chain_bytes = [&](bool argmax) {
-            return chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax, r->W, r->dbytes, argmax)
+        auto chain_bytes = [&](int kind) {
+            return chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax, r->W, r->dbytes, kind)
                 .total;
+        };
+        auto least_bytes = [&]() {
+            return std::min(chain_bytes(kLayoutSlots), chain_bytes(r->table ? kLayoutAny : kLayoutMain));
         };
         // (A wider chain keeps a few bytes more; the largest graphs fit at a
         // narrower one only.)
-        while (c.threads_per_chain == 0 && r->W > 1 &&
-               static_cast<int64_t>(kSmemHeader) + chain_bytes(false) > dynMax)
+        while (c.threads_per_chain == 0 && r->W > 1 && static_cast<int64_t>(kSmemHeader) + least_bytes() > dynMax) {
             r->W /= 2;
-        const uint32_t chainB = chain_bytes(!r->s64), leastB = chain_bytes(false);
+            r->table = true;   // the narrower chain's keys may lack room
+        }
+        const uint32_t chainB = chain_bytes(r->s64 ? kLayoutSlots : r->table ? kLayoutAny : kLayoutMain);
+        const uint32_t leastB = least_bytes();
         const int64_t kWant = std::min<int64_t>(nchains, std::max(1, 8 / r->W));
         if (!csr_in_hbm(fmt) && static_cast<int64_t>(kSmemHeader) + csr_bytes(g, fmt) + kWant * chainB > dynMax) {
             if (c.csr_format != 0 &&
