@@ -1138,20 +1138,40 @@ __device__ __forceinline__ void flip_vertex(const ChainSmem& s, int v, int32_t d
     s.sb[v] = static_cast<unsigned char>(m ^ 0xFFu);
 }
 
+// The best of a wider chain's 2, 4, 8 or 16 partials of one group, four loads in
+// flight together.
+__device__ __forceinline__ unsigned long long best_partial(const unsigned char* part, int warps) {
+    unsigned long long best = 0;
+    for (int w0 = 0; w0 < warps; w0 += 4) {
+        unsigned long long p[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+            p[w] = w0 + w < warps ? *reinterpret_cast<const unsigned long long*>(part + (w0 + w) * kWarpScratch) : 0ull;
+#pragma unroll
+        for (int d = 1; d < 4; d *= 2) {
+#pragma unroll
+            for (int w = 0; w < 4; w += 2 * d) p[w] = p[w + d] > p[w] ? p[w + d] : p[w];
+        }
+        best = p[0] > best ? p[0] : best;
+    }
+    return best;
+}
+
 // FLIP on kPathWarp.  Row r = (t >> laneShift) + q T of the P winners is
 // flipped by its first lane and walked by all 2^laneShift of them; v[q] comes
 // from SELECT's registers (one-warp chains) or the warps' partials.  Returns
 // this thread's part of sum(D before) - sum(D after), which is twice the cut
-// gain once summed over the chain.
+// gain once summed over the chain.  settle() (see run_chain) is called before
+// the first flip, behind the loads that lead to it.
 //
 // With int8 gains nothing a row's walk reads is changed by another row (a
 // flip adds +-1 to its own byte, a walk +-2w to its neighbours': they commute
 // as 32-bit adds, whatever the bytes pass through on the way), so after the
 // gains are read there is one barrier, at the end.  With int32 gains a walk
 // reads its neighbours' new spins, so the flips are fenced off from the walks.
-template <bool kOne, int kRows, class DP, int kFmt, class Loc>
+template <bool kOne, int kRows, class DP, int kFmt, class Loc, class Settle>
 __device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
-                                         int grp, int32_t v[4]) {
+                                         int grp, int32_t v[4], Settle settle) {
     const int sub = t & ((1 << pc.laneShift) - 1);
     uint32_t lo[kRows], hi[kRows], neg[kRows];
     int32_t d[kRows];
@@ -1171,14 +1191,7 @@ __device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr,
             unsigned long long p = 0;
             v[q] = -1;
             if (r < pc.P) {
-                const unsigned char* part = reinterpret_cast<const unsigned char*>(s.slots) + 8 * r;
-                for (int w = 0; w < (T >> 5); w += 2) {
-                    const unsigned long long a = *reinterpret_cast<const unsigned long long*>(part + w * kWarpScratch);
-                    const unsigned long long b =
-                        *reinterpret_cast<const unsigned long long*>(part + (w + 1) * kWarpScratch);
-                    const unsigned long long ab = a > b ? a : b;
-                    p = ab > p ? ab : p;
-                }
+                p = best_partial(reinterpret_cast<const unsigned char*>(s.slots) + 8 * r, T >> 5);
                 const uint32_t low = static_cast<uint32_t>(p);
                 if constexpr (DP::kField) {
                     v[q] = p ? static_cast<int32_t>(~(low >> 9) & 0x7FFFFFu) : -1;
@@ -1198,6 +1211,7 @@ __device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr,
             if (sub == 0) loc += d[q];
         }
     }
+    settle();
     if (kOne || !DP::kField) __syncwarp();
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
@@ -1230,12 +1244,12 @@ __device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr,
 
 // P <= 128 over at least 32 (one-warp chains) or 64 threads: one to four rows,
 // or one or two, a thread.
-template <bool kOne, class DP, int kFmt, class Loc>
+template <bool kOne, class DP, int kFmt, class Loc, class Settle>
 __device__ __forceinline__ Loc flip_warp(const ChainSmem& s, const CsrView& csr, const PhaseCfg& pc, int t, int T,
-                                         int grp, int32_t v[4]) {
-    if (pc.rows == 1) return flip_rows<kOne, 1, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
-    if (!kOne || pc.rows == 2) return flip_rows<kOne, 2, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
-    return flip_rows<kOne, 4, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+                                         int grp, int32_t v[4], Settle settle) {
+    if (pc.rows == 1) return flip_rows<kOne, 1, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v, settle);
+    if (!kOne || pc.rows == 2) return flip_rows<kOne, 2, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v, settle);
+    return flip_rows<kOne, 4, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v, settle);
 }
 
 
@@ -1543,9 +1557,12 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             }
             const bool slots = kS64 || pc.path != kPathWarp;
             if (!kOne || slots) group_sync(grp, T);
-            settle();
-            if (slots) loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
-            else loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v);
+            if (slots) {
+                settle();
+                loc = flip_slots<DP, kFmt, kS64, Loc>(s, csr, pc, t, T, grp);
+            } else {
+                loc = flip_warp<kOne, DP, kFmt, Loc>(s, csr, pc, t, T, grp, v, settle);
+            }
             if (!kOne) {
                 loc = warp_sum(loc);
                 if ((t & 31) == 0) s.red[t >> 5] = loc;
