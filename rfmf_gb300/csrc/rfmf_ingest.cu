@@ -12,11 +12,12 @@
 //     endpoints of the surviving edges renumbered densely in ascending
 //     original id, every row sorted ascending -- then the compact shared-memory
 //     entry formats, B and the weight sum, all without a host CSR.
-//     Steps: endpoint presence marks and an exclusive scan give the dense ids;
-//     a degree histogram and scan give row starts; entries scatter to their
-//     rows tagged with their input index; each row is sorted by (neighbour,
-//     input index) so the first occurrence of a duplicate leads its run;
-//     runs collapse to their first entry and the rows compact.
+//     Steps: one pass checks the edges and finds the largest id; endpoint
+//     presence marks and an exclusive scan give the dense ids; a degree
+//     histogram and scan give row starts; every edge puts one 8-byte key
+//     (neighbour, input index) in each of its two rows; a warp sorts each row
+//     by counting ranks, so the first occurrence of a duplicate leads its run;
+//     the first of each run is emitted in every entry format.
 // Output (reference: src/max_cut.cpp:5-15 cutValueCsr and the
 // Solution-*-partition: lines of src/host_common.cpp:412-422):
 //   * rfmf_batch_cuts: every chain's cut recomputed on the device from its
@@ -290,118 +291,303 @@ __global__ void add_tile_offsets(T* out, const T* offs, int64_t n) {
     }
 }
 
-// Exclusive scan of n values (out may equal in), recursive over tiles.
+// Elements of scan scratch for n values: the tile sums of every level.
+int64_t scan_scratch(int64_t n) {
+    int64_t total = 0;
+    while (n > 1) {
+        n = (n + kScanTile - 1) / kScanTile;
+        total += n + 1;
+    }
+    return total + 1;
+}
+
+// Exclusive scan of n values (out may equal in), recursive over tiles;
+// `sums` holds scan_scratch(n) elements.  Asynchronous on st.
 template <class T>
-int exclusive_scan(const T* in, T* out, int64_t n, cudaStream_t st) {
+int exclusive_scan(const T* in, T* out, int64_t n, T* sums, cudaStream_t st) {
     if (n <= 0) return RFMF_OK;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    DevBuf sums;
-    if (int rc = sums.alloc(static_cast<size_t>(tiles + 1) * sizeof(T))) return rc;
-    scan_tiles<T><<<static_cast<unsigned>(tiles), kScanBlock, 0, st>>>(in, out, sums.as<T>(), n);
+    scan_tiles<T><<<static_cast<unsigned>(tiles), kScanBlock, 0, st>>>(in, out, sums, n);
     CU(cudaGetLastError());
     if (tiles > 1) {
-        if (int rc = exclusive_scan<T>(sums.as<T>(), sums.as<T>(), tiles, st)) return rc;
-        add_tile_offsets<T><<<static_cast<unsigned>(tiles), kScanBlock, 0, st>>>(out, sums.as<T>(), n);
+        if (int rc = exclusive_scan<T>(sums, sums, tiles, sums + tiles + 1, st)) return rc;
+        add_tile_offsets<T><<<static_cast<unsigned>(tiles), kScanBlock, 0, st>>>(out, sums, n);
         CU(cudaGetLastError());
     }
-    CU(cudaStreamSynchronize(st));
     return RFMF_OK;
 }
 
-struct BuildFlags {
+// What one pass over the edge lines finds (zero weights count for the id
+// check only: the parser's rule drops them).
+struct EdgeFacts {
+    unsigned long long firstNegative;   // first edge with a negative id (~0: none)
+    unsigned long long firstBig;        // first edge whose weight does not fit int32
+    long long maxId;                    // largest id of the kept edges
+    unsigned long long kept;
     int selfLoop;
-    int badId;
-    int notUnit;
-    int notSmall;
-    unsigned long long B;
-    long long wsum2;
+    int pad;
 };
 
-__global__ void mark_endpoints(const int64_t* u, const int64_t* v, int64_t E, int64_t maxId,
-                               int32_t* present, BuildFlags* f) {
+// Facts of the surviving entries.
+struct RowFacts {
+    unsigned long long B;
+    long long wsum2;
+    int notUnit;
+    int notSmall;
+    int hubs;   // rows in the hub list
+    int pad;
+};
+
+constexpr int kIngestBlock = 256;
+
+// HBM bound: 24 bytes an edge read once.
+__global__ void check_edges(const int64_t* u, const int64_t* v, const int64_t* w, int64_t E, EdgeFacts* f) {
+    long long maxId = 0;
+    unsigned long long kept = 0;
+    bool loop = false;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < E;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t a = u[i], b = v[i];
-        if (a < 0 || b < 0 || a > maxId || b > maxId) { atomicOr(&f->badId, 1); continue; }
-        if (a == b) { atomicOr(&f->selfLoop, 1); continue; }
-        present[a] = 1;
-        present[b] = 1;
+        const int64_t a = u[i], b = v[i], x = w[i];
+        if (a < 0 || b < 0) {
+            atomicMin(&f->firstNegative, static_cast<unsigned long long>(i));
+            continue;
+        }
+        if (x == 0) continue;
+        if (x > INT32_MAX || x < -static_cast<int64_t>(INT32_MAX)) {
+            atomicMin(&f->firstBig, static_cast<unsigned long long>(i));
+            continue;
+        }
+        ++kept;
+        maxId = max(maxId, static_cast<long long>(a > b ? a : b));
+        loop = loop || a == b;
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        maxId = max(maxId, __shfl_xor_sync(0xFFFFFFFFu, maxId, m));
+        kept += __shfl_xor_sync(0xFFFFFFFFu, kept, m);
+    }
+    const bool any = __any_sync(0xFFFFFFFFu, loop);
+    if ((threadIdx.x & 31) == 0) {
+        if (kept) {
+            atomicMax(&f->maxId, maxId);
+            atomicAdd(&f->kept, kept);
+        }
+        if (any) atomicOr(&f->selfLoop, 1);
     }
 }
 
-__global__ void count_degrees(const int64_t* u, const int64_t* v, int64_t E, const int32_t* dense,
+__global__ void mark_endpoints(const int64_t* u, const int64_t* v, const int64_t* w, int64_t E, int32_t* present) {
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < E;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        if (w[i] == 0) continue;
+        present[u[i]] = 1;
+        present[v[i]] = 1;
+    }
+}
+
+__global__ void count_degrees(const int64_t* u, const int64_t* v, const int64_t* w, int64_t E, const int32_t* dense,
                               int32_t* deg) {
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < E;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        if (w[i] == 0) continue;
         atomicAdd(&deg[dense[u[i]]], 1);
         atomicAdd(&deg[dense[v[i]]], 1);
     }
 }
 
-// Raw directed entry: neighbour, weight, input edge index.
-struct RawEntry {
-    int32_t col;
-    int32_t w;
-    int64_t idx;
-};
+// Directed entry: neighbour in the high half, input edge index in the low one
+// (fewer than 2^32 edge lines); ascending keys are the row's order.
+__device__ __forceinline__ unsigned long long entry_key(int32_t col, int64_t idx) {
+    return (static_cast<unsigned long long>(static_cast<uint32_t>(col)) << 32) | static_cast<uint32_t>(idx);
+}
 
+// cursor[r] starts at row r's first entry.
 __global__ void scatter_entries(const int64_t* u, const int64_t* v, const int64_t* w, int64_t E,
-                                const int32_t* dense, const int32_t* rowStart, int32_t* fill,
-                                RawEntry* ent) {
+                                const int32_t* dense, int32_t* cursor, unsigned long long* ent) {
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < E;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        if (w[i] == 0) continue;
         const int32_t a = dense[u[i]], b = dense[v[i]];
-        const int32_t wi = static_cast<int32_t>(w[i]);
-        const int32_t pa = rowStart[a] + atomicAdd(&fill[a], 1);
-        const int32_t pb = rowStart[b] + atomicAdd(&fill[b], 1);
-        ent[pa] = RawEntry{b, wi, i};
-        ent[pb] = RawEntry{a, wi, i};
+        ent[atomicAdd(&cursor[a], 1)] = entry_key(b, i);
+        ent[atomicAdd(&cursor[b], 1)] = entry_key(a, i);
     }
 }
 
-// One thread per row: insertion sort by (col, idx); then the first entry of
-// each col run survives.  Writes the surviving count of the row and, in the
-// high half, that count padded to four (both are scanned together).
-__global__ void sort_rows(RawEntry* ent, const int32_t* rowStart, int32_t n, uint64_t* keep) {
-    for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const int32_t lo = rowStart[r], hi = rowStart[r + 1];
-        for (int32_t i = lo + 1; i < hi; ++i) {
-            const RawEntry x = ent[i];
-            int32_t j = i - 1;
-            while (j >= lo && (ent[j].col > x.col || (ent[j].col == x.col && ent[j].idx > x.idx))) {
-                ent[j + 1] = ent[j];
-                --j;
+// Rows above this go to a block each (sort_hubs).
+constexpr int kHubRow = 2048;
+
+// Rank of `key` among the d keys of a row.
+__device__ __forceinline__ int rank_in(const unsigned long long* row, int d, unsigned long long key) {
+    int rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < d; ++j) rank += row[j] < key;
+    return rank;
+}
+
+// The surviving entries (first key of each neighbour) of a sorted row: counts
+// them for this thread's stride and folds their weights into the facts.
+struct RowSum {
+    int kept = 0;
+    long long abs = 0, sum = 0;
+    bool notUnit = false, notSmall = false;
+    __device__ __forceinline__ void add(const unsigned long long* row, int i, const int64_t* w) {
+        const unsigned long long k = row[i];
+        if (i > 0 && (row[i - 1] >> 32) == (k >> 32)) return;
+        const int32_t x = static_cast<int32_t>(w[static_cast<uint32_t>(k)]);
+        ++kept;
+        abs += x < 0 ? -static_cast<long long>(x) : x;
+        sum += x;
+        notUnit = notUnit || (x != 1 && x != -1);
+        notSmall = notSmall || x < -32767 || x > 32767;
+    }
+    __device__ __forceinline__ void warp() {
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            kept += __shfl_xor_sync(0xFFFFFFFFu, kept, m);
+            abs += __shfl_xor_sync(0xFFFFFFFFu, abs, m);
+        }
+    }
+};
+
+// Count of survivors and, in the high half, padded to four (both are scanned
+// together).
+__device__ __forceinline__ uint64_t kept_word(int k) {
+    return (static_cast<uint64_t>((k + 3) & ~3) << 32) | static_cast<uint32_t>(k);
+}
+
+// One warp a row: every lane ranks its keys against the whole row (d^2 / 32
+// comparisons on broadcast loads, no moves) and writes them in order, then the
+// row's survivors are counted.  (One thread's insertion sort of 16-byte
+// entries, d^2 / 4 moves through memory, took most of a 481,000-edge build.)
+__global__ void __launch_bounds__(kIngestBlock) sort_rows(const unsigned long long* ent, const int32_t* rowStart,
+                                                          const int32_t* nPtr, const int64_t* w,
+                                                          unsigned long long* out, uint64_t* keep, RowFacts* f,
+                                                          int32_t* hubList) {
+    const int n = *nPtr, lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * kIngestBlock) >> 5;
+    unsigned long long maxB = 0;
+    long long wsum = 0;
+    bool notUnit = false, notSmall = false;
+    for (int r = (blockIdx.x * kIngestBlock + threadIdx.x) >> 5; r < n; r += warps) {
+        const int lo = rowStart[r], d = rowStart[r + 1] - lo;
+        if (d > kHubRow) {
+            if (lane == 0) hubList[atomicAdd(&f->hubs, 1)] = r;
+            continue;
+        }
+        for (int i = lane; i < d; i += 32) {
+            const unsigned long long k = ent[lo + i];
+            out[lo + rank_in(ent + lo, d, k)] = k;
+        }
+        __syncwarp();
+        RowSum s;
+        for (int i = lane; i < d; i += 32) s.add(out + lo, i, w);
+        s.warp();
+        if (lane == 0) keep[r] = kept_word(s.kept);
+        maxB = maxB > static_cast<unsigned long long>(s.abs) ? maxB : static_cast<unsigned long long>(s.abs);
+        wsum += s.sum;
+        notUnit = notUnit || s.notUnit;
+        notSmall = notSmall || s.notSmall;
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) wsum += __shfl_xor_sync(0xFFFFFFFFu, wsum, m);
+    notUnit = __any_sync(0xFFFFFFFFu, notUnit);
+    notSmall = __any_sync(0xFFFFFFFFu, notSmall);
+    if (lane == 0) {
+        if (maxB) atomicMax(&f->B, maxB);
+        if (wsum) atomicAdd(reinterpret_cast<unsigned long long*>(&f->wsum2), static_cast<unsigned long long>(wsum));
+        if (notUnit) atomicOr(&f->notUnit, 1);
+        if (notSmall) atomicOr(&f->notSmall, 1);
+    }
+}
+
+// The rows of the hub list, one block each.
+__global__ void __launch_bounds__(1024) sort_hubs(const unsigned long long* ent, const int32_t* rowStart,
+                                                  const int64_t* w, unsigned long long* out, uint64_t* keep,
+                                                  RowFacts* f, const int32_t* hubList) {
+    __shared__ int kept[32];
+    __shared__ long long abs[32];
+    const int hubs = f->hubs, lane = threadIdx.x & 31;
+    for (int h = blockIdx.x; h < hubs; h += gridDim.x) {
+        const int r = hubList[h], lo = rowStart[r], d = rowStart[r + 1] - lo;
+        for (int i = threadIdx.x; i < d; i += blockDim.x) {
+            const unsigned long long k = ent[lo + i];
+            out[lo + rank_in(ent + lo, d, k)] = k;
+        }
+        __syncthreads();
+        RowSum s;
+        for (int i = threadIdx.x; i < d; i += blockDim.x) s.add(out + lo, i, w);
+        if (s.sum) atomicAdd(reinterpret_cast<unsigned long long*>(&f->wsum2), static_cast<unsigned long long>(s.sum));
+        if (s.notUnit) atomicOr(&f->notUnit, 1);
+        if (s.notSmall) atomicOr(&f->notSmall, 1);
+        s.warp();
+        if (lane == 0) {
+            kept[threadIdx.x >> 5] = s.kept;
+            abs[threadIdx.x >> 5] = s.abs;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int k = 0;
+            long long b = 0;
+            for (int q = 0; q < static_cast<int>(blockDim.x >> 5); ++q) {
+                k += kept[q];
+                b += abs[q];
             }
-            ent[j + 1] = x;
+            keep[r] = kept_word(k);
+            atomicMax(&f->B, static_cast<unsigned long long>(b));
         }
-        int32_t k = 0;
-        for (int32_t i = lo; i < hi; ++i)
-            if (i == lo || ent[i].col != ent[i - 1].col) ++k;
-        keep[r] = (static_cast<uint64_t>((k + 3) & ~3) << 32) | static_cast<uint32_t>(k);
+        __syncthreads();
     }
 }
 
-__global__ void compact_rows(const RawEntry* ent, const int32_t* rowStart, const uint64_t* outStart,
-                             int32_t n, uint32_t* offsets, Edge* edges, BuildFlags* f) {
-    for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const int32_t lo = rowStart[r], hi = rowStart[r + 1];
-        int32_t o = static_cast<int32_t>(outStart[r]);
-        offsets[r] = static_cast<uint32_t>(o);
-        long long b = 0, s = 0;
-        bool unit = true, small = true;
-        for (int32_t i = lo; i < hi; ++i) {
-            if (i != lo && ent[i].col == ent[i - 1].col) continue;
-            const int32_t wi = ent[i].w;
-            edges[o++] = Edge{ent[i].col, wi};
-            b += (wi < 0) ? -static_cast<long long>(wi) : wi;
-            s += wi;
-            unit = unit && (wi == 1 || wi == -1);
-            small = small && (wi >= -32767 && wi <= 32767);
+// The survivors of every sorted row, one warp a row, in all the formats given:
+// {col, w} pairs with their offsets, and the compact rows (start[r]: kept
+// entries before row r, padded entries in the high half) with their row words
+// and padding (the vertex itself, weight +1 or 0).  offsets and rows are
+// filled up to `words`.
+__global__ void __launch_bounds__(kIngestBlock) emit_rows(const unsigned long long* ent, const int32_t* rowStart,
+                                                          const uint64_t* start, int n, int words, const int64_t* w,
+                                                          uint32_t* offsets, Edge* edges, uint32_t* rows,
+                                                          uint16_t* u16, uint32_t* p32) {
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * kIngestBlock) >> 5;
+    for (int r = (blockIdx.x * kIngestBlock + threadIdx.x) >> 5; r < n; r += warps) {
+        const int lo = rowStart[r], d = rowStart[r + 1] - lo;
+        const uint32_t o = static_cast<uint32_t>(start[r]), c = static_cast<uint32_t>(start[r] >> 32);
+        uint32_t k = 0;   // survivors so far
+        for (int i0 = 0; i0 < d; i0 += 32) {
+            const int i = i0 + lane;
+            bool take = false;
+            unsigned long long key = 0;
+            if (i < d) {
+                key = ent[lo + i];
+                take = i == 0 || (ent[lo + i - 1] >> 32) != (key >> 32);
+            }
+            const uint32_t vote = __ballot_sync(0xFFFFFFFFu, take);
+            if (take) {
+                const uint32_t at = k + __popc(vote & ((1u << lane) - 1u));
+                const int32_t col = static_cast<int32_t>(key >> 32);
+                const int32_t x = static_cast<int32_t>(w[static_cast<uint32_t>(key)]);
+                edges[o + at] = Edge{col, x};
+                if (u16) u16[c + at] = static_cast<uint16_t>(col | (x < 0 ? 0x8000 : 0));
+                if (p32) p32[c + at] = (static_cast<uint32_t>(x) << 16) | static_cast<uint32_t>(col);
+            }
+            k += __popc(vote);
         }
-        atomicMax(&f->B, static_cast<unsigned long long>(b));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&f->wsum2), static_cast<unsigned long long>(s));
-        if (!unit) atomicOr(&f->notUnit, 1);
-        if (!small) atomicOr(&f->notSmall, 1);
+        const uint32_t pad = (0u - k) & 3u;
+        if (static_cast<uint32_t>(lane) < pad) {
+            if (u16) u16[c + k + lane] = static_cast<uint16_t>(r);
+            if (p32) p32[c + k + lane] = static_cast<uint32_t>(r);
+        }
+        if (lane == 0) {
+            offsets[r] = o;
+            if (rows) rows[r] = c | pad;
+        }
+    }
+    if (blockIdx.x == 0) {
+        for (int r = n + threadIdx.x; r < words; r += kIngestBlock) {
+            offsets[r] = static_cast<uint32_t>(start[n]);
+            if (rows) rows[r] = static_cast<uint32_t>(start[n] >> 32);
+        }
     }
 }
 
@@ -411,26 +597,14 @@ __global__ void orig_ids(const int32_t* present, const int32_t* dense, int64_t m
         if (present[i]) out[dense[i]] = i;
 }
 
-// The compact entries (u16 and/or p32, whichever are given) and the row words,
-// eight lanes a row: the high half of start[r] is row r's first compact entry.
-__global__ void make_compact(const Edge* edges, const uint32_t* offsets, const uint64_t* start, int32_t n,
-                             uint32_t* rows, uint16_t* u16, uint32_t* p32) {
-    const int sub = threadIdx.x & 7;
-    for (int32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; r < n; r += (gridDim.x * blockDim.x) >> 3) {
-        const uint32_t lo = offsets[r], deg = offsets[r + 1] - lo, o = static_cast<uint32_t>(start[r] >> 32);
-        for (uint32_t k = sub; k < ((deg + 3u) & ~3u); k += 8) {
-            const Edge e = k < deg ? edges[lo + k] : Edge{r, 0};   // padding: the vertex itself
-            if (u16) u16[o + k] = static_cast<uint16_t>(e.col | (e.w < 0 ? 0x8000 : 0));
-            if (p32) p32[o + k] = (static_cast<uint32_t>(e.w) << 16) | static_cast<uint32_t>(e.col);
-        }
-        if (sub == 0) rows[r] = o | ((0u - deg) & 3u);
+// The two halves of the {col, w} pairs.
+__global__ void split_edges(const Edge* edges, int64_t m2, int32_t* col, int32_t* w) {
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < m2;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const Edge e = edges[i];
+        if (col) col[i] = e.col;
+        if (w) w[i] = e.w;
     }
-}
-
-__global__ void fill_tail_u32(uint32_t* p, int64_t from, int64_t to, uint32_t val) {
-    for (int64_t i = from + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < to;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        p[i] = val;
 }
 
 unsigned grid_for(int64_t n) {
@@ -439,89 +613,103 @@ unsigned grid_for(int64_t n) {
 
 }  // namespace
 
+// Parts of one device allocation, each 256-byte aligned.
+class Arena {
+public:
+    template <class T>
+    size_t add(int64_t count) {
+        const size_t at = bytes_;
+        bytes_ += (static_cast<size_t>(count) * sizeof(T) + 255) & ~size_t(255);
+        return at;
+    }
+    int alloc() { return buf_.alloc(bytes_); }
+    template <class T>
+    T* at(size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(buf_.p) + off); }
+
+private:
+    DevBuf buf_;
+    size_t bytes_ = 0;
+};
+
 static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const int64_t* u,
                                      const int64_t* v, const int64_t* w, rfmf_graph** out,
                                      int64_t* n_out) {
     if (!ctx || !out || nedges < 0 || (nedges > 0 && (!u || !v || !w)))
         return fail(RFMF_ERR_INVALID, "bad arguments");
     *out = nullptr;
-    // Zero weights drop (the parser's rule); ids and weights checked.
-    std::vector<int64_t> hu, hv, hw;
-    hu.reserve(static_cast<size_t>(nedges));
-    hv.reserve(static_cast<size_t>(nedges));
-    hw.reserve(static_cast<size_t>(nedges));
-    int64_t maxId = 0;
-    for (int64_t i = 0; i < nedges; ++i) {
-        if (u[i] < 0 || v[i] < 0) return fail(RFMF_ERR_INVALID, "negative vertex id at edge %lld", (long long)i);
-        if (w[i] == 0) continue;
-        if (w[i] > std::numeric_limits<int32_t>::max() || w[i] < -std::numeric_limits<int32_t>::max())
-            return fail(RFMF_ERR_CAPACITY, "weight at edge %lld does not fit int32", (long long)i);
-        maxId = std::max(maxId, std::max(u[i], v[i]));
-        hu.push_back(u[i]);
-        hv.push_back(v[i]);
-        hw.push_back(w[i]);
+    const int64_t E = nedges;
+    CU(cudaSetDevice(ctx->device));
+    cudaStream_t st = ctx->stream;
+    int rc;
+    // The edge lines as they are; ids and weights are checked on the device.
+    Arena in;
+    const size_t oU = in.add<int64_t>(E), oV = in.add<int64_t>(E), oW = in.add<int64_t>(E), oF = in.add<EdgeFacts>(1);
+    if ((rc = in.alloc())) return rc;
+    const int64_t *dU = in.at<int64_t>(oU), *dV = in.at<int64_t>(oV), *dW = in.at<int64_t>(oW);
+    EdgeFacts ef{~0ull, ~0ull, 0, 0, 0, 0};
+    CU(cudaMemcpyAsync(in.at<EdgeFacts>(oF), &ef, sizeof ef, cudaMemcpyHostToDevice, st));
+    if (E) {
+        CU(cudaMemcpyAsync(in.at<int64_t>(oU), u, E * 8, cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(in.at<int64_t>(oV), v, E * 8, cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(in.at<int64_t>(oW), w, E * 8, cudaMemcpyHostToDevice, st));
+        check_edges<<<grid_for(E), kIngestBlock, 0, st>>>(dU, dV, dW, E, in.at<EdgeFacts>(oF));
+        CU(cudaGetLastError());
     }
-    const int64_t E = static_cast<int64_t>(hu.size());
+    CU(cudaMemcpyAsync(&ef, in.at<EdgeFacts>(oF), sizeof ef, cudaMemcpyDeviceToHost, st));
+    CU(cudaStreamSynchronize(st));
+    if (ef.firstNegative != ~0ull && ef.firstNegative <= ef.firstBig)
+        return fail(RFMF_ERR_INVALID, "negative vertex id at edge %lld", (long long)ef.firstNegative);
+    if (ef.firstBig != ~0ull)
+        return fail(RFMF_ERR_CAPACITY, "weight at edge %lld does not fit int32", (long long)ef.firstBig);
+    const int64_t maxId = ef.maxId, kept = static_cast<int64_t>(ef.kept);
     if (maxId >= (int64_t(1) << 28))
         return fail(RFMF_ERR_CAPACITY, "vertex ids up to %lld: the device build takes ids below 2^28",
                     (long long)maxId);
-    if (2 * E >= (int64_t(1) << 31)) return fail(RFMF_ERR_CAPACITY, "too many edges");
-    CU(cudaSetDevice(ctx->device));
-    cudaStream_t st = ctx->stream;
-    const int64_t ids = maxId + 1;
-    DevBuf dU, dV, dW, dPresent, dDense, dFlags;
-    int rc;
-    if ((rc = dU.alloc(E * 8)) || (rc = dV.alloc(E * 8)) || (rc = dW.alloc(E * 8)) ||
-        (rc = dPresent.alloc((ids + 1) * 4)) || (rc = dDense.alloc((ids + 1) * 4)) ||
-        (rc = dFlags.alloc(sizeof(BuildFlags))))
-        return rc;
-    if (E) {
-        CU(cudaMemcpyAsync(dU.p, hu.data(), E * 8, cudaMemcpyHostToDevice, st));
-        CU(cudaMemcpyAsync(dV.p, hv.data(), E * 8, cudaMemcpyHostToDevice, st));
-        CU(cudaMemcpyAsync(dW.p, hw.data(), E * 8, cudaMemcpyHostToDevice, st));
-    }
-    CU(cudaMemsetAsync(dPresent.p, 0, (ids + 1) * 4, st));
-    CU(cudaMemsetAsync(dFlags.p, 0, sizeof(BuildFlags), st));
-    if (E) mark_endpoints<<<grid_for(E), 256, 0, st>>>(dU.as<int64_t>(), dV.as<int64_t>(), E, maxId,
-                                                       dPresent.as<int32_t>(), dFlags.as<BuildFlags>());
-    CU(cudaGetLastError());
+    if (2 * kept >= (int64_t(1) << 31) || E >= (int64_t(1) << 32)) return fail(RFMF_ERR_CAPACITY, "too many edges");
+    if (ef.selfLoop) return fail(RFMF_ERR_INVALID, "self loop in the edge list");
+
+    // Scratch, rows at most one per id and per line end.
+    const int64_t ids = maxId + 1, rowsMax = std::min<int64_t>(ids, 2 * kept) + 1;
+    Arena sc;
+    const size_t oPresent = sc.add<int32_t>(ids + 1), oDeg = sc.add<int32_t>(rowsMax), oKeep = sc.add<uint64_t>(rowsMax),
+                 oRf = sc.add<RowFacts>(1), zeroBytes = sc.add<char>(0), oDense = sc.add<int32_t>(ids + 1),
+                 oRow = sc.add<int32_t>(rowsMax), oCursor = sc.add<int32_t>(rowsMax), oStart = sc.add<uint64_t>(rowsMax),
+                 oEnt = sc.add<unsigned long long>(2 * kept), oSorted = sc.add<unsigned long long>(2 * kept),
+                 oHubs = sc.add<int32_t>(2 * kept / kHubRow + 1), oIds = sc.add<int64_t>(rowsMax),
+                 oSums = sc.add<uint64_t>(scan_scratch(std::max(ids + 1, rowsMax)));
+    if ((rc = sc.alloc())) return rc;
+    int32_t *present = sc.at<int32_t>(oPresent), *dense = sc.at<int32_t>(oDense), *deg = sc.at<int32_t>(oDeg);
+    int32_t *row = sc.at<int32_t>(oRow), *cursor = sc.at<int32_t>(oCursor), *hubs = sc.at<int32_t>(oHubs);
+    uint64_t *keep = sc.at<uint64_t>(oKeep), *start = sc.at<uint64_t>(oStart);
+    unsigned long long *ent = sc.at<unsigned long long>(oEnt), *sorted = sc.at<unsigned long long>(oSorted);
+    RowFacts* rf = sc.at<RowFacts>(oRf);
+    int32_t* sums32 = sc.at<int32_t>(oSums);
+    CU(cudaMemsetAsync(present, 0, zeroBytes, st));   // presence, degrees, kept counts, facts
+    if (E) mark_endpoints<<<grid_for(E), kIngestBlock, 0, st>>>(dU, dV, dW, E, present);
     // dense ids: exclusive scan of presence over ids + 1 slots; n = last value
-    if ((rc = exclusive_scan<int32_t>(dPresent.as<int32_t>(), dDense.as<int32_t>(), ids + 1, st)))
-        return rc;
-    BuildFlags hf{};
-    int32_t n32 = 0;
-    CU(cudaMemcpyAsync(&hf, dFlags.p, sizeof hf, cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(&n32, dDense.as<int32_t>() + ids, 4, cudaMemcpyDeviceToHost, st));
+    if ((rc = exclusive_scan<int32_t>(present, dense, ids + 1, sums32, st))) return rc;
+    if (E) count_degrees<<<grid_for(E), kIngestBlock, 0, st>>>(dU, dV, dW, E, dense, deg);
+    // row starts (slots past the last row hold 2 * kept)
+    if ((rc = exclusive_scan<int32_t>(deg, row, rowsMax, sums32, st))) return rc;
+    CU(cudaMemcpyAsync(cursor, row, rowsMax * 4, cudaMemcpyDeviceToDevice, st));
+    if (E) scatter_entries<<<grid_for(E), kIngestBlock, 0, st>>>(dU, dV, dW, E, dense, cursor, ent);
+    if (kept) {
+        const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((rowsMax + 7) / 8, 8 * ctx->sms));
+        sort_rows<<<blocks, kIngestBlock, 0, st>>>(ent, row, dense + ids, dW, sorted, keep, rf, hubs);
+        if (2 * kept > kHubRow)
+            sort_hubs<<<ctx->sms, 1024, 0, st>>>(ent, row, dW, sorted, keep, rf, hubs);
+    }
+    CU(cudaGetLastError());
+    if ((rc = exclusive_scan<uint64_t>(keep, start, rowsMax, sc.at<uint64_t>(oSums), st))) return rc;
+    RowFacts hf{};
+    int32_t n = 0;
+    uint64_t total = 0;
+    CU(cudaMemcpyAsync(&hf, rf, sizeof hf, cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(&n, dense + ids, 4, cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(&total, start + rowsMax - 1, 8, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
-    if (hf.selfLoop) return fail(RFMF_ERR_INVALID, "self loop in the edge list");
-    const int32_t n = n32;
-    // degrees and row starts (n + 1 slots; slot n becomes 2E)
-    DevBuf dDeg, dRow, dFill, dEnt, dKeep, dOut;
-    if ((rc = dDeg.alloc((static_cast<int64_t>(n) + 1) * 4)) || (rc = dRow.alloc((static_cast<int64_t>(n) + 1) * 4)) ||
-        (rc = dFill.alloc((static_cast<int64_t>(n) + 1) * 4)) || (rc = dEnt.alloc(std::max<int64_t>(2 * E, 1) * sizeof(RawEntry))) ||
-        (rc = dKeep.alloc((static_cast<int64_t>(n) + 1) * 8)) || (rc = dOut.alloc((static_cast<int64_t>(n) + 1) * 8)))
-        return rc;
-    CU(cudaMemsetAsync(dDeg.p, 0, (static_cast<int64_t>(n) + 1) * 4, st));
-    CU(cudaMemsetAsync(dFill.p, 0, (static_cast<int64_t>(n) + 1) * 4, st));
-    CU(cudaMemsetAsync(dKeep.p, 0, (static_cast<int64_t>(n) + 1) * 8, st));
-    if (E) count_degrees<<<grid_for(E), 256, 0, st>>>(dU.as<int64_t>(), dV.as<int64_t>(), E,
-                                                      dDense.as<int32_t>(), dDeg.as<int32_t>());
-    CU(cudaGetLastError());
-    if ((rc = exclusive_scan<int32_t>(dDeg.as<int32_t>(), dRow.as<int32_t>(), static_cast<int64_t>(n) + 1, st)))
-        return rc;
-    if (E) scatter_entries<<<grid_for(E), 256, 0, st>>>(dU.as<int64_t>(), dV.as<int64_t>(), dW.as<int64_t>(), E,
-                                                        dDense.as<int32_t>(), dRow.as<int32_t>(),
-                                                        dFill.as<int32_t>(), dEnt.as<RawEntry>());
-    CU(cudaGetLastError());
-    if (n) sort_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), n, dKeep.as<uint64_t>());
-    CU(cudaGetLastError());
-    if ((rc = exclusive_scan<uint64_t>(dKeep.as<uint64_t>(), dOut.as<uint64_t>(), static_cast<int64_t>(n) + 1, st)))
-        return rc;
-    uint64_t kept = 0;
-    CU(cudaMemcpyAsync(&kept, dOut.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    const int32_t m2 = static_cast<int32_t>(kept);
-    const uint32_t mPad = static_cast<uint32_t>(kept >> 32);   // entries of the padded compact rows
+    const int32_t m2 = static_cast<int32_t>(total);
+    const uint32_t mPad = static_cast<uint32_t>(total >> 32);   // entries of the padded compact rows
 
     auto g = std::unique_ptr<rfmf_graph>(new (std::nothrow) rfmf_graph());
     if (!g) return fail(RFMF_ERR_NOMEM, "host allocation failed");
@@ -529,54 +717,42 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     g->ctx = ctx;
     g->n = n;
     g->m = m2 / 2;
-    const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
-    if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(std::max<int64_t>(m2, 1) * sizeof(Edge)))) return rc;
-    if (n) compact_rows<<<grid_for(n), 256, 0, st>>>(dEnt.as<RawEntry>(), dRow.as<int32_t>(), dOut.as<uint64_t>(), n,
-                                                     g->offsets.as<uint32_t>(), g->edges.as<Edge>(),
-                                                     dFlags.as<BuildFlags>());
-    CU(cudaGetLastError());
-    // offsets[n .. padded end] = m2
-    fill_tail_u32<<<1, 256, 0, st>>>(g->offsets.as<uint32_t>(), n, static_cast<int64_t>(ob / 4), static_cast<uint32_t>(m2));
-    CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(&hf, dFlags.p, sizeof hf, cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
     g->B = static_cast<int64_t>(hf.B);
     g->wsum2 = hf.wsum2;
     if (g->B > std::numeric_limits<int32_t>::max())
         return fail(RFMF_ERR_CAPACITY, "max weighted degree %lld exceeds int32", (long long)g->B);
+    const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
+    if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(std::max<int64_t>(m2, 1) * sizeof(Edge)))) return rc;
     g->unit16 = !hf.notUnit && n <= 32768;
     g->packed32 = !hf.notSmall && n <= 65536 && mPad < (1u << 30);
     if (g->unit16 || g->packed32) {
         g->rowBytes = static_cast<uint32_t>(ob);
         if ((rc = g->rows.alloc(ob))) return rc;
-        if (g->unit16) {
-            g->u16Bytes = align16(mPad * 2u);
-            if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
-            CU(cudaMemsetAsync(g->u16.p, 0, g->u16Bytes, st));
-        }
-        if (g->packed32) {
-            g->p32Bytes = align16(mPad * 4u);
-            if ((rc = g->p32.alloc(g->p32Bytes))) return rc;
-            CU(cudaMemsetAsync(g->p32.p, 0, g->p32Bytes, st));
-        }
-        if (n)
-            make_compact<<<grid_for(8 * static_cast<int64_t>(n)), 256, 0, st>>>(
-                g->edges.as<Edge>(), g->offsets.as<uint32_t>(), dOut.as<uint64_t>(), n, g->rows.as<uint32_t>(),
-                g->unit16 ? g->u16.as<uint16_t>() : nullptr, g->packed32 ? g->p32.as<uint32_t>() : nullptr);
-        fill_tail_u32<<<1, 32, 0, st>>>(g->rows.as<uint32_t>(), n, static_cast<int64_t>(ob / 4), mPad);
     }
+    if (g->unit16) {
+        g->u16Bytes = align16(mPad * 2u);
+        if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
+        CU(cudaMemsetAsync(static_cast<char*>(g->u16.p) + (g->u16.bytes - 16), 0, 16, st));   // the last vector's rest
+    }
+    if (g->packed32) {
+        g->p32Bytes = align16(mPad * 4u);
+        if ((rc = g->p32.alloc(g->p32Bytes))) return rc;
+    }
+    const unsigned blocks = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, 8 * ctx->sms)));
+    emit_rows<<<blocks, kIngestBlock, 0, st>>>(sorted, row, start, n, static_cast<int>(ob / 4), dW,
+                                               g->offsets.as<uint32_t>(), g->edges.as<Edge>(),
+                                               g->rowBytes ? g->rows.as<uint32_t>() : nullptr,
+                                               g->unit16 ? g->u16.as<uint16_t>() : nullptr,
+                                               g->packed32 ? g->p32.as<uint32_t>() : nullptr);
     CU(cudaGetLastError());
     // dense id -> original id, kept on the host with the graph
-    {
-        DevBuf dIds;
-        if ((rc = dIds.alloc(std::max<int64_t>(n, 1) * 8))) return rc;
-        if (n) orig_ids<<<grid_for(ids), 256, 0, st>>>(dPresent.as<int32_t>(), dDense.as<int32_t>(), maxId,
-                                                       dIds.as<int64_t>());
+    g->origIds.resize(static_cast<size_t>(n));
+    if (n) {
+        orig_ids<<<grid_for(ids), kIngestBlock, 0, st>>>(present, dense, maxId, sc.at<int64_t>(oIds));
         CU(cudaGetLastError());
-        g->origIds.resize(static_cast<size_t>(n));
-        if (n) CU(cudaMemcpyAsync(g->origIds.data(), dIds.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CU(cudaStreamSynchronize(st));
+        CU(cudaMemcpyAsync(g->origIds.data(), sc.at<int64_t>(oIds), n * 8, cudaMemcpyDeviceToHost, st));
     }
+    CU(cudaStreamSynchronize(st));
     if (n_out) *n_out = n;
     *out = g.release();
     return RFMF_OK;
@@ -596,12 +772,16 @@ static int rfmf_graph_csr_impl(const rfmf_graph* g, uint32_t* offsets, int32_t* 
     const int64_t m2 = 2 * g->m;
     if (offsets) CU(cudaMemcpy(offsets, g->offsets.p, (g->n + 1) * 4, cudaMemcpyDeviceToHost));
     if ((col || weight) && m2) {
-        std::vector<Edge> e(static_cast<size_t>(m2));
-        CU(cudaMemcpy(e.data(), g->edges.p, m2 * sizeof(Edge), cudaMemcpyDeviceToHost));
-        for (int64_t i = 0; i < m2; ++i) {
-            if (col) col[i] = e[i].col;
-            if (weight) weight[i] = e[i].w;
-        }
+        cudaStream_t st = g->ctx->stream;
+        Arena a;
+        const size_t oCol = a.add<int32_t>(m2), oW = a.add<int32_t>(m2);
+        if (int rc = a.alloc()) return rc;
+        split_edges<<<grid_for(m2), kIngestBlock, 0, st>>>(g->edges.as<Edge>(), m2, col ? a.at<int32_t>(oCol) : nullptr,
+                                                           weight ? a.at<int32_t>(oW) : nullptr);
+        CU(cudaGetLastError());
+        if (col) CU(cudaMemcpyAsync(col, a.at<int32_t>(oCol), m2 * 4, cudaMemcpyDeviceToHost, st));
+        if (weight) CU(cudaMemcpyAsync(weight, a.at<int32_t>(oW), m2 * 4, cudaMemcpyDeviceToHost, st));
+        CU(cudaStreamSynchronize(st));
     }
     return RFMF_OK;
 }
