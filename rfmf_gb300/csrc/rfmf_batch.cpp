@@ -80,6 +80,8 @@ struct rfmf_batch {
     std::vector<uint32_t> phaseP;                // the schedule, host copy
     std::vector<uint64_t> phaseIters;
     DevBuf dGraphs, dScheds, dChains, dPhaseP, dPhaseIters, dBits, dBest;
+    DevBuf dCutPlan;                             // cut groups and their chains (made when first wanted)
+    int cutGroups = 0;
     std::vector<DevBetaRef> betaRefs;            // the context's shared beta tables in use
     std::vector<BatchClass> cls;
     cudaEvent_t fork = nullptr;
@@ -597,6 +599,46 @@ int enqueue_run(rfmf_batch* b, uint64_t sweeps, bool capturing = false) {
 
 }  // namespace
 
+namespace {
+
+// Cuts of every chain's spins, recomputed on the device into out (C values),
+// asynchronously on the context's stream.  The groups of up to 32 chains of a
+// graph are laid out once per batch.
+int enqueue_cuts(rfmf_batch* b, int which, int64_t* out) {
+    cudaStream_t st = b->ctx->stream;
+    const size_t orderBytes = static_cast<size_t>((b->C * 4 + 15) & ~int64_t(15));
+    if (!b->dCutPlan.p) {
+        std::vector<std::vector<int32_t>> of(b->glist.size());
+        for (int64_t i = 0; i < b->C; ++i) of[b->graphOfChain[i]].push_back(static_cast<int32_t>(i));
+        std::vector<int32_t> order;
+        std::vector<CutGroup> groups;
+        for (size_t g = 0; g < of.size(); ++g)
+            for (size_t s = 0; s < of[g].size(); s += 32) {
+                const int cnt = static_cast<int>(std::min<size_t>(32, of[g].size() - s));
+                groups.push_back(CutGroup{static_cast<int32_t>(g), static_cast<int32_t>(order.size()), cnt, 0});
+                order.insert(order.end(), of[g].begin() + s, of[g].begin() + s + cnt);
+            }
+        DevBuf plan;
+        if (int rc = plan.alloc(orderBytes + groups.size() * sizeof(CutGroup))) return rc;
+        CU(cudaMemcpyAsync(plan.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(plan.as<char>() + orderBytes, groups.data(), groups.size() * sizeof(CutGroup),
+                           cudaMemcpyHostToDevice, st));
+        CU(cudaStreamSynchronize(st));
+        b->dCutPlan = std::move(plan);
+        b->cutGroups = static_cast<int>(groups.size());
+    }
+    int64_t maxN = 0;
+    for (const rfmf_graph* g : b->glist) maxN = std::max(maxN, g->n);
+    CU(cudaMemsetAsync(out, 0, static_cast<size_t>(b->C) * sizeof(int64_t), st));
+    CU(launch_chain_cuts(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(),
+                         reinterpret_cast<const CutGroup*>(b->dCutPlan.as<char>() + orderBytes), b->cutGroups,
+                         b->dCutPlan.as<int32_t>(), static_cast<int>(maxN), b->ctx->sms, b->ctx->smemOptin, which, out,
+                         st));
+    return RFMF_OK;
+}
+
+}  // namespace
+
 // Saved chain state a batch starts from (rfmf_batch_restore).
 struct Resume {
     const int8_t* best_spins;
@@ -1056,12 +1098,10 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     if (resume) {
         // The checkpoint's cut values against its spins, recomputed on the
         // device (cutValueCsr, src/max_cut.cpp:5-15).
-        DevBuf d;
-        if ((rc = d.alloc(static_cast<size_t>(2 * C) * sizeof(int64_t)))) return rc;
-        CU(launch_chain_cuts(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(), static_cast<int>(C), 0,
-                             d.as<int64_t>(), st));
-        CU(launch_chain_cuts(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(), static_cast<int>(C), 1,
-                             d.as<int64_t>() + C, st));
+        Scratch d;
+        if ((rc = d.alloc(ctx, static_cast<size_t>(2 * C) * sizeof(int64_t)))) return rc;
+        for (int which = 0; which < 2; ++which)
+            if ((rc = enqueue_cuts(b.get(), which, d.as<int64_t>() + which * C))) return rc;
         std::vector<int64_t> cuts(static_cast<size_t>(2 * C));
         CU(cudaMemcpyAsync(cuts.data(), d.p, cuts.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
@@ -1207,10 +1247,9 @@ static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_s
 static int rfmf_batch_cuts_impl(rfmf_batch* b, int which, int64_t* out_cuts) {
     if (!b || !out_cuts || (which != 0 && which != 1)) return fail(RFMF_ERR_INVALID, "bad arguments");
     if (int rc = rfmf_batch_synchronize(b)) return rc;
-    DevBuf d;
-    if (int rc = d.alloc(b->C * sizeof(int64_t))) return rc;
-    CU(launch_chain_cuts(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(), static_cast<int>(b->C), which,
-                         d.as<int64_t>(), b->ctx->stream));
+    Scratch d;
+    if (int rc = d.alloc(b->ctx, static_cast<size_t>(b->C) * sizeof(int64_t))) return rc;
+    if (int rc = enqueue_cuts(b, which, d.as<int64_t>())) return rc;
     CU(cudaMemcpyAsync(out_cuts, d.p, b->C * sizeof(int64_t), cudaMemcpyDeviceToHost, b->ctx->stream));
     CU(cudaStreamSynchronize(b->ctx->stream));
     return RFMF_OK;
@@ -1222,18 +1261,14 @@ static int rfmf_batch_partitions_impl(rfmf_batch* b, int which, char* out, int64
     for (int64_t n : b->chainN) maxN = std::max(maxN, n);
     if (stride < maxN) return fail(RFMF_ERR_INVALID, "stride %lld < largest n %lld", (long long)stride, (long long)maxN);
     if (int rc = rfmf_batch_synchronize(b)) return rc;
-    // chunks of chains bounded to ~256 MB of device staging and to 65535
-    // chains (one grid row per chain: gridDim.y is at most 65535)
-    const int64_t per = std::max<int64_t>(
-        1, std::min<int64_t>(std::min<int64_t>(b->C, 65535), (int64_t(256) << 20) / std::max<int64_t>(stride, 1)));
-    DevBuf d;
-    if (int rc = d.alloc(static_cast<size_t>(per * stride))) return rc;
+    // chunks of chains bounded to ~256 MB of device staging
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(b->C, (int64_t(256) << 20) / std::max<int64_t>(stride, 1)));
+    Scratch d;
+    if (int rc = d.alloc(b->ctx, static_cast<size_t>(per * stride))) return rc;
     for (int64_t c0 = 0; c0 < b->C; c0 += per) {
         const int64_t cnt = std::min(per, b->C - c0);
-        CU(cudaMemsetAsync(d.p, 0, static_cast<size_t>(cnt * stride), b->ctx->stream));
         CU(launch_chain_partitions(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(), static_cast<int>(c0),
-                                   static_cast<int>(cnt), static_cast<int>(maxN), which, d.as<char>(), stride,
-                                   b->ctx->stream));
+                                   static_cast<int>(cnt), which, d.as<char>(), stride, b->ctx->stream));
         CU(cudaMemcpyAsync(out + c0 * stride, d.p, static_cast<size_t>(cnt * stride), cudaMemcpyDeviceToHost,
                            b->ctx->stream));
         CU(cudaStreamSynchronize(b->ctx->stream));

@@ -282,6 +282,28 @@ bool score_safe_int32(int64_t total, double t0, int64_t B) {
 
 }  // namespace rfmf
 
+namespace rfmf {
+int Scratch::alloc(const rfmf_context* ctx, size_t bytes) {
+    if (bytes < 16) bytes = 16;
+    stream = ctx->stream;
+    pooled = ctx->scratch != nullptr;
+    const cudaError_t e = pooled ? cudaMallocFromPoolAsync(&p, bytes, ctx->scratch, stream) : cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) {
+        p = nullptr;
+        cudaGetLastError();
+        return fail(e == cudaErrorMemoryAllocation ? RFMF_ERR_NOMEM : RFMF_ERR_CUDA, "scratch of %zu bytes failed: %s",
+                    bytes, cudaGetErrorString(e));
+    }
+    return RFMF_OK;
+}
+
+Scratch::~Scratch() {
+    if (!p) return;
+    if (pooled) cudaFreeAsync(p, stream);
+    else cudaFree(p);
+}
+}  // namespace rfmf
+
 // Error channel shared with the other translation units of the library.
 namespace rfmf {
 int set_last_error(int code, const char* msg) { return fail(code, "%s", msg); }
@@ -311,6 +333,17 @@ extern "C" int rfmf_context_create(int device, rfmf_context** out) {
     CU(cudaDeviceGetAttribute(&ctx->smemOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CU(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     gumbel_lut(ctx->lut);
+    int pools = 0;
+    if (cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && pools) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        uint64_t keep = kScratchKeepBytes;
+        if (cudaMemPoolCreate(&ctx->scratch, &props) != cudaSuccess) ctx->scratch = nullptr;
+        else cudaMemPoolSetAttribute(ctx->scratch, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    cudaGetLastError();
     *out = ctx.release();
     return RFMF_OK;
 }
@@ -325,6 +358,10 @@ void let_go(rfmf_context* ctx) {
         ctx->devBeta.clear();
     }
     if (ctx->uploadStream) cudaStreamDestroy(ctx->uploadStream);
+    if (ctx->scratch) {
+        if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+        cudaMemPoolDestroy(ctx->scratch);
+    }
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

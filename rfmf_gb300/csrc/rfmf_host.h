@@ -45,11 +45,18 @@ const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream);
 
-// Output-path kernels (rfmf_ingest.cu).
-cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, int C, int which,
-                              int64_t* out, cudaStream_t st);
-cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count,
-                                    int maxN, int which, char* out, int64_t stride, cudaStream_t st);
+// Output-path kernels (rfmf_ingest.cu).  A cut group: up to 32 chains of one
+// graph, order[first .. first + count).
+struct CutGroup {
+    int32_t graph, first, count, pad;
+};
+// Adds every chain's cut into out (zeroed by the caller).
+cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutGroup* groups, int ngroups,
+                              const int32_t* order, int maxN, int sms, int smemOptin, int which, int64_t* out,
+                              cudaStream_t st);
+// '0'/'1' rows of chains [c0, c0 + count) into out, `stride` bytes each, 0 past n.
+cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count, int which,
+                                    char* out, int64_t stride, cudaStream_t st);
 
 // Error channel: records the message for rfmf_last_error() (per host thread)
 // and returns `code`.
@@ -136,6 +143,23 @@ struct DevBuf {
         }
         return RFMF_OK;
     }
+    template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// Device memory for the length of one call on a context's stream, from the
+// context's scratch pool: allocated and freed in stream order, so it costs no
+// device synchronisation (GB300: cudaMalloc + cudaFree of 4 MB 63 us).  The pool
+// keeps at most kScratchKeepBytes between calls and goes with the context.
+constexpr uint64_t kScratchKeepBytes = uint64_t(64) << 20;
+struct Scratch {
+    void* p = nullptr;
+    cudaStream_t stream = nullptr;
+    bool pooled = false;
+    Scratch() = default;
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch();
+    int alloc(const rfmf_context* ctx, size_t bytes);
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
@@ -266,6 +290,7 @@ struct rfmf_context {
     int64_t devBetaKeepBytes = 0;
     uint64_t devBetaUploads = 0;
     cudaStream_t uploadStream = nullptr;
+    cudaMemPool_t scratch = nullptr;   // see Scratch; null where the device has no pools
     // Measured plans (rfmf_autotune) by batch shape: the chosen config and
     // every candidate's config and microseconds per chain-sweep.
     struct TunedPlan {

@@ -613,7 +613,7 @@ unsigned grid_for(int64_t n) {
 
 }  // namespace
 
-// Parts of one device allocation, each 256-byte aligned.
+// Parts of one scratch allocation, each 256-byte aligned.
 class Arena {
 public:
     template <class T>
@@ -622,12 +622,12 @@ public:
         bytes_ += (static_cast<size_t>(count) * sizeof(T) + 255) & ~size_t(255);
         return at;
     }
-    int alloc() { return buf_.alloc(bytes_); }
+    int alloc(const rfmf_context* ctx) { return buf_.alloc(ctx, bytes_); }
     template <class T>
     T* at(size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(buf_.p) + off); }
 
 private:
-    DevBuf buf_;
+    Scratch buf_;
     size_t bytes_ = 0;
 };
 
@@ -644,7 +644,7 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     // The edge lines as they are; ids and weights are checked on the device.
     Arena in;
     const size_t oU = in.add<int64_t>(E), oV = in.add<int64_t>(E), oW = in.add<int64_t>(E), oF = in.add<EdgeFacts>(1);
-    if ((rc = in.alloc())) return rc;
+    if ((rc = in.alloc(ctx))) return rc;
     const int64_t *dU = in.at<int64_t>(oU), *dV = in.at<int64_t>(oV), *dW = in.at<int64_t>(oW);
     EdgeFacts ef{~0ull, ~0ull, 0, 0, 0, 0};
     CU(cudaMemcpyAsync(in.at<EdgeFacts>(oF), &ef, sizeof ef, cudaMemcpyHostToDevice, st));
@@ -677,7 +677,7 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
                  oEnt = sc.add<unsigned long long>(2 * kept), oSorted = sc.add<unsigned long long>(2 * kept),
                  oHubs = sc.add<int32_t>(2 * kept / kHubRow + 1), oIds = sc.add<int64_t>(rowsMax),
                  oSums = sc.add<uint64_t>(scan_scratch(std::max(ids + 1, rowsMax)));
-    if ((rc = sc.alloc())) return rc;
+    if ((rc = sc.alloc(ctx))) return rc;
     int32_t *present = sc.at<int32_t>(oPresent), *dense = sc.at<int32_t>(oDense), *deg = sc.at<int32_t>(oDeg);
     int32_t *row = sc.at<int32_t>(oRow), *cursor = sc.at<int32_t>(oCursor), *hubs = sc.at<int32_t>(oHubs);
     uint64_t *keep = sc.at<uint64_t>(oKeep), *start = sc.at<uint64_t>(oStart);
@@ -775,7 +775,7 @@ static int rfmf_graph_csr_impl(const rfmf_graph* g, uint32_t* offsets, int32_t* 
         cudaStream_t st = g->ctx->stream;
         Arena a;
         const size_t oCol = a.add<int32_t>(m2), oW = a.add<int32_t>(m2);
-        if (int rc = a.alloc()) return rc;
+        if (int rc = a.alloc(g->ctx)) return rc;
         split_edges<<<grid_for(m2), kIngestBlock, 0, st>>>(g->edges.as<Edge>(), m2, col ? a.at<int32_t>(oCol) : nullptr,
                                                            weight ? a.at<int32_t>(oW) : nullptr);
         CU(cudaGetLastError());
@@ -795,62 +795,168 @@ __device__ __forceinline__ int bit_of(const uint32_t* bits, int v) {
     return (bits[v >> 5] >> (v & 31)) & 1;
 }
 
-// One CTA per chain: cutValueCsr of its end (which 0) or best (which 1)
-// spins -- every directed entry (v, u) with u > v across the cut adds w.
-__global__ void chain_cuts_kernel(const DevChain* chains, const DevGraph* graphs, int C, int which,
-                                  int64_t* out) {
-    __shared__ long long part[32];
-    const int c = blockIdx.x;
-    if (c >= C) return;
-    const DevChain& ch = chains[c];
-    const DevGraph& g = graphs[ch.graph];
-    const uint32_t* bits = which ? ch.bestBits : ch.spinBits;
+// The transpose of the warp's 32 x 32 bits: bit c of lane l's word becomes bit l
+// of lane c's.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
+    uint32_t m = 0x0000FFFFu;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1, m ^= m << s) {
+        const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, s);
+        x = (lane & s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y << s) & ~m);
+    }
+    return x;
+}
+
+// cutValueCsr of up to 32 chains of one graph per CTA (end spins: which 0, best:
+// 1): lane c sums chain c.  The chains' spin bits are transposed into one word
+// per vertex (bit c: chain c) in shared memory.  A warp takes 32 rows at a time and
+// loads their entries 32 together; the words of which chains each entry
+// crosses, transposed, give every lane its chain's entries as a bit mask, and
+// its sum of weights is a population count per bit of the weights (one for
+// +-1).  So 32 entries cost 32 chains about 60 instructions.  A CTA takes the
+// slice blockIdx.y of the rows.  Graphs above tableN vertices read the chains'
+// bits directly.  GB300, 1024 chains each of the 50x60 torus and ER n = 2000
+// d = 19: 25 us; one CTA per chain walking all its entries took 87.
+constexpr int kCutWarps = 8;
+__global__ void __launch_bounds__(32 * kCutWarps) chain_cuts_kernel(const DevChain* chains, const DevGraph* graphs,
+                                                                    const CutGroup* groups, const int32_t* order,
+                                                                    int tableN, int which, int64_t* out) {
+    extern __shared__ uint32_t spins[];
+    __shared__ long long part[kCutWarps][32];
+    const CutGroup group = groups[blockIdx.x];
+    const DevGraph& g = graphs[group.graph];
+    const int n = g.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t* offsets = g.offsets;
+    const Edge* edges = g.edges;
+    int c = -1;
+    const uint32_t* bits = nullptr;
+    if (lane < group.count) {
+        c = order[group.first + lane];
+        bits = which ? chains[c].bestBits : chains[c].spinBits;
+    }
+    const bool table = n <= tableN;
+    if (table) {
+#pragma unroll 4
+        for (int w = warp; w < g.words; w += kCutWarps) {
+            const uint32_t x = bits ? bits[w] : 0u;
+            const uint32_t mine = transpose_bits(x, lane);
+            if (32 * w + lane < n) spins[32 * w + lane] = mine;
+        }
+        __syncthreads();
+    }
+    const int slices = gridDim.y;
+    const int v0 = static_cast<int>(static_cast<int64_t>(n) * blockIdx.y / slices);
+    const int v1 = static_cast<int>(static_cast<int64_t>(n) * (blockIdx.y + 1) / slices);
     long long acc = 0;
-    for (int v = threadIdx.x; v < g.n; v += blockDim.x) {
-        const int sv = bit_of(bits, v);
-        for (uint32_t i = g.offsets[v]; i < g.offsets[v + 1]; ++i) {
-            const Edge e = g.edges[i];
-            if (e.col > v && bit_of(bits, e.col) != sv) acc += e.w;
+    for (int base = v0 + 32 * warp; base < v1; base += 32 * kCutWarps) {
+        const int rows = min(32, v1 - base);
+        const uint32_t off = offsets[base + min(lane, rows)];
+        const uint32_t e1 = rows < 32 ? __shfl_sync(0xFFFFFFFFu, off, rows) : offsets[base + 32];
+        for (uint32_t i0 = __shfl_sync(0xFFFFFFFFu, off, 0); i0 < e1; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const Edge e = i < e1 ? edges[i] : Edge{-1, 0};
+            int r = 0;   // the entry's row: the last one that starts at or before it
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const uint32_t o = __shfl_sync(0xFFFFFFFFu, off, (r + step) & 31);
+                if (r + step < rows && o <= i) r += step;
+            }
+            const int v = base + r;
+            const bool up = e.col > v;
+            if (table) {
+                const uint32_t mine = transpose_bits(up ? spins[v] ^ spins[e.col] : 0u, lane);
+                const uint32_t neg = __ballot_sync(0xFFFFFFFFu, e.w < 0);
+                const uint32_t mag = static_cast<uint32_t>(abs(e.w));
+                uint32_t planes = __reduce_or_sync(0xFFFFFFFFu, up ? mag : 0u);
+                for (; planes; planes &= planes - 1) {
+                    const int k = __ffs(planes) - 1;
+                    const uint32_t has = mine & __ballot_sync(0xFFFFFFFFu, (mag >> k) & 1u);
+                    acc += static_cast<long long>(__popc(has & ~neg) - __popc(has & neg)) << k;
+                }
+            } else {
+                for (uint32_t left = __ballot_sync(0xFFFFFFFFu, up); left; left &= left - 1) {
+                    const int j = __ffs(left) - 1;
+                    const int w = __shfl_sync(0xFFFFFFFFu, e.w, j);
+                    const int vj = __shfl_sync(0xFFFFFFFFu, v, j), uj = __shfl_sync(0xFFFFFFFFu, e.col, j);
+                    if (bits && bit_of(bits, vj) != bit_of(bits, uj)) acc += w;
+                }
+            }
         }
     }
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, m);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    part[warp][lane] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0 && c >= 0) {
         long long t = 0;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += part[w];
-        out[c] = t;
+#pragma unroll
+        for (int w = 0; w < kCutWarps; ++w) t += part[w][lane];
+        if (t) atomicAdd(reinterpret_cast<unsigned long long*>(out + c), static_cast<unsigned long long>(t));
     }
 }
 
-// '0'/'1' per vertex of chains [c0, c0 + gridDim.y) into out (row stride).
-__global__ void chain_partitions_kernel(const DevChain* chains, const DevGraph* graphs, int c0,
-                                        int which, char* out, int64_t stride) {
-    const int c = c0 + blockIdx.y;
-    const DevChain& ch = chains[c];
-    const int n = graphs[ch.graph].n;
-    const uint32_t* bits = which ? ch.bestBits : ch.spinBits;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        out[static_cast<int64_t>(blockIdx.y) * stride + v] = bit_of(bits, v) ? '1' : '0';
+// '0'/'1' per vertex, 16 characters a thread (6.1 MB: 9 us, one character a
+// thread 23): bit k of a nibble moves to byte k of 0x30303030 by one multiply.  The rows are one flat array (a thread's 16
+// bytes are aligned whatever the stride); bytes past n are 0.
+__global__ void chain_partitions_kernel(const DevChain* chains, const DevGraph* graphs, int c0, int count, int which,
+                                        char* out, int64_t stride, int64_t total) {
+    for (int64_t at = 16 * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x); at < total;
+         at += 16 * static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        int r = static_cast<int>(at / stride);
+        int64_t v = at - r * stride;
+        const DevChain* ch = chains + c0 + r;
+        int n = graphs[ch->graph].n;
+        const uint32_t* bits = which ? ch->bestBits : ch->spinBits;
+        if (v + 16 <= n) {
+            const uint32_t lo = bits[v >> 5], hi = (v & 31) > 16 ? bits[(v >> 5) + 1] : 0u;
+            const uint32_t x = __funnelshift_r(lo, hi, static_cast<uint32_t>(v) & 31u);
+            uint4 q;
+            q.x = (((x & 15u) * 0x00204081u) & 0x01010101u) + 0x30303030u;
+            q.y = ((((x >> 4) & 15u) * 0x00204081u) & 0x01010101u) + 0x30303030u;
+            q.z = ((((x >> 8) & 15u) * 0x00204081u) & 0x01010101u) + 0x30303030u;
+            q.w = ((((x >> 12) & 15u) * 0x00204081u) & 0x01010101u) + 0x30303030u;
+            *reinterpret_cast<uint4*>(out + at) = q;
+        } else {
+            for (int k = 0; k < 16 && at + k < total; ++k) {
+                out[at + k] = v < n ? (bit_of(bits, static_cast<int>(v)) ? '1' : '0') : '\0';
+                if (++v == stride && at + k + 1 < total) {
+                    v = 0;
+                    ++ch;
+                    n = graphs[ch->graph].n;
+                    bits = which ? ch->bestBits : ch->spinBits;
+                }
+            }
+        }
+    }
 }
 
 }  // namespace
 
 namespace rfmf {
 
-cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, int C, int which,
-                              int64_t* out, cudaStream_t st) {
-    if (C <= 0) return cudaSuccess;
-    chain_cuts_kernel<<<C, 256, 0, st>>>(chains, graphs, C, which, out);
+cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutGroup* groups, int ngroups,
+                              const int32_t* order, int maxN, int sms, int smemOptin, int which, int64_t* out,
+                              cudaStream_t st) {
+    if (ngroups <= 0) return cudaSuccess;
+    // About four CTAs per SM in all.
+    const int slices = std::max(1, std::min(64, (4 * sms + ngroups - 1) / ngroups));
+    const int tableN = std::min(maxN, (smemOptin - 4096) / 4);
+    const int smem = 4 * tableN;
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&chain_cuts_kernel),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smemOptin - 4096);
+    if (e != cudaSuccess) return e;
+    for (int g0 = 0; g0 < ngroups; g0 += 1 << 20) {
+        const dim3 grid(static_cast<unsigned>(std::min(ngroups - g0, 1 << 20)), static_cast<unsigned>(slices));
+        chain_cuts_kernel<<<grid, 32 * kCutWarps, smem, st>>>(chains, graphs, groups + g0, order, tableN, which, out);
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count,
-                                    int maxN, int which, char* out, int64_t stride, cudaStream_t st) {
+cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count, int which,
+                                    char* out, int64_t stride, cudaStream_t st) {
     if (count <= 0) return cudaSuccess;
-    const dim3 grid(static_cast<unsigned>(std::min(64, (maxN + 255) / 256)), static_cast<unsigned>(count));
-    chain_partitions_kernel<<<grid, 256, 0, st>>>(chains, graphs, c0, which, out, stride);
+    const int64_t total = static_cast<int64_t>(count) * stride;
+    const int64_t blocks = std::min<int64_t>((total + 16 * 256 - 1) / (16 * 256), 1 << 16);
+    chain_partitions_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(chains, graphs, c0, count, which, out,
+                                                                           stride, total);
     return cudaGetLastError();
 }
 
