@@ -52,6 +52,7 @@ struct Request {
     ChainBeta beta;                   // the context's shared device beta tables
     // launch class
     int dbytes = 1, fmt = kCsrGlobal, W = 1;
+    int wMin = 1, wMax = 1;           // widths a window may run it at (wMin <= W <= wMax)
     bool s64 = false;
     int64_t devBytes = 0;             // request_device_bytes: counted against max_device_bytes
     // device state (worker thread only)
@@ -347,16 +348,95 @@ int harvest(rfmf_server* s, Request& r) {
     return RFMF_OK;
 }
 
+// Estimated us per sweep of a request at W warps per chain, few chains per SM.
+// GB300, measured / this, averaged over P = 128, 32, 8 and 1: ER n = 2000 d = 19
+// W = 1 2.5 / 2.9, W = 4 1.8 / 1.9; ER n = 5000 d = 5 3.6 / 4.1 and 2.1 / 2.2;
+// 100x200 torus 11.7 / 11.6 and 4.1 / 4.0, W = 8 3.4 / 2.8.
+double sweep_us(const Request& r, int W) {
+    const double n = static_cast<double>(r.n);
+    double rows = 0.0, sweeps = 0.0;
+    for (size_t p = 0; p < r.phaseP.size(); ++p) {
+        if (!r.phaseP[p]) continue;
+        rows += static_cast<double>(r.phaseIters[p]) * std::min(static_cast<double>(r.phaseP[p]), n);
+        sweeps += static_cast<double>(r.phaseIters[p]);
+    }
+    return 1.5 + 0.5e-3 * (n + rows / std::max(sweeps, 1.0) * 2.0 * static_cast<double>(r.g->m) / std::max(n, 1.0)) / W;
+}
+
+// Requests on several graphs running side by side: a window lasts as long as its
+// slowest request, so each gets the narrowest width that keeps it within the
+// least time that 14 warps per SM allow all of them, and graphs of 4096 vertices
+// on walk their rows in HBM, where their CSR copies crowd out the others'
+// chains.  Up to ten chains per SM: beyond, every width is down to one warp and
+// the copies pay.  True when it applies; false leaves the requests' own widths
+// (the load at their submission) and formats.  GB300, ms for 2,400 sweeps, own /
+// this: eight graphs n 5000..20,000, 330 chains 20.0 / 10.9, 790 28.5 / 19.9, 1300
+// 32.9 / 27.0 (2600: 52.9 / 65.5); eight graphs n 800..12,000 x 64 11.5 / 10.1, x
+// 128 25.6 / 17.9; 32 graphs n 2000..9000 x 16 13.1 / 10.0; 16 graphs n 800..1633
+// 10.1 / 8.5.  With 16 warps per SM the second was 22.3, with rows in shared
+// memory where they fit 24.1, with every graph's in HBM the last but one 9.9 and
+// four graphs n 800..3000 7.6 instead of 5.9.
+constexpr int64_t kMixedHbmN = 4096;
+bool mixed_widths(const rfmf_server* s, std::vector<int>& width) {
+    const std::vector<ReqPtr>& run = s->running;
+    const int64_t sms = std::max(s->ctx->sms, 1);
+    int64_t chains = 0;
+    bool mixed = false;
+    width.clear();
+    for (const ReqPtr& r : run) {
+        width.push_back(r->W);
+        chains += r->C;
+        mixed = mixed || r->graphSlot != run[0]->graphSlot;
+    }
+    if (!mixed || s->lc.csr_format || s->lc.threads_per_chain || chains > 10 * sms) return false;
+    std::vector<std::vector<double>> us(run.size());   // at wMin, 2 wMin, ..
+    std::vector<double> taus;
+    for (size_t i = 0; i < run.size(); ++i)
+        for (int W = run[i]->wMin; W <= run[i]->wMax; W *= 2) {
+            us[i].push_back(sweep_us(*run[i], W));
+            taus.push_back(us[i].back());
+        }
+    std::sort(taus.begin(), taus.end());
+    std::vector<int> trial(run.size());
+    auto fits = [&](double tau) {
+        int64_t warps = 0;
+        for (size_t i = 0; i < run.size(); ++i) {
+            size_t w = 0;
+            while (w < us[i].size() && us[i][w] > tau) ++w;
+            if (w == us[i].size()) return false;
+            trial[i] = run[i]->wMin << w;
+            warps += run[i]->C * trial[i];
+        }
+        return warps <= 14 * sms;
+    };
+    size_t lo = 0, hi = taus.size();   // the least tau that fits is in [lo, hi]
+    while (lo < hi) {
+        const size_t mid = (lo + hi) / 2;
+        if (fits(taus[mid])) hi = mid; else lo = mid + 1;
+    }
+    if (lo == taus.size() || !fits(taus[lo])) return false;
+    width = trial;
+    return true;
+}
+
 // One window over the running requests: one launch per launch class, the
 // classes side by side on their own streams (a class that fills only part
 // of the GPU no longer leaves the rest idle while the next one waits).
 // Each class has its own work items, item order and queue/error words.
 int run_window(rfmf_server* s, int64_t& launches, float& ms) {
     std::map<ClassKey, std::vector<Request*>> classes;
-    for (const ReqPtr& r : s->running) classes[ClassKey{r->dbytes, r->fmt, r->W, r->s64}].push_back(r.get());
+    std::vector<int> width;
+    const bool mixed = mixed_widths(s, width);
+    for (size_t i = 0; i < s->running.size(); ++i) {
+        Request* r = s->running[i].get();
+        classes[ClassKey{r->dbytes, mixed && r->n >= kMixedHbmN ? hbm_format(r->g) : r->fmt, width[i], r->s64}].push_back(r);
+    }
     launches = 0;
     ms = 0.0f;
     const int ncls = static_cast<int>(classes.size());
+    double warps = 0.0;
+    for (const auto& kv : classes)
+        for (const Request* r : kv.second) warps += static_cast<double>(r->C) * kv.first.W;
     int64_t need = 0;
     for (const ReqPtr& r : s->running) need += r->C;
     if (need > s->itemCap) {
@@ -397,7 +477,7 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
     std::vector<int32_t> order;
     int ci = 0;
     for (auto& kv : classes) {
-        const ClassKey& k = kv.first;
+        ClassKey k = kv.first;
         std::vector<Request*>& reqs = kv.second;
         int maxN = 0, maxWords = 0, pmax = 1;
         int layout = k.s64 ? kLayoutSlots : kLayoutMain;
@@ -409,12 +489,19 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
             if (r->table && layout == kLayoutMain) layout = kLayoutAny;
             csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
         }
+        auto chain_bytes = [&](int kind) { return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total; };
+        // The largest copy beside the largest graph's chain may not fit though
+        // each request fits by itself: the class then walks HBM.
+        if (s->lc.csr_format == 0 && !csr_in_hbm(k.fmt) && static_cast<int64_t>(kSmemHeader) + csrB +
+                std::min(chain_bytes(layout), chain_bytes(kLayoutSlots)) > s->ctx->smemOptin) {
+            k.fmt = k.fmt == kCsrUnit16 ? kCsrGlobal16 : kCsrGlobal32;
+            csrB = 0;
+        }
         const void* kern = kernel_ptr(k.dbytes, k.fmt, k.s64, k.W);
         if (int rc = ensure_attr(s, kern)) return rc;
         cudaFuncAttributes fa{};
         CU(cudaFuncGetAttributes(&fa, kern));
         const int64_t dynMax = s->ctx->smemOptin - static_cast<int64_t>(fa.sharedSizeBytes);
-        auto chain_bytes = [&](int kind) { return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total; };
         uint32_t chainB = chain_bytes(layout);
         const int kCap = std::min(std::min(16 / k.W, k.W > 1 ? 15 : 16), fa.maxThreadsPerBlock / (32 * k.W));
         const int64_t room = dynMax - kSmemHeader - csrB;
@@ -425,31 +512,45 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         const int Kmax = room > 0 ? static_cast<int>(std::min<int64_t>(kCap, room / chainB)) : 0;
         if (Kmax < 1)
             return fail(RFMF_ERR_CAPACITY, "launch class needs %u B CSR + %u B per chain", csrB, chainB);
-        int occ = 0, Kshape = Kmax;
-        for (; Kshape >= 1; --Kshape) {
-            const size_t smem = kSmemHeader + csrB + static_cast<size_t>(Kshape) * chainB;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * k.W * Kshape, smem) !=
-                cudaSuccess) {
+        auto resident = [&](int K) {
+            int blocks = 0;
+            const size_t smem = kSmemHeader + csrB + static_cast<size_t>(K) * chainB;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, 32 * k.W * K, smem) != cudaSuccess) {
                 cudaGetLastError();
-                occ = 0;
+                blocks = 0;
             }
-            if (occ > 0) break;
-        }
-        if (Kshape < 1) return fail(RFMF_ERR_CAPACITY, "no resident configuration for a launch class");
+            return blocks;
+        };
+        int Kshape = Kmax, occ = resident(Kshape);
+        while (occ == 0 && Kshape > 1) occ = resident(--Kshape);
+        if (occ == 0) return fail(RFMF_ERR_CAPACITY, "no resident configuration for a launch class");
         // Chains grouped by graph; items of K chains, K the smallest that
         // keeps all items resident (else Kshape).
         std::map<int, std::vector<int32_t>> byGraph;
         for (Request* r : reqs)
             for (int64_t c = 0; c < r->C; ++c)
                 byGraph[r->graphSlot].push_back(static_cast<int32_t>(r->slot0 + c));
-        const int64_t slotsRes = static_cast<int64_t>(occ) * s->ctx->sms;
+        int64_t slotsRes = static_cast<int64_t>(occ) * s->ctx->sms;
         auto items_for = [&](int K) {
             int64_t it = 0;
             for (auto& g : byGraph) it += (static_cast<int64_t>(g.second.size()) + K - 1) / K;
             return it;
         };
         int K = 1;
-        while (K < Kshape && items_for(K) > slotsRes) ++K;
+        if (ncls == 1) {
+            while (K < Kshape && items_for(K) > slotsRes) ++K;
+        } else {
+            // CTAs of the items' own size, so that the classes fill the SMs
+            // together: the smallest that keeps this class's items resident in
+            // its share of them.
+            double mine = 0.0;
+            for (Request* r : reqs) mine += static_cast<double>(r->C) * k.W;
+            while (K < Kshape &&
+                   static_cast<double>(items_for(K)) > resident(K) * static_cast<double>(s->ctx->sms) * mine / warps)
+                ++K;
+            Kshape = K;
+            slotsRes = static_cast<int64_t>(resident(K)) * s->ctx->sms;
+        }
         const size_t item0 = items.size(), order0 = order.size();
         for (auto& g : byGraph) {
             const std::vector<int32_t>& ch = g.second;
@@ -864,6 +965,23 @@ static int rfmf_submit_impl(rfmf_server* s, const rfmf_graph* g, int64_t nchains
             return fail(RFMF_ERR_CAPACITY, "one chain needs %u B of shared memory", leastB);
     }
     r->fmt = fmt;
+    // Other widths that its score path and shared memory allow.
+    r->wMin = r->wMax = r->W;
+    if (c.threads_per_chain == 0 && !r->s64 && !r->table) {
+        auto safe = [&](int W) {
+            for (int64_t k = 0; k < nchains; ++k)
+                if (!compact_key_safe(static_cast<int64_t>(total), t0s[k], g->B, key_bits(g->n, 32 * W))) return false;
+            return true;
+        };
+        while (r->wMin > 1 && safe(r->wMin / 2)) r->wMin /= 2;
+        const int widest = choose_warps(static_cast<int>(g->n), c, nchains, s->ctx->sms);
+        while (2 * r->wMax <= widest) {
+            const uint32_t b = chain_layout(static_cast<int>(g->n), static_cast<int>(r->words), r->pmax, 2 * r->wMax,
+                                            r->dbytes, kLayoutMain).total;
+            if (static_cast<int64_t>(kSmemHeader) + b > s->ctx->smemOptin - 1024) break;
+            r->wMax *= 2;
+        }
+    }
     if (nchains * r->words > (int64_t(1) << 34)) return fail(RFMF_ERR_CAPACITY, "request too large");
     r->initBits.assign(static_cast<size_t>(nchains * r->words), 0u);
     for (int64_t k = 0; k < nchains; ++k)

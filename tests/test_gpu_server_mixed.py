@@ -1,0 +1,62 @@
+"""Requests on several graphs in one window: each runs at its own width and, from
+4096 vertices on, walks its rows in HBM, in windows whose widths change as
+requests come and go.  The results must stay those of a standalone call."""
+import numpy as np
+import pytest
+
+from conftest import chains_for
+
+pytestmark = pytest.mark.gpu
+
+MIXES = {
+    # the largest graph wide, the small ones narrow; both sides of 4096 vertices
+    "sizes": [("torus", 4095, 40, 1), ("torus", 4100, 30, 1), ("torus", 14000, 12, 1), ("er", 700, 200, 1),
+              ("er", 65, 3, 1)],
+    # a copy that leaves little room beside a class mate's larger chains
+    "crowded": [("dense", 1200, 2, 1), ("torus", 4000, 2, 1), ("er", 900, 1, 1)],
+    # int32 gains and 32-bit entries beside int8
+    "weights": [("er", 900, 24, 300), ("torus", 5000, 24, 1), ("torus", 5000, 16, 300)],
+    # more than ten chains per SM: the requests' own widths, several classes
+    "many": [("er", 300, 900, 1), ("torus", 4200, 300, 1), ("er", 600, 800, 40)],
+}
+
+
+def _graph(rfmf, kind, n, wmax, seed):
+    if kind == "torus":
+        rows = next(k for k in range(int(n ** 0.5), 0, -1) if n % k == 0)
+        g = rfmf.torus(rows, n // rows, signed=True, seed=seed)
+    else:
+        g = rfmf.erdos_renyi_degree(n, 8 if kind == "er" else 76, signed=True, seed=seed)
+    if wmax > 1:
+        rng = np.random.default_rng(seed)
+        m = {}
+        src = np.repeat(np.arange(g.n), np.diff(g.offsets.astype(np.int64)))
+        w = np.empty_like(g.weight)
+        for i, (a, b) in enumerate(zip(src, g.col)):
+            key = (min(a, b), max(a, b))
+            if key not in m:
+                m[key] = int(rng.integers(1, wmax + 1)) * (1 if rng.random() < 0.5 else -1)
+            w[i] = m[key]
+        g.weight = w
+    return g
+
+
+@pytest.mark.parametrize("name", sorted(MIXES))
+def test_mixed_requests_match_standalone(rfmf, ctx, name):
+    srv = rfmf.Server(ctx, window_sweeps=37)
+    reqs = []
+    for k, (kind, n, C, wmax) in enumerate(MIXES[name]):
+        g = _graph(rfmf, kind, n, wmax, 11 + k)
+        init, solver = chains_for(g, list(range(1000 * k, 1000 * k + C)))
+        t0s = [(35.0, 70.0, 200.0, 400.0)[c % 4] * (1 if wmax == 1 else 100) for c in range(C)]
+        reqs.append((g, rfmf.DeviceGraph(ctx, g), init, solver, t0s, [128, 16, 1], [40 + 30 * k, 25, 20]))
+    ids = [srv.submit(dg, init, t0s, ph, it, solver) for _, dg, init, solver, t0s, ph, it in reqs]
+    for rid, (g, dg, init, solver, t0s, ph, it) in zip(ids, reqs):
+        st = srv.wait(rid, timeout=300)
+        assert st["state"] == "done"
+        a = srv.result(rid)
+        b = rfmf.anneal_gpu(ctx, dg, g.max_weighted_degree(), init, t0s, ph, it, solver)
+        assert np.array_equal(a.end_spins, b.end_spins)
+        assert np.array_equal(a.best_spins, b.best_spins)
+        assert np.array_equal(a.best_vals, b.best_vals)
+        assert np.array_equal(a.final_vals, b.final_vals)
