@@ -49,6 +49,7 @@ struct BatchClass {
     int dbytes = 1, fmt = kCsrGlobal, warps = 1;
     int baseWarps = 1;           // the planner's width; `warps` may double per phase
     int K = 1, threads = 32, grid = 0, occ = 1, nitems = 0, pmax = 1;
+    double share = 1.0;          // of the SMs, among classes whose widths were chosen together
     size_t smem = 0;
     std::vector<int> graphs;                      // batch graph indices
     std::vector<std::vector<int32_t>> chainsOf;   // per class graph: chain ids
@@ -92,6 +93,7 @@ struct rfmf_batch {
     int64_t launches = 0;        // kernel launches enqueued (captured ones when replayed)
     rfmf_launch_config cfg{};    // the creation config (re-planning per phase)
     bool phaseWarps = false;     // the one class's width follows the phase
+    bool shared = false;         // widths chosen together: each class gets its share of the SMs
     ~rfmf_batch() {
         if (graphExec) cudaGraphExecDestroy(graphExec);
         for (BatchClass& k : cls) {
@@ -180,9 +182,18 @@ int plan_class(rfmf_batch& b, BatchClass& k, const rfmf_launch_config& c, bool e
     // Smallest uniform K whose items all fit the resident CTA slots.
     int Kuni = c.chains_per_cta ? Kshape : 1;
     if (exact) {
+        if (b.shared) {
+            double all = 0.0, mine = 0.0;
+            for (const BatchClass& o : b.cls)
+                for (const auto& ch : o.chainsOf) {
+                    all += static_cast<double>(ch.size()) * o.warps;
+                    if (&o == &k) mine += static_cast<double>(ch.size()) * o.warps;
+                }
+            k.share = mine / all;
+        }
         for (; Kuni < Kshape; ++Kuni) {
             const int o = occ_for(Kuni);
-            if (o > 0 && items_for(Kuni) <= static_cast<int64_t>(o) * sms) break;
+            if (o > 0 && static_cast<double>(items_for(Kuni)) <= k.share * o * sms) break;
         }
         Kshape = Kuni;
         occ = occ_for(Kshape);
@@ -353,7 +364,7 @@ double item_cost(const rfmf_batch& b, const BatchClass& k, size_t q, uint32_t P,
 bool plan_balanced(const rfmf_batch& b, const BatchClass& k, uint32_t P, std::vector<int>& kg) {
     const size_t G = k.graphs.size();
     const bool alone = b.cls.size() == 1;
-    const int64_t slots = static_cast<int64_t>(k.occ) * b.ctx->sms;
+    const int64_t slots = static_cast<int64_t>(k.share * k.occ * b.ctx->sms);
     // One graph: its uniform items are right unless even full ones need
     // more than one round (then the list schedule decides, as below).
     if (G == 0 || (G == 1 && !(alone && (static_cast<int64_t>(k.chainsOf[0].size()) + k.K - 1) / k.K > slots)))
@@ -721,9 +732,9 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     using Key = std::tuple<int, int, int, int>;   // dbytes, fmt, W, s64
     std::map<Key, int> classOf;
     std::vector<int> graphClass(G);
-    // hbm: every graph's rows are walked in HBM; width: warps per chain of all
-    // graphs (0: the rule for each).
-    auto classify = [&](bool hbm, int width) -> int {
+    // Graphs of at least hbmN vertices walk their rows in HBM; width: warps per
+    // chain of each graph (empty: the rule for each).
+    auto classify = [&](int64_t hbmN, const std::vector<int>& width) -> int {
         classOf.clear();
         b->cls.clear();
         for (size_t gi = 0; gi < G; ++gi) {
@@ -776,7 +787,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 } else if (c.csr_format == 2) {
                     if (!g->packed32) return fail(RFMF_ERR_INVALID, "packed32 CSR needs |w| < 2^15 and n <= 65536");
                     pk.fmt = kCsrPacked32;
-                } else if (c.csr_format == 0 && !hbm) {
+                } else if (c.csr_format == 0 && g->n < hbmN) {
                     if (g->unit16 && fits(kCsrUnit16)) pk.fmt = kCsrUnit16;
                     else if (g->packed32 && fits(kCsrPacked32)) pk.fmt = kCsrPacked32;
                 }
@@ -791,7 +802,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 pk.resident = std::max<int64_t>(0, std::min<int64_t>({perSm, warpCap, room / chainB}));
                 return RFMF_OK;
             };
-            int W = width ? width : choose_warps(static_cast<int>(g->n), c, b->C, ctx->sms);
+            int W = width.size() ? width[gi] : choose_warps(static_cast<int>(g->n), c, b->C, ctx->sms);
             Pick pk;
             if (int rc = pick(W, pk)) return rc;
             // When shared memory (not the chain count) keeps an SM's chains from
@@ -802,7 +813,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             // one-warp chains per SM: deeper queues keep every warp slot busy
             // anyway and one warp per chain does more per slot (512 graphs x 64
             // chains: 1.52e8 -> 1.44e8 when widened).
-            if (c.threads_per_chain == 0 && width == 0 && perSm <= 32) {
+            if (c.threads_per_chain == 0 && width.empty() && perSm <= 32) {
                 while (W < kMaxAutoWarps && pk.resident < perSm) {
                     Pick wider;
                     if (int rc = pick(2 * W, wider)) return rc;
@@ -832,7 +843,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         }
         return RFMF_OK;
     };
-    if (int rc = classify(false, 0)) return rc;
+    if (int rc = classify(INT64_MAX, {})) return rc;
     // A shared-memory class's CTA holds the class's largest CSR beside K
     // chains sized for its largest graph.  While that leaves room for fewer
     // chains than a CTA should hold (as above, over the class), the graph
@@ -911,26 +922,58 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     };
     if (c.csr_format == 0) spread();
     // Several classes share the SMs, each sized as if alone: their CSR copies
-    // crowd the chains out of shared memory.  Up to two chains per SM, and from
-    // sixteen on, such a batch walks every graph's rows in HBM instead; between
-    // two and five per SM, at four warps per chain for all, so that (but for
-    // gain widths) it is one class whose items the work queue levels.  Only
-    // with graphs whose copies are large (4096 vertices).  GB300, ms for 1,200
-    // sweeps, before / this: 16 graphs n 807..14,000 x 4 chains 3.4 / 3.5, x 16
-    // 5.1 / 4.1, x 48 10.3 / 7.2, x 160 19.8 / 15.5, x 300 26.8 / 23.7; three
-    // sparse graphs x 64 4.9 / 4.2, x 256 13.7 / 9.7; four graphs n 11,000 to
-    // 17,000 x 200 14.1 / 12.6; 64 graphs x 64 18.5 / 15.1 (between five and
-    // sixteen per SM neither form is always ahead: 64 graphs x 16 7.9 / 8.8, 16
-    // graphs x 96 12.9 / 11.9).
+    // crowd the chains out of shared memory, and the narrowest class may hold the
+    // largest graph.  With graphs whose copies are large (4096 vertices), by the
+    // chains per SM:
+    // - up to two, and from sixteen on: every graph's rows in HBM, widths as they
+    //   were;
+    // - from two to 5.25: in HBM, four warps per chain for all, so that (but for
+    //   gain widths) it is one class whose items the work queue levels;
+    // - up to twelve: widths chosen together (common_widths), rows in HBM from
+    //   4096 vertices on, while the chains leave a fifth of the SMs' shared memory
+    //   free (else they come in rounds, which classes of full CTAs do better).
+    // GB300, ms for 1,200 sweeps, before / HBM: 16 graphs n 807..14,000 x 4 chains
+    // 3.4 / 3.5, x 16 5.1 / 4.1; 64 graphs x 64 18.5 / 15.1.  For 2,400 sweeps,
+    // before / four warps / widths together: those 16 graphs x 20 18.1 / 8.1 /
+    // 9.0, x 32 18.7 / 9.9 / 9.3, x 48 21.2 / 14.4 / 12.9 (44.7 and 47.7 for 8,000
+    // once costs are learned), x 64 23.4 / - / 14.2, x 96 29.3 / - / 22.2; three sparse graphs n 5000..20,000 x 128 - / 12.5 /
+    // 12.0, x 256 27.4 / 19.4 / 20.3, x 400 (97% of shared memory) 33.1 / - /
+    // 37.7; 64 graphs n 600..14,000 x 8 19.6 / 10.3 / 11.3, x 16 25.1 / - / 16.4;
+    // eight graphs n 5000..20,000 x 128 34.7 / - / 26.0.
     if (b->cls.size() > 1 && c.csr_format == 0 && c.threads_per_chain == 0) {
-        int64_t maxN = 0;
-        for (const rfmf_graph* g : b->glist) maxN = std::max(maxN, g->n);
         const int64_t sms = std::max(ctx->sms, 1);
         const bool few = b->C <= 2 * sms, some = 4 * b->C <= 21 * sms, many = b->C >= 16 * sms;
-        if (maxN >= 4096 && (few || some || many)) {
-            if (classify(true, !few && some ? kMaxAutoWarps : 0) != RFMF_OK) {
-                // int32 scores asked for that this width has no room for
-                if (int rc = classify(false, 0)) return rc;
+        int64_t maxN = 0, bytes = 0;
+        std::vector<WidthAsk> asks;
+        for (size_t gi = 0; gi < G; ++gi) {
+            const rfmf_graph* g = b->glist[gi];
+            const int n = static_cast<int>(g->n);
+            const int64_t chains = static_cast<int64_t>(chainsOfGraph[gi].size());
+            auto safe = [&](int W) {
+                for (int32_t ch : chainsOfGraph[gi])
+                    if (!compact_key_safe(static_cast<int64_t>(total), t0s[ch], g->B, key_bits(g->n, 32 * W)))
+                        return false;
+                return true;
+            };
+            const int widest = choose_warps(n, c, chains, ctx->sms);
+            int least = widest;
+            if (c.score_path != 2 && safe(widest))
+                while (least > 1 && safe(least / 2)) least /= 2;
+            asks.push_back(width_ask(g, chains, least, widest, b->phaseP, b->phaseIters));
+            const int dbytes = c.gain_width ? c.gain_width : (g->B <= 127 ? 1 : 4);
+            bytes += chains * chain_layout(n, (n + 31) / 32, 1, 2, dbytes, kLayoutMain).total;
+            maxN = std::max(maxN, g->n);
+        }
+        std::vector<int> width;
+        const bool together = !some && b->C <= 12 * sms && bytes <= 4 * sms * (static_cast<int64_t>(ctx->smemOptin) / 5) &&
+                              maxN >= 4096 && common_widths(asks, ctx->sms, width);
+        if (maxN >= 4096 && (few || some || many || together)) {
+            const int rc = together     ? classify(kMixedHbmN, width)
+                           : few || many ? classify(0, {})
+                                         : classify(0, std::vector<int>(G, kMaxAutoWarps));
+            b->shared = together && rc == RFMF_OK;
+            if (rc != RFMF_OK) {   // int32 scores asked for that such a width has no room for
+                if (int rc2 = classify(INT64_MAX, {})) return rc2;
                 spread();
             }
         }

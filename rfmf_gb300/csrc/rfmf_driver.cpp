@@ -685,6 +685,58 @@ int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms)
     return W;
 }
 
+WidthAsk width_ask(const rfmf_graph* g, int64_t chains, int least, int widest, const std::vector<uint32_t>& phaseP,
+                   const std::vector<uint64_t>& phaseIters) {
+    const double n = static_cast<double>(std::max<int64_t>(g->n, 1));
+    double rows = 0.0, sweeps = 0.0;
+    for (size_t p = 0; p < phaseP.size(); ++p) {
+        if (!phaseP[p]) continue;
+        rows += static_cast<double>(phaseIters[p]) * std::min(static_cast<double>(phaseP[p]), n);
+        sweeps += static_cast<double>(phaseIters[p]);
+    }
+    return WidthAsk{chains, least, widest, n, rows / std::max(sweeps, 1.0) * 2.0 * static_cast<double>(g->m) / n};
+}
+
+// Chains of several graphs running side by side: the launches last as long as
+// the slowest graph's, so each graph gets the narrowest width that keeps it
+// within the least time per sweep that 14 warps per SM allow all of them.  Time
+// is estimated as 1.5 us + 0.5 ns per vertex and winner-row entry, the latter
+// over the chain's warps.  GB300, measured / estimated, few chains per SM,
+// averaged over P = 128, 32, 8 and 1: ER n = 2000 d = 19 W = 1 2.5 / 2.9, W = 4
+// 1.8 / 1.9; ER n = 5000 d = 5 3.6 / 4.1 and 2.1 / 2.2; 100x200 torus 11.7 / 11.6
+// and 4.1 / 4.0, W = 8 3.4 / 2.8.  False, and `width` as it was, where even the
+// narrowest widths hold more warps.
+bool common_widths(const std::vector<WidthAsk>& asks, int sms, std::vector<int>& width) {
+    std::vector<std::vector<double>> us(asks.size());   // at least, 2 least, ..
+    std::vector<double> taus;
+    for (size_t i = 0; i < asks.size(); ++i)
+        for (int W = asks[i].least; W <= asks[i].widest; W *= 2) {
+            us[i].push_back(asks[i].us(W));
+            taus.push_back(us[i].back());
+        }
+    std::sort(taus.begin(), taus.end());
+    std::vector<int> trial(asks.size());
+    auto fits = [&](double tau) {
+        int64_t warps = 0;
+        for (size_t i = 0; i < asks.size(); ++i) {
+            size_t w = 0;
+            while (w < us[i].size() && us[i][w] > tau) ++w;
+            if (w == us[i].size()) return false;
+            trial[i] = asks[i].least << w;
+            warps += asks[i].chains * trial[i];
+        }
+        return warps <= 14 * static_cast<int64_t>(sms);
+    };
+    size_t lo = 0, hi = taus.size();   // the least time that fits is in [lo, hi]
+    while (lo < hi) {
+        const size_t mid = (lo + hi) / 2;
+        if (fits(taus[mid])) hi = mid; else lo = mid + 1;
+    }
+    if (lo == taus.size() || !fits(taus[lo])) return false;
+    width = trial;
+    return true;
+}
+
 // Bits of the block-iteration field of the compact int32 key (kernel
 // key_bits): ceil(log2(blocks per thread)), at least 4.
 int key_bits(int64_t n, int T) {

@@ -111,6 +111,18 @@ constexpr int kMaxLatencyWarps = 8;   // widest chain the planner picks for few 
 // SM's four schedulers (warp w issues from scheduler w mod 4).
 inline int sched_level(int chains, int warps) { return (chains * warps + 3) / 4; }
 int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms);
+// One graph's chains among those that run side by side (see common_widths).
+struct WidthAsk {
+    int64_t chains;
+    int least, widest;   // widths its score path and shared memory allow
+    double n, entries;   // vertices; entries of a sweep's winner rows, averaged over the phases
+    double us(int W) const { return 1.5 + 0.5e-3 * (n + entries) / W; }   // per sweep
+};
+WidthAsk width_ask(const rfmf_graph* g, int64_t chains, int least, int widest, const std::vector<uint32_t>& phaseP,
+                   const std::vector<uint64_t>& phaseIters);
+bool common_widths(const std::vector<WidthAsk>& asks, int sms, std::vector<int>& width);
+// Graphs of at least this many vertices walk their rows in HBM there.
+constexpr int64_t kMixedHbmN = 4096;
 int key_bits(int64_t n, int T);
 bool compact_key_safe(int64_t total, double t0, int64_t B, int kb);
 

@@ -348,75 +348,32 @@ int harvest(rfmf_server* s, Request& r) {
     return RFMF_OK;
 }
 
-// Estimated us per sweep of a request at W warps per chain, few chains per SM.
-// GB300, measured / this, averaged over P = 128, 32, 8 and 1: ER n = 2000 d = 19
-// W = 1 2.5 / 2.9, W = 4 1.8 / 1.9; ER n = 5000 d = 5 3.6 / 4.1 and 2.1 / 2.2;
-// 100x200 torus 11.7 / 11.6 and 4.1 / 4.0, W = 8 3.4 / 2.8.
-double sweep_us(const Request& r, int W) {
-    const double n = static_cast<double>(r.n);
-    double rows = 0.0, sweeps = 0.0;
-    for (size_t p = 0; p < r.phaseP.size(); ++p) {
-        if (!r.phaseP[p]) continue;
-        rows += static_cast<double>(r.phaseIters[p]) * std::min(static_cast<double>(r.phaseP[p]), n);
-        sweeps += static_cast<double>(r.phaseIters[p]);
-    }
-    return 1.5 + 0.5e-3 * (n + rows / std::max(sweeps, 1.0) * 2.0 * static_cast<double>(r.g->m) / std::max(n, 1.0)) / W;
-}
-
-// Requests on several graphs running side by side: a window lasts as long as its
-// slowest request, so each gets the narrowest width that keeps it within the
-// least time that 14 warps per SM allow all of them, and graphs of 4096 vertices
-// on walk their rows in HBM, where their CSR copies crowd out the others'
-// chains.  Up to ten chains per SM: beyond, every width is down to one warp and
-// the copies pay.  True when it applies; false leaves the requests' own widths
-// (the load at their submission) and formats.  GB300, ms for 2,400 sweeps, own /
-// this: eight graphs n 5000..20,000, 330 chains 20.0 / 10.9, 790 28.5 / 19.9, 1300
-// 32.9 / 27.0 (2600: 52.9 / 65.5); eight graphs n 800..12,000 x 64 11.5 / 10.1, x
-// 128 25.6 / 17.9; 32 graphs n 2000..9000 x 16 13.1 / 10.0; 16 graphs n 800..1633
-// 10.1 / 8.5.  With 16 warps per SM the second was 22.3, with rows in shared
-// memory where they fit 24.1, with every graph's in HBM the last but one 9.9 and
-// four graphs n 800..3000 7.6 instead of 5.9.
-constexpr int64_t kMixedHbmN = 4096;
+// Requests on several graphs running side by side get their widths together
+// (common_widths), and the larger graphs walk their rows in HBM, where their CSR
+// copies crowd out the others' chains.  Up to ten chains per SM: beyond, every
+// width is down to one warp and the copies pay.  True when it applies; false
+// leaves the requests' own widths (the load at their submission) and formats.
+// GB300, ms for 2,400 sweeps, own / this: eight graphs n 5000..20,000, 330 chains
+// 20.0 / 10.9, 790 28.5 / 19.9, 1300 32.9 / 27.0 (2600: 52.9 / 65.5); eight
+// graphs n 800..12,000 x 64 11.5 / 10.1, x 128 25.6 / 17.9; 32 graphs n 2000..9000
+// x 16 13.1 / 10.0; 16 graphs n 800..1633 10.1 / 8.5.  With 16 warps per SM the
+// second was 22.3, with rows in shared memory where they fit 24.1; every graph's
+// in HBM made four graphs n 800..3000 7.6 instead of 5.9.
 bool mixed_widths(const rfmf_server* s, std::vector<int>& width) {
     const std::vector<ReqPtr>& run = s->running;
-    const int64_t sms = std::max(s->ctx->sms, 1);
     int64_t chains = 0;
     bool mixed = false;
+    std::vector<WidthAsk> asks;
     width.clear();
     for (const ReqPtr& r : run) {
         width.push_back(r->W);
         chains += r->C;
         mixed = mixed || r->graphSlot != run[0]->graphSlot;
     }
-    if (!mixed || s->lc.csr_format || s->lc.threads_per_chain || chains > 10 * sms) return false;
-    std::vector<std::vector<double>> us(run.size());   // at wMin, 2 wMin, ..
-    std::vector<double> taus;
-    for (size_t i = 0; i < run.size(); ++i)
-        for (int W = run[i]->wMin; W <= run[i]->wMax; W *= 2) {
-            us[i].push_back(sweep_us(*run[i], W));
-            taus.push_back(us[i].back());
-        }
-    std::sort(taus.begin(), taus.end());
-    std::vector<int> trial(run.size());
-    auto fits = [&](double tau) {
-        int64_t warps = 0;
-        for (size_t i = 0; i < run.size(); ++i) {
-            size_t w = 0;
-            while (w < us[i].size() && us[i][w] > tau) ++w;
-            if (w == us[i].size()) return false;
-            trial[i] = run[i]->wMin << w;
-            warps += run[i]->C * trial[i];
-        }
-        return warps <= 14 * sms;
-    };
-    size_t lo = 0, hi = taus.size();   // the least tau that fits is in [lo, hi]
-    while (lo < hi) {
-        const size_t mid = (lo + hi) / 2;
-        if (fits(taus[mid])) hi = mid; else lo = mid + 1;
-    }
-    if (lo == taus.size() || !fits(taus[lo])) return false;
-    width = trial;
-    return true;
+    if (!mixed || s->lc.csr_format || s->lc.threads_per_chain || chains > 10 * static_cast<int64_t>(s->ctx->sms))
+        return false;
+    for (const ReqPtr& r : run) asks.push_back(width_ask(r->g, r->C, r->wMin, r->wMax, r->phaseP, r->phaseIters));
+    return common_widths(asks, s->ctx->sms, width);
 }
 
 // One window over the running requests: one launch per launch class, the

@@ -1,6 +1,6 @@
-"""Requests on several graphs in one window: each runs at its own width and, from
-4096 vertices on, walks its rows in HBM, in windows whose widths change as
-requests come and go.  The results must stay those of a standalone call."""
+"""Several graphs side by side, as requests of one window and as one batch: each
+runs at a width chosen with the others' and, from 4096 vertices on, walks its
+rows in HBM.  The results must stay those of a standalone call."""
 import numpy as np
 import pytest
 
@@ -60,3 +60,35 @@ def test_mixed_requests_match_standalone(rfmf, ctx, name):
         assert np.array_equal(a.best_spins, b.best_spins)
         assert np.array_equal(a.best_vals, b.best_vals)
         assert np.array_equal(a.final_vals, b.final_vals)
+
+
+@pytest.mark.parametrize("wmax", [1, 60])
+def test_mixed_batch_matches_standalone(rfmf, ctx, wmax):
+    # between 5.25 and 12 chains per SM: widths chosen together
+    mix = [("torus", 4100, 300, wmax), ("torus", 14000, 40, 1), ("er", 700, 520, wmax)]
+    sets, dgs, init, solver, t0s = [], [], [], [], []
+    for k, (kind, n, C, w) in enumerate(mix):
+        g = _graph(rfmf, kind, n, w, 31 + k)
+        dg = rfmf.DeviceGraph(ctx, g)
+        i, s = chains_for(g, list(range(1000 * k, 1000 * k + C)))
+        t = [(35.0, 70.0, 200.0, 400.0)[c % 4] * (1 if w == 1 else 50) for c in range(C)]
+        sets.append((g, dg, i, s, t))
+        dgs += [dg] * C
+        init += list(i)
+        solver += list(s)
+        t0s += t
+    ph, it = [128, 16, 1], [40, 25, 20]
+    b = rfmf.Batch(ctx, dgs, t0s, solver, init, ph, it)
+    for sweeps in (13, 40, 32):   # windows that cut phases
+        b.run(sweeps)
+    r = b.read()
+    b.close()
+    at = 0
+    for g, dg, i, s, t in sets:
+        a = rfmf.anneal_gpu(ctx, dg, g.max_weighted_degree(), i, t, ph, it, s)
+        C = len(t)
+        assert np.array_equal(np.stack(r["end_spins"][at:at + C]), a.end_spins)
+        assert np.array_equal(np.stack(r["best_spins"][at:at + C]), a.best_spins)
+        assert np.array_equal(r["best_vals"][at:at + C], a.best_vals)
+        assert np.array_equal(r["cur_vals"][at:at + C], a.final_vals)
+        at += C
