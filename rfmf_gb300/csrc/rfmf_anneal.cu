@@ -1771,11 +1771,31 @@ const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps) {
     return dbytes == 1 ? kernel_for<1>(fmt, s64, warps) : kernel_ptr_i32(fmt, s64, warps);
 }
 
+// Rows walked in HBM pass through the L1 that the SM's chains leave: a launch
+// that has the GPU to itself (sms > 0) asks for no more shared memory than its
+// resident CTAs hold, as otherwise 28 KB of L1 are left whatever they hold.
+// GB300, 28 KB / as asked: 150 chains of a planar graph n = 3000 in 8-byte pairs
+// 17.0 / 16.1 ms, 16 graphs n 807..14,000 x 48 44.7 / 42.0, 80 of the 100x200
+// torus 52.8 / 52.1; ER n = 5000 x 256 at P = 128 2.88 / 2.40 us per sweep, full
+// SMs the same.
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
-                          int threads, size_t smem, cudaStream_t stream) {
+                          int threads, size_t smem, cudaStream_t stream, int sms) {
     void* args[] = {const_cast<DevLaunch*>(&L)};
-    return cudaLaunchKernel(kernel_ptr(dbytes, fmt, s64, L.warpsPerChain), dim3(grid), dim3(threads), args, smem,
-                            stream);
+    cudaLaunchAttribute split{};
+    split.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    if (sms > 0 && csr_in_hbm(fmt)) {
+        constexpr size_t kSmBytes = 228 << 10, kCtaBytes = 1 << 10;   // shared memory of an SM; a CTA's own part
+        const size_t held = static_cast<size_t>((grid + sms - 1) / sms) * (smem + kCtaBytes);
+        split.val.sharedMemCarveout = static_cast<unsigned>(held < kSmBytes ? (100 * held + kSmBytes - 1) / kSmBytes : 100);
+        cfg.attrs = &split;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelExC(&cfg, kernel_ptr(dbytes, fmt, s64, L.warpsPerChain), args);
 }
 #endif
 

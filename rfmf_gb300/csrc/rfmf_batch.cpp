@@ -560,7 +560,8 @@ int launch_window(rfmf_batch* b, uint64_t sweeps) {
         DevLaunch L = k.L;
         L.window = sweeps;
         CU(cudaMemsetAsync(L.queue, 0, sizeof(int32_t), st));
-        CU(launch_anneal(L, k.dbytes, k.fmt, k.score64, k.grid, k.threads, k.smem, st));
+        CU(launch_anneal(L, k.dbytes, k.fmt, k.score64, k.grid, k.threads, k.smem, st,
+                         fork ? 0 : b->ctx->sms));
         if (fork) {
             CU(cudaEventRecord(k.done, st));
             CU(cudaStreamWaitEvent(main, k.done, 0));

@@ -43,7 +43,7 @@ inline void host_alloc_point() {
 // Kernel entry points (rfmf_anneal.cu).
 const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
-                          int threads, size_t smem, cudaStream_t stream);
+                          int threads, size_t smem, cudaStream_t stream, int sms);
 
 // Output-path kernels (rfmf_ingest.cu).  A cut group: up to 32 chains of one
 // graph, order[first .. first + count).

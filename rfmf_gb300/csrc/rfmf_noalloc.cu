@@ -53,7 +53,7 @@ int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms)
 int key_bits(int64_t n, int T);
 const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
-                          int threads, size_t smem, cudaStream_t stream);
+                          int threads, size_t smem, cudaStream_t stream, int sms);
 }  // namespace rfmf
 
 using namespace rfmf;
@@ -358,7 +358,7 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     for (int i = 0; i < 16; ++i)
         L.lut[i] = static_cast<int32_t>(std::lround(-std::log(-std::log((2.0 * i + 1.0) / 32.0)) * 1048576.0));
     const int grid = static_cast<int>(std::min<int64_t>(nitems, static_cast<int64_t>(occ) * sms));
-    e = launch_anneal(L, dbytes, kCsrGlobal, s64, grid, 32 * W * K, smem, st);
+    e = launch_anneal(L, dbytes, kCsrGlobal, s64, grid, 32 * W * K, smem, st, sms);
     // Cut values out: the int64 fields of the chain records, strided.
     if (e == cudaSuccess)
         e = cudaMemcpy2DAsync(d_cur, sizeof(int64_t), base + kOffChains + offsetof(DevChain, cur),

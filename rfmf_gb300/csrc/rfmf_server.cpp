@@ -560,7 +560,8 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         const Plan& pl = plans[c];
         cudaStream_t st = fork ? s->clsStreams[c] : s->stream;
         if (fork) CU(cudaStreamWaitEvent(st, s->fork, 0));
-        CU(launch_anneal(pl.L, pl.k.dbytes, pl.k.fmt, pl.k.s64, pl.grid, pl.threads, pl.smem, st));
+        CU(launch_anneal(pl.L, pl.k.dbytes, pl.k.fmt, pl.k.s64, pl.grid, pl.threads, pl.smem, st,
+                         fork ? 0 : s->ctx->sms));
         if (fork) {
             CU(cudaEventRecord(s->clsDone[c], st));
             CU(cudaStreamWaitEvent(s->stream, s->clsDone[c], 0));
