@@ -1446,26 +1446,22 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     }
 
     const ChainKeys keys = make_keys(ch.solverSeed);
-    // Beta cursor: the current run and the next one as uniform values, the one
-    // after as loads in flight (read-only path), so that a change of run costs
-    // neither a dependent global load nor a reduction before SELECT.
+    // Beta cursor: lane l holds run `run` + l of the table (the last runs' ends
+    // are past the window), loaded a segment of sweeps ahead.
+    const int lane = t & 31;
     const int64_t* __restrict__ bEnd = uniform(ch.betaEnd);
     const int32_t* __restrict__ bVal = uniform(ch.betaVal);
     const int64_t nRuns = uniform(ch.betaRuns);
-    uint64_t betaNext = ~uint64_t(0), nextEnd = ~uint64_t(0), pfEnd = ~uint64_t(0);
-    int32_t beta = 0, nextVal = 0, pfVal = 0;
-    if (s1 > s0) {
-        betaNext = uniform(static_cast<uint64_t>(__ldg(bEnd + run)));
-        beta = uniform(__ldg(bVal + run));
-        if (run + 1 < nRuns) {
-            nextEnd = uniform(static_cast<uint64_t>(__ldg(bEnd + run + 1)));
-            nextVal = uniform(__ldg(bVal + run + 1));
+    uint64_t runEnd = ~uint64_t(0);
+    int32_t runVal = 0;
+    auto load_runs = [&]() {
+        runEnd = ~uint64_t(0);
+        if (run + lane < nRuns) {
+            runEnd = static_cast<uint64_t>(__ldg(bEnd + run + lane));
+            runVal = __ldg(bVal + run + lane);
         }
-        if (run + 2 < nRuns) {
-            pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 2));
-            pfVal = __ldg(bVal + run + 2);
-        }
-    }
+    };
+    load_runs();
     uint64_t improved = 0;
     using Loc = typename std::conditional<DP::kField, int32_t, int64_t>::type;
     // The last sweep's gain is settled when the next one is about to flip (or
@@ -1528,33 +1524,34 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         uint32_t left = kPaceEvery - paced;
         if (phaseEnd > sw && phaseEnd - sw < left) left = static_cast<uint32_t>(phaseEnd - sw);
         if (s1 - sw < left) left = static_cast<uint32_t>(s1 - sw);
-        // The sweep of them at which the beta run changes, if any does (runs
-        // are never empty: one step of the cursor per sweep).
-        auto turn_in = [&]() { return betaNext - sw < kPaceEvery ? static_cast<uint32_t>(betaNext - sw) : ~0u; };
-        uint32_t toTurn = sw >= betaNext ? 0u : turn_in();
+        // Their betas, one to a lane: sweep sw + l takes the first run that ends
+        // past it (runs are never empty, so that is one of the 32 at hand).
+        // A beta lasts one sweep for most of a schedule (t0 = 35: until sweep
+        // 30,000).  Against a cursor that moved with the sweeps (two loads, three
+        // warp reductions and 64-bit compares a run), GB300, us per sweep at P =
+        // 1: 32 chains of ER n = 800 1.165 / 1.081, four one-warp chains of ER n =
+        // 256 0.858 / 0.782, 1024 of ER n = 2000 2.09 / 1.98; 80 of the 100x200
+        // torus 2.91 / 2.76.
+        int32_t betas;
+        {
+            const uint64_t room = runEnd - sw;
+            const uint32_t ends = room < 64 ? static_cast<uint32_t>(room) : 64u;
+            int at = 0;
+#pragma unroll
+            for (int step = 16; step; step >>= 1)
+                if (__shfl_sync(0xFFFFFFFFu, ends, at + step - 1) <= static_cast<uint32_t>(lane)) at += step;
+            betas = __shfl_sync(0xFFFFFFFFu, runVal, at);
+            run += __popc(__ballot_sync(0xFFFFFFFFu, ends <= left));
+            load_runs();
+        }
+        const uint32_t segment = left;
         do {
-            const bool turn = toTurn == 0;
-            if (turn) {
-                ++run;
-                betaNext = nextEnd;
-                beta = nextVal;
-                toTurn = turn_in();
-            }
-            --toTurn;
+            const int32_t beta = __shfl_sync(0xFFFFFFFFu, betas, static_cast<int>(segment - left));
             int32_t v[4];
             if constexpr (kS64) select64<DP>(s, lut, n, pc, beta, sc, keys, t, T, grp);
             else select32<kOne, DP>(s, lut, kc, n, pc, beta, sc, keys, t, T, v);
             ++sw;
             sc = make_sweep(sw + 1, keys);
-            if (turn) {
-                nextEnd = uniform(pfEnd);
-                nextVal = uniform(pfVal);
-                pfEnd = ~uint64_t(0);
-                if (run + 2 < nRuns) {
-                    pfEnd = static_cast<uint64_t>(__ldg(bEnd + run + 2));
-                    pfVal = __ldg(bVal + run + 2);
-                }
-            }
             const bool slots = kS64 || pc.path != kPathWarp;
             if (!kOne || slots) group_sync(grp, T);
             if (slots) {
