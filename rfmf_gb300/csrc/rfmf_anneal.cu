@@ -221,6 +221,9 @@ struct D32 {
     __device__ static __forceinline__ int32_t get(const unsigned char* D, const unsigned char*, int v) {
         return reinterpret_cast<const int32_t*>(D)[v];
     }
+    __device__ static __forceinline__ int32_t get_as(const unsigned char* D, uint32_t, int v) {
+        return reinterpret_cast<const int32_t*>(D)[v];
+    }
     __device__ static __forceinline__ void set(unsigned char* D, const unsigned char*, int v, int32_t d) {
         reinterpret_cast<int32_t*>(D)[v] = d;
     }
@@ -312,6 +315,10 @@ struct D8 {
     }
     __device__ static __forceinline__ int32_t get(const unsigned char* D, const unsigned char* sb, int v) {
         return static_cast<int32_t>(D[v] ^ sb[v]) - 128;
+    }
+    // The same for a vertex whose spin is known (neg: -1).
+    __device__ static __forceinline__ int32_t get_as(const unsigned char* D, uint32_t neg, int v) {
+        return static_cast<int32_t>(D[v] ^ (neg ? 0xFFu : 0u)) - 128;
     }
     __device__ static __forceinline__ void set(unsigned char* D, const unsigned char* sb, int v, int32_t d) {
         D[v] = static_cast<unsigned char>((d + 128) ^ sb[v]);
@@ -539,7 +546,7 @@ __device__ __forceinline__ KeyCfg key_cfg(int n, int S, int t, const int32_t* lu
     kc.full = uniform(((n + 7) >> 3) / S);
     kc.extra = uniform(((n + 7) >> 3) % S);
     const int i = t & 15;
-    kc.tkLane = lut[i] * (1 << kc.kb) - i * static_cast<int32_t>(kc.mulF);
+    kc.tkLane = lut[i] * (1 << kc.kb) - i * static_cast<int32_t>(kc.mulF) + (1 << kc.kb) - 1;
     return kc;
 }
 
@@ -791,7 +798,7 @@ __device__ __forceinline__ void select_warp(int32_t acc[8], const ChainSmem& s, 
     for (int j = 0; j < 8; ++j) acc[j] = INT32_MIN;
     const int32_t betaK = beta * (1 << kc.kb);
     // Per-sweep part of the table register: (2^kb - 1) - bias * beta * 2^kb.
-    const int32_t tkBase = static_cast<int32_t>(static_cast<uint32_t>(kc.tkLane) + (1u << kc.kb) - 1u -
+    const int32_t tkBase = static_cast<int32_t>(static_cast<uint32_t>(kc.tkLane) -
                                                 static_cast<uint32_t>(DP::kBias) * static_cast<uint32_t>(betaK));
     select_blocks<kF0, DP>(acc, s, sc, keys, n, t, S, iters, betaK, tkBase, kc);
 }
@@ -1238,7 +1245,7 @@ __device__ __forceinline__ Loc flip_rows(const ChainSmem& s, const CsrView& csr,
     if (kRows == 1 && pc.P == 1) return 2 * loc;   // a lone winner's gain just changes sign
 #pragma unroll
     for (int q = 0; q < kRows; ++q)
-        if (v[q] >= 0 && sub == 0) loc -= DP::get(s.D, s.sb, v[q]);
+        if (v[q] >= 0 && sub == 0) loc -= DP::get_as(s.D, neg[q], v[q]);
     return loc;
 }
 
@@ -1469,13 +1476,20 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     // SELECT, and wider chains pass the warps' sums through s.red under
     // SELECT's own barrier instead of one more.
     Loc loc = 0;
+    // The cut as its distance below the best, in a gain's type: with int8 gains
+    // (n < 2^23, B <= 127) no two cuts are 2^30 apart, so a best further off is
+    // never reached.
+    constexpr int64_t kFar = DP::kField ? int64_t(1) << 30 : INT64_MAX / 2;
+    Loc behind = static_cast<Loc>(best < cur - kFar ? -kFar : best > cur + kFar ? kFar : best - cur);
+    int64_t top = cur + behind;
     auto settle = [&]() {
         Loc gain;
         if constexpr (kOne) gain = warp_sum(loc);
         else gain = warp_sum(static_cast<Loc>((t & 31) < (T >> 5) ? s.red[t & 31] : 0));
-        cur += gain / 2;
-        if (cur > best) {
-            best = cur;
+        behind -= gain >> 1;
+        if (behind < 0) {
+            top -= behind;
+            behind = 0;
             ++improved;
             for (int w = t; w < words; w += T) s.best[w] = s.bits[w];
             group_sync(grp, T);
@@ -1577,8 +1591,8 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
         ch.bestBits[w] = s.best[w];
     }
     if (t == 0) {
-        ch.cur = cur;
-        ch.best = best;
+        ch.cur = top - behind;
+        ch.best = best > top ? best : top;
         ch.sweepsDone = s1;
         ch.improvedSweeps += improved;
     }
