@@ -468,7 +468,9 @@ struct PhaseCfg {
     int rows;       // FLIP: rows a thread takes part in on kPathWarp (1 to 4)
     int S;          // block stride (T but on kPathWarp; above 32 a one-warp chain
                     //    plays several warps)
-    int step;       // kPathWarp: 256 mod P, a warp's shift of the groups
+    int shares;     // kPathWarp off the main path: 256 mod P, a warp's shift of the
+                    //    groups, and from bit 8 the lanes that share a group's
+                    //    accumulators (0 when 256 % P == 0)
     int warpG;      // kPathWarp: (256 warp) mod P
 };
 
@@ -493,7 +495,7 @@ __device__ __forceinline__ PhaseCfg phase_cfg(int P, int n, int t, int T, bool o
     c.S = uniform(warp ? S : T);
     const bool priv = (8 * T) % P == 0 && key_bits(n, T) <= kbMax;
     c.path = uniform(static_cast<int>(warp ? kPathWarp : priv ? kPathPrivate : kPathVertex));
-    c.step = uniform(256 % P);
+    c.shares = uniform(256 % P);
     c.warpG = uniform((8 * (t & ~31)) % P);
     int sh = 0;
     while ((2 << sh) * P <= T && sh < 5) ++sh;
@@ -705,15 +707,29 @@ __device__ __forceinline__ void warp_argmax(const int32_t acc[8], int32_t* scr, 
     }
 }
 
+// Lanes that share a group of warp_argmax_any: 32 / P for a P below 16 that does
+// not divide 32, never more (a division a sweep cost 110 cycles).
+__constant__ unsigned char kShare[129] = {
+    1, 15, 15, 10, 8, 6, 5, 4, 4, 3, 3, 2, 2, 2, 2, 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
+    1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
+    1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
+    1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1,
+};
+
 // The same for any P <= 128: class c = a mod P (the group but for the warp's
 // shift).  With P <= 32, 32 / P lanes share a class and fold pairwise into its
 // first lane; four reads go out together.
-__device__ __forceinline__ void warp_argmax_any(const int32_t acc[8], int32_t* scr, int lane, int P, int32_t key[4],
-                                                int32_t at[4]) {
-    *reinterpret_cast<int4*>(scr + 4 * lane) = make_int4(acc[0], acc[1], acc[2], acc[3]);
-    *reinterpret_cast<int4*>(scr + kHalf + 4 * lane) = make_int4(acc[4], acc[5], acc[6], acc[7]);
+//
+// Accumulators lie at their own number here: lane-consecutive reads at any P,
+// each address one add, where the halves of warp_argmax took seven
+// instructions a read.  GB300, us per sweep before / now: 300 four-warp chains
+// of a weighted ER n = 1500 P = 100 2.85 / 2.70, P = 12 1.90 / 1.77; 1024
+// one-warp chains of ER n = 2000 P = 60 4.40 / 4.19, P = 5 2.98 / 2.80.
+__device__ __forceinline__ void warp_argmax_any(const int32_t acc[8], int32_t* scr, int lane, int P, int share,
+                                                int32_t key[4], int32_t at[4]) {
+    *reinterpret_cast<int4*>(scr + 8 * lane) = make_int4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<int4*>(scr + 8 * lane + 4) = make_int4(acc[4], acc[5], acc[6], acc[7]);
     __syncwarp();
-    int share = P <= 32 ? 32 / P : 1;
     const int width = share * P;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -721,13 +737,11 @@ __device__ __forceinline__ void warp_argmax_any(const int32_t acc[8], int32_t* s
         at[q] = 0;
         const int c = lane + 32 * q;
         if (c < width) {
+#pragma unroll 1
             for (int a = c; a < 256; a += 4 * width) {
                 int32_t k[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int x = a + i * width < 256 ? a + i * width : a;   // past the end: the first again
-                    k[i] = scr[4 * (x >> 3) + (x & 3) + kHalf * ((x >> 2) & 1)];
-                }
+                for (int i = 0; i < 4; ++i) k[i] = a + i * width < 256 ? scr[a + i * width] : INT32_MIN;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (k[i] > key[q]) {
@@ -885,7 +899,7 @@ __device__ __forceinline__ void select32_general(const ChainSmem& s, const int32
         }
         int32_t* scr = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(s.slots) +
                                                   (kOne ? 0 : (t >> 5) * kWarpScratch));
-        warp_argmax_any(acc, scr, lane, P, key, at);
+        warp_argmax_any(acc, scr, lane, P, kShare[P], key, at);
         if (!kOne || S <= 32) {
             warp_winners<kOne, DP>(s, pc, kc, scr, first, lane, S, key, at, v);
             return;
@@ -901,7 +915,8 @@ __device__ __forceinline__ void select32_general(const ChainSmem& s, const int32
                 if (first == 0 || mine > table[g]) table[g] = mine;
             }
         }
-        shift = shift + pc.step < P ? shift + pc.step : shift + pc.step - P;
+        const int step = pc.shares;
+        shift = shift + step < P ? shift + step : shift + step - P;
         __syncwarp();
         if (first + 32 >= S) {
 #pragma unroll
@@ -924,7 +939,7 @@ template <bool kOne, class DP>
 __device__ __forceinline__ void select32(const ChainSmem& s, const int32_t* lut, const KeyCfg& kc, int n,
                                          const PhaseCfg& pc, int32_t beta, const SweepConst& sc,
                                          const ChainKeys& keys, int t, int T, int32_t v[4]) {
-    if (pc.path != kPathWarp || pc.step != 0) {
+    if (pc.path != kPathWarp || pc.shares != 0) {
         select32_general<kOne, DP>(s, lut, kc, n, pc, beta, sc, keys, t, T, v);
         return;
     }
@@ -1443,7 +1458,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     const bool table = L.layout != kLayoutMain;
     PhaseCfg pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
     KeyCfg kc = key_cfg(n, pc.S, t, lut);
-    if (!table && (pc.path != kPathWarp || pc.step != 0)) {
+    if (!table && (pc.path != kPathWarp || pc.shares != 0)) {
         // The host plans a table for every schedule that needs one.
         if (t == 0) {
             raise_error(L, kDevBadItem, ci);
@@ -1513,7 +1528,7 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
             const bool warp = pc.path == kPathWarp;
             pc = phase_cfg(P, n, t, T, kOne, kbMax, slotsOnly);
             kc = key_cfg(n, pc.S, t, lut);
-            if (!table && (pc.path != kPathWarp || pc.step != 0)) {
+            if (!table && (pc.path != kPathWarp || pc.shares != 0)) {
                 if (t == 0) raise_error(L, kDevBadItem, ci);
                 break;
             }
