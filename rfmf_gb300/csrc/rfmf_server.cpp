@@ -114,8 +114,9 @@ struct SlotRanges {
 struct ClassKey {
     int dbytes, fmt, W;
     bool s64;
+    bool table;   // kept apart where widths are chosen together: a group table beside the largest chain may not fit
     bool operator<(const ClassKey& o) const {
-        return std::tie(dbytes, fmt, W, s64) < std::tie(o.dbytes, o.fmt, o.W, o.s64);
+        return std::tie(dbytes, fmt, W, s64, table) < std::tie(o.dbytes, o.fmt, o.W, o.s64, o.table);
     }
 };
 
@@ -386,7 +387,8 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
     const bool mixed = mixed_widths(s, width);
     for (size_t i = 0; i < s->running.size(); ++i) {
         Request* r = s->running[i].get();
-        classes[ClassKey{r->dbytes, mixed && r->n >= kMixedHbmN ? hbm_format(r->g) : r->fmt, width[i], r->s64}].push_back(r);
+        classes[ClassKey{r->dbytes, mixed && r->n >= kMixedHbmN ? hbm_format(r->g) : r->fmt, width[i], r->s64,
+                         mixed && r->table}].push_back(r);
     }
     launches = 0;
     ms = 0.0f;

@@ -16,6 +16,8 @@ MIXES = {
     "crowded": [("dense", 1200, 2, 1), ("torus", 4000, 2, 1), ("er", 900, 1, 1)],
     # int32 gains and 32-bit entries beside int8
     "weights": [("er", 900, 24, 300), ("torus", 5000, 24, 1), ("torus", 5000, 16, 300)],
+    # one schedule off the kernel's main path (P = 300) beside two on it
+    "table": [("er", 500, 30, 1), ("torus", 14000, 12, 1), ("torus", 4100, 20, 1)],
     # more than ten chains per SM: the requests' own widths, several classes
     "many": [("er", 300, 900, 1), ("torus", 4200, 300, 1), ("er", 600, 800, 40)],
 }
@@ -49,7 +51,8 @@ def test_mixed_requests_match_standalone(rfmf, ctx, name):
         g = _graph(rfmf, kind, n, wmax, 11 + k)
         init, solver = chains_for(g, list(range(1000 * k, 1000 * k + C)))
         t0s = [(35.0, 70.0, 200.0, 400.0)[c % 4] * (1 if wmax == 1 else 100) for c in range(C)]
-        reqs.append((g, rfmf.DeviceGraph(ctx, g), init, solver, t0s, [128, 16, 1], [40 + 30 * k, 25, 20]))
+        reqs.append((g, rfmf.DeviceGraph(ctx, g), init, solver, t0s, [300 if name == "table" and k == 0 else 128, 16, 1],
+                     [40 + 30 * k, 25, 20]))
     ids = [srv.submit(dg, init, t0s, ph, it, solver) for _, dg, init, solver, t0s, ph, it in reqs]
     for rid, (g, dg, init, solver, t0s, ph, it) in zip(ids, reqs):
         st = srv.wait(rid, timeout=300)
