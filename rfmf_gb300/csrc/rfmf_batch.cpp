@@ -491,11 +491,11 @@ int rebalance(rfmf_batch* b, uint32_t P, bool* changed = nullptr) {
 // vertices, while that leaves an SM few enough warps: 10 from one or two warps
 // per chain, 8 from four, or 16 from four when the rows hold four times the
 // vertices.  GB300, us per sweep at P = 128, narrow / doubled: from one warp ER
-// n = 1500 d = 12 600 chains (8 warps per SM) 5.06 / 3.98, ER n = 2000 d = 19 700
-// chains (9) 4.50 / 4.47 and 1024 chains (14) 4.58 / 5.15; from four ER n = 800
-// d = 48 (rows 7.7 times the vertices) 32 chains 2.98 / 2.51, 300 chains (16)
-// 3.37 / 3.14, ER n = 2000 64 chains 2.34 / 2.11, 200 chains (11; 1.2 times)
-// 2.58 / 2.67.
+// n = 1500 d = 12 600 chains (8 warps per SM) 2.96 / 2.90, ER n = 2000 d = 19 700
+// chains (9) 4.26 / 4.05 and 1024 chains (14) 4.30 / 4.73; from four ER n = 800
+// d = 48 (rows 7.7 times the vertices) 32 chains 2.77 / 2.35, 300 chains (16)
+// 3.14 / 2.94, ER n = 2000 64 chains 2.12 / 1.93, 200 chains (11; 1.2 times)
+// 2.39 / 2.57.
 bool wide_phase(const rfmf_graph* g, uint32_t P, int warps, int64_t warpsPerSm) {
     const double n = static_cast<double>(g->n);
     const double rows = std::min(static_cast<double>(P), n);

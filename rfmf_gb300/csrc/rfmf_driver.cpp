@@ -658,17 +658,17 @@ namespace rfmf {
 // eight up to 8 (one chain per SM) on graphs of at least 6144 vertices and up
 // to 16 from 16384 on.  GB300, us per sweep summed over P = 128, 32, 8 and 1 at
 // 1 / 2 / 4 / 8 warps:
-//   ER n = 2000 d = 19   200 chains 10.1 / 8.9 / 7.8 / 8.6, 400 10.1 / 10.2 /
-//                        9.0 / 17, 700 12.3 / 11.9 / 17.7, 1024 12.4 / 13.6
-//   50x60 torus          400 chains 9.8 / 9.7 / 9.0, 700 12.5 / 11.7 / 17.7,
-//                        1024 12.5 / 13.6
-//   ER n = 800 d = 48    32 chains 10.9 / 9.8 / 7.4 / 7.1, 300 10.9 / 9.8 / 8.4
-//   ER n = 5000 d = 5    80 chains 14.3 / 10.5 / 8.3 / 7.6, 256 14.2 / 10.6 /
-//                        9.4 / 10.1, 600 14.2 / 12.9 / 12.8
-//   70x100 torus         80 chains 16.8 / 12.4 / 8.5 / 8.3, 300 16.8 / 12.4 /
-//                        10.3 / 11.1, 600 16.9 / 15.3 / 14.7
-//   100x200 torus        80 chains 46.8 / 27.5 / 16.4 / 13.7, 256 - / 27.6 /
-//                        20.8 / 19.2, 400 - / 35.4 / 25.7 / 38.1
+//   ER n = 2000 d = 19   200 chains 8.9 / 7.7 / 6.9 / 8.0, 400 8.9 / 9.1 / 8.0 /
+//                        15.8, 700 11.1 / 10.8 / 15.8, 1024 11.2 / 12.7 / 18.1
+//   50x60 torus          400 chains 8.7 / 8.7 / 7.9 / 15.9, 700 11.2 / 10.7 /
+//                        15.7, 1024 11.2 / 12.9 / 18.0
+//   ER n = 800 d = 48    32 chains 9.6 / 8.4 / 6.5 / 6.3, 300 9.7 / 8.4 / 7.4 / 8.0
+//   ER n = 5000 d = 5    80 chains 13.0 / 9.3 / 6.8 / 6.7, 256 13.0 / 9.4 / 8.2 /
+//                        9.3, 600 13.0 / 11.8 / 11.9 / 18.6
+//   70x100 torus         80 chains 15.6 / 10.6 / 7.5 / 7.4, 300 15.6 / 10.6 / 9.3 /
+//                        10.4, 600 15.7 / 14.0 / 14.2 / 20.9
+//   100x200 torus        80 chains 40.0 / 24.1 / 14.5 / 12.4, 256 40.1 / 24.2 /
+//                        19.1 / 18.1, 400 40.2 / 32.6 / 24.0 / 35.9
 // (sixteen warps lost to eight everywhere.)
 int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms) {
     if (c.threads_per_chain) return c.threads_per_chain / 32;
@@ -702,9 +702,9 @@ WidthAsk width_ask(const rfmf_graph* g, int64_t chains, int least, int widest, c
 // within the least time per sweep that 14 warps per SM allow all of them.  Time
 // is estimated as 1.5 us + 0.5 ns per vertex and winner-row entry, the latter
 // over the chain's warps.  GB300, measured / estimated, few chains per SM,
-// averaged over P = 128, 32, 8 and 1: ER n = 2000 d = 19 W = 1 2.5 / 2.9, W = 4
-// 1.8 / 1.9; ER n = 5000 d = 5 3.6 / 4.1 and 2.1 / 2.2; 100x200 torus 11.7 / 11.6
-// and 4.1 / 4.0, W = 8 3.4 / 2.8.  False, and `width` as it was, where even the
+// averaged over P = 128, 32, 8 and 1: ER n = 2000 d = 19 W = 1 2.2 / 2.9, W = 4
+// 1.5 / 1.9; ER n = 5000 d = 5 3.3 / 4.1 and 1.7 / 2.2; 100x200 torus 10.0 / 11.6
+// and 3.6 / 4.0, W = 8 3.1 / 2.8.  False, and `width` as it was, where even the
 // narrowest widths hold more warps.
 bool common_widths(const std::vector<WidthAsk>& asks, int sms, std::vector<int>& width) {
     std::vector<std::vector<double>> us(asks.size());   // at least, 2 least, ..

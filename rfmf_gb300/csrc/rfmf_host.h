@@ -399,7 +399,7 @@ struct rfmf_graph {
     // and ER n = 2000 d = 19, phases 128..1): 1.49 us + 1.0 ns per vertex +
     // 1.4 ns per winner-row entry (min(P, n) rows of mean degree 2m/n), the
     // vertex and entry terms spread over the chain's warps, scaled by level
-    // as above.  Within 5% of the measured sweep on both graphs at every P.
+    // as above (the kernel has since become some 5% faster, alike for all).  Within 5% of the measured sweep on both graphs at every P.
     double model_cost(int warps, uint32_t P, int level) const {
         const double nn = static_cast<double>(n > 0 ? n : 1);
         const double rows = std::min(static_cast<double>(P > 0 ? P : 1), nn);
