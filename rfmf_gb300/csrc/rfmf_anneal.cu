@@ -1648,19 +1648,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
     return ok != 0;
 }
 
-// Stage graph g's compact CSR into shared memory: thread 0 arms the mbarrier
-// with the byte count and issues the bulk copies (<= 64 KB each); every
-// thread waits on the phase with a bounded poll.  Returns this thread's
-// outcome (false: its polls ran out); the caller makes it CTA-uniform and
-// advances the phase.
+// Stage graph g's row words and compact entries (kUnit: 16 bits, else 32) into
+// shared memory: thread 0 arms the mbarrier with the byte count and issues the
+// bulk copies (<= 64 KB each); every thread waits on the phase with a bounded
+// poll.  Returns this thread's outcome (false: its polls ran out); the caller
+// makes it CTA-uniform and advances the phase.
+template <bool kUnit>
 __device__ bool stage_csr(const DevGraph& g, unsigned char* dst, uint64_t* mbar, uint32_t phase) {
-    const uint32_t total = g.rowBytes + g.entBytes;
+    const uint32_t entBytes = kUnit ? g.u16Bytes : g.p32Bytes;
+    const uint32_t total = g.rowBytes + entBytes;
     if (threadIdx.x == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(mbar, total);
         const unsigned char* srcs[2] = {reinterpret_cast<const unsigned char*>(g.rows),
-                                        static_cast<const unsigned char*>(g.compact)};
-        const uint32_t sizes[2] = {g.rowBytes, g.entBytes};
+                                        kUnit ? reinterpret_cast<const unsigned char*>(g.u16)
+                                              : reinterpret_cast<const unsigned char*>(g.p32)};
+        const uint32_t sizes[2] = {g.rowBytes, entBytes};
         uint32_t o = 0;
         for (int k = 0; k < 2; ++k) {
             for (uint32_t c = 0; c < sizes[k]; c += 65536u) {
@@ -1721,12 +1724,14 @@ __global__ void __launch_bounds__(512, 1) rfmf_anneal_kernel(const DevLaunch L) 
         CsrView csr;
         if constexpr (csr_in_hbm(kFmt)) {
             csr.off = (kFmt == kCsrGlobal) ? g.offsets : g.rows;
-            csr.ent = (kFmt == kCsrGlobal) ? static_cast<const void*>(g.edges) : g.compact;
+            csr.ent = (kFmt == kCsrGlobal)    ? static_cast<const void*>(g.edges)
+                      : Csr<kFmt>::kUnit ? static_cast<const void*>(g.u16)
+                                         : static_cast<const void*>(g.p32);
         } else {
             if (item.graph != loaded) {
                 // All threads agree on the outcome, so that a chain's
                 // barriers never see part of its warp group leave.
-                if (!__syncthreads_and(stage_csr(g, csrBase, mbar, phase))) {
+                if (!__syncthreads_and(stage_csr<Csr<kFmt>::kUnit>(g, csrBase, mbar, phase))) {
                     // The copy may still be in flight.  Report it, then stay
                     // resident for a second, longer bounded wait: a CTA that
                     // retired with a copy outstanding would leave its target

@@ -732,7 +732,6 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     // reference's.
     using Key = std::tuple<int, int, int, int>;   // dbytes, fmt, W, s64
     std::map<Key, int> classOf;
-    std::vector<int> graphClass(G);
     // Graphs of at least hbmN vertices walk their rows in HBM; width: warps per
     // chain of each graph (empty: the rule for each).
     auto classify = [&](int64_t hbmN, const std::vector<int>& width) -> int {
@@ -837,7 +836,6 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 k.score64 = s64;
                 k.pmax = static_cast<int>(std::max<uint64_t>(1, maxP));
             }
-            graphClass[gi] = it->second;
             BatchClass& k = b->cls[it->second];
             k.graphs.push_back(static_cast<int>(gi));
             k.chainsOf.push_back(chainsOfGraph[gi]);
@@ -907,19 +905,13 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 }
                 b->cls[it->second].graphs.push_back(gi);
                 b->cls[it->second].chainsOf.push_back(std::move(chains));
-                graphClass[gi] = it->second;
             }
         }
-        // Drop classes emptied by the moves and renumber.
-        std::vector<int> remap(b->cls.size(), -1);
+        // Drop classes emptied by the moves.
         std::vector<BatchClass> kept;
-        for (size_t ci = 0; ci < b->cls.size(); ++ci) {
-            if (b->cls[ci].graphs.empty()) continue;
-            remap[ci] = static_cast<int>(kept.size());
-            kept.push_back(std::move(b->cls[ci]));
-        }
+        for (BatchClass& k : b->cls)
+            if (!k.graphs.empty()) kept.push_back(std::move(k));
         b->cls = std::move(kept);
-        for (size_t gi = 0; gi < G; ++gi) graphClass[gi] = remap[graphClass[gi]];
     };
     if (c.csr_format == 0) spread();
     // Several classes share the SMs, each sized as if alone: their CSR copies
@@ -1018,20 +1010,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     b->betaRefs = cb.refs;
 
     std::vector<DevGraph> hg(G);
-    for (size_t gi = 0; gi < G; ++gi) {
-        const rfmf_graph* g = b->glist[gi];
-        const int fmt = b->cls[graphClass[gi]].fmt;
-        hg[gi].offsets = g->offsets.as<uint32_t>();
-        hg[gi].edges = g->edges.as<Edge>();
-        hg[gi].rows = g->rows.as<uint32_t>();
-        hg[gi].compact = compact_entries(g, fmt);
-        hg[gi].n = static_cast<int32_t>(g->n);
-        hg[gi].words = static_cast<int32_t>((g->n + 31) / 32);
-        hg[gi].B = g->B;
-        hg[gi].wsum2 = g->wsum2;
-        hg[gi].rowBytes = g->rowBytes;
-        hg[gi].entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;
-    }
+    for (size_t gi = 0; gi < G; ++gi) hg[gi] = device_graph(b->glist[gi]);
 
     // Per-chain spin words and initial state.
     b->chainN.resize(C);

@@ -48,13 +48,16 @@ struct DevGraph {
     const uint32_t* offsets;   // n + 1 (padded to 16 B)
     const Edge*     edges;     // 2m  {col, weight}
     const uint32_t* rows;      // n + 1 row words of the compact entries (padded to 16 B)
-    const void*     compact;   // compact entries of the launch's format, rows padded to four (16 B in all)
+    const uint16_t* u16;       // compact entries by width, rows padded to four (16 B in all); null: the
+    const uint32_t* p32;       //   graph has none.  A record serves every format, as launches of several
+                               //   formats may share it
     int32_t         n;
     int32_t         words;     // ceil(n / 32): spin bit-words per chain
     int64_t         B;         // max weighted degree: no gain exceeds it
     int64_t         wsum2;     // sum of weight over directed entries (2 * sum over edges)
     uint32_t        rowBytes;  // bytes of rows, multiple of 16
-    uint32_t        entBytes;  // bytes of compact entries, multiple of 16
+    uint32_t        u16Bytes;  // bytes of u16 and of p32, multiples of 16
+    uint32_t        p32Bytes;
 };
 
 // One schedule: phases (group counts P) and sweeps per phase, shared by the

@@ -464,12 +464,22 @@ inline int64_t packed_csr_bytes(const rfmf_graph* g, int fmt) {
     return ((4 * (g->n + 1) + 15) & ~int64_t(15)) + ((2 * g->m * (fmt == kCsrUnit16 ? 2 : 4) + 15) & ~int64_t(15));
 }
 
-// The entry array a launch of format `fmt` reads for graph g (the 8-byte
-// pairs are DevGraph::edges).
-inline const void* compact_entries(const rfmf_graph* g, int fmt) {
-    if (fmt == kCsrUnit16 || fmt == kCsrGlobal16) return g->u16.p;
-    if (fmt == kCsrPacked32 || fmt == kCsrGlobal32) return g->p32.p;
-    return nullptr;
+// The graph's device record, the same for launches of any format.
+inline DevGraph device_graph(const rfmf_graph* g) {
+    DevGraph d{};
+    d.offsets = g->offsets.as<uint32_t>();
+    d.edges = g->edges.as<Edge>();
+    d.rows = g->rows.as<uint32_t>();
+    d.u16 = g->u16.as<uint16_t>();
+    d.p32 = g->p32.as<uint32_t>();
+    d.n = static_cast<int32_t>(g->n);
+    d.words = static_cast<int32_t>((g->n + 31) / 32);
+    d.B = g->B;
+    d.wsum2 = g->wsum2;
+    d.rowBytes = g->rowBytes;
+    d.u16Bytes = g->u16Bytes;
+    d.p32Bytes = g->p32Bytes;
+    return d;
 }
 
 }  // namespace rfmf

@@ -271,14 +271,10 @@ static int rfmf_anneal_noalloc_impl(int device, void* stream, int64_t n,
     DevGraph g{};
     g.offsets = d_offsets;
     g.edges = reinterpret_cast<const Edge*>(d_edges);
-    g.rows = nullptr;
-    g.compact = nullptr;
     g.n = static_cast<int32_t>(n);
     g.words = words;
     g.B = max_weighted_deg;
     g.wsum2 = 0;
-    g.rowBytes = 0;
-    g.entBytes = 0;
     DevSchedule sch{reinterpret_cast<const uint32_t*>(base + kOffPhaseP),
                     reinterpret_cast<const uint64_t*>(base + kOffPhaseIters),
                     static_cast<int32_t>(nphases), 0};

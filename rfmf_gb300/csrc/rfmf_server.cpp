@@ -198,21 +198,6 @@ int ensure_attr(rfmf_server* s, const void* k) {
     return RFMF_OK;
 }
 
-DevGraph dev_graph(const rfmf_graph* g, int fmt) {
-    DevGraph d{};
-    d.offsets = g->offsets.as<uint32_t>();
-    d.edges = g->edges.as<Edge>();
-    d.rows = g->rows.as<uint32_t>();
-    d.compact = compact_entries(g, fmt);
-    d.n = static_cast<int32_t>(g->n);
-    d.words = static_cast<int32_t>((g->n + 31) / 32);
-    d.B = g->B;
-    d.wsum2 = g->wsum2;
-    d.rowBytes = g->rowBytes;
-    d.entBytes = csr_bytes(g, fmt) ? csr_bytes(g, fmt) - g->rowBytes : 0;
-    return d;
-}
-
 // Device state of a newly admitted request (worker thread).
 int admit(rfmf_server* s, Request& r) {
     host_alloc_point();
@@ -257,7 +242,7 @@ int admit(rfmf_server* s, Request& r) {
                 s->graphCap = cap;
             }
         }
-        const DevGraph dg = dev_graph(r.g, r.fmt);
+        const DevGraph dg = device_graph(r.g);
         CU(cudaMemcpyAsync(s->dGraphs.as<DevGraph>() + slot, &dg, sizeof dg, cudaMemcpyHostToDevice, st));
         s->graphSlotOf[r.g] = {slot, 1};
         r.graphSlot = slot;
