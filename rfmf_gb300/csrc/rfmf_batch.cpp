@@ -83,6 +83,8 @@ struct rfmf_batch {
     DevBuf dGraphs, dScheds, dChains, dPhaseP, dPhaseIters, dBits, dBest;
     DevBuf dCutPlan;                             // cut groups and their chains (made when first wanted)
     int cutGroups = 0;
+    bool lowBest = false;                        // restored, not run yet: a chain's best is below its cut
+    DevBuf dOwnBest;                             // then: see lift_best
     std::vector<DevBetaRef> betaRefs;            // the context's shared beta tables in use
     std::vector<BatchClass> cls;
     cudaEvent_t fork = nullptr;
@@ -576,6 +578,16 @@ int launch_window(rfmf_batch* b, uint64_t sweeps) {
 // the cut (a chain's sweeps are a function of its sweep index alone).
 int enqueue_run(rfmf_batch* b, uint64_t sweeps, bool capturing = false) {
     if (capturing) return launch_window(b, sweeps);
+    if (b->lowBest && sweeps == 0) return RFMF_OK;   // nothing to move
+    if (b->lowBest) {   // the first sweep by itself
+        cudaStream_t st = b->ctx->stream;
+        DevChain* chains = b->dChains.as<DevChain>();
+        b->lowBest = false;
+        CU(lift_best(chains, b->C, b->dOwnBest.as<int64_t>(), st));
+        if (int rc = enqueue_run(b, 1)) return rc;
+        CU(settle_best(chains, b->dGraphs.as<DevGraph>(), b->C, b->dOwnBest.as<int64_t>(), st));
+        if (--sweeps == 0) return RFMF_OK;
+    }
     const int64_t perWindow = static_cast<int64_t>(b->cls.size());
     uint64_t left = std::min<uint64_t>(sweeps, b->total - std::min(b->total, b->hostDone));
     bool split = b->phaseWarps;
@@ -1039,6 +1051,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 return fail(RFMF_ERR_INVALID, "chain %lld: %llu sweeps done, the schedule has %llu", (long long)i,
                             (unsigned long long)resume->sweeps_done[i], (unsigned long long)total);
             least = std::min<uint64_t>(least, resume->sweeps_done[i]);
+            b->lowBest = b->lowBest || (resume->best_vals[i] < resume->cur_vals[i] && resume->sweeps_done[i] < total);
             pack_spins(resume->best_spins + sp, b->chainN[i], bestBits.data() + b->chainWordOff[i]);
             sp += static_cast<size_t>(b->chainN[i]);
         }
@@ -1053,6 +1066,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     if ((rc = b->dPhaseIters.alloc(std::max<int64_t>(nphases, 1) * sizeof(uint64_t)))) return rc;
     if ((rc = b->dBits.alloc(bits.size() * sizeof(uint32_t)))) return rc;
     if ((rc = b->dBest.alloc(bits.size() * sizeof(uint32_t)))) return rc;
+    if (b->lowBest && (rc = b->dOwnBest.alloc(C * sizeof(int64_t)))) return rc;
     for (BatchClass& k : b->cls) {
         const int64_t kc = static_cast<int64_t>(k.order.size());
         if ((rc = k.dItems.alloc(kc * sizeof(DevItem))) || (rc = k.dOrder.alloc(kc * sizeof(int32_t))) ||
@@ -1152,6 +1166,12 @@ static int rfmf_batch_run_impl(rfmf_batch* b, uint64_t sweeps) {
 static int rfmf_batch_run_graph_impl(rfmf_batch* b, uint64_t sweeps, int launches, int replays) {
     if (!b || launches <= 0 || replays < 0) return fail(RFMF_ERR_INVALID, "bad arguments");
     CU(cudaSetDevice(b->ctx->device));
+    if (b->lowBest && sweeps == 0) return RFMF_OK;
+    if (b->lowBest && replays > 0) {   // the first replay's windows as they are (see enqueue_run)
+        for (int i = 0; i < launches; ++i)
+            if (int rc = enqueue_run(b, sweeps)) return rc;
+        --replays;
+    }
     auto capture = [&]() -> int {
         if (b->graphExec) { cudaGraphExecDestroy(b->graphExec); b->graphExec = nullptr; }
         cudaGraph_t graph = nullptr;

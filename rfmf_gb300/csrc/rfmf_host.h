@@ -58,6 +58,14 @@ cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, co
 cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count, int which,
                                     char* out, int64_t stride, cudaStream_t st);
 
+// A restored chain whose best cut lies below its current one: best moves after a
+// sweep only, while the sweep kernel takes the better of the two at once.  Before
+// the chain's first sweep, lift_best sets best to the current cut and keeps the
+// chain's own in own[c] (kUnsetCut: nothing to do); after it, settle_best puts
+// the better of the chain's own and that sweep's cut in its place.
+cudaError_t lift_best(DevChain* chains, int64_t count, int64_t* own, cudaStream_t st);
+cudaError_t settle_best(DevChain* chains, const DevGraph* graphs, int64_t count, const int64_t* own, cudaStream_t st);
+
 // Error channel: records the message for rfmf_last_error() (per host thread)
 // and returns `code`.
 int fail(int code, const char* fmt, ...);

@@ -928,9 +928,48 @@ __global__ void chain_partitions_kernel(const DevChain* chains, const DevGraph* 
     }
 }
 
+__global__ void lift_best_kernel(DevChain* chains, int64_t count, int64_t* own) {
+    for (int64_t c = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; c < count;
+         c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        DevChain& ch = chains[c];
+        const bool low = ch.best < ch.cur && ch.sweepsDone < ch.sweepsTotal;
+        own[c] = low ? ch.best : kUnsetCut;
+        if (low) ch.best = ch.cur;
+    }
+}
+
+// A warp a chain.  (A best that the sweep did raise is right as it is.)
+__global__ void settle_best_kernel(DevChain* chains, const DevGraph* graphs, int64_t count, const int64_t* own) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * blockDim.x >> 5;
+    for (int64_t c = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; c < count; c += warps) {
+        const int64_t best = own[c];
+        DevChain& ch = chains[c];
+        if (best == kUnsetCut || ch.improvedSweeps != 0) continue;
+        const bool better = ch.cur > best;
+        if (better)
+            for (int w = lane; w < graphs[ch.graph].words; w += 32) ch.bestBits[w] = ch.spinBits[w];
+        __syncwarp();
+        if (lane == 0) {
+            ch.best = better ? ch.cur : best;
+            ch.improvedSweeps = better;
+        }
+    }
+}
+
 }  // namespace
 
 namespace rfmf {
+
+cudaError_t lift_best(DevChain* chains, int64_t count, int64_t* own, cudaStream_t st) {
+    lift_best_kernel<<<grid_for(count), 256, 0, st>>>(chains, count, own);
+    return cudaGetLastError();
+}
+
+cudaError_t settle_best(DevChain* chains, const DevGraph* graphs, int64_t count, const int64_t* own, cudaStream_t st) {
+    settle_best_kernel<<<grid_for(32 * count), 256, 0, st>>>(chains, graphs, count, own);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutGroup* groups, int ngroups,
                               const int32_t* order, int maxN, int sms, int smemOptin, int which, int64_t* out,
