@@ -113,6 +113,10 @@ int64_t dyn_smem_max(const rfmf_context* ctx, const void* kern, cudaFuncAttribut
     return static_cast<int64_t>(ctx->smemOptin) - static_cast<int64_t>(fa.sharedSizeBytes);
 }
 
+// Whether `warps` per chain leave a CTA room for the chains asked for (c.chains_per_cta;
+// plan_class's limit).  A width that the planner chooses never refuses them.
+bool width_ok(const rfmf_launch_config& c, int warps) { return c.chains_per_cta <= 16 / warps; }
+
 // Plan one class: chains per CTA K, CTA shape, grid.  `exact` sizes the CTA
 // to the chosen K (several classes share SMs); otherwise the CTA keeps the
 // largest K that fits as headroom for per-graph item sizes.
@@ -815,6 +819,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
                 return RFMF_OK;
             };
             int W = width.size() ? width[gi] : choose_warps(static_cast<int>(g->n), c, b->C, ctx->sms);
+            while (c.threads_per_chain == 0 && W > 1 && !width_ok(c, W)) W /= 2;
             Pick pk;
             if (int rc = pick(W, pk)) return rc;
             // When shared memory (not the chain count) keeps an SM's chains from
@@ -826,7 +831,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             // anyway and one warp per chain does more per slot (512 graphs x 64
             // chains: 1.52e8 -> 1.44e8 when widened).
             if (c.threads_per_chain == 0 && width.empty() && perSm <= 32) {
-                while (W < kMaxAutoWarps && pk.resident < perSm) {
+                while (W < kMaxAutoWarps && pk.resident < perSm && width_ok(c, 2 * W)) {
                     Pick wider;
                     if (int rc = pick(2 * W, wider)) return rc;
                     if (2 * W * wider.resident <= W * pk.resident) break;
@@ -1004,7 +1009,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     b->cfg = c;
     for (BatchClass& k : b->cls) k.baseWarps = k.warps;
     if (b->cls.size() == 1 && b->cls[0].graphs.size() == 1 && c.threads_per_chain == 0 &&
-        2 * b->cls[0].warps <= kMaxLatencyWarps) {
+        2 * b->cls[0].warps <= kMaxLatencyWarps && width_ok(c, 2 * b->cls[0].warps)) {
         for (uint32_t P : b->phaseP)
             b->phaseWarps = b->phaseWarps || (P && wide_phase(b->glist[b->cls[0].graphs[0]], P, b->cls[0].baseWarps, doubled_load(*b, b->cls[0])));
     }
