@@ -362,18 +362,51 @@ bool mixed_widths(const rfmf_server* s, std::vector<int>& width) {
     return common_widths(asks, s->ctx->sms, width);
 }
 
+// What a class of requests needs in a CTA: its largest graph's chain with the most
+// groups (in the least layout, too) beside its largest CSR copy.
+struct ClassNeed {
+    int maxN = 0, maxWords = 0, pmax = 1, layout = kLayoutMain;
+    uint32_t csrB = 0;
+    ClassNeed(const ClassKey& k, const std::vector<Request*>& reqs) : layout(k.s64 ? kLayoutSlots : kLayoutMain) {
+        for (const Request* r : reqs) {
+            maxN = std::max<int>(maxN, static_cast<int>(r->n));
+            maxWords = std::max<int>(maxWords, static_cast<int>(r->words));
+            pmax = std::max(pmax, r->pmax);
+            if (r->table && layout == kLayoutMain) layout = kLayoutAny;
+            csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
+        }
+    }
+    uint32_t chain_bytes(const ClassKey& k, int kind) const {
+        return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total;
+    }
+    int64_t least_bytes(const ClassKey& k, bool copy) const {
+        return static_cast<int64_t>(kSmemHeader) + (copy ? csrB : 0u) +
+               std::min(chain_bytes(k, layout), chain_bytes(k, kLayoutSlots));
+    }
+};
+
 // One window over the running requests: one launch per launch class, the
 // classes side by side on their own streams (a class that fills only part
 // of the GPU no longer leaves the rest idle while the next one waits).
 // Each class has its own work items, item order and queue/error words.
 int run_window(rfmf_server* s, int64_t& launches, float& ms) {
-    std::map<ClassKey, std::vector<Request*>> classes;
+    std::multimap<ClassKey, std::vector<Request*>> classes;
     std::vector<int> width;
     const bool mixed = mixed_widths(s, width);
     for (size_t i = 0; i < s->running.size(); ++i) {
         Request* r = s->running[i].get();
-        classes[ClassKey{r->dbytes, mixed && r->n >= kMixedHbmN ? hbm_format(r->g) : r->fmt, width[i], r->s64,
-                         mixed && r->table}].push_back(r);
+        const ClassKey key{r->dbytes, mixed && r->n >= kMixedHbmN ? hbm_format(r->g) : r->fmt, width[i], r->s64,
+                           mixed && r->table};
+        // A request fits a CTA by itself, but the largest of each need among
+        // several may not: the first class of its key that holds it too, else one
+        // of its own.  (A copy can give way to HBM walks unless it was asked for.)
+        auto of = classes.equal_range(key);
+        for (; of.first != of.second; ++of.first) {
+            of.first->second.push_back(r);
+            if (ClassNeed(key, of.first->second).least_bytes(key, s->lc.csr_format != 0) <= s->ctx->smemOptin) break;
+            of.first->second.pop_back();
+        }
+        if (of.first == of.second) classes.emplace(key, std::vector<Request*>{r});
     }
     launches = 0;
     ms = 0.0f;
@@ -423,21 +456,14 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
     for (auto& kv : classes) {
         ClassKey k = kv.first;
         std::vector<Request*>& reqs = kv.second;
-        int maxN = 0, maxWords = 0, pmax = 1;
-        int layout = k.s64 ? kLayoutSlots : kLayoutMain;
-        uint32_t csrB = 0;
-        for (Request* r : reqs) {
-            maxN = std::max<int>(maxN, static_cast<int>(r->n));
-            maxWords = std::max<int>(maxWords, static_cast<int>(r->words));
-            pmax = std::max(pmax, r->pmax);
-            if (r->table && layout == kLayoutMain) layout = kLayoutAny;
-            csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
-        }
-        auto chain_bytes = [&](int kind) { return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total; };
-        // The largest copy beside the largest graph's chain may not fit though
-        // each request fits by itself: the class then walks HBM.
-        if (s->lc.csr_format == 0 && !csr_in_hbm(k.fmt) && static_cast<int64_t>(kSmemHeader) + csrB +
-                std::min(chain_bytes(layout), chain_bytes(kLayoutSlots)) > s->ctx->smemOptin) {
+        const ClassNeed needs(k, reqs);
+        const int maxN = needs.maxN, maxWords = needs.maxWords, pmax = needs.pmax;
+        int layout = needs.layout;
+        uint32_t csrB = needs.csrB;
+        auto chain_bytes = [&](int kind) { return needs.chain_bytes(k, kind); };
+        // The largest copy does not fit beside the largest graph's chain: the
+        // class walks HBM.
+        if (s->lc.csr_format == 0 && !csr_in_hbm(k.fmt) && needs.least_bytes(k, true) > s->ctx->smemOptin) {
             k.fmt = k.fmt == kCsrUnit16 ? kCsrGlobal16 : kCsrGlobal32;
             csrB = 0;
         }
