@@ -577,11 +577,15 @@ static int rfmf_graph_create_impl(rfmf_context* ctx, int64_t n, const uint32_t* 
     for (uint64_t i = 0; i < m2; ++i) he[i] = Edge{col[i], weight[i]};
     int rc = g->offsets.alloc(ob);
     if (rc) return rc;
-    rc = g->edges.alloc(m2 * sizeof(Edge));
+    rc = g->edges.alloc(rfmf_graph::edge_bytes(static_cast<int64_t>(m2)));
     if (rc) return rc;
     cudaStream_t st = ctx->stream;
     CU(cudaMemcpyAsync(g->offsets.p, ho.data(), ob, cudaMemcpyHostToDevice, st));
-    if (m2) CU(cudaMemcpyAsync(g->edges.p, he.data(), m2 * sizeof(Edge), cudaMemcpyHostToDevice, st));
+    if (m2) {
+        CU(cudaMemcpyAsync(g->edges.p, he.data(), m2 * sizeof(Edge), cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(g->cols(), col, m2 * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(g->weights(), weight, m2 * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    }
     std::vector<uint32_t> hr, h32;
     std::vector<uint16_t> h16;
     if (g->unit16 || g->packed32) {

@@ -362,7 +362,12 @@ struct rfmf_graph {
     int64_t n = 0, m = 0, B = 0, wsum2 = 0;
     bool unit16 = false, packed32 = false;
     uint32_t rowBytes = 0, u16Bytes = 0, p32Bytes = 0;
+    // edges: the 2m {col, weight} pairs, behind them the 2m neighbour ids and the
+    // 2m weights by themselves, which rfmf_graph_csr copies out.
     rfmf::DevBuf offsets, edges, rows, u16, p32;
+    static size_t edge_bytes(int64_t m2) { return static_cast<size_t>(m2) * (sizeof(rfmf::Edge) + 8); }
+    int32_t* cols() const { return reinterpret_cast<int32_t*>(edges.as<rfmf::Edge>() + 2 * m); }
+    int32_t* weights() const { return cols() + 2 * m; }
     // Learned costs: device time per sweep of one work item, by plan (warps
     // per chain, CSR format), phase group count P and scheduler level (the
     // warps an item puts on each of the SM's four schedulers,

@@ -540,14 +540,15 @@ __global__ void __launch_bounds__(1024) sort_hubs(const unsigned long long* ent,
 }
 
 // The survivors of every sorted row, one warp a row, in all the formats given:
-// {col, w} pairs with their offsets, and the compact rows (start[r]: kept
+// {col, w} pairs with their offsets and their two halves, and the compact rows (start[r]: kept
 // entries before row r, padded entries in the high half) with their row words
 // and padding (the vertex itself, weight +1 or 0).  offsets and rows are
 // filled up to `words`.
 __global__ void __launch_bounds__(kIngestBlock) emit_rows(const unsigned long long* ent, const int32_t* rowStart,
                                                           const uint64_t* start, int n, int words, const int64_t* w,
-                                                          uint32_t* offsets, Edge* edges, uint32_t* rows,
-                                                          uint16_t* u16, uint32_t* p32) {
+                                                          uint32_t* offsets, Edge* edges, int32_t* cols,
+                                                          int32_t* weights, uint32_t* rows, uint16_t* u16,
+                                                          uint32_t* p32) {
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * kIngestBlock) >> 5;
     for (int r = (blockIdx.x * kIngestBlock + threadIdx.x) >> 5; r < n; r += warps) {
@@ -568,6 +569,8 @@ __global__ void __launch_bounds__(kIngestBlock) emit_rows(const unsigned long lo
                 const int32_t col = static_cast<int32_t>(key >> 32);
                 const int32_t x = static_cast<int32_t>(w[static_cast<uint32_t>(key)]);
                 edges[o + at] = Edge{col, x};
+                cols[o + at] = col;
+                weights[o + at] = x;
                 if (u16) u16[c + at] = static_cast<uint16_t>(col | (x < 0 ? 0x8000 : 0));
                 if (p32) p32[c + at] = (static_cast<uint32_t>(x) << 16) | static_cast<uint32_t>(col);
             }
@@ -595,16 +598,6 @@ __global__ void orig_ids(const int32_t* present, const int32_t* dense, int64_t m
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i <= maxId;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x)
         if (present[i]) out[dense[i]] = i;
-}
-
-// The two halves of the {col, w} pairs.
-__global__ void split_edges(const Edge* edges, int64_t m2, int32_t* col, int32_t* w) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < m2;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const Edge e = edges[i];
-        if (col) col[i] = e.col;
-        if (w) w[i] = e.w;
-    }
 }
 
 unsigned grid_for(int64_t n) {
@@ -722,7 +715,7 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     if (g->B > std::numeric_limits<int32_t>::max())
         return fail(RFMF_ERR_CAPACITY, "max weighted degree %lld exceeds int32", (long long)g->B);
     const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
-    if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(std::max<int64_t>(m2, 1) * sizeof(Edge)))) return rc;
+    if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(rfmf_graph::edge_bytes(m2)))) return rc;
     g->unit16 = !hf.notUnit && n <= 32768;
     g->packed32 = !hf.notSmall && n <= 65536 && mPad < (1u << 30);
     if (g->unit16 || g->packed32) {
@@ -740,7 +733,7 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     }
     const unsigned blocks = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, 8 * ctx->sms)));
     emit_rows<<<blocks, kIngestBlock, 0, st>>>(sorted, row, start, n, static_cast<int>(ob / 4), dW,
-                                               g->offsets.as<uint32_t>(), g->edges.as<Edge>(),
+                                               g->offsets.as<uint32_t>(), g->edges.as<Edge>(), g->cols(), g->weights(),
                                                g->rowBytes ? g->rows.as<uint32_t>() : nullptr,
                                                g->unit16 ? g->u16.as<uint16_t>() : nullptr,
                                                g->packed32 ? g->p32.as<uint32_t>() : nullptr);
@@ -771,18 +764,9 @@ static int rfmf_graph_csr_impl(const rfmf_graph* g, uint32_t* offsets, int32_t* 
     CU(cudaSetDevice(g->ctx->device));
     const int64_t m2 = 2 * g->m;
     if (offsets) CU(cudaMemcpy(offsets, g->offsets.p, (g->n + 1) * 4, cudaMemcpyDeviceToHost));
-    if ((col || weight) && m2) {
-        cudaStream_t st = g->ctx->stream;
-        Arena a;
-        const size_t oCol = a.add<int32_t>(m2), oW = a.add<int32_t>(m2);
-        if (int rc = a.alloc(g->ctx)) return rc;
-        split_edges<<<grid_for(m2), kIngestBlock, 0, st>>>(g->edges.as<Edge>(), m2, col ? a.at<int32_t>(oCol) : nullptr,
-                                                           weight ? a.at<int32_t>(oW) : nullptr);
-        CU(cudaGetLastError());
-        if (col) CU(cudaMemcpyAsync(col, a.at<int32_t>(oCol), m2 * 4, cudaMemcpyDeviceToHost, st));
-        if (weight) CU(cudaMemcpyAsync(weight, a.at<int32_t>(oW), m2 * 4, cudaMemcpyDeviceToHost, st));
-        CU(cudaStreamSynchronize(st));
-    }
+    // Plain copies: they need no device memory and wait for no launch.
+    if (col && m2) CU(cudaMemcpy(col, g->cols(), m2 * 4, cudaMemcpyDeviceToHost));
+    if (weight && m2) CU(cudaMemcpy(weight, g->weights(), m2 * 4, cudaMemcpyDeviceToHost));
     return RFMF_OK;
 }
 
