@@ -60,7 +60,7 @@ struct BatchClass {
     bool balanced = false;       // items sized from graph costs (learned or modelled)
     uint64_t pendingSweeps = 0;  // sweeps of the last launch, whose item times are unread
     uint32_t pendingP = 0;       // its phase P (0: it spanned several phases)
-    DevBuf dItems, dOrder, dItemNs, dCtl;
+    DevBuf dItems, dOrder, dItemNs;
     DevLaunch L{};
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
@@ -81,8 +81,13 @@ struct rfmf_batch {
     std::vector<uint32_t> phaseP;                // the schedule, host copy
     std::vector<uint64_t> phaseIters;
     DevBuf dGraphs, dScheds, dChains, dPhaseP, dPhaseIters, dBits, dBest;
-    DevBuf dCutPlan;                             // cut groups and their chains (made when first wanted)
-    int cutGroups = 0;
+    DevBuf dCtl;                                 // per class: queue head, error, its item, unused
+    // The cut items and their chains, made when first wanted; the host copy stays
+    // for the upload, which is not waited for.
+    Scratch dCutPlan;
+    std::vector<char> cutPlan;
+    int cutSmall = 0, cutItems = 0;
+    bool cutAdds = false;                        // some items are slices
     bool lowBest = false;                        // restored, not run yet: a chain's best is below its cut
     DevBuf dOwnBest;                             // then: see lift_best
     std::vector<DevBetaRef> betaRefs;            // the context's shared beta tables in use
@@ -630,38 +635,55 @@ int enqueue_run(rfmf_batch* b, uint64_t sweeps, bool capturing = false) {
 namespace {
 
 // Cuts of every chain's spins, recomputed on the device into out (C values),
-// asynchronously on the context's stream.  The groups of up to 32 chains of a
-// graph are laid out once per batch.
-int enqueue_cuts(rfmf_batch* b, int which, int64_t* out) {
+// asynchronously on the context's stream; ctl, if given, receives the classes'
+// control words.  The items are laid out once per batch.
+int enqueue_cuts(rfmf_batch* b, int which, int64_t* out, int32_t* ctl) {
     cudaStream_t st = b->ctx->stream;
     const size_t orderBytes = static_cast<size_t>((b->C * 4 + 15) & ~int64_t(15));
-    if (!b->dCutPlan.p) {
-        std::vector<std::vector<int32_t>> of(b->glist.size());
-        for (int64_t i = 0; i < b->C; ++i) of[b->graphOfChain[i]].push_back(static_cast<int32_t>(i));
-        std::vector<int32_t> order;
-        std::vector<CutGroup> groups;
-        for (size_t g = 0; g < of.size(); ++g)
-            for (size_t s = 0; s < of[g].size(); s += 32) {
-                const int cnt = static_cast<int>(std::min<size_t>(32, of[g].size() - s));
-                groups.push_back(CutGroup{static_cast<int32_t>(g), static_cast<int32_t>(order.size()), cnt, 0});
-                order.insert(order.end(), of[g].begin() + s, of[g].begin() + s + cnt);
-            }
-        DevBuf plan;
-        if (int rc = plan.alloc(orderBytes + groups.size() * sizeof(CutGroup))) return rc;
-        CU(cudaMemcpyAsync(plan.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
-        CU(cudaMemcpyAsync(plan.as<char>() + orderBytes, groups.data(), groups.size() * sizeof(CutGroup),
-                           cudaMemcpyHostToDevice, st));
-        CU(cudaStreamSynchronize(st));
-        b->dCutPlan = std::move(plan);
-        b->cutGroups = static_cast<int>(groups.size());
-    }
     int64_t maxN = 0;
     for (const rfmf_graph* g : b->glist) maxN = std::max(maxN, g->n);
-    CU(cudaMemsetAsync(out, 0, static_cast<size_t>(b->C) * sizeof(int64_t), st));
+    if (!b->cutItems) {
+        const size_t G = b->glist.size();
+        std::vector<std::vector<int32_t>> of(G);
+        for (int64_t i = 0; i < b->C; ++i) of[b->graphOfChain[i]].push_back(static_cast<int32_t>(i));
+        int64_t groups = 0;
+        for (const auto& chains : of) groups += (static_cast<int64_t>(chains.size()) + 31) / 32;
+        std::vector<int32_t> order;
+        std::vector<CutItem> items;
+        int small = 0;
+        bool adds = false;
+        for (int large = 0; large < 2; ++large) {
+            for (size_t g = 0; g < G; ++g) {
+                if ((b->glist[g]->n > kCutSmallN) != (large == 1)) continue;
+                const int slices = cut_slices(b->glist[g]->n, groups, b->ctx->sms);
+                adds = adds || slices > 1;
+                for (size_t s = 0; s < of[g].size(); s += 32) {
+                    const int cnt = static_cast<int>(std::min<size_t>(32, of[g].size() - s));
+                    for (int k = 0; k < slices; ++k)
+                        items.push_back(CutItem{static_cast<int32_t>(g), static_cast<int32_t>(order.size()),
+                                                static_cast<int16_t>(cnt), static_cast<int16_t>(k),
+                                                static_cast<int16_t>(slices), 0});
+                    order.insert(order.end(), of[g].begin() + s, of[g].begin() + s + cnt);
+                }
+            }
+            if (!large) small = static_cast<int>(items.size());
+        }
+        b->cutPlan.resize(orderBytes + items.size() * sizeof(CutItem));
+        std::memcpy(b->cutPlan.data(), order.data(), order.size() * 4);
+        std::memcpy(b->cutPlan.data() + orderBytes, items.data(), items.size() * sizeof(CutItem));
+        if (!b->dCutPlan.p)
+            if (int rc = b->dCutPlan.alloc(b->ctx, b->cutPlan.size())) return rc;
+        CU(cudaMemcpyAsync(b->dCutPlan.p, b->cutPlan.data(), b->cutPlan.size(), cudaMemcpyHostToDevice, st));
+        b->cutAdds = adds;
+        b->cutSmall = small;
+        b->cutItems = static_cast<int>(items.size());
+    }
+    if (b->cutAdds) CU(cudaMemsetAsync(out, 0, static_cast<size_t>(b->C) * sizeof(int64_t), st));
+    const char* plan = b->dCutPlan.as<char>();
     CU(launch_chain_cuts(b->dChains.as<DevChain>(), b->dGraphs.as<DevGraph>(),
-                         reinterpret_cast<const CutGroup*>(b->dCutPlan.as<char>() + orderBytes), b->cutGroups,
-                         b->dCutPlan.as<int32_t>(), static_cast<int>(maxN), b->ctx->sms, b->ctx->smemOptin, which, out,
-                         st));
+                         reinterpret_cast<const CutItem*>(plan + orderBytes), b->cutSmall, b->cutItems,
+                         reinterpret_cast<const int32_t*>(plan), maxN, b->ctx->smemOptin, which, out,
+                         ctl ? b->dCtl.as<int32_t>() : nullptr, 4 * static_cast<int>(b->cls.size()), ctl, st));
     return RFMF_OK;
 }
 
@@ -1075,9 +1097,10 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     for (BatchClass& k : b->cls) {
         const int64_t kc = static_cast<int64_t>(k.order.size());
         if ((rc = k.dItems.alloc(kc * sizeof(DevItem))) || (rc = k.dOrder.alloc(kc * sizeof(int32_t))) ||
-            (rc = k.dItemNs.alloc(kc * sizeof(uint64_t))) || (rc = k.dCtl.alloc(4 * sizeof(int32_t))))
+            (rc = k.dItemNs.alloc(kc * sizeof(uint64_t))))
             return rc;
     }
+    if ((rc = b->dCtl.alloc(b->cls.size() * 4 * sizeof(int32_t)))) return rc;
     if (b->cls.size() > 1) {
         CU(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
         for (BatchClass& k : b->cls) {
@@ -1117,9 +1140,10 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     CU(cudaMemcpyAsync(b->dBits.p, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync(b->dBest.p, resume ? bestBits.data() : bits.data(), bits.size() * sizeof(uint32_t),
                        cudaMemcpyHostToDevice, st));
-    for (BatchClass& k : b->cls) {
+    CU(cudaMemsetAsync(b->dCtl.p, 0, b->cls.size() * 4 * sizeof(int32_t), st));
+    for (size_t ci = 0; ci < b->cls.size(); ++ci) {
+        BatchClass& k = b->cls[ci];
         if ((rc = upload_items(*b, k))) return rc;
-        CU(cudaMemsetAsync(k.dCtl.p, 0, 4 * sizeof(int32_t), st));
         DevLaunch& L = k.L;
         L.graphs = b->dGraphs.as<DevGraph>();
         L.scheds = b->dScheds.as<DevSchedule>();
@@ -1130,9 +1154,9 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         L.itemNs = k.dItemNs.as<uint64_t>();
         L.ngraphs = static_cast<int32_t>(G);
         L.nscheds = 1;
-        L.queue = k.dCtl.as<int32_t>();
-        L.error = k.dCtl.as<int32_t>() + 1;
-        L.errorItem = k.dCtl.as<int32_t>() + 2;
+        L.queue = b->dCtl.as<int32_t>() + 4 * ci;
+        L.error = L.queue + 1;
+        L.errorItem = L.queue + 2;
         L.window = 0;
         std::memcpy(L.lut, ctx->lut, sizeof L.lut);
     }
@@ -1143,7 +1167,7 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
         Scratch d;
         if ((rc = d.alloc(ctx, static_cast<size_t>(2 * C) * sizeof(int64_t)))) return rc;
         for (int which = 0; which < 2; ++which)
-            if ((rc = enqueue_cuts(b.get(), which, d.as<int64_t>() + which * C))) return rc;
+            if ((rc = enqueue_cuts(b.get(), which, d.as<int64_t>() + which * C, nullptr))) return rc;
         std::vector<int64_t> cuts(static_cast<size_t>(2 * C));
         CU(cudaMemcpyAsync(cuts.data(), d.p, cuts.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
@@ -1243,14 +1267,11 @@ static int rfmf_batch_stats_impl(rfmf_batch* b, uint64_t* improved_sweeps) {
     return RFMF_OK;
 }
 
-static int rfmf_batch_synchronize_impl(rfmf_batch* b) {
-    if (!b) return fail(RFMF_ERR_INVALID, "batch is NULL");
-    CU(cudaSetDevice(b->ctx->device));
-    CU(cudaStreamSynchronize(b->ctx->stream));
-    for (BatchClass& k : b->cls) {
-        if (int rc = harvest_item_times(*b, k)) return rc;
-        int32_t ctl[4];
-        CU(cudaMemcpy(ctl, k.dCtl.p, sizeof ctl, cudaMemcpyDeviceToHost));
+// After the stream is idle: what the launches taught, and the first device error
+// in the classes' control words.
+static int finish_launches(rfmf_batch* b, const int32_t* ctl) {
+    for (size_t ci = 0; ci < b->cls.size(); ++ci, ctl += 4) {
+        if (int rc = harvest_item_times(*b, b->cls[ci])) return rc;
         if (ctl[1] != kDevOk) {
             static const char* names[] = {"ok", "carried cut value disagrees with the spins",
                                           "beta table shorter than the window", "bad work item",
@@ -1262,6 +1283,15 @@ static int rfmf_batch_synchronize_impl(rfmf_batch* b) {
         }
     }
     return RFMF_OK;
+}
+
+static int rfmf_batch_synchronize_impl(rfmf_batch* b) {
+    if (!b) return fail(RFMF_ERR_INVALID, "batch is NULL");
+    CU(cudaSetDevice(b->ctx->device));
+    std::vector<int32_t> ctl(4 * b->cls.size());
+    CU(cudaMemcpyAsync(ctl.data(), b->dCtl.p, ctl.size() * 4, cudaMemcpyDeviceToHost, b->ctx->stream));
+    CU(cudaStreamSynchronize(b->ctx->stream));
+    return finish_launches(b, ctl.data());
 }
 
 static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_spins,
@@ -1294,12 +1324,17 @@ static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_s
 
 static int rfmf_batch_cuts_impl(rfmf_batch* b, int which, int64_t* out_cuts) {
     if (!b || !out_cuts || (which != 0 && which != 1)) return fail(RFMF_ERR_INVALID, "bad arguments");
-    if (int rc = rfmf_batch_synchronize(b)) return rc;
+    CU(cudaSetDevice(b->ctx->device));
+    // The cuts and, behind them, the control words: one wait for both.
+    const size_t C = static_cast<size_t>(b->C), bytes = C * sizeof(int64_t) + b->cls.size() * 4 * sizeof(int32_t);
+    std::vector<int64_t> got((bytes + 7) / 8);
     Scratch d;
-    if (int rc = d.alloc(b->ctx, static_cast<size_t>(b->C) * sizeof(int64_t))) return rc;
-    if (int rc = enqueue_cuts(b, which, d.as<int64_t>())) return rc;
-    CU(cudaMemcpyAsync(out_cuts, d.p, b->C * sizeof(int64_t), cudaMemcpyDeviceToHost, b->ctx->stream));
+    if (int rc = d.alloc(b->ctx, bytes)) return rc;
+    if (int rc = enqueue_cuts(b, which, d.as<int64_t>(), reinterpret_cast<int32_t*>(d.as<int64_t>() + C))) return rc;
+    CU(cudaMemcpyAsync(got.data(), d.p, bytes, cudaMemcpyDeviceToHost, b->ctx->stream));
     CU(cudaStreamSynchronize(b->ctx->stream));
+    if (int rc = finish_launches(b, reinterpret_cast<const int32_t*>(got.data() + C))) return rc;
+    std::copy(got.begin(), got.begin() + static_cast<std::ptrdiff_t>(C), out_cuts);
     return RFMF_OK;
 }
 

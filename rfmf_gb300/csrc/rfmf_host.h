@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -45,15 +46,28 @@ const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
 cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
                           int threads, size_t smem, cudaStream_t stream, int sms);
 
-// Output-path kernels (rfmf_ingest.cu).  A cut group: up to 32 chains of one
-// graph, order[first .. first + count).
-struct CutGroup {
-    int32_t graph, first, count, pad;
+// Output-path kernels (rfmf_ingest.cu).  A cut item, one CTA's work: up to 32
+// chains of one graph, order[first .. first + count), over slice `slice` of
+// `slices` of its rows.
+struct CutItem {
+    int32_t graph, first;
+    int16_t count, slice, slices, pad;
 };
-// Adds every chain's cut into out (zeroed by the caller).
-cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutGroup* groups, int ngroups,
-                              const int32_t* order, int maxN, int sms, int smemOptin, int which, int64_t* out,
-                              cudaStream_t st);
+// Graphs of at most this many vertices come first among the items: their CTAs do
+// not reserve shared memory for the largest graph's vertex table.
+constexpr int64_t kCutSmallN = 4096;
+// Slices of a graph's rows: about four CTAs per SM over all `groups` of a batch,
+// but at least 32 rows a warp.
+inline int cut_slices(int64_t n, int64_t groups, int sms) {
+    const int64_t want = std::max<int64_t>(1, std::min<int64_t>(64, (4 * static_cast<int64_t>(sms) + groups - 1) / groups));
+    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, (n + 255) / 256)));
+}
+// Every chain's cut into out: stored by an item of one slice, added by others
+// (out is then zeroed by the caller).  ctl (may be null): `words` words that the
+// first CTA copies to ctlOut, to come back with the cuts.
+cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutItem* items, int nsmall,
+                              int nitems, const int32_t* order, int64_t maxN, int smemOptin, int which, int64_t* out,
+                              const int32_t* ctl, int words, int32_t* ctlOut, cudaStream_t st);
 // '0'/'1' rows of chains [c0, c0 + count) into out, `stride` bytes each, 0 past n.
 cudaError_t launch_chain_partitions(const DevChain* chains, const DevGraph* graphs, int c0, int count, int which,
                                     char* out, int64_t stride, cudaStream_t st);

@@ -856,17 +856,22 @@ __device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
 // loads their entries 32 together; the words of which chains each entry
 // crosses, transposed, give every lane its chain's entries as a bit mask, and
 // its sum of weights is a population count per bit of the weights (one for
-// +-1).  So 32 entries cost 32 chains about 60 instructions.  A CTA takes the
-// slice blockIdx.y of the rows.  Graphs above tableN vertices read the chains'
-// bits directly.  GB300, 1024 chains each of the 50x60 torus and ER n = 2000
-// d = 19: 25 us; one CTA per chain walking all its entries took 87.
+// +-1).  So 32 entries cost 32 chains about 60 instructions.  Graphs above tableN
+// vertices read the chains' bits directly.  GB300, 1024 chains each of the 50x60
+// torus and ER n = 2000 d = 19: 25 us; one CTA per chain walking all its entries
+// took 87.  (Every slice builds the whole vertex table: slices are kept to 256
+// rows at least.)
 constexpr int kCutWarps = 8;
 __global__ void __launch_bounds__(32 * kCutWarps) chain_cuts_kernel(const DevChain* chains, const DevGraph* graphs,
-                                                                    const CutGroup* groups, const int32_t* order,
-                                                                    int tableN, int which, int64_t* out) {
+                                                                    const CutItem* items, const int32_t* order,
+                                                                    int tableN, int which, int64_t* out,
+                                                                    const int32_t* ctl, int ctlWords,
+                                                                    int32_t* ctlOut) {
     extern __shared__ uint32_t spins[];
     __shared__ long long part[kCutWarps][32];
-    const CutGroup group = groups[blockIdx.x];
+    if (ctl && blockIdx.x == 0)
+        for (int w = threadIdx.x; w < ctlWords; w += 32 * kCutWarps) ctlOut[w] = ctl[w];
+    const CutItem group = items[blockIdx.x];
     const DevGraph& g = graphs[group.graph];
     const int n = g.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t* offsets = g.offsets;
@@ -887,17 +892,17 @@ __global__ void __launch_bounds__(32 * kCutWarps) chain_cuts_kernel(const DevCha
         }
         __syncthreads();
     }
-    const int slices = gridDim.y;
-    const int v0 = static_cast<int>(static_cast<int64_t>(n) * blockIdx.y / slices);
-    const int v1 = static_cast<int>(static_cast<int64_t>(n) * (blockIdx.y + 1) / slices);
+    const int v0 = static_cast<int>(static_cast<int64_t>(n) * group.slice / group.slices);
+    const int v1 = static_cast<int>(static_cast<int64_t>(n) * (group.slice + 1) / group.slices);
     long long acc = 0;
     for (int base = v0 + 32 * warp; base < v1; base += 32 * kCutWarps) {
         const int rows = min(32, v1 - base);
         const uint32_t off = offsets[base + min(lane, rows)];
         const uint32_t e1 = rows < 32 ? __shfl_sync(0xFFFFFFFFu, off, rows) : offsets[base + 32];
-        for (uint32_t i0 = __shfl_sync(0xFFFFFFFFu, off, 0); i0 < e1; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const Edge e = i < e1 ? edges[i] : Edge{-1, 0};
+        const uint32_t e0 = __shfl_sync(0xFFFFFFFFu, off, 0);
+        for (uint32_t k = 0; k < e1 - e0; k += 32) {   // (e0 + k may pass 2^32 in the last round)
+            const uint32_t i = e0 + k + lane;
+            const Edge e = k + lane < e1 - e0 ? edges[i] : Edge{-1, 0};
             int r = 0;   // the entry's row: the last one that starts at or before it
 #pragma unroll
             for (int step = 16; step > 0; step >>= 1) {
@@ -932,7 +937,8 @@ __global__ void __launch_bounds__(32 * kCutWarps) chain_cuts_kernel(const DevCha
         long long t = 0;
 #pragma unroll
         for (int w = 0; w < kCutWarps; ++w) t += part[w][lane];
-        if (t) atomicAdd(reinterpret_cast<unsigned long long*>(out + c), static_cast<unsigned long long>(t));
+        if (group.slices == 1) out[c] = t;
+        else if (t) atomicAdd(reinterpret_cast<unsigned long long*>(out + c), static_cast<unsigned long long>(t));
     }
 }
 
@@ -1014,21 +1020,21 @@ cudaError_t settle_best(DevChain* chains, const DevGraph* graphs, int64_t count,
     return cudaGetLastError();
 }
 
-cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutGroup* groups, int ngroups,
-                              const int32_t* order, int maxN, int sms, int smemOptin, int which, int64_t* out,
-                              cudaStream_t st) {
-    if (ngroups <= 0) return cudaSuccess;
-    // About four CTAs per SM in all.
-    const int slices = std::max(1, std::min(64, (4 * sms + ngroups - 1) / ngroups));
-    const int tableN = std::min(maxN, (smemOptin - 4096) / 4);
-    const int smem = 4 * tableN;
+cudaError_t launch_chain_cuts(const DevChain* chains, const DevGraph* graphs, const CutItem* items, int nsmall,
+                              int nitems, const int32_t* order, int64_t maxN, int smemOptin, int which, int64_t* out,
+                              const int32_t* ctl, int words, int32_t* ctlOut, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&chain_cuts_kernel),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, smemOptin - 4096);
     if (e != cudaSuccess) return e;
-    for (int g0 = 0; g0 < ngroups; g0 += 1 << 20) {
-        const dim3 grid(static_cast<unsigned>(std::min(ngroups - g0, 1 << 20)), static_cast<unsigned>(slices));
-        chain_cuts_kernel<<<grid, 32 * kCutWarps, smem, st>>>(chains, graphs, groups + g0, order, tableN, which, out);
-    }
+    auto launch = [&](const CutItem* from, int count, int64_t largest) {
+        if (count <= 0) return;
+        const int tableN = static_cast<int>(std::min<int64_t>(largest, (smemOptin - 4096) / 4));
+        chain_cuts_kernel<<<static_cast<unsigned>(count), 32 * kCutWarps, 4 * tableN, st>>>(
+            chains, graphs, from, order, tableN, which, out, ctl, words, ctlOut);
+        ctl = nullptr;
+    };
+    launch(items, nsmall, std::min(maxN, kCutSmallN));
+    launch(items + nsmall, nitems - nsmall, maxN);
     return cudaGetLastError();
 }
 
