@@ -264,31 +264,37 @@ struct ItemCand {
 
 // The list-schedule makespan of sizes idx[q] (indices into cand[q]): items
 // of the chosen size plus one remainder item per graph, longest first, each
-// to the slot that frees first.
+// to the slot that frees first.  Items of one length and slots free at one time
+// are taken together, so that it costs a few steps a graph.
 double list_makespan(const std::vector<std::vector<ItemCand>>& cand, const std::vector<int64_t>& chains,
                      const std::vector<size_t>& idx, int64_t slots) {
-    std::vector<double> items;
+    using Group = std::pair<double, int64_t>;   // item time and items; time free and slots
+    std::vector<Group> items;
+    items.reserve(2 * cand.size());
     for (size_t q = 0; q < cand.size(); ++q) {
         const ItemCand& c = cand[q][idx[q]];
         const int64_t full = chains[q] / c.K, rest = chains[q] % c.K;
-        items.insert(items.end(), static_cast<size_t>(full), c.ns);
+        if (full) items.emplace_back(c.ns, full);
         if (rest) {
             size_t r = 0;
             while (cand[q][r].K < rest) ++r;   // the level of a partial item
-            items.push_back(cand[q][r].ns);
+            items.emplace_back(cand[q][r].ns, 1);
         }
     }
-    std::sort(items.begin(), items.end(), std::greater<double>());
-    const size_t S = static_cast<size_t>(std::max<int64_t>(1, std::min<int64_t>(slots, static_cast<int64_t>(items.size()))));
-    std::priority_queue<double, std::vector<double>, std::greater<double>> freeAt;
-    for (size_t i = 0; i < S; ++i) freeAt.push(0.0);
+    std::sort(items.begin(), items.end(), std::greater<Group>());
+    std::priority_queue<Group, std::vector<Group>, std::greater<Group>> freeAt;
+    freeAt.emplace(0.0, std::max<int64_t>(slots, 1));
     double span = 0.0;
-    for (double t : items) {
-        const double f = freeAt.top() + t;
-        freeAt.pop();
-        freeAt.push(f);
-        span = std::max(span, f);
-    }
+    for (Group it : items)
+        while (it.second > 0) {
+            const Group at = freeAt.top();
+            freeAt.pop();
+            const int64_t used = std::min(at.second, it.second);
+            it.second -= used;
+            if (at.second > used) freeAt.emplace(at.first, at.second - used);
+            freeAt.emplace(at.first + it.first, used);
+            span = std::max(span, at.first + it.first);
+        }
     return span;
 }
 
@@ -323,17 +329,35 @@ bool balance_items(const std::vector<std::vector<ItemCand>>& cand, const std::ve
         return true;
     }
     if (!rounds) return false;
-    // More than one round: descend from the largest sizes (at most 2000
-    // schedule evaluations, a few hundred ms for the largest classes).
-    std::vector<size_t> idx(G);
-    for (size_t q = 0; q < G; ++q) idx[q] = cand[q].size() - 1;
+    // More than one round: descend from the largest sizes, lowering one of the
+    // graphs with the longest items at a time.  Planning comes before every launch
+    // whose items it sizes, so it is kept short: kEvals schedules, some 5 us each
+    // for 64 graphs.  (Every graph a step and 2000 schedules of single items took
+    // 2.2 ms a launch for 64 graphs x 12 chains: 800 sweeps in 16 launches took 35 ms
+    // instead of 4.4.)
+    constexpr int kEvals = 64;
+    constexpr size_t kTry = 8;
+    std::vector<size_t> idx(G), order(G);
+    for (size_t q = 0; q < G; ++q) {
+        idx[q] = cand[q].size() - 1;
+        order[q] = q;
+    }
     double best = list_makespan(cand, chains, idx, slots);
     int evals = 1;
-    for (bool improved = true; improved && evals < 2000;) {
+    for (bool improved = true; improved && evals < kEvals;) {
         improved = false;
+        const size_t tried = std::min(kTry, G);
+        std::partial_sort(order.begin(), order.begin() + static_cast<std::ptrdiff_t>(tried), order.end(),
+                          [&](size_t a, size_t z) {
+                              const bool la = idx[a] > 0, lz = idx[z] > 0;   // the others cannot be lowered
+                              if (la != lz) return la;
+                              const double ta = cand[a][idx[a]].ns, tz = cand[z][idx[z]].ns;
+                              return ta != tz ? ta > tz : a < z;
+                          });
         size_t bestQ = G;
-        for (size_t q = 0; q < G && evals < 2000; ++q) {
-            if (idx[q] == 0) continue;
+        for (size_t k = 0; k < tried && evals < kEvals; ++k) {
+            const size_t q = order[k];
+            if (idx[q] == 0) break;
             --idx[q];
             const double m = list_makespan(cand, chains, idx, slots);
             ++evals;
