@@ -331,12 +331,12 @@ bool balance_items(const std::vector<std::vector<ItemCand>>& cand, const std::ve
     if (!rounds) return false;
     // More than one round: descend from the largest sizes, lowering one of the
     // graphs with the longest items at a time.  Planning comes before every launch
-    // whose items it sizes, so it is kept short: kEvals schedules, some 5 us each
-    // for 64 graphs.  (Every graph a step and 2000 schedules of single items took
-    // 2.2 ms a launch for 64 graphs x 12 chains: 800 sweeps in 16 launches took 35 ms
-    // instead of 4.4.)
-    constexpr int kEvals = 64;
-    constexpr size_t kTry = 8;
+    // whose items it sizes, so it is kept short: at most `most` schedules, some 0.1
+    // us a graph each.  (Every graph a step and 2000 schedules of single items took
+    // 2.2 ms a launch for 64 graphs x 12 chains: 800 sweeps in 16 launches took 35
+    // ms instead of 4.8.)
+    const int most = static_cast<int>(std::max<size_t>(16, std::min<size_t>(512, 4096 / G)));
+    constexpr size_t kTry = 16;
     std::vector<size_t> idx(G), order(G);
     for (size_t q = 0; q < G; ++q) {
         idx[q] = cand[q].size() - 1;
@@ -344,7 +344,7 @@ bool balance_items(const std::vector<std::vector<ItemCand>>& cand, const std::ve
     }
     double best = list_makespan(cand, chains, idx, slots);
     int evals = 1;
-    for (bool improved = true; improved && evals < kEvals;) {
+    for (bool improved = true; improved && evals < most;) {
         improved = false;
         const size_t tried = std::min(kTry, G);
         std::partial_sort(order.begin(), order.begin() + static_cast<std::ptrdiff_t>(tried), order.end(),
@@ -355,7 +355,7 @@ bool balance_items(const std::vector<std::vector<ItemCand>>& cand, const std::ve
                               return ta != tz ? ta > tz : a < z;
                           });
         size_t bestQ = G;
-        for (size_t k = 0; k < tried && evals < kEvals; ++k) {
+        for (size_t k = 0; k < tried && evals < most; ++k) {
             const size_t q = order[k];
             if (idx[q] == 0) break;
             --idx[q];
