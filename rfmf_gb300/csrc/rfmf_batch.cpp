@@ -984,22 +984,29 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
     // - up to two, and from sixteen on: every graph's rows in HBM, widths as they
     //   were;
     // - from two to 5.25: in HBM, four warps per chain for all, so that (but for
-    //   gain widths) it is one class whose items the work queue levels;
-    // - up to twelve: widths chosen together (common_widths), rows in HBM from
-    //   4096 vertices on, while the chains leave a fifth of the SMs' shared memory
-    //   free (else they come in rounds, which classes of full CTAs do better).
+    //   gain widths) it is one class whose items the work queue levels.  Where one
+    //   graph's chains are over two thirds of the vertices, they alone decide the
+    //   time, and widths are chosen together;
+    // - up to nine: widths chosen together (common_widths), rows in HBM from 4096
+    //   vertices on, while the chains leave a fifth of the SMs' shared memory free
+    //   (else they come in rounds, which classes of full CTAs do better);
+    // - up to twelve: together if the graphs' sizes are within a factor of two,
+    //   else four warps for all: nearly all warps are then taken at one warp per
+    //   chain, and the largest graph is left as slow as that makes it.
     // GB300, ms for 1,200 sweeps, before / HBM: 16 graphs n 807..14,000 x 4 chains
     // 3.4 / 3.5, x 16 5.1 / 4.1; 64 graphs x 64 18.5 / 15.1.  For 2,400 sweeps,
-    // before / four warps / widths together: those 16 graphs x 20 18.1 / 8.1 /
-    // 9.0, x 32 18.7 / 9.9 / 9.3, x 48 21.2 / 14.4 / 12.9 (44.7 and 47.7 for 8,000
-    // once costs are learned), x 64 23.4 / - / 14.2, x 96 29.3 / - / 22.2; three sparse graphs n 5000..20,000 x 128 - / 12.5 /
-    // 12.0, x 256 27.4 / 19.4 / 20.3, x 400 (97% of shared memory) 33.1 / - /
-    // 37.7; 64 graphs n 600..14,000 x 8 19.6 / 10.3 / 11.3, x 16 25.1 / - / 16.4;
-    // eight graphs n 5000..20,000 x 128 34.7 / - / 26.0.
+    // before / four warps / widths together: those 16 graphs x 24 13.5 / 7.5 / 8.6,
+    // x 48 17.8 / 11.5 / 12.5, x 64 21.1 / 14.1 / 15.0, x 96 26.0 / 19.9 / 23.2;
+    // three sparse graphs n 5000..20,000 x 128 13.3 / 12.0 / 11.5, x 256 25.2 / 18.6
+    // / 19.9; 64 graphs n 600..14,000 x 12 14.0 / 12.0 / 12.3, x 24 18.1 / 19.5 / 27.0;
+    // eight graphs n 5000..20,000 x 128 33.8 / 21.4 / 24.7, x 200 41.3 / 31.9 / 34.2;
+    // ER n = 700 and the 100x200 torus x 300 12.6 / 18.6 / 12.4; six graphs n
+    // 500..1500 and that torus x 80 10.8 / 15.1 / 8.9, x 220 19.4 / 19.3 / 23.3; six
+    // graphs n 5000..5300 x 300 27.7 / 23.0 / 20.8.
     if (b->cls.size() > 1 && c.csr_format == 0 && c.threads_per_chain == 0) {
         const int64_t sms = std::max(ctx->sms, 1);
         const bool few = b->C <= 2 * sms, some = 4 * b->C <= 21 * sms, many = b->C >= 16 * sms;
-        int64_t maxN = 0, bytes = 0;
+        int64_t maxN = 0, minN = INT64_MAX, bytes = 0, vertices = 0, most = 0;
         std::vector<WidthAsk> asks;
         for (size_t gi = 0; gi < G; ++gi) {
             const rfmf_graph* g = b->glist[gi];
@@ -1019,11 +1026,17 @@ static int rfmf_batch_create_impl(rfmf_context* ctx, int64_t C, const rfmf_graph
             const int dbytes = c.gain_width ? c.gain_width : (g->B <= 127 ? 1 : 4);
             bytes += chains * chain_layout(n, (n + 31) / 32, 1, 2, dbytes, kLayoutMain).total;
             maxN = std::max(maxN, g->n);
+            minN = std::min(minN, g->n);
+            most = std::max(most, chains * g->n);
+            vertices += chains * g->n;
         }
         std::vector<int> width;
-        const bool together = !some && b->C <= 12 * sms && bytes <= 4 * sms * (static_cast<int64_t>(ctx->smemOptin) / 5) &&
-                              maxN >= 4096 && common_widths(asks, ctx->sms, width);
-        if (maxN >= 4096 && (few || some || many || together)) {
+        const bool one = 3 * most > 2 * vertices, uneven = maxN >= 2 * minN;
+        const bool together = (some ? !few && one : b->C <= (uneven ? 9 : 12) * sms) &&
+                              bytes <= 4 * sms * (static_cast<int64_t>(ctx->smemOptin) / 5) && maxN >= 4096 &&
+                              common_widths(asks, ctx->sms, width);
+        const bool four = some || (uneven && b->C > 9 * sms && b->C <= 12 * sms);
+        if (maxN >= 4096 && (few || four || many || together)) {
             const int rc = together     ? classify(kMixedHbmN, width)
                            : few || many ? classify(0, {})
                                          : classify(0, std::vector<int>(G, kMaxAutoWarps));
