@@ -337,7 +337,10 @@ int harvest(rfmf_server* s, Request& r) {
 // Requests on several graphs running side by side get their widths together
 // (common_widths), and the larger graphs walk their rows in HBM, where their CSR
 // copies crowd out the others' chains.  Up to ten chains per SM: beyond, every
-// width is down to one warp and the copies pay.  True when it applies; false
+// width is down to one warp and the copies pay.  And while the chains leave a tenth
+// of the SMs' shared memory free: else they come in rounds, which classes of full
+// CTAs do better (1,200 sweeps, own / this: a tree of n = 10,000 and the 70x100
+// torus x 700, 86% of it, 15.1 / 14.1, x 750, 92%, 15.1 / 17.6).  True when it applies; false
 // leaves the requests' own widths (the load at their submission) and formats.
 // GB300, ms for 2,400 sweeps, own / this: eight graphs n 5000..20,000, 330 chains
 // 20.0 / 10.9, 790 28.5 / 19.9, 1300 32.9 / 27.0 (2600: 52.9 / 65.5); eight
@@ -347,16 +350,18 @@ int harvest(rfmf_server* s, Request& r) {
 // in HBM made four graphs n 800..3000 7.6 instead of 5.9.
 bool mixed_widths(const rfmf_server* s, std::vector<int>& width) {
     const std::vector<ReqPtr>& run = s->running;
-    int64_t chains = 0;
+    int64_t chains = 0, bytes = 0;
     bool mixed = false;
     std::vector<WidthAsk> asks;
     width.clear();
     for (const ReqPtr& r : run) {
         width.push_back(r->W);
         chains += r->C;
+        bytes += r->C * chain_layout(static_cast<int>(r->n), static_cast<int>(r->words), 1, 2, r->dbytes, kLayoutMain).total;
         mixed = mixed || r->graphSlot != run[0]->graphSlot;
     }
-    if (!mixed || s->lc.csr_format || s->lc.threads_per_chain || chains > 10 * static_cast<int64_t>(s->ctx->sms))
+    if (!mixed || s->lc.csr_format || s->lc.threads_per_chain || chains > 10 * static_cast<int64_t>(s->ctx->sms) ||
+        bytes > 9 * static_cast<int64_t>(s->ctx->sms) * (s->ctx->smemOptin / 10))
         return false;
     for (const ReqPtr& r : run) asks.push_back(width_ask(r->g, r->C, r->wMin, r->wMax, r->phaseP, r->phaseIters));
     return common_widths(asks, s->ctx->sms, width);
