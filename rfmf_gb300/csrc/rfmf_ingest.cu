@@ -677,6 +677,26 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
         return fail(RFMF_ERR_INVALID, "bad arguments");
     *out = nullptr;
     const int64_t E = nedges;
+    // More lines than a graph can keep (below 2^30): those of weight zero do not
+    // get device memory, nor a number in the entries' 32 bits.
+    if (E >= (int64_t(1) << 30)) {
+        std::vector<int64_t> keep[3];
+        int64_t largest = 0, kept = 0;
+        for (int64_t i = 0; i < E; ++i) {
+            if (u[i] < 0 || v[i] < 0) return fail(RFMF_ERR_INVALID, "negative vertex id at edge %lld", (long long)i);
+            if (w[i] == 0) continue;
+            if (w[i] > INT32_MAX || w[i] < -static_cast<int64_t>(INT32_MAX))
+                return fail(RFMF_ERR_CAPACITY, "weight at edge %lld does not fit int32", (long long)i);
+            largest = std::max(largest, std::max(u[i], v[i]));
+            if (++kept >= (int64_t(1) << 30)) continue;
+            keep[0].push_back(u[i]);
+            keep[1].push_back(v[i]);
+            keep[2].push_back(w[i]);
+        }
+        if (largest < (int64_t(1) << 28) && kept >= (int64_t(1) << 30)) return fail(RFMF_ERR_CAPACITY, "too many edges");
+        return rfmf_graph_from_edges_impl(ctx, static_cast<int64_t>(keep[0].size()), keep[0].data(), keep[1].data(),
+                                          keep[2].data(), out, n_out);
+    }
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     int rc;
@@ -704,7 +724,6 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     if (maxId >= (int64_t(1) << 28))
         return fail(RFMF_ERR_CAPACITY, "vertex ids up to %lld: the device build takes ids below 2^28",
                     (long long)maxId);
-    if (2 * kept >= (int64_t(1) << 31) || E >= (int64_t(1) << 32)) return fail(RFMF_ERR_CAPACITY, "too many edges");
     if (ef.selfLoop) return fail(RFMF_ERR_INVALID, "self loop in the edge list");
 
     // Scratch, rows at most one per id and per line end.
