@@ -185,8 +185,11 @@ typedef struct rfmf_launch_config {
     int s_width;           /* 32 or 64; accepted (the per-vertex gain width is gain_width) */
     int threads_per_chain; /* 0 = auto, else 32, 64, 128 or 256 (one chain's warp group) */
     int score_path;        /* 0 = gate (src/host_common.cpp:296-312), 1 = int32, 2 = int64 */
-    int chains_per_cta;    /* 0 = auto, else chains sharing one CTA's copy of the graph */
-    int csr_format;        /* 0 = auto, 1 = unit16 (shared), 2 = packed32 (shared),
+    int chains_per_cta;    /* 0 = auto, else chains sharing one CTA's copy of the graph (1..16, at
+                              most 16 / warps per chain when threads_per_chain is given) */
+    int csr_format;        /* 0 = auto, 1 = unit16 (shared), 2 = packed32 (shared; 1 and 2 are
+                              walked in HBM instead where rows padded to four entries do
+                              not fit beside a chain but packed ones would),
                               3 = HBM (the graph's most compact entries: 2, 4 or 8 bytes),
                               4 = HBM with 8-byte {col, weight} entries */
     int gain_width;        /* 0 = auto, 1 = int8 (needs B <= 127), 4 = int32 */
@@ -264,7 +267,8 @@ int rfmf_batch_read(rfmf_batch* b, int8_t* end_spins, int8_t* best_spins,
  * running it to the end of the schedule gives exactly the results of one
  * uninterrupted run.  The cut values are recomputed from the spins on the
  * device and a checkpoint whose values disagree is refused
- * (RFMF_ERR_INVALID).  The improved-sweeps statistic restarts at 0.
+ * (RFMF_ERR_INVALID).  A best below the current cut is taken as it is: best
+ * moves after a sweep only.  The improved-sweeps statistic restarts at 0.
  */
 int rfmf_batch_restore(rfmf_context* ctx, int64_t nchains, const rfmf_graph* const* graphs,
                        const double* t0s, const uint64_t* solver_seeds, int64_t nphases,

@@ -25,17 +25,19 @@
 //     hoisted (rounds 1-3 lose 3 multiplies and 3 xors per block) and three
 //     vertex blocks are in flight per thread.
 //   * The group argmax keeps eight register accumulators per thread (one per
-//     Philox lane j) whenever every thread's lane j lands in one group.  For
-//     256 % P == 0, P <= 128 each warp transposes its 256 accumulators through
-//     shared memory and reduces them in registers; the winners stay there
-//     (one-warp chains) or pass through one partial per warp and group.  Other
-//     P go through shared-memory slots with atomics.
+//     Philox lane j), the block stride chosen so that each lands in one group.
+//     For P <= 128 each warp passes its 256 accumulators through shared memory
+//     and reduces them without atomics; the winners stay in registers (one-warp
+//     chains) or pass through one partial per warp and group.  Larger P, int64
+//     scores, strides that a chain's threads do not reach, and chains with no
+//     room for the scratch go through shared-memory slots with atomics.
 //   * FLIP has no winner-winner correction walk.  With D kept per vertex,
 //     negating the winners' D and scattering 2*w*s_b*s_x into D[x] over the
 //     winners' rows leaves every winner holding D_final, and the cut gain of
 //     the whole flip set is exactly (sum delta_pre - sum D_final) / 2: the
 //     same integer the reference's corr[] formulation (src/anneal_kernels.cu:
-//     133-192, 420-440) adds up.  Row walks issue their loads four at a time.
+//     133-192, 420-440) adds up.  Compact rows are walked as vectors of four
+//     entries, 8-byte pairs four loads at a time.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -431,9 +433,10 @@ __device__ __forceinline__ int64_t group_sum(int64_t v, const ChainSmem& s, int 
 }
 
 // Exact warp sums with redux.sync.  int8 gains: the winners' gains of a sweep
-// sum to at most 2 * 127 * P, far inside int32.  int32 gains: a lane's |v| is
-// below 2^34, split into a low 24-bit part and the rest so that neither sum
-// of 32 lanes leaves int32.
+// sum to at most 2 * 127 * P, far inside int32.  int32 gains: a lane's v is split
+// into its low 24 bits, whose sum over 32 lanes is below 2^29, and the rest, whose
+// sum stays in int32 while |v| < 2^50: a lane adds at most 2 * 2^31 a winner, and
+// the fewer than 2^17 vertices that a chain's shared memory holds over 32 lanes.
 __device__ __forceinline__ int32_t warp_sum(int32_t v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
 __device__ __forceinline__ int64_t warp_sum(int64_t v) {
     const int32_t lo = __reduce_add_sync(0xFFFFFFFFu, static_cast<int32_t>(v & 0xFFFFFF));
@@ -468,9 +471,8 @@ struct PhaseCfg {
     int rows;       // FLIP: rows a thread takes part in on kPathWarp (1 to 4)
     int S;          // block stride (T but on kPathWarp; above 32 a one-warp chain
                     //    plays several warps)
-    int shares;     // kPathWarp off the main path: 256 mod P, a warp's shift of the
-                    //    groups, and from bit 8 the lanes that share a group's
-                    //    accumulators (0 when 256 % P == 0)
+    int shares;     // 256 mod P: how far each warp's groups are shifted from the one
+                    //    before; 0 on kPathWarp's main path
     int warpG;      // kPathWarp: (256 warp) mod P
 };
 
@@ -1491,9 +1493,10 @@ __device__ void run_chain(const DevLaunch& L, const ChainSmem& s, const CsrView&
     // SELECT, and wider chains pass the warps' sums through s.red under
     // SELECT's own barrier instead of one more.
     Loc loc = 0;
-    // The cut as its distance below the best, in a gain's type: with int8 gains
-    // (n < 2^23, B <= 127) no two cuts are 2^30 apart, so a best further off is
-    // never reached.
+    // The cut as its distance below the best, in a gain's type.  With int8 gains no
+    // two cuts of a graph are n B / 2 apart, below 2^23 (B <= 127, and a chain's
+    // shared memory holds fewer than 2^17 vertices), so that it is exact in int32;
+    // a best further off than 2^30 cannot be one, and is never reached.
     constexpr int64_t kFar = DP::kField ? int64_t(1) << 30 : INT64_MAX / 2;
     Loc behind = static_cast<Loc>(best < cur - kFar ? -kFar : best > cur + kFar ? kFar : best - cur);
     int64_t top = cur + behind;

@@ -138,7 +138,9 @@ struct WidthAsk {
     int64_t chains;
     int least, widest;   // widths its score path and shared memory allow
     double n, entries;   // vertices; entries of a sweep's winner rows, averaged over the phases
-    double us(int W) const { return 1.5 + 0.5e-3 * (n + entries) / W; }   // per sweep
+    // Time per sweep with few warps per SM, where latency shows (model_cost is that
+    // of a full SM); figures beside common_widths.
+    double us(int W) const { return 1.5 + 0.5e-3 * (n + entries) / W; }
 };
 WidthAsk width_ask(const rfmf_graph* g, int64_t chains, int least, int widest, const std::vector<uint32_t>& phaseP,
                    const std::vector<uint64_t>& phaseIters);
@@ -426,7 +428,9 @@ struct rfmf_graph {
     // and ER n = 2000 d = 19, phases 128..1): 1.49 us + 1.0 ns per vertex +
     // 1.4 ns per winner-row entry (min(P, n) rows of mean degree 2m/n), the
     // vertex and entry terms spread over the chain's warps, scaled by level
-    // as above (the kernel has since become some 5% faster, alike for all).  Within 5% of the measured sweep on both graphs at every P.
+    // as above.  The fit was within 5% of an earlier kernel's sweep on both graphs
+    // at every P; today's takes 0.86 to 1.01 of the model on them (0.98 at P = 128,
+    // 0.87 to 0.94 at P = 1).  What counts is the ratio between graphs.
     double model_cost(int warps, uint32_t P, int level) const {
         const double nn = static_cast<double>(n > 0 ? n : 1);
         const double rows = std::min(static_cast<double>(P > 0 ? P : 1), nn);

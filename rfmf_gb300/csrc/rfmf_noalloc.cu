@@ -43,18 +43,7 @@
 #include <new>
 #include <vector>
 
-#include "../../include/rfmf.h"
-#include "rfmf_device.h"
-
-namespace rfmf {
-int set_last_error(int code, const char* msg);
-int fail(int code, const char* fmt, ...);
-int choose_warps(int maxN, const rfmf_launch_config& c, int64_t chains, int sms);
-int key_bits(int64_t n, int T);
-const void* kernel_ptr(int dbytes, int fmt, bool s64, int warps);
-cudaError_t launch_anneal(const DevLaunch& L, int dbytes, int fmt, bool s64, int grid,
-                          int threads, size_t smem, cudaStream_t stream, int sms);
-}  // namespace rfmf
+#include "rfmf_host.h"
 
 using namespace rfmf;
 

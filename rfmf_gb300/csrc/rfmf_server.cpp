@@ -114,7 +114,7 @@ struct SlotRanges {
 struct ClassKey {
     int dbytes, fmt, W;
     bool s64;
-    bool table;   // kept apart where widths are chosen together: a group table beside the largest chain may not fit
+    bool table;   // kept apart where widths are chosen together: the others' chains then hold no group table
     bool operator<(const ClassKey& o) const {
         return std::tie(dbytes, fmt, W, s64, table) < std::tie(o.dbytes, o.fmt, o.W, o.s64, o.table);
     }
