@@ -378,10 +378,14 @@ struct rfmf_graph {
     int64_t n = 0, m = 0, B = 0, wsum2 = 0;
     bool unit16 = false, packed32 = false;
     uint32_t rowBytes = 0, u16Bytes = 0, p32Bytes = 0;
-    // edges: the 2m {col, weight} pairs, behind them the 2m neighbour ids and the
-    // 2m weights by themselves, which rfmf_graph_csr copies out.
-    rfmf::DevBuf offsets, edges, rows, u16, p32;
-    static size_t edge_bytes(int64_t m2) { return static_cast<size_t>(m2) * (sizeof(rfmf::Edge) + 8); }
+    // offsets: the plain offsets, behind them (rowBytes > 0) the row words.
+    // edges: the 2m {col, weight} pairs; behind them (halves) the 2m neighbour ids
+    // and the 2m weights by themselves, which rfmf_graph_csr copies out.  Graphs
+    // built from an edge list have them; one made from a CSR, whose owner has it,
+    // does not hold it twice.
+    rfmf::DevBuf offsets, edges, u16, p32;
+    bool halves = false;
+    uint32_t* row_words() const { return rowBytes ? offsets.as<uint32_t>() + rowBytes / 4 : nullptr; }
     int32_t* cols() const { return reinterpret_cast<int32_t*>(edges.as<rfmf::Edge>() + 2 * m); }
     int32_t* weights() const { return cols() + 2 * m; }
     // Learned costs: device time per sweep of one work item, by plan (warps
@@ -500,7 +504,7 @@ inline DevGraph device_graph(const rfmf_graph* g) {
     DevGraph d{};
     d.offsets = g->offsets.as<uint32_t>();
     d.edges = g->edges.as<Edge>();
-    d.rows = g->rows.as<uint32_t>();
+    d.rows = g->row_words();
     d.u16 = g->u16.as<uint16_t>();
     d.p32 = g->p32.as<uint32_t>();
     d.n = static_cast<int32_t>(g->n);

@@ -793,13 +793,12 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     if (g->B > std::numeric_limits<int32_t>::max())
         return fail(RFMF_ERR_CAPACITY, "max weighted degree %lld exceeds int32", (long long)g->B);
     const uint64_t ob = (static_cast<uint64_t>(n + 1) * 4u + 15u) & ~uint64_t(15);
-    if ((rc = g->offsets.alloc(ob)) || (rc = g->edges.alloc(rfmf_graph::edge_bytes(m2)))) return rc;
+    g->halves = true;
+    if ((rc = g->edges.alloc(static_cast<size_t>(m2) * (sizeof(Edge) + 8)))) return rc;
     g->unit16 = !hf.notUnit && n <= 32768;
     g->packed32 = !hf.notSmall && n <= 65536 && mPad < (1u << 30);
-    if (g->unit16 || g->packed32) {
-        g->rowBytes = static_cast<uint32_t>(ob);
-        if ((rc = g->rows.alloc(ob))) return rc;
-    }
+    if (g->unit16 || g->packed32) g->rowBytes = static_cast<uint32_t>(ob);
+    if ((rc = g->offsets.alloc(ob + g->rowBytes))) return rc;
     if (g->unit16) {
         g->u16Bytes = align16(mPad * 2u);
         if ((rc = g->u16.alloc(g->u16Bytes))) return rc;
@@ -812,7 +811,7 @@ static int rfmf_graph_from_edges_impl(rfmf_context* ctx, int64_t nedges, const i
     const unsigned blocks = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, 8 * ctx->sms)));
     emit_rows<<<blocks, kIngestBlock, 0, st>>>(sorted, row, start, n, static_cast<int>(ob / 4), dW,
                                                g->offsets.as<uint32_t>(), g->edges.as<Edge>(), g->cols(), g->weights(),
-                                               g->rowBytes ? g->rows.as<uint32_t>() : nullptr,
+                                               g->row_words(),
                                                g->unit16 ? g->u16.as<uint16_t>() : nullptr,
                                                g->packed32 ? g->p32.as<uint32_t>() : nullptr);
     CU(cudaGetLastError());
@@ -843,8 +842,23 @@ static int rfmf_graph_csr_impl(const rfmf_graph* g, uint32_t* offsets, int32_t* 
     const int64_t m2 = 2 * g->m;
     if (offsets) CU(cudaMemcpy(offsets, g->offsets.p, (g->n + 1) * 4, cudaMemcpyDeviceToHost));
     // Plain copies: they need no device memory and wait for no launch.
-    if (col && m2) CU(cudaMemcpy(col, g->cols(), m2 * 4, cudaMemcpyDeviceToHost));
-    if (weight && m2) CU(cudaMemcpy(weight, g->weights(), m2 * 4, cudaMemcpyDeviceToHost));
+    if (g->halves) {
+        if (col && m2) CU(cudaMemcpy(col, g->cols(), m2 * 4, cudaMemcpyDeviceToHost));
+        if (weight && m2) CU(cudaMemcpy(weight, g->weights(), m2 * 4, cudaMemcpyDeviceToHost));
+        return RFMF_OK;
+    }
+    if (!col && !weight) return RFMF_OK;
+    constexpr int64_t kPart = int64_t(1) << 16;   // split a cache-sized part at a time
+    const std::unique_ptr<Edge[]> part(new Edge[static_cast<size_t>(std::min(m2, kPart))]);
+    for (int64_t at = 0; at < m2; at += kPart) {
+        const int64_t cnt = std::min(kPart, m2 - at);
+        CU(cudaMemcpy(part.get(), g->edges.as<Edge>() + at, static_cast<size_t>(cnt) * sizeof(Edge),
+                      cudaMemcpyDeviceToHost));
+        if (col)
+            for (int64_t i = 0; i < cnt; ++i) col[at + i] = part[i].col;
+        if (weight)
+            for (int64_t i = 0; i < cnt; ++i) weight[at + i] = part[i].w;
+    }
     return RFMF_OK;
 }
 
