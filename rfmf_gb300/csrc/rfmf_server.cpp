@@ -372,14 +372,15 @@ bool mixed_widths(const rfmf_server* s, std::vector<int>& width) {
 struct ClassNeed {
     int maxN = 0, maxWords = 0, pmax = 1, layout = kLayoutMain;
     uint32_t csrB = 0;
-    ClassNeed(const ClassKey& k, const std::vector<Request*>& reqs) : layout(k.s64 ? kLayoutSlots : kLayoutMain) {
-        for (const Request* r : reqs) {
-            maxN = std::max<int>(maxN, static_cast<int>(r->n));
-            maxWords = std::max<int>(maxWords, static_cast<int>(r->words));
-            pmax = std::max(pmax, r->pmax);
-            if (r->table && layout == kLayoutMain) layout = kLayoutAny;
-            csrB = std::max(csrB, csr_bytes(r->g, k.fmt));
-        }
+    explicit ClassNeed(const ClassKey& k) : layout(k.s64 ? kLayoutSlots : kLayoutMain) {}
+    ClassNeed with(const ClassKey& k, const Request& r) const {
+        ClassNeed c = *this;
+        c.maxN = std::max<int>(maxN, static_cast<int>(r.n));
+        c.maxWords = std::max<int>(maxWords, static_cast<int>(r.words));
+        c.pmax = std::max(pmax, r.pmax);
+        if (r.table && layout == kLayoutMain) c.layout = kLayoutAny;
+        c.csrB = std::max(csrB, csr_bytes(r.g, k.fmt));
+        return c;
     }
     uint32_t chain_bytes(const ClassKey& k, int kind) const {
         return chain_layout(maxN, maxWords, pmax, k.W, k.dbytes, kind).total;
@@ -395,7 +396,11 @@ struct ClassNeed {
 // of the GPU no longer leaves the rest idle while the next one waits).
 // Each class has its own work items, item order and queue/error words.
 int run_window(rfmf_server* s, int64_t& launches, float& ms) {
-    std::multimap<ClassKey, std::vector<Request*>> classes;
+    struct Class {
+        ClassNeed need;
+        std::vector<Request*> reqs;
+    };
+    std::multimap<ClassKey, Class> classes;
     std::vector<int> width;
     const bool mixed = mixed_widths(s, width);
     for (size_t i = 0; i < s->running.size(); ++i) {
@@ -407,18 +412,20 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
         // of its own.  (A copy can give way to HBM walks unless it was asked for.)
         auto of = classes.equal_range(key);
         for (; of.first != of.second; ++of.first) {
-            of.first->second.push_back(r);
-            if (ClassNeed(key, of.first->second).least_bytes(key, s->lc.csr_format != 0) <= s->ctx->smemOptin) break;
-            of.first->second.pop_back();
+            const ClassNeed need = of.first->second.need.with(key, *r);
+            if (need.least_bytes(key, s->lc.csr_format != 0) > s->ctx->smemOptin) continue;
+            of.first->second.need = need;
+            of.first->second.reqs.push_back(r);
+            break;
         }
-        if (of.first == of.second) classes.emplace(key, std::vector<Request*>{r});
+        if (of.first == of.second) classes.emplace(key, Class{ClassNeed(key).with(key, *r), {r}});
     }
     launches = 0;
     ms = 0.0f;
     const int ncls = static_cast<int>(classes.size());
     double warps = 0.0;
     for (const auto& kv : classes)
-        for (const Request* r : kv.second) warps += static_cast<double>(r->C) * kv.first.W;
+        for (const Request* r : kv.second.reqs) warps += static_cast<double>(r->C) * kv.first.W;
     int64_t need = 0;
     for (const ReqPtr& r : s->running) need += r->C;
     if (need > s->itemCap) {
@@ -460,8 +467,8 @@ int run_window(rfmf_server* s, int64_t& launches, float& ms) {
     int ci = 0;
     for (auto& kv : classes) {
         ClassKey k = kv.first;
-        std::vector<Request*>& reqs = kv.second;
-        const ClassNeed needs(k, reqs);
+        std::vector<Request*>& reqs = kv.second.reqs;
+        const ClassNeed& needs = kv.second.need;
         const int maxN = needs.maxN, maxWords = needs.maxWords, pmax = needs.pmax;
         int layout = needs.layout;
         uint32_t csrB = needs.csrB;
