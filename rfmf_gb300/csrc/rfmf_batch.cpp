@@ -1331,12 +1331,10 @@ static int rfmf_batch_synchronize_impl(rfmf_batch* b) {
     return finish_launches(b, ctl.data());
 }
 
-static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_spins,
-                               int64_t* cur_vals, int64_t* best_vals, uint64_t* sweeps_done) {
-    if (!b) return fail(RFMF_ERR_INVALID, "batch is NULL");
-    host_alloc_point();
-    int rc = rfmf_batch_synchronize(b);
-    if (rc) return rc;
+// The chains' state, the launches being finished.
+static int copy_state(rfmf_batch* b, int8_t* end_spins, int8_t* best_spins, int64_t* cur_vals, int64_t* best_vals,
+                      uint64_t* sweeps_done) {
+    int rc;
     std::vector<DevChain> hc(b->C);
     CU(cudaMemcpy(hc.data(), b->dChains.p, b->C * sizeof(DevChain), cudaMemcpyDeviceToHost));
     auto unpack = [&](const DevBuf& src, int8_t* dst) -> int {
@@ -1357,6 +1355,14 @@ static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_s
         if (sweeps_done) sweeps_done[i] = hc[i].sweepsDone;
     }
     return RFMF_OK;
+}
+
+static int rfmf_batch_read_impl(rfmf_batch* b, int8_t* end_spins, int8_t* best_spins,
+                               int64_t* cur_vals, int64_t* best_vals, uint64_t* sweeps_done) {
+    if (!b) return fail(RFMF_ERR_INVALID, "batch is NULL");
+    host_alloc_point();
+    if (int rc = rfmf_batch_synchronize(b)) return rc;
+    return copy_state(b, end_spins, best_spins, cur_vals, best_vals, sweeps_done);
 }
 
 static int rfmf_batch_cuts_impl(rfmf_batch* b, int which, int64_t* out_cuts) {
@@ -1492,7 +1498,8 @@ static int rfmf_anneal_impl(rfmf_context* ctx, const rfmf_graph* g, int64_t max_
     cudaEventDestroy(e1);
     if (rc) return rc;
     if (kernel_ms) *kernel_ms = ms;
-    return rfmf_batch_read(b, end_spins, best_spins, kernel_final_vals, kernel_best_vals, nullptr);
+    host_alloc_point();
+    return copy_state(b, end_spins, best_spins, kernel_final_vals, kernel_best_vals, nullptr);
 }
 
 // ---------------------------------------------------------------- autotune
