@@ -933,7 +933,7 @@ __global__ void __launch_bounds__(32 * kCutWarps) chain_cuts_kernel(const DevCha
         const uint32_t off = offsets[base + min(lane, rows)];
         const uint32_t e1 = rows < 32 ? __shfl_sync(0xFFFFFFFFu, off, rows) : offsets[base + 32];
         const uint32_t e0 = __shfl_sync(0xFFFFFFFFu, off, 0);
-        for (uint32_t k = 0; k < e1 - e0; k += 32) {   // (e0 + k may pass 2^32 in the last round)
+        for (uint32_t k = 0; k < e1 - e0; k += 32) {   // (e0 + k may pass 2^32 with the last 32)
             const uint32_t i = e0 + k + lane;
             const Edge e = k + lane < e1 - e0 ? edges[i] : Edge{-1, 0};
             int r = 0;   // the entry's row: the last one that starts at or before it
